@@ -1,82 +1,325 @@
 // True 32-bit matrix product on the FP32 pipes (FFMA only; no tensor-core or TF32 mode):
 //   C[M,N] = alpha * A[M,K] * W[N,K]^T (+ bias[N])
 // A and W are row-major with K contiguous (the layout of activations and of checkpoint weights).
-// Every output element is one accumulator that adds its K products in index order, in every
-// tile shape, so a row's result is bit-identical whatever else is in the batch.
+//
+// One order of summation for every shape, so that a row's result is bit-identical whatever else is in the batch: K is cut
+// into chunks of 64; in a chunk the products at even and at odd k are two chains of fused multiply-adds in the order of k
+// (one packed instruction serves both), the chunk's sum is even + odd, and the chunks' sums are added in their order. Chunks
+// are what the kernels below spread over threads: no sum ever waits for K products in a row, and the rounding error is that
+// of chains of 32 and K / 64 instead of one of K.
+//
+// Up to 16 rows the kernel is bound by the bytes of W (gemm_f32_rows_kernel); beyond, by the FP32 pipes and, where there
+// are few tiles, by how many SMs get one (gemm_f32_tile_kernel).
 #include "common.cuh"
 
-template <int BM, int BN, int TM, int TN>
-__global__ void __launch_bounds__(256) gemm_f32_kernel(const float* __restrict__ A, int lda, const float* __restrict__ W, int ldw,
-                                                       float* __restrict__ C, int ldc, const float* __restrict__ bias, float alpha,
-                                                       int M, int N, int K) {
-    constexpr int BK = 16;
-    static_assert((BM / TM) * (BN / TN) == 256, "256 threads");
-    __shared__ float As[BK][BM + 4];
-    __shared__ float Ws[BK][BN + 4];
-    const int tid = threadIdx.x;
-    const int tx = tid % (BN / TN), ty = tid / (BN / TN);
-    const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
-    float acc[TM][TN];
-#pragma unroll
-    for (int i = 0; i < TM; ++i)
-#pragma unroll
-        for (int j = 0; j < TN; ++j) acc[i][j] = 0.f;
+constexpr int F32_CHUNK = 64;
 
-    for (int k0 = 0; k0 < K; k0 += BK) {
-        for (int idx = tid; idx < BM * BK; idx += 256) {
-            const int r = idx / BK, k = idx - r * BK;
-            const int gm = m0 + r, gk = k0 + k;
-            As[k][r] = (gm < M && gk < K) ? A[(size_t)gm * lda + gk] : 0.f;
-        }
-        for (int idx = tid; idx < BN * BK; idx += 256) {
-            const int r = idx / BK, k = idx - r * BK;
-            const int gn = n0 + r, gk = k0 + k;
-            Ws[k][r] = (gn < N && gk < K) ? W[(size_t)gn * ldw + gk] : 0.f;
-        }
-        __syncthreads();
+__device__ __forceinline__ void f32_cp16(uint32_t dst, const void* src, int bytes) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst), "l"(src), "r"(bytes));
+}
+__device__ __forceinline__ void f32_cp4(uint32_t dst, const void* src, int bytes) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(dst), "l"(src), "r"(bytes));
+}
+__device__ __forceinline__ void f32_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
+template <int N> __device__ __forceinline__ void f32_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
+
+// Four floats row[k .. k+3] to shared memory, zeros past K. VEC: row + k is 16-byte aligned. (A copy of no bytes still names
+// an address inside the row.)
+template <bool VEC>
+__device__ __forceinline__ void f32_cp_piece(uint32_t dst, const float* row, int k, int K) {
+    if (VEC) {
+        const int left = K - k;
+        f32_cp16(dst, row + (left > 0 ? k : 0), left >= 4 ? 16 : left > 0 ? left * 4 : 0);
+    } else {
 #pragma unroll
-        for (int k = 0; k < BK; ++k) {
-            float a[TM], b[TN];
-#pragma unroll
-            for (int i = 0; i < TM; ++i) a[i] = As[k][ty * TM + i];
-#pragma unroll
-            for (int j = 0; j < TN; ++j) b[j] = Ws[k][tx * TN + j];
-#pragma unroll
-            for (int i = 0; i < TM; ++i)
-#pragma unroll
-                for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
-        }
-        __syncthreads();
-    }
-#pragma unroll
-    for (int i = 0; i < TM; ++i) {
-        const int gm = m0 + ty * TM + i;
-        if (gm >= M) continue;
-#pragma unroll
-        for (int j = 0; j < TN; ++j) {
-            const int gn = n0 + tx * TN + j;
-            if (gn >= N) continue;
-            float v = alpha * acc[i][j];
-            if (bias) v += bias[gn];
-            C[(size_t)gm * ldc + gn] = v;
-        }
+        for (int i = 0; i < 4; ++i) f32_cp4(dst + 4 * i, row + (k + i < K ? k + i : 0), k + i < K ? 4 : 0);
     }
 }
 
+struct F32Pair { il_f2 lo, hi; };                 // floats k, k+1 and k+2, k+3
+__device__ __forceinline__ F32Pair f32_ld4(const float* p) {
+    const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(p);
+    return F32Pair{v.x, v.y};
+}
+__device__ __forceinline__ float f32_halves(il_f2 v) {
+    float a, b;
+    il_f2_get(v, a, b);
+    return __fadd_rn(a, b);
+}
+
+// ---- up to 16 rows: W streamed once -------------------------------------------------------------------------------------
+// A block owns 8 rows of W. K is taken in rounds of 16 chunks: asynchronous copies bring the round's 32 KB of W (and the rows of
+// A) to shared memory, a thread sums one chunk of one W row with all M rows of A, and the chunk sums are added in order.
+// The next round's copies are in flight meanwhile, and the first round's W is asked for before the wait for the kernel in
+// front where the caller says that W is no kernel's output (`early`). Rows and chunks are padded so that the eight lanes of a load phase hit eight banks groups.
+// Measured, one row, weights not in cache: 8,192 x 1,024 in 10.3 us (3.3 TB/s), 73,448 x 1,024 in 69 us (4.4 TB/s); one accumulator
+// that walked all of K with plain loads took 740 us on average over a step's products of 1,024 and 4,096 k.
+constexpr int FR_ROWS = 8, FR_CHUNKS = 16, FR_ROUND = FR_CHUNKS * F32_CHUNK, FR_CS = F32_CHUNK + 4;
+constexpr int FR_WS = FR_CHUNKS * FR_CS + 4, FR_XS = FR_CHUNKS * FR_CS, FR_THREADS = FR_ROWS * FR_CHUNKS;
+__host__ __device__ constexpr int fr_stage_floats(int M) { return FR_ROWS * FR_WS + M * FR_XS; }
+__host__ __device__ constexpr int fr_smem_floats(int M, int stages) { return stages * fr_stage_floats(M) + M * FR_CHUNKS * FR_ROWS; }
+
+template <int MT, bool VEC>
+__global__ void __launch_bounds__(FR_THREADS) gemm_f32_rows_kernel(const float* A, int lda, const float* __restrict__ W, int ldw,
+                                                                   float* __restrict__ C, int ldc, const float* __restrict__ bias, float alpha,
+                                                                   int M, int N, int K, int stages, int early) {
+    extern __shared__ __align__(16) float sm[];
+    const int tid = threadIdx.x, n0 = blockIdx.x * FR_ROWS;
+    const int n = tid & 7, c = tid >> 3;
+    const int stage_f = fr_stage_floats(M);
+    float* red = sm + (size_t)stages * stage_f;   // [M][FR_CHUNKS][FR_ROWS]
+    const int rounds = (K + FR_ROUND - 1) / FR_ROUND;
+
+    auto load_w = [&](int r) {
+        const uint32_t base = (uint32_t)__cvta_generic_to_shared(sm + (size_t)(r % stages) * stage_f);
+#pragma unroll 4
+        for (int i = 0; i < FR_ROWS * FR_ROUND / 4 / FR_THREADS; ++i) {
+            const int idx = tid + i * FR_THREADS, row = idx / (FR_ROUND / 4), kk = (idx % (FR_ROUND / 4)) * 4;
+            const int gn = min(n0 + row, N - 1);  // rows past the end are computed and dropped
+            f32_cp_piece<VEC>(base + 4u * (row * FR_WS + (kk / F32_CHUNK) * FR_CS + kk % F32_CHUNK), W + (size_t)gn * ldw, r * FR_ROUND + kk, K);
+        }
+    };
+    auto load_x = [&](int r) {
+        const uint32_t base = (uint32_t)__cvta_generic_to_shared(sm + (size_t)(r % stages) * stage_f + FR_ROWS * FR_WS);
+        for (int idx = tid; idx < M * (FR_ROUND / 4); idx += FR_THREADS) {
+            const int row = idx / (FR_ROUND / 4), kk = (idx % (FR_ROUND / 4)) * 4;
+            f32_cp_piece<VEC>(base + 4u * (row * FR_XS + (kk / F32_CHUNK) * FR_CS + kk % F32_CHUNK), A + (size_t)row * lda, r * FR_ROUND + kk, K);
+        }
+    };
+    if (early) load_w(0);
+    il_pdl_wait();
+    if (!early) load_w(0);
+    load_x(0);
+    f32_commit();
+    if (rounds > 1) load_w(1), load_x(1);
+    f32_commit();
+
+    const int on = tid & 7, om = tid >> 3;        // the output this thread adds up (om < M)
+    float tot = 0.f;
+    for (int r = 0; r < rounds; ++r) {
+        f32_wait<1>();
+        __syncthreads();
+        const float* st = sm + (size_t)(r % stages) * stage_f;
+        const float* w = st + n * FR_WS + c * FR_CS;
+        const float* x = st + FR_ROWS * FR_WS + c * FR_CS;
+        il_f2 acc[MT];
+#pragma unroll
+        for (int m = 0; m < MT; ++m) acc[m] = 0ull;
+#pragma unroll 4
+        for (int k = 0; k < F32_CHUNK; k += 4) {
+            const F32Pair wv = f32_ld4(w + k);
+#pragma unroll
+            for (int m = 0; m < MT; ++m) {
+                const F32Pair xv = f32_ld4(x + (m < M ? m : 0) * FR_XS + k);
+                acc[m] = il_f2_fma(wv.lo, xv.lo, acc[m]);
+                acc[m] = il_f2_fma(wv.hi, xv.hi, acc[m]);
+            }
+        }
+#pragma unroll
+        for (int m = 0; m < MT; ++m)
+            if (m < M) red[(m * FR_CHUNKS + c) * FR_ROWS + n] = f32_halves(acc[m]);
+        __syncthreads();
+        if (r + 2 < rounds) load_w(r + 2), load_x(r + 2);
+        f32_commit();
+        if (om < M) {
+#pragma unroll
+            for (int i = 0; i < FR_CHUNKS; ++i) tot = __fadd_rn(tot, red[(om * FR_CHUNKS + i) * FR_ROWS + on]);
+        }
+    }
+    il_pdl_tail();
+    if (om < M && n0 + on < N) C[(size_t)om * ldc + n0 + on] = __fmaf_rn(alpha, tot, bias ? bias[n0 + on] : 0.f);
+}
+
+// ---- more rows: tiles of 32 WM x 32 WN, K dealt out to KG groups of warps ------------------------------------------------------
+// Eight warps; a warp holds 32 x 32 outputs (a lane 8 x 4: rows l/8 + 4i, columns l%8 + 8j) of one group's chunks, fed by a ring
+// of stages of 16 k for every group, 16-byte asynchronous copies, rows padded to 20 floats (a lane's loads run along k, where the
+// packed multiply-adds want their pairs, and no two lanes of a phase share a bank group). With KG > 1 the groups' chunk sums meet in
+// shared memory after every round of KG chunks and are added in the order of the chunks.
+constexpr int FT_BK = 16, FT_RS = FT_BK + 4, FT_THREADS = 256;
+template <int WM, int WN, int KG> struct FtShape {
+    static_assert(WM * WN * KG == 8, "eight warps");
+    static constexpr int BM = 32 * WM, BN = 32 * WN, STAGES = KG > 1 ? 3 : 4;
+    static constexpr int STAGE = KG * (BM + BN) * FT_RS, RSR = BN + 8;
+    static constexpr int SMEM = (STAGES * STAGE + (KG > 1 ? KG * BM * RSR : BM * BN)) * 4;
+    static constexpr int BLOCKS = 2 * SMEM <= 224 * 1024 ? 2 : 1;     // an SM's worth: two where both fit
+};
+
+template <int WM, int WN, int KG, bool VEC>
+__global__ void __launch_bounds__(FT_THREADS, FtShape<WM, WN, KG>::BLOCKS) gemm_f32_tile_kernel(const float* A, int lda, const float* __restrict__ W, int ldw,
+                                                                   float* __restrict__ C, int ldc, const float* __restrict__ bias, float alpha,
+                                                                   int M, int N, int K) {
+    using S = FtShape<WM, WN, KG>;
+    constexpr int BM = S::BM, BN = S::BN, ST = S::STAGES, GROUP = (BM + BN) * FT_RS;
+    extern __shared__ __align__(16) float sm[];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int g = warp / (WM * WN), wm = warp % (WM * WN) / WN, wn = warp % WN;
+    const int lm = lane >> 3, ln = lane & 7;
+    const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
+    const int steps = ((K + F32_CHUNK * KG - 1) / (F32_CHUNK * KG)) * (F32_CHUNK / FT_BK);
+
+    auto load = [&](int s) {
+        const uint32_t base = (uint32_t)__cvta_generic_to_shared(sm + (size_t)(s % ST) * S::STAGE);
+        const int k_round = (s / (F32_CHUNK / FT_BK)) * KG * F32_CHUNK + (s % (F32_CHUNK / FT_BK)) * FT_BK;
+#pragma unroll
+        for (int i = 0; i < KG * (BM + BN) * 4 / FT_THREADS; ++i) {
+            const int idx = tid + i * FT_THREADS, gg = idx / ((BM + BN) * 4), rem = idx % ((BM + BN) * 4), row = rem >> 2, q = rem & 3;
+            const float* src = row < BM ? A + (size_t)min(m0 + row, M - 1) * lda : W + (size_t)min(n0 + row - BM, N - 1) * ldw;
+            f32_cp_piece<VEC>(base + 4u * (gg * GROUP + row * FT_RS + q * 4), src, k_round + gg * F32_CHUNK + q * 4, K);
+        }
+    };
+    il_pdl_wait();
+#pragma unroll
+    for (int s = 0; s < ST - 1; ++s) {
+        if (s < steps) load(s);
+        f32_commit();
+    }
+    il_f2 acc[8][4];
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) acc[i][j] = 0ull;
+    // The sums over chunks. KG 1: this lane's outputs, kept in shared memory (one column a thread) - they are touched once in 64
+    // k, and 32 registers fewer let two blocks share an SM. Else outputs tid + 256 i of the tile, in registers.
+    constexpr int OUT = BM * BN / FT_THREADS;
+    float* red = sm + ST * S::STAGE;              // KG 1: [32][256]; else [KG][BM][RSR]
+    float tot[KG > 1 ? OUT : 1];
+#pragma unroll
+    for (int i = 0; i < OUT; ++i) {
+        if (KG > 1) tot[KG > 1 ? i : 0] = 0.f;
+        else red[i * FT_THREADS + tid] = 0.f;
+    }
+    for (int s = 0; s < steps; ++s) {
+        f32_wait<ST - 2>();
+        __syncthreads();
+        if (s + ST - 1 < steps) load(s + ST - 1);
+        f32_commit();
+        const float* st = sm + (size_t)(s % ST) * S::STAGE + g * GROUP;
+        const float* ap = st + (wm * 32 + lm) * FT_RS;
+        const float* bp = st + (BM + wn * 32 + ln) * FT_RS;
+#pragma unroll
+        for (int k = 0; k < FT_BK; k += 4) {
+            F32Pair b[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) b[j] = f32_ld4(bp + 8 * j * FT_RS + k);
+#pragma unroll
+            for (int i = 0; i < 8; i += 2) {
+                const F32Pair a0 = f32_ld4(ap + 4 * i * FT_RS + k), a1 = f32_ld4(ap + 4 * (i + 1) * FT_RS + k);
+#pragma unroll
+                for (int j = 0; j < 4; ++j) acc[i][j] = il_f2_fma(a0.lo, b[j].lo, acc[i][j]);
+#pragma unroll
+                for (int j = 0; j < 4; ++j) acc[i + 1][j] = il_f2_fma(a1.lo, b[j].lo, acc[i + 1][j]);
+#pragma unroll
+                for (int j = 0; j < 4; ++j) acc[i][j] = il_f2_fma(a0.hi, b[j].hi, acc[i][j]);
+#pragma unroll
+                for (int j = 0; j < 4; ++j) acc[i + 1][j] = il_f2_fma(a1.hi, b[j].hi, acc[i + 1][j]);
+            }
+        }
+        if (s % (F32_CHUNK / FT_BK) == F32_CHUNK / FT_BK - 1) {       // a chunk is done
+            if (KG == 1) {
+#pragma unroll
+                for (int i = 0; i < 8; ++i)
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        float* t = red + (i * 4 + j) * FT_THREADS + tid;
+                        *t = __fadd_rn(*t, f32_halves(acc[i][j]));
+                        acc[i][j] = 0ull;
+                    }
+            } else {
+                float* mine = red + ((size_t)g * BM + wm * 32 + lm) * S::RSR + wn * 32 + ln;
+#pragma unroll
+                for (int i = 0; i < 8; ++i)
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        mine[4 * i * S::RSR + 8 * j] = f32_halves(acc[i][j]);
+                        acc[i][j] = 0ull;
+                    }
+                __syncthreads();
+#pragma unroll
+                for (int gg = 0; gg < KG; ++gg)
+#pragma unroll
+                    for (int i = 0; i < OUT; ++i) {
+                        const int e = tid + i * FT_THREADS;
+                        tot[KG > 1 ? i : 0] = __fadd_rn(tot[KG > 1 ? i : 0], red[((size_t)gg * BM + e / BN) * S::RSR + e % BN]);
+                    }
+            }
+        }
+    }
+    il_pdl_tail();
+#pragma unroll
+    for (int i = 0; i < OUT; ++i) {
+        const int e = tid + i * FT_THREADS;
+        const int row = KG == 1 ? wm * 32 + lm + 4 * (i / 4) : e / BN, col = KG == 1 ? wn * 32 + ln + 8 * (i % 4) : e % BN;
+        const int gm = m0 + row, gn = n0 + col;
+        if (gm < M && gn < N) C[(size_t)gm * ldc + gn] = __fmaf_rn(alpha, KG > 1 ? tot[KG > 1 ? i : 0] : red[i * FT_THREADS + tid], bias ? bias[gn] : 0.f);
+    }
+}
+
+struct F32Args {
+    const float *A, *W, *bias;
+    float* C;
+    int lda, ldw, ldc, M, N, K, early;
+    float alpha;
+    cudaStream_t stream;
+};
+
+// Dynamic shared memory beyond 48 KB is asked for once per device and kernel.
+static cudaError_t f32_allow_smem(const void* kernel, int bytes, bool* done) {
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    if (dev < 0 || dev >= 64) return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    if (!done[dev]) {
+        e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+        if (e == cudaSuccess) done[dev] = true;
+    }
+    return e;
+}
+
+template <int MT, bool VEC> static cudaError_t f32_launch_rows(const F32Args& a) {
+    static bool done[64];
+    const int stages = a.K > FR_ROUND ? 2 : 1;
+    cudaError_t e = f32_allow_smem((const void*)gemm_f32_rows_kernel<MT, VEC>, fr_smem_floats(MT, 2) * 4, done);
+    if (e != cudaSuccess) return e;
+    return il_launch(gemm_f32_rows_kernel<MT, VEC>, dim3((a.N + FR_ROWS - 1) / FR_ROWS), dim3(FR_THREADS), (size_t)fr_smem_floats(a.M, stages) * 4,
+                     a.stream, a.A, a.lda, a.W, a.ldw, a.C, a.ldc, a.bias, a.alpha, a.M, a.N, a.K, stages, a.early);
+}
+
+template <int WM, int WN, int KG, bool VEC> static cudaError_t f32_launch_tile(const F32Args& a) {
+    using S = FtShape<WM, WN, KG>;
+    static bool done[64];
+    cudaError_t e = f32_allow_smem((const void*)gemm_f32_tile_kernel<WM, WN, KG, VEC>, S::SMEM, done);
+    if (e != cudaSuccess) return e;
+    return il_launch(gemm_f32_tile_kernel<WM, WN, KG, VEC>, dim3((a.N + S::BN - 1) / S::BN, (a.M + S::BM - 1) / S::BM), dim3(FT_THREADS), (size_t)S::SMEM,
+                     a.stream, a.A, a.lda, a.W, a.ldw, a.C, a.ldc, a.bias, a.alpha, a.M, a.N, a.K);
+}
+
+template <bool VEC> static cudaError_t f32_dispatch(const F32Args& a) {
+    if (a.M <= 16)
+        return a.M == 1 ? f32_launch_rows<1, VEC>(a) : a.M == 2 ? f32_launch_rows<2, VEC>(a) : a.M <= 4 ? f32_launch_rows<4, VEC>(a)
+             : a.M <= 8 ? f32_launch_rows<8, VEC>(a) : f32_launch_rows<16, VEC>(a);
+    // The tile by what a wave of blocks was measured to take (us for K = 1,024 on a B200): one block on an SM, two on an SM.
+    //   128 x 64: 78, 138    64 x 64 (K in 2): 50, 74    64 x 32 (K in 4): 25, 49    32 x 32 (K in 8): 14, 28
+    // Large tiles do more work a byte, small ones give more SMs work: 61 rows to 1,024 columns 78 / 42 / 25 / 14 us, 2,048 rows to
+    // 8,192 columns 908 / 954 / 1,309 / 1,425 us (37.9 TFLOP/s; one accumulator a product and plain loads took 389 us and 1.7 ms).
+    const auto cost = [&](int bm, int bn, float one, float two) {
+        const long long tiles = (long long)((a.M + bm - 1) / bm) * ((a.N + bn - 1) / bn), rest = tiles % 296;
+        return (float)(tiles / 296) * two + (rest == 0 ? 0.f : rest <= 148 ? one : two);
+    };
+    const float c0 = cost(128, 64, 78.f, 138.f), c1 = cost(64, 64, 50.f, 74.f), c2 = cost(64, 32, 25.f, 49.f), c3 = cost(32, 32, 14.f, 28.f);
+    if (c3 <= c2 && c3 <= c1 && c3 <= c0) return f32_launch_tile<1, 1, 8, VEC>(a);
+    if (c2 <= c1 && c2 <= c0) return f32_launch_tile<2, 1, 4, VEC>(a);
+    if (c1 <= c0) return f32_launch_tile<2, 2, 2, VEC>(a);
+    return f32_launch_tile<4, 2, 1, VEC>(a);
+}
+
 IL_EXPORT int il_gemm_f32(const float* A, int lda, const float* W, int ldw, float* C, int ldc, const float* bias,
-                          float alpha, int M, int N, int K, cudaStream_t stream) {
+                          float alpha, int M, int N, int K, int w_static, cudaStream_t stream) {
     if (M <= 0 || N <= 0) return IL_OK;
     if (K <= 0 || lda < K || ldw < K || ldc < N) return IL_BAD_ARG;
-    if (M <= 16) {
-        dim3 grid((N + 255) / 256, (M + 15) / 16);
-        gemm_f32_kernel<16, 256, 1, 16><<<grid, 256, 0, stream>>>(A, lda, W, ldw, C, ldc, bias, alpha, M, N, K);
-    } else if (M <= 64) {
-        dim3 grid((N + 63) / 64, (M + 63) / 64);
-        gemm_f32_kernel<64, 64, 4, 4><<<grid, 256, 0, stream>>>(A, lda, W, ldw, C, ldc, bias, alpha, M, N, K);
-    } else {
-        dim3 grid((N + 127) / 128, (M + 127) / 128);
-        gemm_f32_kernel<128, 128, 8, 8><<<grid, 256, 0, stream>>>(A, lda, W, ldw, C, ldc, bias, alpha, M, N, K);
-    }
+    const F32Args a{A, W, bias, C, lda, ldw, ldc, M, N, K, w_static, alpha, stream};
+    const bool vec = !(lda & 3) && !(ldw & 3) && !((uintptr_t)A & 15) && !((uintptr_t)W & 15);
+    const cudaError_t e = vec ? f32_dispatch<true>(a) : f32_dispatch<false>(a);
+    if (e != cudaSuccess) return 1000 + (int)e;
     IL_LAUNCH_CHECK();
     return IL_OK;
 }

@@ -572,8 +572,9 @@ def gate_pack(y: torch.Tensor, head_dim: int, gate: Optional[torch.Tensor], g_of
 
 
 def gemm_f32(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, alpha: float = 1.0,
-             bias: Optional[torch.Tensor] = None) -> None:
-    """out[M,N] = alpha * a[M,K] @ w[N,K]^T (+ bias), all float32, FP32 pipes only."""
+             bias: Optional[torch.Tensor] = None, w_static: bool = False) -> None:
+    """out[M,N] = alpha * a[M,K] @ w[N,K]^T (+ bias), all float32, FP32 pipes only. `w_static`: w is a model's weight, not what
+    the kernel launched just before writes, and may be read while that kernel still runs."""
     _need_cuda(a, w, out, bias)
     M, K = a.shape
     N = w.shape[0]
@@ -586,9 +587,9 @@ def gemm_f32(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, alpha: float =
     if bias is not None and (bias.dtype != torch.float32 or bias.numel() != N):
         raise KernelError("gemm_f32: bias float32 [N]")
     f = _fn("gemm_f32", "il_gemm_f32", [_c_void_p, _c_int, _c_void_p, _c_int, _c_void_p, _c_int, _c_void_p, _c_float,
-                                        _c_int, _c_int, _c_int, _c_void_p])
+                                        _c_int, _c_int, _c_int, _c_int, _c_void_p])
     _check(f(_ptr(a), a.stride(0), _ptr(w), w.stride(0), _ptr(out), out.stride(0), _ptr(bias), alpha, M, N, K,
-             _stream()), "gemm_f32")
+             int(w_static), _stream()), "gemm_f32")
 
 
 _ones_k = {}

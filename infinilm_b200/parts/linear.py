@@ -42,7 +42,7 @@ class Linear:
     def __call__(self, x: torch.Tensor, out: torch.Tensor, out_f32: bool = False) -> torch.Tensor:
         """x [M,in] -> out [M,out]. `out_f32`: out is float32 even on the bfloat16 path."""
         if self.dtype == torch.float32:
-            ops.gemm_f32(x, self.weight, out, self.alpha, self.bias)
+            ops.gemm_f32(x, self.weight, out, self.alpha, self.bias, w_static=True)
             return out
         if ops.skinny_ok(x.shape[0], self.in_features):
             # a few rows (decode): the weight-streaming kernel of this package

@@ -97,6 +97,27 @@ def test_gemm_f32(cuda_device, M, N, K):
     assert torch.equal(out1[0], out[M - 1])
 
 
+@pytest.mark.parametrize("M", [1, 2, 3, 8, 9, 16, 17, 33, 65, 300])
+@pytest.mark.parametrize("N,K,off", [(8, 64, 0), (9, 63, 0), (31, 1024, 0), (70, 1028, 4), (33, 4100, 0), (1300, 130, 1)])
+def test_gemm_f32_shapes(cuda_device, M, N, K, off):
+    """Every kernel and tile of the dispatch at the edges of chunks (64), rounds (1,024) and tiles, aligned rows and not. A sum is
+    made of chains of at most 32 products and of K / 64 chunk sums, so its error is below (32 + K / 64 + 4) 2^-24 times the sum
+    of the products' sizes (the 4: the two halves, alpha and the bias); and one row alone gives the same bits."""
+    g = torch.Generator(device="cuda").manual_seed(M * 7 + N)
+    a = torch.randn(M, K + 8, device="cuda", generator=g)[:, off:off + K]
+    w = torch.randn(N, K + 8, device="cuda", generator=g)[:, off:off + K]
+    b = torch.randn(N, device="cuda", generator=g)
+    out, again = torch.full((M, N + 3), float("nan"), device="cuda"), torch.empty(M, N, device="cuda")
+    ops.gemm_f32(a, w, out[:, :N], 0.7, b)
+    ref, size = 0.7 * (a.double() @ w.double().t()) + b.double(), 0.7 * (a.double().abs() @ w.double().abs().t()) + b.double().abs()
+    assert bool(((out[:, :N].double() - ref).abs() <= (32 + math.ceil(K / 64) + 4) * 2.0 ** -24 * size).all())
+    assert bool(out[:, N:].isnan().all())
+    ops.gemm_f32(a, w, again, 0.7, b, w_static=True)
+    one = torch.empty(1, N, device="cuda")
+    ops.gemm_f32(a[M - 1:M], w, one, 0.7, b)
+    assert torch.equal(again, out[:, :N]) and torch.equal(one[0], out[M - 1, :N])
+
+
 # -- rope + cache write --------------------------------------------------------------------------
 def _paged_setup(E, lens, nkv, hd, page, dtype, seed, n_extra_pages=3):
     """Random block tables over shuffled pages for entries with the given kv lengths."""
