@@ -1,7 +1,6 @@
-// Plain attention over the paged cache: one warp per (token, query head), keys visited one by
-// one with an online softmax in f32. It takes any mix of prompt portions and single decoded
-// tokens, any head size up to 1024, any number of heads and groups, and an optional window.
-// It is the attention of the 32-bit path and the reference beside the fast bfloat16 kernels.
+// Plain attention over the paged cache. It takes any mix of prompt portions and single decoded tokens, any head size up to
+// 1024, any number of heads and groups, any page size and an optional window. It is the attention of the 32-bit path and the
+// reference beside the fast bfloat16 kernels; all arithmetic is f32.
 // With `sink` (one f32 number per query head) the softmax's denominator also holds exp(sink[head]): a key without a
 // value whose score is the number itself, not multiplied by `scale`.
 //
@@ -13,8 +12,215 @@
 // normalised over the keys. CAP: the scaled score s becomes cap * tanh(s / cap) (a soft cap; the sink is not capped).
 #include "common.cuh"
 
-// A lane holds head_dim / 32 elements of the query and of the output: 8 (head_dim <= 256) or 32 (<= 1024).
-template <typename TA, int AP_MAX_PER_LANE, bool SIG, bool CAP>
+// ---- head sizes up to 256: tiles of 32 keys -----------------------------------------------------------------------------------
+// A block serves one token and up to 8 query heads of one kv head (HW), a warp a head; with fewer heads, or few tokens in the
+// step, several warps share a head and take tiles of 32 keys in turn (KS of them, merged at the end). All warps of the block
+// read the same keys and values from shared memory, where asynchronous copies bring the next round while this one is
+// worked on (bfloat16, and sizes whose rows are not whole 16-byte pieces, are widened by plain loads instead). In the scores a lane
+// is a key, in the weighted sum a pair of columns. What bounds it is the chain of a tile - scores, maximum, exponentials, sum -
+// where one key at a time paid that chain and a trip to memory for every key.
+constexpr int AT_KEYS = 32;
+__host__ __device__ constexpr int at_row(int hdp) { return hdp + 4; }          // floats of a staged row: an odd number of 16-byte pieces
+__host__ __device__ constexpr int at_round_floats(int hdp, int ks) { return 2 * ks * AT_KEYS * at_row(hdp); }
+
+template <typename TA, int HDP, bool SIG, bool CAP>
+__global__ void attn_tile_kernel(const TA* qkv, int row_stride, TA* __restrict__ out, const TA* cache, const int* __restrict__ block_table,
+                                 int bt_stride, const int* __restrict__ tok_pos, const int* __restrict__ tok_entry, int page_size, int page_shift,
+                                 int nh, int nkv, int hd, float scale, int window, const float* __restrict__ sink,
+                                 const float* __restrict__ dist_bias, int dist_far, float cap, int HW, int KS, int async) {
+    extern __shared__ __align__(16) float sm[];
+    il_pdl_wait();
+    constexpr int RS = at_row(HDP), PIECES = HDP / 4, NV = (HDP + 63) / 64;
+    const int G = nh / nkv, n_hb = (G + HW - 1) / HW;
+    const int t = blockIdx.x, g = blockIdx.y / n_hb, hb = blockIdx.y - g * n_hb;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, n_thr = blockDim.x;
+    const int hs = warp % HW, ks = warp / HW;
+    const int hj = hb * HW + hs;                  // head within the group
+    const bool live = hj < G;
+    const int j = g * G + (live ? hj : 0);
+    const int round_f = at_round_floats(HDP, KS), half_f = KS * AT_KEYS * RS;
+    float* qs = sm + 2 * round_f + (size_t)hs * HDP;             // this head's query
+    float* ps = sm + 2 * round_f + HW * HDP + warp * AT_KEYS;    // this warp's weights of a tile
+    const int pos = tok_pos[t];
+    const int* bt = block_table + (size_t)tok_entry[t] * bt_stride;
+    const int lo = il_mask_lo(pos, window), n_keys = pos - lo + 1;
+    const int per_round = KS * AT_KEYS, rounds = (n_keys + per_round - 1) / per_round;
+    const size_t page_elems = (size_t)2 * nkv * page_size * hd, v_off = (size_t)nkv * page_size * hd;
+    auto load = [&](int r) {                      // keys lo + r * per_round ..: K rows, then V rows; rows past the last key are zero
+        float* dst0 = sm + (r & 1) * round_f;
+        for (int i = tid; i < per_round * PIECES; i += n_thr) {
+            const int row = i / PIECES, d = (i % PIECES) * 4, kk = r * per_round + row;
+            const bool in = kk < n_keys && d < hd;
+            const int kp = lo + (kk < n_keys ? kk : 0);
+            const int pi = page_shift >= 0 ? kp >> page_shift : kp / page_size;
+            const TA* src = cache + (size_t)bt[pi] * page_elems + ((size_t)g * page_size + (kp - pi * page_size)) * hd + (d < hd ? d : 0);
+            float* dst = dst0 + row * RS + d;
+            if (sizeof(TA) == 4 && async) {
+                const int bytes = in ? 16 : 0;
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src), "r"(bytes));
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"((uint32_t)__cvta_generic_to_shared(dst + half_f)), "l"(src + v_off), "r"(bytes));
+            } else {
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    const bool ok = in && d + e < hd;
+                    dst[e] = ok ? il_to_f(src[e]) : 0.f;
+                    dst[half_f + e] = ok ? il_to_f(src[v_off + e]) : 0.f;
+                }
+            }
+        }
+        asm volatile("cp.async.commit_group;\n" ::: "memory");
+    };
+    load(0);
+    const TA* qrow = qkv + (size_t)t * row_stride + (size_t)j * hd;
+    if (ks == 0)
+        for (int d = lane; d < HDP; d += 32) qs[d] = d < hd ? il_to_f(qrow[d]) : 0.f;
+    float m = -INFINITY, l = 0.f;                 // l: this lane's keys only
+    il_f2 acc[NV];
+#pragma unroll
+    for (int v = 0; v < NV; ++v) acc[v] = 0ull;
+    for (int r = 0; r < rounds; ++r) {
+        asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+        __syncthreads();                          // the round is there, and nobody reads the other half any more
+        if (r + 1 < rounds) load(r + 1);
+        const float* kr = sm + (r & 1) * round_f + (ks * AT_KEYS + lane) * RS;
+        const int kk = r * per_round + ks * AT_KEYS + lane;
+        const bool in = kk < n_keys;
+        if (r * per_round + ks * AT_KEYS >= n_keys) continue;        // (warp-uniform: a tile without keys)
+        il_f2 s2[2] = {0ull, 0ull};
+#pragma unroll 8
+        for (int d = 0; d < HDP; d += 4) {
+            const ulonglong2 a = *reinterpret_cast<const ulonglong2*>(kr + d), b = *reinterpret_cast<const ulonglong2*>(qs + d);
+            s2[0] = il_f2_fma(a.x, b.x, s2[0]);
+            s2[1] = il_f2_fma(a.y, b.y, s2[1]);
+        }
+        float d0, d1;
+        il_f2_get(il_f2_add(s2[0], s2[1]), d0, d1);
+        float s = (d0 + d1) * scale;
+        if (CAP) s = cap * tanhf(s / cap);
+        if (dist_bias && in) s += dist_bias[(size_t)min(n_keys - 1 - kk, dist_far) * nh + j];
+        float p;
+        if constexpr (SIG) {
+            p = in ? 1.f / (1.f + expf(-s)) : 0.f;
+        } else {
+            const float mn = fmaxf(m, il_warp_max(in ? s : -INFINITY));
+            const float corr = expf(m - mn);      // exp(-inf) = 0 on the first tile
+            p = in ? expf(s - mn) : 0.f;
+            l = l * corr + p;
+            m = mn;
+            const il_f2 c2 = il_f2_dup(corr);
+#pragma unroll
+            for (int v = 0; v < NV; ++v) acc[v] = il_f2_mul(acc[v], c2);
+        }
+        ps[lane] = p;
+        __syncwarp();
+        const float* vr = sm + (r & 1) * round_f + half_f + ks * AT_KEYS * RS + 2 * lane;
+#pragma unroll 2
+        for (int key = 0; key < AT_KEYS; key += 4) {
+            const float4 w = *reinterpret_cast<const float4*>(ps + key);
+            const float wk[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+#pragma unroll
+                for (int v = 0; v < NV; ++v)
+                    if (HDP >= 64 || 2 * lane < HDP)
+                        acc[v] = il_f2_fma(il_f2_dup(wk[e]), *reinterpret_cast<const il_f2*>(vr + (key + e) * RS + 64 * v), acc[v]);
+        }
+        __syncwarp();                             // ps is written again in the next round
+    }
+    if (!SIG) l = il_warp_sum(l);
+    if (KS > 1) {                                 // the warps of a head: maxima, sums and weighted sums through shared memory
+        __syncthreads();
+        float* part = sm + (size_t)warp * (HDP + 4);
+        if (lane == 0) part[HDP] = m, part[HDP + 1] = l;
+#pragma unroll
+        for (int v = 0; v < NV; ++v)
+            if (HDP >= 64 || 2 * lane < HDP) *reinterpret_cast<il_f2*>(part + 2 * lane + 64 * v) = acc[v];
+        __syncthreads();
+        if (ks != 0) return;
+        const float m0 = m;
+        for (int i = 1; i < KS; ++i) m = fmaxf(m, sm[(size_t)(i * HW + hs) * (HDP + 4) + HDP]);
+        if (!SIG) {
+            const float c = expf(m0 - m);
+            l *= c;
+#pragma unroll
+            for (int v = 0; v < NV; ++v) acc[v] = il_f2_mul(acc[v], il_f2_dup(c));
+        }
+        for (int i = 1; i < KS; ++i) {
+            const float* other = sm + (size_t)(i * HW + hs) * (HDP + 4);
+            const float mi = other[HDP];
+            const float c = SIG ? 1.f : mi == -INFINITY && m != -INFINITY ? 0.f : expf(mi - m);
+            l += c * other[HDP + 1];
+#pragma unroll
+            for (int v = 0; v < NV; ++v)
+                if (HDP >= 64 || 2 * lane < HDP)
+                    acc[v] = il_f2_fma(il_f2_dup(c), *reinterpret_cast<const il_f2*>(other + 2 * lane + 64 * v), acc[v]);
+        }
+    }
+    if (!live) return;
+    if (sink) l += expf(sink[j] - m);             // (+inf when the sink towers over every score: the row is then zero)
+    const float inv = SIG ? 1.f : 1.f / l;
+    TA* orow = out + (size_t)t * nh * hd + (size_t)j * hd;
+#pragma unroll
+    for (int v = 0; v < NV; ++v) {
+        float a, b;
+        il_f2_get(acc[v], a, b);
+        const int d = 2 * lane + 64 * v;
+        if (d < hd) orow[d] = il_from_f<TA>(a * inv);
+        if (d + 1 < hd) orow[d + 1] = il_from_f<TA>(b * inv);
+    }
+}
+
+struct AtArgs {
+    const void *qkv, *cache;
+    void* out;
+    const int *block_table, *tok_pos, *tok_entry;
+    const float *sink, *dist_bias;
+    int row_stride, bt_stride, page_size, T, nh, nkv, hd, window, dist_far;
+    float scale, cap;
+    cudaStream_t stream;
+};
+
+template <typename TA, int HDP, bool SIG, bool CAP>
+static cudaError_t at_launch(const AtArgs& a) {
+    const int G = a.nh / a.nkv, HW = G < 8 ? G : 8, n_hb = (G + HW - 1) / HW;
+    const long long blocks = (long long)a.T * a.nkv * n_hb;
+    // Warps of a block: 8; 16 where the step has too few (token, kv head) pairs to give every SM two blocks. As many of them share a
+    // head as shared memory holds tiles for.
+    const int warps = blocks < 2 * 148 ? 16 : 8, fit = HDP <= 32 ? 8 : HDP == 64 ? 4 : HDP == 128 ? 2 : 1;
+    int KS = warps / HW;
+    KS = KS > fit ? fit : KS < 1 ? 1 : KS;
+    int shift = -1;
+    if ((a.page_size & (a.page_size - 1)) == 0)
+        for (shift = 0; (1 << shift) < a.page_size; ++shift) {}
+    const int async = sizeof(TA) == 4 && a.hd % 4 == 0 && !((uintptr_t)a.cache & 15);
+    constexpr int fit_c = HDP <= 32 ? 8 : HDP == 64 ? 4 : HDP == 128 ? 2 : 1;
+    constexpr int smem_max = (2 * at_round_floats(HDP, fit_c) + 8 * HDP + 64 * AT_KEYS) * 4;
+    const int smem = (2 * at_round_floats(HDP, KS) + HW * HDP + HW * KS * AT_KEYS) * 4;
+    static bool done[64];
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    if (dev < 0 || dev >= 64 || !done[dev]) {
+        e = cudaFuncSetAttribute(attn_tile_kernel<TA, HDP, SIG, CAP>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_max);
+        if (e != cudaSuccess) return e;
+        if (dev >= 0 && dev < 64) done[dev] = true;
+    }
+    return il_launch(attn_tile_kernel<TA, HDP, SIG, CAP>, dim3(a.T, a.nkv * n_hb), dim3(HW * KS * 32), (size_t)smem, a.stream, (const TA*)a.qkv, a.row_stride,
+                     (TA*)a.out, (const TA*)a.cache, a.block_table, a.bt_stride, a.tok_pos, a.tok_entry, a.page_size, shift, a.nh, a.nkv, a.hd, a.scale,
+                     a.window, a.sink, a.dist_bias, a.dist_far, a.cap, HW, KS, async);
+}
+template <typename TA, bool SIG, bool CAP> static cudaError_t at_sizes(const AtArgs& a) {
+    return a.hd <= 32 ? at_launch<TA, 32, SIG, CAP>(a) : a.hd <= 64 ? at_launch<TA, 64, SIG, CAP>(a)
+         : a.hd <= 128 ? at_launch<TA, 128, SIG, CAP>(a) : at_launch<TA, 256, SIG, CAP>(a);
+}
+template <typename TA> static cudaError_t at_modes(const AtArgs& a, int sigmoid) {
+    return sigmoid ? at_sizes<TA, true, false>(a) : a.cap > 0.f ? at_sizes<TA, false, true>(a) : at_sizes<TA, false, false>(a);
+}
+
+// ---- head sizes beyond 256: one warp per (token, query head), keys one by one with an online softmax -------------------------------
+// A lane holds head_dim / 32 elements of the query and of the output.
+constexpr int AP_MAX_PER_LANE = 32;
+template <typename TA, bool SIG, bool CAP>
 __global__ void attn_plain_kernel(const TA* __restrict__ qkv, int row_stride, TA* __restrict__ out,
                                   const TA* __restrict__ cache, const int* __restrict__ block_table, int bt_stride,
                                   const int* __restrict__ tok_pos, const int* __restrict__ tok_entry, int page_size,
@@ -90,23 +296,27 @@ IL_EXPORT int il_attn_plain(const void* qkv, int act_kind, int row_stride, void*
     if ((dist_bias && dist_far < 0) || (sigmoid && sink) || (cap > 0.f && (sigmoid || dist_bias))) return IL_BAD_ARG;
     if (nh <= 0 || nkv <= 0 || nh % nkv != 0 || hd <= 0 || page_size <= 0) return IL_BAD_ARG;
     if (hd > 1024) return IL_UNSUPPORTED;
+    if (act_kind != IL_F32 && act_kind != IL_BF16) return IL_BAD_ARG;
+    if (hd <= 256) {
+        const AtArgs a{qkv, cache, out, block_table, tok_pos, tok_entry, sink, dist_bias, row_stride, bt_stride, page_size, T, nh, nkv, hd, window,
+                       dist_far, scale, cap, stream};
+        const cudaError_t e = act_kind == IL_F32 ? at_modes<float>(a, sigmoid) : at_modes<__nv_bfloat16>(a, sigmoid);
+        if (e != cudaSuccess) return 1000 + (int)e;
+        IL_LAUNCH_CHECK();
+        return IL_OK;
+    }
     const int warps = 4;
     dim3 grid(T, (nh + warps - 1) / warps);
-#define AP_LAUNCH1(TA, N, S, C)                                                                                                             \
-    attn_plain_kernel<TA, N, S, C><<<grid, warps * 32, 0, stream>>>((const TA*)qkv, row_stride, (TA*)out, (const TA*)cache, block_table, bt_stride, \
-                                                              tok_pos, tok_entry, page_size, nh, nkv, hd, scale, window, sink, dist_bias, dist_far, cap)
-#define AP_LAUNCH(TA, N)                                            \
-    do {                                                            \
-        if (sigmoid) AP_LAUNCH1(TA, N, true, false);                \
-        else if (cap > 0.f) AP_LAUNCH1(TA, N, false, true);         \
-        else AP_LAUNCH1(TA, N, false, false);                       \
+#define AP_LAUNCH1(TA, S, C)                                                                                                                     \
+    attn_plain_kernel<TA, S, C><<<grid, warps * 32, 0, stream>>>((const TA*)qkv, row_stride, (TA*)out, (const TA*)cache, block_table, bt_stride, \
+                                                                 tok_pos, tok_entry, page_size, nh, nkv, hd, scale, window, sink, dist_bias, dist_far, cap)
+#define AP_LAUNCH(TA)                                    \
+    do {                                                 \
+        if (sigmoid) AP_LAUNCH1(TA, true, false);        \
+        else if (cap > 0.f) AP_LAUNCH1(TA, false, true); \
+        else AP_LAUNCH1(TA, false, false);               \
     } while (0)
-    if (act_kind == IL_F32) {
-        if (hd <= 256) AP_LAUNCH(float, 8); else AP_LAUNCH(float, 32);
-    } else if (act_kind == IL_BF16) {
-        if (hd <= 256) AP_LAUNCH(__nv_bfloat16, 8); else AP_LAUNCH(__nv_bfloat16, 32);
-    } else
-        return IL_BAD_ARG;
+    if (act_kind == IL_F32) AP_LAUNCH(float); else AP_LAUNCH(__nv_bfloat16);
 #undef AP_LAUNCH
 #undef AP_LAUNCH1
     IL_LAUNCH_CHECK();

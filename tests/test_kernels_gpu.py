@@ -345,6 +345,17 @@ def test_attention_plain(cuda_device, dtype, nh, nkv, hd, window, page):
     close(out.cpu(), c["ref"], dtype)
 
 
+@pytest.mark.parametrize("nh,nkv,hd", [(9, 1, 64), (1, 1, 10), (5, 1, 36), (12, 4, 256), (2, 2, 300)])
+@pytest.mark.parametrize("starts,qlens", [([33, 0, 31, 300], [1, 1, 2, 1]), ([0, 70], [90, 260])])
+def test_attention_plain_tiles(cuda_device, nh, nkv, hd, starts, qlens):
+    """Tiles of 32 keys at their edges (1, 32, 33, 34 keys and many tiles), more heads a kv head than a block takes, warps that
+    share a head (few tokens), rows that are not whole 16-byte pieces, and the size behind the tiled kernel's last."""
+    c = _attn_case("float32", nh, nkv, hd, starts, qlens, None, 12, dominate=True)
+    out = torch.full((c["T"], nh * hd), float("nan"), device="cuda")
+    ops.attention_plain(c["qkv"], out, c["cache"], c["bt"], c["tok_pos"], c["tok_entry"], c["page"], nh, nkv, hd, 1 / math.sqrt(hd))
+    close(out.cpu(), c["ref"], "float32")
+
+
 @pytest.mark.parametrize("nh,nkv,hd", SHAPES)
 @pytest.mark.parametrize("window", [None, 21])
 def test_attention_prefill_bf16(cuda_device, nh, nkv, hd, window):
