@@ -215,8 +215,9 @@ static inline bool il_pdl_enabled() {
     return on == 1;
 }
 
+// programmatic false: an ordinary launch, for a kernel that would read, before its wait, what the kernel in front may have written.
 template <typename... KArgs, typename... Args>
-static inline cudaError_t il_launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args... args) {
+static inline cudaError_t il_launch_as(bool programmatic, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = block;
@@ -226,8 +227,12 @@ static inline cudaError_t il_launch(void (*kernel)(KArgs...), dim3 grid, dim3 bl
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = il_pdl_enabled() ? 1 : 0;
+    cfg.numAttrs = programmatic && il_pdl_enabled() ? 1 : 0;
     return cudaLaunchKernelEx(&cfg, kernel, KArgs(args)...);
+}
+template <typename... KArgs, typename... Args>
+static inline cudaError_t il_launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args... args) {
+    return il_launch_as(true, kernel, grid, block, smem, stream, args...);
 }
 #define IL_LAUNCH(kernel, grid, block, smem, stream, ...)                                                \
     do {                                                                                                   \

@@ -20,11 +20,74 @@ __device__ __forceinline__ uint4 gs_ld_stream(const void* p) {
     asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];\n" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
     return v;
 }
-__device__ __forceinline__ uint4 gs_ld(const void* p) { return *reinterpret_cast<const uint4*>(p); }
+// Activations: what the kernel in front wrote. A volatile load stays behind the wait for that kernel, whatever is known of the pointer.
+__device__ __forceinline__ uint4 gs_ld(const void* p) {
+    uint4 v;
+    asm volatile("ld.global.v4.u32 {%0,%1,%2,%3}, [%4];\n" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+    return v;
+}
 __device__ __forceinline__ void gs_mma(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
     asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
                  : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
+
+// One round of a warp's loads: K blocks kb0, kb0 + WARPS, ..; weights 16 bytes of two rows a lane, activations 16 bytes of one row.
+template <int U, int WARPS>
+__device__ __forceinline__ void gs_round_w(uint4 (&a)[U][2], const __nv_bfloat16* const (&wrow)[2], int kb0, int c, int K) {
+    const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+        const int k = (kb0 + u * WARPS) * 32 + c * 8;
+        a[u][0] = k < K ? gs_ld_stream(wrow[0] + k) : zero;
+        a[u][1] = k < K ? gs_ld_stream(wrow[1] + k) : zero;
+    }
+}
+template <int NT, int U, int WARPS>
+__device__ __forceinline__ void gs_round_x(uint4 (&b)[U][NT], const __nv_bfloat16* const (&xrow)[NT], int kb0, int c, int K) {
+    const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+        const int k = (kb0 + u * WARPS) * 32 + c * 8;
+#pragma unroll
+        for (int t = 0; t < NT; ++t) b[u][t] = (k < K && xrow[t]) ? gs_ld(xrow[t] + k) : zero;
+    }
+}
+// The whole round, activations between the weights, for the kernels that wait first and take several rounds (their loads in this
+// order and left to the compiler: asked for one kind after the other the 8B step at batch 8 took 4% longer).
+template <int NT, int U, int WARPS>
+__device__ __forceinline__ void gs_round_both(uint4 (&a)[U][2], uint4 (&b)[U][NT], const __nv_bfloat16* const (&wrow)[2],
+                                              const __nv_bfloat16* const (&xrow)[NT], int kb0, int c, int K) {
+    const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+        const int k = (kb0 + u * WARPS) * 32 + c * 8;
+        const bool ok = k < K;
+        a[u][0] = ok ? gs_ld_stream(wrow[0] + k) : zero;
+        a[u][1] = ok ? gs_ld_stream(wrow[1] + k) : zero;
+#pragma unroll
+        for (int t = 0; t < NT; ++t) b[u][t] = (ok && xrow[t]) ? *reinterpret_cast<const uint4*>(xrow[t] + k) : zero;
+    }
+}
+template <int NT, int U>
+__device__ __forceinline__ void gs_round_mma(float (&acc)[NT][4], const uint4 (&a)[U][2], const uint4 (&b)[U][NT]) {
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+#pragma unroll
+        for (int t = 0; t < NT; ++t) {
+            gs_mma(acc[t], a[u][0].x, a[u][1].x, a[u][0].y, a[u][1].y, b[u][t].x, b[u][t].y);
+            gs_mma(acc[t], a[u][0].z, a[u][1].z, a[u][0].w, a[u][1].w, b[u][t].z, b[u][t].w);
+        }
+}
+// A kernel's wait for the one in front. EARLY kernels have asked for their first round of weights before it, and let the kernel behind
+// them do the same as soon as they start (never before their own wait: a chain of waiting kernels would fill the SMs).
+template <bool EARLY> __device__ __forceinline__ void gs_begin() {
+    il_pdl_begin();
+    if (EARLY) il_pdl_launch_dependents();
+}
+template <bool EARLY> __device__ __forceinline__ void gs_tail() {
+    if (!EARLY) il_pdl_tail();
+}
+
 template <typename TO> __device__ __forceinline__ void gs_store(TO* p, float v);
 template <> __device__ __forceinline__ void gs_store<float>(float* p, float v) { *p = v; }
 template <> __device__ __forceinline__ void gs_store<__nv_bfloat16>(__nv_bfloat16* p, float v) { *p = __float2bfloat16_rn(v); }
@@ -64,6 +127,12 @@ __device__ __forceinline__ void gs_norm_finish(float* rstd_s, const float (&pv)[
     }
 }
 
+// Where all of K is one round of loads (1,024 columns with four blocks an SM, else 2,048), the weights are asked for before the wait
+// for the kernel in front (EARLY): what is left behind it is one trip to L2 for the activations. One request on the 0.5B sizes: 13.4
+// -> 10.2 ms for 24 tokens together with the resid form's 16 warps and attention in one split; eight on Gopitar at 2,048 columns 24.9
+// -> 24.5 ms. With K in several rounds (4,096 at 8B sizes) asking early lost 4%: registers held through the wait.
+constexpr int GS_EARLY_K(int U) { return GS_WARPS * U * 32; }
+
 // What the epilogue of ACT_GELU_TANH_ROW multiplies by: row ids[m] of a table (bfloat16), columns off .. off + dim; columns of the
 // product from dim on give 0.
 struct GsRowMul {
@@ -75,80 +144,60 @@ __host__ __device__ constexpr bool gs_gated(int glu) { return glu >= IL_ACT_SILU
 
 // NT: 8-row groups of x (1: M <= 8, 2: M <= 16). GLU: 0 plain, 4 plain with relu(.)^2, 5 plain with gelu_tanh(.) * a table's row; 1 SwiGLU, 2 the same with the tanh form of GELU as the gate, 3 with the clamped gate (act_limit, act_alpha) (W holds N gate rows, then N up rows). U: blocks in flight.
 // NRM: the activations may come without their norm's 1/rms (`ni`); the SwiGLU form always can, the plain form as a variant of its own.
-template <int NT, int GLU, int U, typename TO, bool NRM = gs_gated(GLU)>
-__global__ void __launch_bounds__(GS_WARPS * 32, 2) gemm_skinny_kernel(const __nv_bfloat16* __restrict__ x, int ldx,
+template <int NT, int GLU, int U, typename TO, bool NRM, bool EARLY>
+__global__ void __launch_bounds__(GS_WARPS * 32, EARLY && NT == 1 && U == 4 ? 4 : 2) gemm_skinny_kernel(const __nv_bfloat16* __restrict__ x, int ldx,
                                                                     const __nv_bfloat16* __restrict__ W, int ldw, TO* __restrict__ out,
                                                                     int ldo, const float* __restrict__ bias, float alpha, int M, int N, int K,
                                                                     const GsNormIn ni, float act_limit, float act_alpha, const GsRowMul rm) {
-    constexpr int NW = 1;
     constexpr bool GATED = gs_gated(GLU);
     constexpr int ROWS = GATED ? 8 : 16;           // outputs per activation row and tile: 16 rows, or 8 gate rows with their 8 up rows
-    __shared__ float part[GS_WARPS][NW][NT][16][8];
+    __shared__ float part[GS_WARPS][NT][16][8];
     __shared__ float rstd_s[NT * 8];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int r = lane >> 2, c = lane & 3;
     const int n0 = blockIdx.x * ROWS;
-    const __nv_bfloat16* wrow[NW][2];
+    const __nv_bfloat16* wrow[2];
 #pragma unroll
-    for (int s = 0; s < NW; ++s)
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            int n = GATED ? n0 + r : n0 + r + 8 * h;
-            if (n > N - 1) n = N - 1;             // rows past the end are computed and dropped
-            wrow[s][h] = W + ((size_t)(GATED ? h : 0) * N + n) * ldw;
-        }
-    il_pdl_begin();
+    for (int h = 0; h < 2; ++h) {
+        int n = GATED ? n0 + r : n0 + r + 8 * h;
+        if (n > N - 1) n = N - 1;                 // rows past the end are computed and dropped
+        wrow[h] = W + ((size_t)(GATED ? h : 0) * N + n) * ldw;
+    }
+    uint4 a[U][2], b[U][NT];
+    if (EARLY) gs_round_w<U, GS_WARPS>(a, wrow, warp, c, K);
+    gs_begin<EARLY>();
     float pv[NT][8];
     if (NRM) gs_norm_fetch<NT>(pv, ni, M, warp, lane);
     const __nv_bfloat16* xrow[NT];
 #pragma unroll
     for (int t = 0; t < NT; ++t) xrow[t] = (t * 8 + r < M) ? x + (size_t)(t * 8 + r) * ldx : nullptr;
 
-    float acc[NW][NT][4];
+    float acc[NT][4];
 #pragma unroll
-    for (int s = 0; s < NW; ++s)
+    for (int t = 0; t < NT; ++t)
 #pragma unroll
-        for (int t = 0; t < NT; ++t)
-#pragma unroll
-            for (int j = 0; j < 4; ++j) acc[s][t][j] = 0.f;
+        for (int j = 0; j < 4; ++j) acc[t][j] = 0.f;
 
     const int nkb = (K + 31) >> 5;
-    const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
-    for (int kb0 = warp; kb0 < nkb; kb0 += GS_WARPS * U) {
-        uint4 a[U][NW][2], b[U][NT];
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-            const int k = (kb0 + u * GS_WARPS) * 32 + c * 8;
-            const bool ok = k < K;
-#pragma unroll
-            for (int s = 0; s < NW; ++s) {
-                a[u][s][0] = ok ? gs_ld_stream(wrow[s][0] + k) : zero;
-                a[u][s][1] = ok ? gs_ld_stream(wrow[s][1] + k) : zero;
-            }
-#pragma unroll
-            for (int t = 0; t < NT; ++t) b[u][t] = (ok && xrow[t]) ? gs_ld(xrow[t] + k) : zero;
+    if (EARLY) {                                  // all of K is one round
+        gs_round_x<NT, U, GS_WARPS>(b, xrow, warp, c, K);
+        gs_round_mma<NT, U>(acc, a, b);
+    } else {
+        for (int kb0 = warp; kb0 < nkb; kb0 += GS_WARPS * U) {
+            uint4 a[U][2], b[U][NT];
+            gs_round_both<NT, U, GS_WARPS>(a, b, wrow, xrow, kb0, c, K);
+            gs_round_mma<NT, U>(acc, a, b);
         }
-#pragma unroll
-        for (int u = 0; u < U; ++u)
-#pragma unroll
-            for (int s = 0; s < NW; ++s)
-#pragma unroll
-                for (int t = 0; t < NT; ++t) {
-                    gs_mma(acc[s][t], a[u][s][0].x, a[u][s][1].x, a[u][s][0].y, a[u][s][1].y, b[u][t].x, b[u][t].y);
-                    gs_mma(acc[s][t], a[u][s][0].z, a[u][s][1].z, a[u][s][0].w, a[u][s][1].w, b[u][t].z, b[u][t].w);
-                }
     }
-    il_pdl_tail();
+    gs_tail<EARLY>();
     if (NRM) gs_norm_finish<NT>(rstd_s, pv, ni, warp, lane);
 #pragma unroll
-    for (int s = 0; s < NW; ++s)
-#pragma unroll
-        for (int t = 0; t < NT; ++t) {
-            part[warp][s][t][r][c * 2] = acc[s][t][0];
-            part[warp][s][t][r][c * 2 + 1] = acc[s][t][1];
-            part[warp][s][t][r + 8][c * 2] = acc[s][t][2];
-            part[warp][s][t][r + 8][c * 2 + 1] = acc[s][t][3];
-        }
+    for (int t = 0; t < NT; ++t) {
+        part[warp][t][r][c * 2] = acc[t][0];
+        part[warp][t][r][c * 2 + 1] = acc[t][1];
+        part[warp][t][r + 8][c * 2] = acc[t][2];
+        part[warp][t][r + 8][c * 2 + 1] = acc[t][3];
+    }
     __syncthreads();
     for (int idx = threadIdx.x; idx < NT * 8 * ROWS; idx += GS_WARPS * 32) {
         const int nl = idx % ROWS, m = idx / ROWS;   // consecutive threads: consecutive output columns
@@ -158,8 +207,8 @@ __global__ void __launch_bounds__(GS_WARPS * 32, 2) gemm_skinny_kernel(const __n
         float s0 = 0.f, s1 = 0.f;
 #pragma unroll
         for (int w = 0; w < GS_WARPS; ++w) {
-            s0 += part[w][0][t][nl][mc];
-            if (GATED) s1 += part[w][0][t][nl + 8][mc];
+            s0 += part[w][t][nl][mc];
+            if (GATED) s1 += part[w][t][nl + 8][mc];
         }
         const float an = NRM ? __fmul_rn(alpha, rstd_s[m]) : alpha;     // the norm's 1/rms, where the activations came without it
         float y = __fmaf_rn(an, s0, bias ? bias[n] : 0.f);      // spelled out as one fused multiply-add: the same bits from every build of this line
@@ -178,22 +227,28 @@ __global__ void __launch_bounds__(GS_WARPS * 32, 2) gemm_skinny_kernel(const __n
 
 template <int NT, int GLU, typename TO, bool NRM = gs_gated(GLU)>
 static cudaError_t gs_launch(const void* x, int ldx, const void* W, int ldw, void* out, int ldo, const float* bias, float alpha, int M, int N,
-                      int K, cudaStream_t stream, const GsNormIn& ni = GsNormIn{nullptr, 0, 0.f, 0.f}, float act_limit = 0.f,
+                      int K, bool w_static, cudaStream_t stream, const GsNormIn& ni = GsNormIn{nullptr, 0, 0.f, 0.f}, float act_limit = 0.f,
                       float act_alpha = 0.f, const GsRowMul& rm = GsRowMul{nullptr, nullptr, 0, 0, 0, 0}) {
-    constexpr int U = NT == 1 ? 8 : 4;
-    constexpr int ROWS = gs_gated(GLU) ? 8 : 16;
-    return il_launch(gemm_skinny_kernel<NT, GLU, U, TO, NRM>, dim3((N + ROWS - 1) / ROWS), dim3(GS_WARPS * 32), 0, stream,
-              (const __nv_bfloat16*)x, ldx, (const __nv_bfloat16*)W, ldw, (TO*)out, ldo, bias, alpha, M, N, K, ni, act_limit, act_alpha, rm);
+    constexpr int U = NT == 1 ? 8 : 4, ROWS = gs_gated(GLU) ? 8 : 16;
+    const auto go = [&](auto kernel, bool early) {
+        return il_launch_as(w_static || !early, kernel, dim3((N + ROWS - 1) / ROWS), dim3(GS_WARPS * 32), 0, stream, (const __nv_bfloat16*)x, ldx, (const __nv_bfloat16*)W,
+                         ldw, (TO*)out, ldo, bias, alpha, M, N, K, ni, act_limit, act_alpha, rm);
+    };
+    if (K <= GS_EARLY_K(4)) return go(gemm_skinny_kernel<NT, GLU, 4, TO, NRM, true>, true);
+    if (K <= GS_EARLY_K(U)) return go(gemm_skinny_kernel<NT, GLU, U, TO, NRM, true>, true);
+    return go(gemm_skinny_kernel<NT, GLU, U, TO, NRM, false>, false);
 }
 
 // glu = 1: W is [2N, K] (N gate rows, then N up rows), bias [2N], out[M,N] = silu(alpha*x.Wg^T + bg) * (alpha*x.Wu^T + bu);
 // glu = 2: the same with gelu_tanh in place of silu; glu = 3: the clamped gate with its two numbers; glu = 4: W is [N, K] and
 // out[M,N] = relu(alpha*x.W^T + b)^2. (These write bfloat16.)
+// w_static: W was written long before (a model's weights), not by the kernel in front of this one in the stream: kernels that ask for
+// weights before their wait are then launched to overlap with that kernel, else as an ordinary launch.
 // norm_partial (may be null): x is residual * norm weight and still wants its 1/rms, from these sums of squares
 // [M][n_partial] (n_partial <= 256, H = the width they were summed over).
 IL_EXPORT int il_gemm_skinny(const void* x, int ldx, const void* W, int ldw, void* out, int out_kind, int ldo, const float* bias,
                              float alpha, int M, int N, int K, int glu, const float* norm_partial, int n_partial, int norm_h,
-                             float norm_eps, float act_limit, float act_alpha, cudaStream_t stream) {
+                             float norm_eps, float act_limit, float act_alpha, int w_static, cudaStream_t stream) {
     if (M <= 0 || N <= 0) return IL_OK;
     if (norm_partial && (n_partial <= 0 || n_partial > GS_NORM_MAX_PARTIALS || norm_h <= 0)) return IL_UNSUPPORTED;
     const GsNormIn ni{norm_partial, n_partial, norm_partial ? 1.f / (float)norm_h : 0.f, norm_eps};
@@ -202,25 +257,25 @@ IL_EXPORT int il_gemm_skinny(const void* x, int ldx, const void* W, int ldw, voi
     if (glu && out_kind != IL_BF16) return IL_UNSUPPORTED;
     cudaError_t e;
     if (M <= 8) {
-        if (glu == 4 && norm_partial) e = gs_launch<1, 4, __nv_bfloat16, true>(x, ldx, W, ldw, out, ldo, bias, alpha, M, N, K, stream, ni);
-        else if (glu == 4) e = gs_launch<1, 4, __nv_bfloat16>(x, ldx, W, ldw, out, ldo, bias, alpha, M, N, K, stream);
-        else if (glu == 3) e = gs_launch<1, 3, __nv_bfloat16>(x, ldx, W, ldw, out, ldo, bias, alpha, M, N, K, stream, ni, act_limit, act_alpha);
-        else if (glu == 2) e = gs_launch<1, 2, __nv_bfloat16>(x, ldx, W, ldw, out, ldo, bias, alpha, M, N, K, stream, ni);
-        else if (glu) e = gs_launch<1, 1, __nv_bfloat16>(x, ldx, W, ldw, out, ldo, bias, alpha, M, N, K, stream, ni);
-        else if (norm_partial && out_kind == IL_BF16) e = gs_launch<1, 0, __nv_bfloat16, true>(x, ldx, W, ldw, out, ldo, bias, alpha, M, N, K, stream, ni);
-        else if (norm_partial) e = gs_launch<1, 0, float, true>(x, ldx, W, ldw, out, ldo, bias, alpha, M, N, K, stream, ni);
-        else if (out_kind == IL_BF16) e = gs_launch<1, 0, __nv_bfloat16>(x, ldx, W, ldw, out, ldo, bias, alpha, M, N, K, stream);
-        else e = gs_launch<1, 0, float>(x, ldx, W, ldw, out, ldo, bias, alpha, M, N, K, stream);
+        if (glu == 4 && norm_partial) e = gs_launch<1, 4, __nv_bfloat16, true>(x, ldx, W, ldw, out, ldo, bias, alpha, M, N, K, w_static != 0, stream, ni);
+        else if (glu == 4) e = gs_launch<1, 4, __nv_bfloat16>(x, ldx, W, ldw, out, ldo, bias, alpha, M, N, K, w_static != 0, stream);
+        else if (glu == 3) e = gs_launch<1, 3, __nv_bfloat16>(x, ldx, W, ldw, out, ldo, bias, alpha, M, N, K, w_static != 0, stream, ni, act_limit, act_alpha);
+        else if (glu == 2) e = gs_launch<1, 2, __nv_bfloat16>(x, ldx, W, ldw, out, ldo, bias, alpha, M, N, K, w_static != 0, stream, ni);
+        else if (glu) e = gs_launch<1, 1, __nv_bfloat16>(x, ldx, W, ldw, out, ldo, bias, alpha, M, N, K, w_static != 0, stream, ni);
+        else if (norm_partial && out_kind == IL_BF16) e = gs_launch<1, 0, __nv_bfloat16, true>(x, ldx, W, ldw, out, ldo, bias, alpha, M, N, K, w_static != 0, stream, ni);
+        else if (norm_partial) e = gs_launch<1, 0, float, true>(x, ldx, W, ldw, out, ldo, bias, alpha, M, N, K, w_static != 0, stream, ni);
+        else if (out_kind == IL_BF16) e = gs_launch<1, 0, __nv_bfloat16>(x, ldx, W, ldw, out, ldo, bias, alpha, M, N, K, w_static != 0, stream);
+        else e = gs_launch<1, 0, float>(x, ldx, W, ldw, out, ldo, bias, alpha, M, N, K, w_static != 0, stream);
     } else {
-        if (glu == 4 && norm_partial) e = gs_launch<2, 4, __nv_bfloat16, true>(x, ldx, W, ldw, out, ldo, bias, alpha, M, N, K, stream, ni);
-        else if (glu == 4) e = gs_launch<2, 4, __nv_bfloat16>(x, ldx, W, ldw, out, ldo, bias, alpha, M, N, K, stream);
-        else if (glu == 3) e = gs_launch<2, 3, __nv_bfloat16>(x, ldx, W, ldw, out, ldo, bias, alpha, M, N, K, stream, ni, act_limit, act_alpha);
-        else if (glu == 2) e = gs_launch<2, 2, __nv_bfloat16>(x, ldx, W, ldw, out, ldo, bias, alpha, M, N, K, stream, ni);
-        else if (glu) e = gs_launch<2, 1, __nv_bfloat16>(x, ldx, W, ldw, out, ldo, bias, alpha, M, N, K, stream, ni);
-        else if (norm_partial && out_kind == IL_BF16) e = gs_launch<2, 0, __nv_bfloat16, true>(x, ldx, W, ldw, out, ldo, bias, alpha, M, N, K, stream, ni);
-        else if (norm_partial) e = gs_launch<2, 0, float, true>(x, ldx, W, ldw, out, ldo, bias, alpha, M, N, K, stream, ni);
-        else if (out_kind == IL_BF16) e = gs_launch<2, 0, __nv_bfloat16>(x, ldx, W, ldw, out, ldo, bias, alpha, M, N, K, stream);
-        else e = gs_launch<2, 0, float>(x, ldx, W, ldw, out, ldo, bias, alpha, M, N, K, stream);
+        if (glu == 4 && norm_partial) e = gs_launch<2, 4, __nv_bfloat16, true>(x, ldx, W, ldw, out, ldo, bias, alpha, M, N, K, w_static != 0, stream, ni);
+        else if (glu == 4) e = gs_launch<2, 4, __nv_bfloat16>(x, ldx, W, ldw, out, ldo, bias, alpha, M, N, K, w_static != 0, stream);
+        else if (glu == 3) e = gs_launch<2, 3, __nv_bfloat16>(x, ldx, W, ldw, out, ldo, bias, alpha, M, N, K, w_static != 0, stream, ni, act_limit, act_alpha);
+        else if (glu == 2) e = gs_launch<2, 2, __nv_bfloat16>(x, ldx, W, ldw, out, ldo, bias, alpha, M, N, K, w_static != 0, stream, ni);
+        else if (glu) e = gs_launch<2, 1, __nv_bfloat16>(x, ldx, W, ldw, out, ldo, bias, alpha, M, N, K, w_static != 0, stream, ni);
+        else if (norm_partial && out_kind == IL_BF16) e = gs_launch<2, 0, __nv_bfloat16, true>(x, ldx, W, ldw, out, ldo, bias, alpha, M, N, K, w_static != 0, stream, ni);
+        else if (norm_partial) e = gs_launch<2, 0, float, true>(x, ldx, W, ldw, out, ldo, bias, alpha, M, N, K, w_static != 0, stream, ni);
+        else if (out_kind == IL_BF16) e = gs_launch<2, 0, __nv_bfloat16>(x, ldx, W, ldw, out, ldo, bias, alpha, M, N, K, w_static != 0, stream);
+        else e = gs_launch<2, 0, float>(x, ldx, W, ldw, out, ldo, bias, alpha, M, N, K, w_static != 0, stream);
     }
     if (e != cudaSuccess) return 1000 + (int)e;
     IL_LAUNCH_CHECK();
@@ -229,14 +284,14 @@ IL_EXPORT int il_gemm_skinny(const void* x, int ldx, const void* W, int ldw, voi
 
 // out[m, n] = gelu_tanh(x . W^T) * table[ids[m], off + n] (bfloat16; columns n >= dim give 0): the gate of a token's own table row.
 IL_EXPORT int il_gemm_skinny_gelu_row(const void* x, int ldx, const void* W, int ldw, void* out, int ldo, int M, int N, int K, const int* ids,
-                                      const void* table, int ldt, int off, int dim, int vocab, cudaStream_t stream) {
+                                      const void* table, int ldt, int off, int dim, int vocab, int w_static, cudaStream_t stream) {
     if (M <= 0 || N <= 0) return IL_OK;
     if (M > 16 || K <= 0 || (K & 7) || (ldx & 7) || (ldw & 7) || ldx < K || ldw < K || ldo < N) return IL_UNSUPPORTED;
     if (!ids || !table || dim <= 0 || dim > N || off < 0 || off + dim > ldt || vocab <= 0) return IL_BAD_ARG;
     const GsNormIn ni{nullptr, 0, 0.f, 0.f};
     const GsRowMul rm{ids, (const __nv_bfloat16*)table, ldt, off, dim, vocab};
-    const cudaError_t e = M <= 8 ? gs_launch<1, 5, __nv_bfloat16>(x, ldx, W, ldw, out, ldo, nullptr, 1.f, M, N, K, stream, ni, 0.f, 0.f, rm)
-                                 : gs_launch<2, 5, __nv_bfloat16>(x, ldx, W, ldw, out, ldo, nullptr, 1.f, M, N, K, stream, ni, 0.f, 0.f, rm);
+    const cudaError_t e = M <= 8 ? gs_launch<1, 5, __nv_bfloat16>(x, ldx, W, ldw, out, ldo, nullptr, 1.f, M, N, K, w_static != 0, stream, ni, 0.f, 0.f, rm)
+                                 : gs_launch<2, 5, __nv_bfloat16>(x, ldx, W, ldw, out, ldo, nullptr, 1.f, M, N, K, w_static != 0, stream, ni, 0.f, 0.f, rm);
     if (e != cudaSuccess) return 1000 + (int)e;
     IL_LAUNCH_CHECK();
     return IL_OK;
@@ -260,7 +315,7 @@ struct GsRope {
     float mscale;
 };
 
-template <int NT, int U>
+template <int NT, int U, bool EARLY>
 __global__ void __launch_bounds__(GS_WARPS * 32, 2) gemm_skinny_rope_kernel(const __nv_bfloat16* x, int ldx,
                                                                          const __nv_bfloat16* __restrict__ W, int ldw,
                                                                          __nv_bfloat16* __restrict__ out, int ldo,
@@ -281,6 +336,8 @@ __global__ void __launch_bounds__(GS_WARPS * 32, 2) gemm_skinny_rope_kernel(cons
     const __nv_bfloat16* wrow[2];
 #pragma unroll
     for (int h = 0; h < 2; ++h) wrow[h] = W + (size_t)(n_lo + r + h * step) * ldw;
+    uint4 a[U][2], b[U][NT];
+    if (EARLY) gs_round_w<U, GS_WARPS>(a, wrow, warp, c, K);
     // positions, slots and angles come with the step's descriptors: made ready while the kernel before still runs
     for (int i = threadIdx.x; i < NT * 8 * 8; i += GS_WARPS * 32) {
         const int m = i >> 3, nl = i & 7;
@@ -303,7 +360,7 @@ __global__ void __launch_bounds__(GS_WARPS * 32, 2) gemm_skinny_rope_kernel(cons
         }
         slot[m] = off;
     }
-    il_pdl_begin();
+    gs_begin<EARLY>();
     float pv[NT][8];
     gs_norm_fetch<NT>(pv, ni, M, warp, lane);
     const __nv_bfloat16* xrow[NT];
@@ -315,28 +372,18 @@ __global__ void __launch_bounds__(GS_WARPS * 32, 2) gemm_skinny_rope_kernel(cons
 #pragma unroll
         for (int q = 0; q < 4; ++q) acc[t][q] = 0.f;
     const int nkb = (K + 31) >> 5;
-    const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
-    for (int kb0 = warp; kb0 < nkb; kb0 += GS_WARPS * U) {
-        uint4 a[U][2], b[U][NT];
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-            const int k = (kb0 + u * GS_WARPS) * 32 + c * 8;
-            const bool ok = k < K;
-            a[u][0] = ok ? gs_ld_stream(wrow[0] + k) : zero;
-            a[u][1] = ok ? gs_ld_stream(wrow[1] + k) : zero;
-#pragma unroll
-            for (int t = 0; t < NT; ++t) b[u][t] = (ok && xrow[t]) ? gs_ld(xrow[t] + k) : zero;
+    if (EARLY) {                                  // all of K is one round
+        gs_round_x<NT, U, GS_WARPS>(b, xrow, warp, c, K);
+        gs_round_mma<NT, U>(acc, a, b);
+    } else {
+        for (int kb0 = warp; kb0 < nkb; kb0 += GS_WARPS * U) {
+            uint4 a[U][2], b[U][NT];
+            gs_round_both<NT, U, GS_WARPS>(a, b, wrow, xrow, kb0, c, K);
+            __syncwarp();                         // keeps every load above issued before the first product waits for one
+            gs_round_mma<NT, U>(acc, a, b);
         }
-        __syncwarp();                             // keeps every load above issued before the first product waits for one
-#pragma unroll
-        for (int u = 0; u < U; ++u)
-#pragma unroll
-            for (int t = 0; t < NT; ++t) {
-                gs_mma(acc[t], a[u][0].x, a[u][1].x, a[u][0].y, a[u][1].y, b[u][t].x, b[u][t].y);
-                gs_mma(acc[t], a[u][0].z, a[u][1].z, a[u][0].w, a[u][1].w, b[u][t].z, b[u][t].w);
-            }
     }
-    il_pdl_tail();
+    gs_tail<EARLY>();
     gs_norm_finish<NT>(rstd_s, pv, ni, warp, lane);
 #pragma unroll
     for (int t = 0; t < NT; ++t) {
@@ -381,7 +428,7 @@ __global__ void __launch_bounds__(GS_WARPS * 32, 2) gemm_skinny_rope_kernel(cons
 IL_EXPORT int il_gemm_skinny_rope(const void* x, int ldx, const void* W, int ldw, void* out, int ldo, const float* bias, float alpha,
                                   int M, int K, const int* tok_pos, const int* tok_entry, const int* block_table, int bt_stride,
                                   void* cache, int page_size, int nh, int nkv, int hd, int rot, const float* inv_freq, float mscale,
-                                  const float* norm_partial, int n_partial, int norm_h, float norm_eps, cudaStream_t stream) {
+                                  const float* norm_partial, int n_partial, int norm_h, float norm_eps, int w_static, cudaStream_t stream) {
     if (M <= 0) return IL_OK;
     if (norm_partial && (n_partial <= 0 || n_partial > GS_NORM_MAX_PARTIALS || norm_h <= 0)) return IL_UNSUPPORTED;
     const GsNormIn ni{norm_partial, n_partial, norm_partial ? 1.f / (float)norm_h : 0.f, norm_eps};
@@ -390,13 +437,14 @@ IL_EXPORT int il_gemm_skinny_rope(const void* x, int ldx, const void* W, int ldw
     if (nh <= 0 || nkv <= 0 || hd <= 0 || (hd & 15) || rot < 0 || rot > hd || (rot & 15) || page_size <= 0) return IL_UNSUPPORTED;
     if (rot > 0 && !inv_freq) return IL_BAD_ARG;
     GsRope rp{tok_pos, tok_entry, block_table, bt_stride, (__nv_bfloat16*)cache, page_size, nh, nkv, hd, rot, inv_freq, mscale};
-    cudaError_t e;
-    if (M <= 8)
-        e = il_launch(gemm_skinny_rope_kernel<1, 8>, dim3(N / 16), dim3(GS_WARPS * 32), 0, stream, (const __nv_bfloat16*)x, ldx,
-                      (const __nv_bfloat16*)W, ldw, (__nv_bfloat16*)out, ldo, bias, alpha, M, K, rp, ni);
-    else
-        e = il_launch(gemm_skinny_rope_kernel<2, 4>, dim3(N / 16), dim3(GS_WARPS * 32), 0, stream, (const __nv_bfloat16*)x, ldx,
-                      (const __nv_bfloat16*)W, ldw, (__nv_bfloat16*)out, ldo, bias, alpha, M, K, rp, ni);
+    const auto go = [&](auto kernel, bool early) {
+        return il_launch_as(w_static || !early, kernel, dim3(N / 16), dim3(GS_WARPS * 32), 0, stream, (const __nv_bfloat16*)x, ldx, (const __nv_bfloat16*)W, ldw,
+                         (__nv_bfloat16*)out, ldo, bias, alpha, M, K, rp, ni);
+    };
+    const cudaError_t e = M <= 8 ? (K <= GS_EARLY_K(4)   ? go(gemm_skinny_rope_kernel<1, 4, true>, true)
+                                    : K <= GS_EARLY_K(8) ? go(gemm_skinny_rope_kernel<1, 8, true>, true)
+                                                         : go(gemm_skinny_rope_kernel<1, 8, false>, false))
+                                 : (K <= GS_EARLY_K(4) ? go(gemm_skinny_rope_kernel<2, 4, true>, true) : go(gemm_skinny_rope_kernel<2, 4, false>, false));
     if (e != cudaSuccess) return 1000 + (int)e;
     IL_LAUNCH_CHECK();
     return IL_OK;
@@ -407,14 +455,14 @@ IL_EXPORT int il_gemm_skinny_rope(const void* x, int ldx, const void* W, int ldw
 // y = alpha * x . W^T (+ bias), rounded to bfloat16 as the product alone would store it; resid += bscale * y (float32, in
 // place); xw = resid * norm_w as bfloat16; sumsq[m][block] = sum of resid^2 over the block's 16 columns. N = the width of
 // the residual stream. What add_rmsnorm does, but for the division by the rms, which the next product applies.
-template <int NT, int U>
-__global__ void __launch_bounds__(GS_WARPS * 32, 2) gemm_skinny_resid_kernel(const __nv_bfloat16* __restrict__ x, int ldx,
+template <int NT, int U, int WARPS, bool EARLY>
+__global__ void __launch_bounds__(WARPS * 32, WARPS > 8 ? 1 : 2) gemm_skinny_resid_kernel(const __nv_bfloat16* __restrict__ x, int ldx,
                                                                           const __nv_bfloat16* __restrict__ W, int ldw,
                                                                           const float* __restrict__ bias, float alpha, int M, int N, int K,
                                                                           float* resid, float bscale, const void* __restrict__ norm_w,
                                                                           int norm_w_kind, __nv_bfloat16* __restrict__ xw,
                                                                           float* __restrict__ sumsq) {
-    __shared__ float part[GS_WARPS][NT][16][8];
+    __shared__ float part[WARPS][NT][16][8];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int r = lane >> 2, c = lane & 3;
     const int n0 = blockIdx.x * 16;
@@ -425,7 +473,9 @@ __global__ void __launch_bounds__(GS_WARPS * 32, 2) gemm_skinny_resid_kernel(con
         if (n > N - 1) n = N - 1;                 // rows past the end are computed and dropped
         wrow[h] = W + (size_t)n * ldw;
     }
-    il_pdl_begin();
+    uint4 a[U][2], b[U][NT];
+    if (EARLY) gs_round_w<U, WARPS>(a, wrow, warp, c, K);
+    gs_begin<EARLY>();
     // What the epilogue adds to - the residual, the norm's weight, the bias of this thread's (row, column) - is asked for
     // now: read after the main loop it cost the kernel a round trip to memory at its very end.
     const int e_nl = threadIdx.x & 15, e_m = threadIdx.x >> 4, e_n = n0 + e_nl;
@@ -442,27 +492,16 @@ __global__ void __launch_bounds__(GS_WARPS * 32, 2) gemm_skinny_resid_kernel(con
 #pragma unroll
         for (int q = 0; q < 4; ++q) acc[t][q] = 0.f;
     const int nkb = (K + 31) >> 5;
-    const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
-    for (int kb0 = warp; kb0 < nkb; kb0 += GS_WARPS * U) {
-        uint4 a[U][2], b[U][NT];
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-            const int k = (kb0 + u * GS_WARPS) * 32 + c * 8;
-            const bool ok = k < K;
-            a[u][0] = ok ? gs_ld_stream(wrow[0] + k) : zero;
-            a[u][1] = ok ? gs_ld_stream(wrow[1] + k) : zero;
-#pragma unroll
-            for (int t = 0; t < NT; ++t) b[u][t] = (ok && xrow[t]) ? gs_ld(xrow[t] + k) : zero;
-        }
-#pragma unroll
-        for (int u = 0; u < U; ++u)
-#pragma unroll
-            for (int t = 0; t < NT; ++t) {
-                gs_mma(acc[t], a[u][0].x, a[u][1].x, a[u][0].y, a[u][1].y, b[u][t].x, b[u][t].y);
-                gs_mma(acc[t], a[u][0].z, a[u][1].z, a[u][0].w, a[u][1].w, b[u][t].z, b[u][t].w);
-            }
+    if (EARLY) {
+        gs_round_x<NT, U, WARPS>(b, xrow, warp, c, K);
+        gs_round_mma<NT, U>(acc, a, b);
     }
-    il_pdl_tail();
+    for (int kb0 = warp + (EARLY ? WARPS * U : 0); kb0 < nkb; kb0 += WARPS * U) {
+        uint4 a[U][2], b[U][NT];
+        gs_round_both<NT, U, WARPS>(a, b, wrow, xrow, kb0, c, K);
+        gs_round_mma<NT, U>(acc, a, b);
+    }
+    gs_tail<EARLY>();
 #pragma unroll
     for (int t = 0; t < NT; ++t) {
         part[warp][t][r][c * 2] = acc[t][0];
@@ -481,7 +520,7 @@ __global__ void __launch_bounds__(GS_WARPS * 32, 2) gemm_skinny_resid_kernel(con
     if (m < M && n < N) {
         float s0 = 0.f;
 #pragma unroll
-        for (int w = 0; w < GS_WARPS; ++w) s0 += part[w][t][nl][mc];
+        for (int w = 0; w < WARPS; ++w) s0 += part[w][t][nl][mc];
         const float y = __bfloat162float(__float2bfloat16_rn(alpha * s0 + e_bias));
         h = e_resid + bscale * y;
         resid[(size_t)m * N + n] = h;
@@ -498,18 +537,26 @@ __global__ void __launch_bounds__(GS_WARPS * 32, 2) gemm_skinny_resid_kernel(con
 // N = width of the residual stream; sumsq gets [M][ceil(N / 16)] floats (at most 256 a row: N <= 4096).
 IL_EXPORT int il_gemm_skinny_resid(const void* x, int ldx, const void* W, int ldw, const float* bias, float alpha, int M, int N, int K,
                                    float* resid, float bscale, const void* norm_w, int norm_w_kind, void* xw, float* sumsq,
-                                   cudaStream_t stream) {
+                                   int w_static, cudaStream_t stream) {
     if (M <= 0 || N <= 0) return IL_OK;
     if (M > 16 || K <= 0 || (K & 7) || (ldx & 7) || (ldw & 7) || ldx < K || ldw < K) return IL_UNSUPPORTED;
     if ((N + 15) / 16 > GS_NORM_MAX_PARTIALS || !resid || !norm_w || !xw || !sumsq) return IL_UNSUPPORTED;
     if (norm_w_kind != IL_F32 && norm_w_kind != IL_BF16) return IL_BAD_ARG;
+    const auto go = [&](auto kernel, int warps, bool early) {
+        return il_launch_as(w_static || !early, kernel, dim3((N + 15) / 16), dim3(warps * 32), 0, stream, (const __nv_bfloat16*)x, ldx, (const __nv_bfloat16*)W, ldw, bias, alpha,
+                         M, N, K, resid, bscale, norm_w, norm_w_kind, (__nv_bfloat16*)xw, sumsq);
+    };
+    const bool wide = K > GS_EARLY_K(8) && (N + 15) / 16 <= 148;      // fewer blocks than SMs: 16 warps a block
     cudaError_t e;
     if (M <= 8)
-        e = il_launch(gemm_skinny_resid_kernel<1, 8>, dim3((N + 15) / 16), dim3(GS_WARPS * 32), 0, stream, (const __nv_bfloat16*)x, ldx,
-                      (const __nv_bfloat16*)W, ldw, bias, alpha, M, N, K, resid, bscale, norm_w, norm_w_kind, (__nv_bfloat16*)xw, sumsq);
+        e = wide                   ? go(gemm_skinny_resid_kernel<1, 8, 16, true>, 16, true)
+            : K <= GS_EARLY_K(4)   ? go(gemm_skinny_resid_kernel<1, 4, GS_WARPS, true>, GS_WARPS, true)
+            : K <= GS_EARLY_K(8)   ? go(gemm_skinny_resid_kernel<1, 8, GS_WARPS, true>, GS_WARPS, true)
+                                   : go(gemm_skinny_resid_kernel<1, 8, GS_WARPS, false>, GS_WARPS, false);
     else
-        e = il_launch(gemm_skinny_resid_kernel<2, 4>, dim3((N + 15) / 16), dim3(GS_WARPS * 32), 0, stream, (const __nv_bfloat16*)x, ldx,
-                      (const __nv_bfloat16*)W, ldw, bias, alpha, M, N, K, resid, bscale, norm_w, norm_w_kind, (__nv_bfloat16*)xw, sumsq);
+        e = wide                 ? go(gemm_skinny_resid_kernel<2, 4, 16, true>, 16, true)
+            : K <= GS_EARLY_K(4) ? go(gemm_skinny_resid_kernel<2, 4, GS_WARPS, true>, GS_WARPS, true)
+                                 : go(gemm_skinny_resid_kernel<2, 4, GS_WARPS, false>, GS_WARPS, false);
     if (e != cudaSuccess) return 1000 + (int)e;
     IL_LAUNCH_CHECK();
     return IL_OK;

@@ -213,9 +213,10 @@ def gelu_row(z: torch.Tensor, ids: torch.Tensor, table: torch.Tensor, off: int, 
              _stream()), "gelu_row")
 
 
-def gemm_skinny_gelu_row(x: torch.Tensor, w: torch.Tensor, ids: torch.Tensor, table: torch.Tensor, off: int, dim: int, out: torch.Tensor) -> None:
+def gemm_skinny_gelu_row(x: torch.Tensor, w: torch.Tensor, ids: torch.Tensor, table: torch.Tensor, off: int, dim: int, out: torch.Tensor,
+                         w_static: bool = False) -> None:
     """out[m, n] = gelu_tanh(x @ w^T)[m, n] * table[ids[m], off + n] for n < dim (0 behind them): up to 16 bfloat16 rows, the
-    weight-streaming product with that in its epilogue."""
+    weight-streaming product with that in its epilogue. w_static: as for gemm_skinny."""
     _need_cuda(x, w, ids, table, out)
     M, K = x.shape
     N = w.shape[0]
@@ -225,9 +226,9 @@ def gemm_skinny_gelu_row(x: torch.Tensor, w: torch.Tensor, ids: torch.Tensor, ta
     if x.stride(1) != 1 or w.stride(1) != 1 or out.stride(1) != 1:
         raise KernelError("gemm_skinny_gelu_row: innermost dimension must be contiguous")
     f = _fn("gemm_skinny", "il_gemm_skinny_gelu_row", [_c_void_p, _c_int, _c_void_p, _c_int, _c_void_p, _c_int, _c_int, _c_int, _c_int, _c_void_p,
-                                                       _c_void_p, _c_int, _c_int, _c_int, _c_int, _c_void_p])
+                                                       _c_void_p, _c_int, _c_int, _c_int, _c_int, _c_int, _c_void_p])
     _check(f(_ptr(x), x.stride(0), _ptr(w), w.stride(0), _ptr(out), out.stride(0), M, N, K, _ptr(ids), _ptr(table), table.stride(0), off, dim,
-             table.shape[0], _stream()), "gemm_skinny_gelu_row")
+             table.shape[0], int(w_static), _stream()), "gemm_skinny_gelu_row")
 
 
 def add_bias(y: torch.Tensor, bias: torch.Tensor) -> None:
@@ -849,11 +850,13 @@ def _norm_args(norm_in: Optional[NormedInput], M: int):
 
 
 def gemm_skinny(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, alpha: float = 1.0,
-                bias: Optional[torch.Tensor] = None, glu: int = 0, norm_in: Optional[NormedInput] = None, act_params=None) -> None:
+                bias: Optional[torch.Tensor] = None, glu: int = 0, norm_in: Optional[NormedInput] = None, act_params=None,
+                w_static: bool = False) -> None:
     """out[M,N] = alpha * x[M,K] @ w[N,K]^T (+ bias) for M <= 16 bfloat16 rows; out bfloat16 or float32.
     glu (True, or ACT_SILU / ACT_GELU_TANH / ACT_CLAMPED with act_params): w is [2N,K] (gate rows, then up rows) and out[M,N] = act(gate) * up;
     ACT_RELU2: w is [N,K] and out is relu(.)^2 of the product (bfloat16).
-    norm_in: x is `norm_in.xw`, and the results are divided by the rms that its sums give."""
+    norm_in: x is `norm_in.xw`, and the results are divided by the rms that its sums give.
+    w_static: w is a model's weight, not what the kernel launched just before writes, and may be read while that kernel still runs."""
     _need_cuda(x, w, out, bias)
     M, K = x.shape
     N = w.shape[0] // 2 if glu and int(glu) != ACT_RELU2 else w.shape[0]
@@ -865,11 +868,11 @@ def gemm_skinny(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, alpha: floa
         raise KernelError("gemm_skinny: bias float32, one per weight row")
     f = _fn("gemm_skinny", "il_gemm_skinny", [_c_void_p, _c_int, _c_void_p, _c_int, _c_void_p, _c_int, _c_int, _c_void_p,
                                               _c_float, _c_int, _c_int, _c_int, _c_int, _c_void_p, _c_int, _c_int, _c_float,
-                                              _c_float, _c_float, _c_void_p])
+                                              _c_float, _c_float, _c_int, _c_void_p])
     limit, act_alpha = _act_args(glu, act_params)
     np_, nb, nw, ne = _norm_args(norm_in, M)
     _check(f(_ptr(x), x.stride(0), _ptr(w), w.stride(0), _ptr(out), kind_of(out.dtype), out.stride(0), _ptr(bias), alpha,
-             M, N, K, int(glu), np_, nb, nw, ne, limit, act_alpha, _stream()), "gemm_skinny")
+             M, N, K, int(glu), np_, nb, nw, ne, limit, act_alpha, int(w_static), _stream()), "gemm_skinny")
 
 
 def skinny_resid_ok(M: int, K: int, width: int) -> bool:
@@ -879,10 +882,11 @@ def skinny_resid_ok(M: int, K: int, width: int) -> bool:
 
 def gemm_skinny_resid(x: torch.Tensor, w: torch.Tensor, alpha: float, bias: Optional[torch.Tensor], resid: torch.Tensor,
                       branch_scale: float, norm_weight: torch.Tensor, eps: float, xw: torch.Tensor,
-                      sumsq: torch.Tensor) -> NormedInput:
+                      sumsq: torch.Tensor, w_static: bool = False) -> NormedInput:
     """The last product of a branch (up to 16 bfloat16 rows) with the residual add and the next RMSNorm's inputs in its
     epilogue: resid (float32 [M,H], in place) += branch_scale * bf16(alpha * x @ w^T + bias); xw = resid * norm_weight;
-    sumsq[m][b] = sum of resid[m]^2 over columns 16b..16b+15. Returns what the next product needs to finish the norm."""
+    sumsq[m][b] = sum of resid[m]^2 over columns 16b..16b+15. Returns what the next product needs to finish the norm.
+    w_static: as for gemm_skinny."""
     _need_cuda(x, w, bias, resid, norm_weight, xw, sumsq)
     M, K = x.shape
     H = w.shape[0]
@@ -899,9 +903,9 @@ def gemm_skinny_resid(x: torch.Tensor, w: torch.Tensor, alpha: float, bias: Opti
         raise KernelError("gemm_skinny_resid: bias float32 [H]")
     _contig("resid", resid), _contig("xw", xw), _contig("sumsq", sumsq), _contig("norm_weight", norm_weight)
     f = _fn("gemm_skinny", "il_gemm_skinny_resid", [_c_void_p, _c_int, _c_void_p, _c_int, _c_void_p, _c_float, _c_int, _c_int, _c_int,
-                                                    _c_void_p, _c_float, _c_void_p, _c_int, _c_void_p, _c_void_p, _c_void_p])
+                                                    _c_void_p, _c_float, _c_void_p, _c_int, _c_void_p, _c_void_p, _c_int, _c_void_p])
     _check(f(_ptr(x), x.stride(0), _ptr(w), w.stride(0), _ptr(bias), alpha, M, H, K, _ptr(resid), branch_scale, _ptr(norm_weight),
-             kind_of(norm_weight.dtype), _ptr(xw), _ptr(sumsq), _stream()), "gemm_skinny_resid")
+             kind_of(norm_weight.dtype), _ptr(xw), _ptr(sumsq), int(w_static), _stream()), "gemm_skinny_resid")
     return NormedInput(xw, sumsq, H, eps)
 
 
@@ -913,9 +917,11 @@ def skinny_rope_ok(M: int, K: int, head_dim: int, rot_dim: int) -> bool:
 def gemm_skinny_rope(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, alpha: float, bias: Optional[torch.Tensor],
                      tok_pos: torch.Tensor, tok_entry: torch.Tensor, block_table: torch.Tensor, cache: Optional[torch.Tensor],
                      page_size: int, n_heads: int, n_kv_heads: int, head_dim: int, rot_dim: int,
-                     inv_freq: Optional[torch.Tensor], mscale: float, norm_in: Optional[NormedInput] = None) -> None:
+                     inv_freq: Optional[torch.Tensor], mscale: float, norm_in: Optional[NormedInput] = None,
+                     w_static: bool = False) -> None:
     """The q/k/v projection of up to 16 bfloat16 rows with what `rope_store` does in its epilogue: out[M, (heads + 2
-    kv_heads) * head_dim] = alpha * x @ w^T (+ bias), q and k rotated, k and v written to their cache slots (if `cache`)."""
+    kv_heads) * head_dim] = alpha * x @ w^T (+ bias), q and k rotated, k and v written to their cache slots (if `cache`).
+    w_static: as for gemm_skinny."""
     _need_cuda(x, w, out, bias, tok_pos, tok_entry, block_table, cache, inv_freq)
     M, K = x.shape
     N = (n_heads + 2 * n_kv_heads) * head_dim
@@ -937,11 +943,11 @@ def gemm_skinny_rope(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, alpha:
     f = _fn("gemm_skinny", "il_gemm_skinny_rope",
             [_c_void_p, _c_int, _c_void_p, _c_int, _c_void_p, _c_int, _c_void_p, _c_float, _c_int, _c_int, _c_void_p, _c_void_p,
              _c_void_p, _c_int, _c_void_p, _c_int, _c_int, _c_int, _c_int, _c_int, _c_void_p, _c_float, _c_void_p, _c_int, _c_int,
-             _c_float, _c_void_p])
+             _c_float, _c_int, _c_void_p])
     np_, nb, nw, ne = _norm_args(norm_in, M)
     _check(f(_ptr(x), x.stride(0), _ptr(w), w.stride(0), _ptr(out), out.stride(0), _ptr(bias), alpha, M, K, _ptr(tok_pos),
              _ptr(tok_entry), _ptr(block_table), block_table.shape[1], _ptr(cache), page_size, n_heads, n_kv_heads, head_dim,
-             rot_dim, _ptr(inv_freq), mscale, np_, nb, nw, ne, _stream()), "gemm_skinny_rope")
+             rot_dim, _ptr(inv_freq), mscale, np_, nb, nw, ne, int(w_static), _stream()), "gemm_skinny_rope")
 
 
 def skinny_ok(M: int, K: int) -> bool:

@@ -43,6 +43,9 @@ class PagedAttend:
     FAST_MAX_GROUP = 64
     _warned_plain = False
 
+    # Up to here one split, which writes the output itself: more would save each warp a few pages, but cost the merge's launch
+    # (0.5B sizes, one request of 64 cached tokens: 3.6 us a layer in one split, 3.6 + 2.3 in four with their merge).
+    ONE_SPLIT_PAGES = 16
     WAVE_FILL = 2.0 / 3.0                         # share of the blocks the device holds at once that the splits aim at
 
     def __init__(self, dtype, n_heads: int, n_kv_heads: int, head_dim: int, scale: float, window: Optional[int] = None,
@@ -69,7 +72,10 @@ class PagedAttend:
     def decode_splits(self, base: int, max_pages: int, resident: int) -> int:
         """Splits of the keys for `base` blocks per split: as many as fill the wanted share of one wave of blocks
         (`resident`: what the device runs at once, from the occupancy query), never more - a second, part-filled wave
-        costs more in partials than it gains - and at least four pages a split."""
+        costs more in partials than it gains - and at least four pages a split.
+        A few pages are one split: its block writes the output itself."""
+        if max_pages <= self.ONE_SPLIT_PAGES:
+            return 1
         target = max(1, int(resident * self.WAVE_FILL))
         return max(1, min(target // base, (max_pages + 3) // 4, 128))
 
@@ -195,7 +201,7 @@ class Attention(Mixer):
             normed = isinstance(x, ops.NormedInput)
             ops.gemm_skinny_rope(x.xw if normed else x, self.qkv.weight, qkv, self.qkv.alpha, self.qkv.bias, ctx.tok_pos,
                                  ctx.tok_entry, cache.block_table, store, cache.page_size, self.nh, self.nkv, self.hd,
-                                 pos.rot_dim, pos.inv_freq, pos.mscale, norm_in=x if normed else None)
+                                 pos.rot_dim, pos.inv_freq, pos.mscale, norm_in=x if normed else None, w_static=True)
         else:
             self.qkv(x, qkv)
             if pos.has_transform:                 # an encoding that is no rotary table changes q and k itself
@@ -207,7 +213,7 @@ class Attention(Mixer):
         if tail is not None:                      # o_proj adds into the residual and prepares the next norm itself
             return ops.gemm_skinny_resid(out, self.o_proj.weight, self.o_proj.alpha, self.o_proj.bias, tail.resid, tail.scale,
                                          tail.norm.weight, tail.norm.eps, ctx.ws.rows("xw_mixer", T, self.hidden, self.dtype),
-                                         ctx.ws.rows("sumsq_mixer", T, (self.hidden + 15) // 16, torch.float32))
+                                         ctx.ws.rows("sumsq_mixer", T, (self.hidden + 15) // 16, torch.float32), w_static=True)
         return self.o_proj(out, ctx.ws.rows("branch", T, self.hidden, self.dtype))
 
     def attend(self, qkv, out, ctx, cache) -> None:

@@ -105,7 +105,7 @@ class ConvGatedAttention(Mixer):
         T, hd = x.shape[0], self.hd
         proj = ctx.ws.rows("cga_proj", T, self.n_proj_pad, self.dtype)
         if isinstance(x, ops.NormedInput):
-            ops.gemm_skinny(x.xw, self.proj.weight, proj, 1.0, self.proj.bias, norm_in=x)
+            ops.gemm_skinny(x.xw, self.proj.weight, proj, 1.0, self.proj.bias, norm_in=x, w_static=True)
         else:
             self.proj(x, proj)
         qkv = ctx.ws.rows("cga_qkv", T, (self.nh + 2 * self.nkv) * hd, self.dtype)
@@ -126,7 +126,7 @@ class ConvGatedAttention(Mixer):
         if tail is not None:
             return ops.gemm_skinny_resid(att, self.o_proj.weight, self.o_proj.alpha, self.o_proj.bias, tail.resid, tail.scale,
                                          tail.norm.weight, tail.norm.eps, ctx.ws.rows("xw_mixer", T, self.hidden, self.dtype),
-                                         ctx.ws.rows("sumsq_mixer", T, (self.hidden + 15) // 16, torch.float32))
+                                         ctx.ws.rows("sumsq_mixer", T, (self.hidden + 15) // 16, torch.float32), w_static=True)
         return self.o_proj(att, ctx.ws.rows("cga_branch", T, self.hidden, self.dtype))
 
 

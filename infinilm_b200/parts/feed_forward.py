@@ -68,14 +68,14 @@ class SwiGLU(FeedForward):
             # decode: gate and up rows streamed together, SiLU(gate)*up in the epilogue
             act = ctx.ws.rows("ffn_act", T, self.inter, self.dtype)
             if isinstance(x, ops.NormedInput):
-                ops.gemm_skinny(x.xw, self.gate_up.weight, act, 1.0, self.gate_up.bias, glu=self.act, norm_in=x, act_params=self.act_params)
+                ops.gemm_skinny(x.xw, self.gate_up.weight, act, 1.0, self.gate_up.bias, glu=self.act, norm_in=x, act_params=self.act_params, w_static=True)
             else:
-                ops.gemm_skinny(x, self.gate_up.weight, act, 1.0, self.gate_up.bias, glu=self.act, act_params=self.act_params)
+                ops.gemm_skinny(x, self.gate_up.weight, act, 1.0, self.gate_up.bias, glu=self.act, act_params=self.act_params, w_static=True)
             if tail is not None:                  # down adds into the residual and prepares the next norm itself
                 return ops.gemm_skinny_resid(act, self.down.weight, self.down.alpha, self.down.bias, tail.resid, tail.scale,
                                              tail.norm.weight, tail.norm.eps,
                                              ctx.ws.rows("xw_ffn", T, self.hidden, self.dtype),
-                                             ctx.ws.rows("sumsq_ffn", T, (self.hidden + 15) // 16, torch.float32))
+                                             ctx.ws.rows("sumsq_ffn", T, (self.hidden + 15) // 16, torch.float32), w_static=True)
             return self.down(act, ctx.ws.rows("ffn_branch", T, self.hidden, self.dtype))
         act = ctx.ws.rows("ffn_act", T, self.inter, self.dtype)
         if self.dtype == torch.bfloat16 and ops.mid_ok(T, self.hidden):
@@ -119,7 +119,7 @@ class SquaredReLU(FeedForward):
         act = ctx.ws.rows("ffn_act", T, self.inter, self.dtype)
         if self.dtype == torch.bfloat16 and ops.skinny_ok(T, self.hidden):      # the activation in the product's epilogue
             normed = isinstance(x, ops.NormedInput)
-            ops.gemm_skinny(x.xw if normed else x, self.up.weight, act, glu=ops.ACT_RELU2, norm_in=x if normed else None)
+            ops.gemm_skinny(x.xw if normed else x, self.up.weight, act, glu=ops.ACT_RELU2, norm_in=x if normed else None, w_static=True)
         elif self.dtype == torch.bfloat16 and ops.mid_ok(T, self.hidden):
             ops.gemm_mid(x, self.up.weight, act, glu=ops.ACT_RELU2)
         else:
@@ -128,7 +128,7 @@ class SquaredReLU(FeedForward):
         if tail is not None:                      # down adds into the residual and prepares the next norm itself
             return ops.gemm_skinny_resid(act, self.down.weight, self.down.alpha, self.down.bias, tail.resid, tail.scale,
                                          tail.norm.weight, tail.norm.eps, ctx.ws.rows("xw_ffn", T, self.hidden, self.dtype),
-                                         ctx.ws.rows("sumsq_ffn", T, (self.hidden + 15) // 16, torch.float32))
+                                         ctx.ws.rows("sumsq_ffn", T, (self.hidden + 15) // 16, torch.float32), w_static=True)
         return self.down(act, ctx.ws.rows("ffn_branch", T, self.hidden, self.dtype))
 
 

@@ -131,7 +131,7 @@ class LatentAttention(Mixer):
         ws, dt = ctx.ws, self.dtype
         if isinstance(x, ops.NormedInput):       # rows whose norm the branch before left unfinished: this product divides by the rms
             proj = ws.rows("lat_down", T, self.n_down, dt)
-            ops.gemm_skinny(x.xw, self.down.weight, proj, self.down.alpha, self.down.bias, norm_in=x)
+            ops.gemm_skinny(x.xw, self.down.weight, proj, self.down.alpha, self.down.bias, norm_in=x, w_static=True)
         else:
             proj = self.down(x, ws.rows("lat_down", T, self.n_down, dt))
         cq = None if self.direct_q else ws.rows("lat_cq", T, self.qr, dt)
@@ -170,7 +170,7 @@ class LatentAttention(Mixer):
         if tail is not None:                      # the output product adds into the residual and prepares the next norm itself
             return ops.gemm_skinny_resid(o, self.out.weight, self.out.alpha, self.out.bias, tail.resid, tail.scale, tail.norm.weight,
                                          tail.norm.eps, ws.rows("xw_mixer", T, self.hidden, dt),
-                                         ws.rows("sumsq_mixer", T, (self.hidden + 15) // 16, torch.float32))
+                                         ws.rows("sumsq_mixer", T, (self.hidden + 15) // 16, torch.float32), w_static=True)
         return self.out(o, ws.rows("branch", T, self.hidden, dt))
 
 

@@ -46,7 +46,7 @@ class Linear:
             return out
         if ops.skinny_ok(x.shape[0], self.in_features):
             # a few rows (decode): the weight-streaming kernel of this package
-            ops.gemm_skinny(x, self.weight, out, self.alpha, self.bias)
+            ops.gemm_skinny(x, self.weight, out, self.alpha, self.bias, w_static=True)
             return out
         if self.use_tc5 and x.shape[0] <= self.MID_ROWS and ops.mid_ok(x.shape[0], self.in_features):
             # 17..64 rows: tiles of weight rows by blocks of activation rows over all of K, nothing cut along K

@@ -47,7 +47,7 @@ class _FusableEnds:
 
     def _project(self, x, out):
         if isinstance(x, ops.NormedInput):
-            ops.gemm_skinny(x.xw, self.proj.weight, out, 1.0, None, norm_in=x)
+            ops.gemm_skinny(x.xw, self.proj.weight, out, 1.0, None, norm_in=x, w_static=True)
             return out
         return self.proj(x, out, out_f32=True)
 
@@ -56,7 +56,7 @@ class _FusableEnds:
         if tail is not None:
             return ops.gemm_skinny_resid(gated, self.o_proj.weight, self.o_proj.alpha, None, tail.resid, tail.scale, tail.norm.weight,
                                          tail.norm.eps, ctx.ws.rows("xw_mixer", T, self.hidden, self.dtype),
-                                         ctx.ws.rows("sumsq_mixer", T, (self.hidden + 15) // 16, torch.float32))
+                                         ctx.ws.rows("sumsq_mixer", T, (self.hidden + 15) // 16, torch.float32), w_static=True)
         return self.o_proj(gated, ctx.ws.rows(tag, T, self.hidden, self.dtype))
 
 

@@ -47,7 +47,7 @@ class TokenInput(Part):
         T = x.shape[0]
         g = ctx.ws.rows("token_gated", T, self.dim_pad, self.dtype)
         if self.dtype == torch.bfloat16 and ops.skinny_ok(T, self.hidden):
-            ops.gemm_skinny_gelu_row(x, self.gate.weight, ctx.token_ids, table, self.offset, self.dim, g)
+            ops.gemm_skinny_gelu_row(x, self.gate.weight, ctx.token_ids, table, self.offset, self.dim, g, w_static=True)
         else:
             z = self.gate(x, ctx.ws.rows("token_gate", T, self.dim_pad, torch.float32), out_f32=True)
             ops.gelu_row(z, ctx.token_ids, table, self.offset, self.dim, g)

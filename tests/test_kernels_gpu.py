@@ -575,6 +575,28 @@ def test_gemm_skinny(cuda_device, M, N, K, out_dtype):
     assert torch.equal(out1[0], out[M - 1])
 
 
+@pytest.mark.parametrize("M", [1, 8, 9, 16])
+@pytest.mark.parametrize("N,K", [(23, 8), (160, 1016), (2400, 1024), (40, 1032), (2368, 2048), (33, 2056), (2384, 2056), (64, 8200)])
+def test_gemm_skinny_weights_before_the_wait(cuda_device, M, N, K):
+    """K at the edges of one round of loads (1,024 and 2,048) and beyond, for the plain product and the one that adds into the
+    residual (148 and 149 blocks: 16 warps a block or 8); weights declared static give the same bits."""
+    g = torch.Generator(device="cuda").manual_seed(M + K)
+    x = torch.randn(M, K, device="cuda", generator=g).bfloat16()
+    w = (torch.randn(N, K, device="cuda", generator=g) / math.sqrt(K)).bfloat16()
+    resid, nw = torch.randn(M, N, device="cuda", generator=g), torch.ones(N, device="cuda")
+    ref = x.double() @ w.double().t()
+    outs = []
+    for static in (False, True):
+        out = torch.full((M, N), float("nan"), device="cuda")
+        ops.gemm_skinny(x, w, out, w_static=static)
+        r, xw, sq = resid.clone(), torch.empty(M, N, device="cuda", dtype=torch.bfloat16), torch.empty(M, (N + 15) // 16, device="cuda")
+        ops.gemm_skinny_resid(x, w, 1.0, None, r, 0.5, nw, 1e-5, xw, sq, w_static=static)
+        outs.append((out, r, xw, sq))
+    close(outs[0][0], ref.float(), "float32")
+    close(outs[0][1], (resid.double() + 0.5 * ref).float(), "bfloat16", scale=ref.abs().max().float())      # the branch is rounded to bfloat16
+    assert all(torch.equal(a, b) for a, b in zip(*outs))
+
+
 @pytest.mark.parametrize("M,I,K", [(1, 160, 64), (8, 264, 200), (13, 320, 192), (4, 16384, 4096)])
 def test_gemm_skinny_swiglu(cuda_device, M, I, K):
     g = torch.Generator(device="cuda").manual_seed(10)
