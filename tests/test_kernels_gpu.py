@@ -593,7 +593,7 @@ def test_gemm_skinny_weights_before_the_wait(cuda_device, M, N, K):
         ops.gemm_skinny_resid(x, w, 1.0, None, r, 0.5, nw, 1e-5, xw, sq, w_static=static)
         outs.append((out, r, xw, sq))
     close(outs[0][0], ref.float(), "float32")
-    close(outs[0][1], (resid.double() + 0.5 * ref).float(), "bfloat16", scale=ref.abs().max().float())      # the branch is rounded to bfloat16
+    close(outs[0][1], (resid.double() + 0.5 * ref).float(), "bfloat16", scale=ref.abs().max().float().cpu())      # the branch is rounded to bfloat16
     assert all(torch.equal(a, b) for a, b in zip(*outs))
 
 
