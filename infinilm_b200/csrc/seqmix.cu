@@ -388,16 +388,17 @@ __global__ void __launch_bounds__(SR_THREADS) matrix_state_scan_reg_kernel(
     const int part = tid & (split - 1), col_l = tid >> log_split, c = blockIdx.z * cpb + col_l;
     // Which tokens this block walks. Plain form (seg_len 0): entry e0 + blockIdx.x, all of it. Segmented form (the decayed
     // sum of long portions): blockIdx.x counts segments of seg_len tokens, entry after entry; segment p of an entry starts
-    // from nothing (p > 0) and leaves what it gathered in seg_state, and a second pass (MODE 2) adds what the state at the
-    // segment's start contributes: S is linear in its start, o_t += decay^(t - t0 + 1) S_start^T q_t.
-    int e = e0 + blockIdx.x, q0, n, p = 0, n_seg = 1, first_tile = 0;
+    // from nothing (p > 0) and leaves what it gathered in seg_state, decay_prefix_kernel turns these into the states at the
+    // segments' ends, and a second pass (MODE 2) adds what the state at the segment's start contributes: S is linear in its
+    // start, o_t += decay^(t - t0 + 1) S_start^T q_t. (Key sizes of 33 to 128 run both passes as decay_segment_kernel.)
+    int e = e0 + blockIdx.x, q0, n, p = 0, n_seg = 1;
     if (seg_len > 0) {
         int tile = blockIdx.x;
         for (e = e0;; ++e) {
             if (e >= e0 + n_ent) return;          // a surplus block (the grid is a bound)
             const int a = qstart[e], cnt = (qstart[e + 1] - a + seg_len - 1) / seg_len;
             if (tile < cnt) {
-                p = tile, n_seg = cnt, first_tile = blockIdx.x - tile;
+                p = tile, n_seg = cnt;
                 break;
             }
             tile -= cnt;
@@ -442,23 +443,7 @@ __global__ void __launch_bounds__(SR_THREADS) matrix_state_scan_reg_kernel(
     };
     const size_t head_f = (size_t)dim * vdim;     // floats of one head's state
     if (MODE == 2) {
-        // the state at this segment's start: what the segments before it gathered, each decayed over those behind it
-        const float dseg = powf(dec, (float)seg_len);
-        load_cols(seg_state + ((size_t)first_tile * H + h) * head_f, S);
-        for (int j = 1; j < p; ++j) {
-            float L[DPT];
-            load_cols(seg_state + ((size_t)(first_tile + j) * H + h) * head_f, L);
-#pragma unroll
-            for (int i = 0; i < DPT; ++i) S[i] = fmaf(dseg, S[i], L[i]);
-        }
-        if (p == n_seg - 1) {                     // the last segment also leaves the request's state: its start decayed over it, plus its own
-            float L[DPT];
-            load_cols(seg_state + ((size_t)(first_tile + p) * H + h) * head_f, L);
-            const float dn = powf(dec, (float)n);
-#pragma unroll
-            for (int i = 0; i < DPT; ++i) L[i] = fmaf(dn, S[i], L[i]);
-            store_cols(state + (size_t)write_slots[e] * slot_stride + (size_t)h * head_f, L);
-        }
+        load_cols(seg_state + ((size_t)(blockIdx.x - 1) * H + h) * head_f, S);       // where the segment before ended (decay_prefix_kernel)
     } else if (p == 0) {
         load_cols(state + (size_t)read_slots[e] * slot_stride + (size_t)h * head_f, S);
     } else {
@@ -662,6 +647,239 @@ static void sr_launch(dim3 grid, size_t smem, cudaStream_t stream, const float* 
                                                                                     ldo, log_split, e0, n_ent, seg_len, seg_state, ld_g);
 }
 
+// ---- the decayed sum of long portions: segments ------------------------------------------------------------------------------
+// Which segment of which entry block `tile` of a bound on their number walks; false: none.
+struct DsSegment { int e, p, n_seg, q0, n; };
+__device__ __forceinline__ bool ds_find(int tile, int e0, int n_ent, int seg_len, const int* __restrict__ qstart, DsSegment& s) {
+    for (int e = e0; e < e0 + n_ent; ++e) {
+        const int a = qstart[e], len = qstart[e + 1] - a, cnt = (len + seg_len - 1) / seg_len;
+        if (tile < cnt) {
+            s = DsSegment{e, tile, cnt, a + tile * seg_len, min(seg_len, len - tile * seg_len)};
+            return true;
+        }
+        tile -= cnt;
+    }
+    return false;
+}
+
+// seg_state, segment by segment what each gathered from nothing (the first: from the request's state), becomes the state at each
+// segment's end: E_0 = L_0, E_j = decay^seg_len E_(j-1) + L_j; the last one, decayed over its own length, is the request's state.
+// A thread per element of a head's state, eight segments asked for at a time. (Each block of the second pass used to add up all the
+// segments before its own: 390 MB of reads a layer for two portions of 2,100 and 2,900 tokens, where this pass moves 80.)
+__global__ void decay_prefix_kernel(const float* __restrict__ decay, float* state, size_t slot_stride, const int* __restrict__ write_slots,
+                                    const int* __restrict__ qstart, int H, int head_f, int e0, int seg_len, float* seg_state) {
+    const int e = e0 + blockIdx.z, h = blockIdx.y, i = blockIdx.x * blockDim.x + threadIdx.x;
+    int first = 0;
+    for (int f = e0; f < e; ++f) first += (qstart[f + 1] - qstart[f] + seg_len - 1) / seg_len;
+    const int len = qstart[e + 1] - qstart[e], n_seg = (len + seg_len - 1) / seg_len;
+    if (n_seg < 2 || i >= head_f) return;         // (one segment: the first pass left the request's state itself)
+    const float dec = decay[h], dseg = powf(dec, (float)seg_len), dlast = powf(dec, (float)(len - (n_seg - 1) * seg_len));
+    float* p = seg_state + ((size_t)first * H + h) * head_f + i;
+    const size_t step = (size_t)H * head_f;
+    float S = p[0];
+    for (int j0 = 1; j0 < n_seg; j0 += 8) {
+        float L[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) L[j] = j0 + j < n_seg ? p[(j0 + j) * step] : 0.f;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            if (j0 + j < n_seg - 1) {
+                S = fmaf(dseg, S, L[j]);
+                p[(j0 + j) * step] = S;
+            } else if (j0 + j == n_seg - 1) {
+                state[(size_t)write_slots[e] * slot_stride + (size_t)h * head_f + i] = fmaf(dlast, S, L[j]);
+            }
+        }
+    }
+}
+
+// Both passes for key sizes of 33 to 128. What bounds the register form above is shared memory: 8 loads of 16 bytes of q and k for
+// 48 multiply-adds of a lane's 16 rows of one column. Here a lane holds 16 rows of FOUR columns, so each load serves four times
+// the arithmetic, which runs two rows an instruction (packed f32); a head is two blocks instead of eight, so the inputs'
+// activation fits into the staging (no pass of its own); and the outputs of 8 tokens are summed over the lanes of a column by
+// halving (28 shuffles for 32 outputs) and leave as 16 bytes a lane. SECOND: o_t += decay^(t - t0 + 1) S_start^T q_t.
+// Measured at 16 heads of 128 x 128, portions of 2,100 and 2,900 tokens, a layer: 110 + 11 (prefix) + 57 us; the register form took
+// 279 + 142 us, and the activation's own pass 45. The arithmetic alone is about 130 us at the FP32 pipes' rate.
+constexpr int DS_COLS = 4, DS_CHUNK = 8, DS_ROWS = 16, DS_SEG = DS_ROWS + 4;
+template <int LOG_SPLIT, bool SECOND>
+__global__ void __launch_bounds__(SR_THREADS) decay_segment_kernel(const float* __restrict__ q, const float* __restrict__ k, const float* __restrict__ v,
+                                                                   int ld_q, int ld_k, int ld_v, int H, int G, int dim, int vdim, int in_act,
+                                                                   const float* __restrict__ decay, float* state, size_t slot_stride,
+                                                                   const int* __restrict__ read_slots, const int* __restrict__ write_slots,
+                                                                   const int* __restrict__ qstart, float* out, int ldo, int e0, int n_ent,
+                                                                   int seg_len, float* seg_state) {
+    constexpr int SPLIT = 1 << LOG_SPLIT, CPB = (SR_THREADS / SPLIT) * DS_COLS, ROW_F = DS_SEG * SPLIT, TPT = SR_THREADS / DS_CHUNK;
+    constexpr int NQ = SPLIT, NV = CPB / TPT, TOK = DS_CHUNK / SPLIT;     // staged values a thread; tokens a lane holds in the end
+    static_assert(TPT == DS_ROWS, "a staging thread's entries fall into one lane segment each");
+    __shared__ __align__(16) float qs[DS_CHUNK * ROW_F], ks[SECOND ? 4 : DS_CHUNK * ROW_F], vs[SECOND ? 4 : DS_CHUNK * CPB];
+    const int h = blockIdx.y, tid = threadIdx.x, part = tid & (SPLIT - 1), cg = tid >> LOG_SPLIT;
+    const int cb = blockIdx.z * CPB, c0 = cb + cg * DS_COLS, d0 = part * DS_ROWS;
+    DsSegment sg;
+    if (!ds_find(blockIdx.x, e0, n_ent, seg_len, qstart, sg)) return;      // a surplus block (the grid is a bound)
+    if (SECOND && sg.p == 0) return;              // the first segment started from the request's own state: nothing to add
+    const int hq = h / (H / G), n = sg.n, q0 = sg.q0;
+    const float dec = decay[h];
+    const il_f2 dec2 = il_f2_dup(dec);
+    const size_t head_f = (size_t)dim * vdim;
+    il_f2 S[DS_COLS][DS_ROWS / 2];
+    const float* src = SECOND ? seg_state + ((size_t)(blockIdx.x - 1) * H + h) * head_f
+                              : sg.p == 0 ? state + (size_t)read_slots[sg.e] * slot_stride + (size_t)h * head_f : nullptr;
+    const bool rows4 = (dim & 3) == 0;            // a column's rows lie together: 16 bytes a load where that keeps them aligned
+#pragma unroll
+    for (int c = 0; c < DS_COLS; ++c)
+#pragma unroll
+        for (int i = 0; i < DS_ROWS; i += 4) {
+            float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (src && c0 + c < vdim) {
+                const float* at = src + (size_t)(c0 + c) * dim + d0 + i;
+                if (rows4) {
+                    if (d0 + i < dim) x = *reinterpret_cast<const float4*>(at);
+                } else {
+                    x = make_float4(d0 + i < dim ? at[0] : 0.f, d0 + i + 1 < dim ? at[1] : 0.f, d0 + i + 2 < dim ? at[2] : 0.f,
+                                    d0 + i + 3 < dim ? at[3] : 0.f);
+                }
+            }
+            S[c][i / 2] = il_f2_make(x.x, x.y), S[c][i / 2 + 1] = il_f2_make(x.z, x.w);
+        }
+    const int s_tt = tid / TPT, s_l = tid % TPT;
+    float qr[NQ], kr[NQ], vr[NV];
+    auto fetch = [&](int t0) {
+        const bool tok = t0 + s_tt < n;
+        const size_t row = (size_t)(q0 + t0 + s_tt);
+#pragma unroll
+        for (int j = 0; j < NQ; ++j) {
+            const int d = s_l + j * TPT;
+            const bool ok = tok && d < dim;
+            qr[j] = ok ? q[row * ld_q + hq * dim + d] : 0.f;
+            if (!SECOND) kr[j] = ok ? k[row * ld_k + hq * dim + d] : 0.f;
+        }
+        if (!SECOND)
+#pragma unroll
+            for (int j = 0; j < NV; ++j) vr[j] = tok && cb + s_l + j * TPT < vdim ? v[row * ld_v + h * vdim + cb + s_l + j * TPT] : 0.f;
+    };
+    auto stage = [&]() {
+#pragma unroll
+        for (int j = 0; j < NQ; ++j) {
+            qs[s_tt * ROW_F + j * DS_SEG + s_l] = in_act ? sm_silu_fast(qr[j]) : qr[j];
+            if (!SECOND) ks[s_tt * ROW_F + j * DS_SEG + s_l] = in_act ? sm_silu_fast(kr[j]) : kr[j];
+        }
+        if (!SECOND)
+#pragma unroll
+            for (int j = 0; j < NV; ++j) vs[s_tt * CPB + s_l + j * TPT] = in_act ? sm_silu_fast(vr[j]) : vr[j];
+    };
+    const bool out4 = (ldo & 3) == 0 && (vdim & 3) == 0 && !((uintptr_t)out & 15);
+    const int tok0 = LOG_SPLIT == 3 ? part : LOG_SPLIT == 2 ? part * 2 : part * 4;       // the tokens this lane ends up with
+    fetch(0);
+    stage();
+    __syncthreads();
+    for (int t0 = 0; t0 < n; t0 += DS_CHUNK) {
+        if (t0 + DS_CHUNK < n) fetch(t0 + DS_CHUNK);
+        float old[TOK][DS_COLS];
+        if (SECOND) {                             // what the first pass wrote, asked for before the products
+#pragma unroll
+            for (int j = 0; j < TOK; ++j) {
+                const float* at = out + (size_t)(q0 + t0 + tok0 + j) * ldo + h * vdim + c0;
+                const bool in = t0 + tok0 + j < n;
+#pragma unroll
+                for (int c = 0; c < DS_COLS; ++c) old[j][c] = in && c0 + c < vdim ? at[c] : 0.f;
+            }
+        }
+        float o[DS_CHUNK][DS_COLS];
+#pragma unroll
+        for (int tt = 0; tt < DS_CHUNK; ++tt) {
+            const ulonglong2* qq = reinterpret_cast<const ulonglong2*>(qs + tt * ROW_F + part * DS_SEG);
+            const ulonglong2* kk = reinterpret_cast<const ulonglong2*>(ks + (SECOND ? 0 : tt * ROW_F + part * DS_SEG));
+            il_f2 v2[DS_COLS], o2[DS_COLS];
+            if (!SECOND) {
+                const float4 x = *reinterpret_cast<const float4*>(vs + tt * CPB + cg * DS_COLS);
+                v2[0] = il_f2_dup(x.x), v2[1] = il_f2_dup(x.y), v2[2] = il_f2_dup(x.z), v2[3] = il_f2_dup(x.w);
+            }
+#pragma unroll
+            for (int c = 0; c < DS_COLS; ++c) o2[c] = 0ull;
+            if (t0 + tt < n) {                    // (a token beyond the segment's end moves nothing)
+#pragma unroll
+                for (int i = 0; i < DS_ROWS / 4; ++i) {
+                    const ulonglong2 q4 = qq[i];
+                    if (!SECOND) {
+                        const ulonglong2 k4 = kk[i];
+#pragma unroll
+                        for (int c = 0; c < DS_COLS; ++c) {
+                            S[c][2 * i] = il_f2_fma(dec2, S[c][2 * i], il_f2_mul(k4.x, v2[c]));
+                            S[c][2 * i + 1] = il_f2_fma(dec2, S[c][2 * i + 1], il_f2_mul(k4.y, v2[c]));
+                        }
+                    }
+#pragma unroll
+                    for (int c = 0; c < DS_COLS; ++c) o2[c] = il_f2_fma(S[c][2 * i], q4.x, o2[c]);
+#pragma unroll
+                    for (int c = 0; c < DS_COLS; ++c) o2[c] = il_f2_fma(S[c][2 * i + 1], q4.y, o2[c]);
+                }
+            }
+#pragma unroll
+            for (int c = 0; c < DS_COLS; ++c) {
+                float lo, hi;
+                il_f2_get(o2[c], lo, hi);
+                o[tt][c] = lo + hi;
+            }
+        }
+        // over the lanes of a column: each step a lane gives away one half of the tokens it still holds and adds up the other
+#pragma unroll
+        for (int st = LOG_SPLIT - 1, half = DS_CHUNK / 2; st >= 0; --st, half /= 2) {
+            const bool up = part & (1 << st);
+#pragma unroll
+            for (int j = 0; j < DS_CHUNK / 2; ++j)
+                if (j < half) {
+#pragma unroll
+                    for (int c = 0; c < DS_COLS; ++c) {
+                        const float got = __shfl_xor_sync(0xffffffffu, up ? o[j][c] : o[j + half][c], 1 << st);
+                        o[j][c] = (up ? o[j + half][c] : o[j][c]) + got;
+                    }
+                }
+        }
+#pragma unroll
+        for (int j = 0; j < TOK; ++j) {
+            const int t = t0 + tok0 + j;
+            if (t >= n) continue;
+            float* at = out + (size_t)(q0 + t) * ldo + h * vdim + c0;
+            if (SECOND) {                         // token i of the segment sees its start through i + 1 decays
+                const float pw = powf(dec, (float)(t + 1));
+#pragma unroll
+                for (int c = 0; c < DS_COLS; ++c) o[j][c] = fmaf(pw, o[j][c], old[j][c]);
+            }
+            if (out4 && c0 + DS_COLS <= vdim) {
+                *reinterpret_cast<float4*>(at) = make_float4(o[j][0], o[j][1], o[j][2], o[j][3]);
+            } else {
+#pragma unroll
+                for (int c = 0; c < DS_COLS; ++c)
+                    if (c0 + c < vdim) at[c] = o[j][c];
+            }
+        }
+        __syncthreads();                          // everyone has read this chunk
+        if (t0 + DS_CHUNK < n) stage();
+        __syncthreads();
+    }
+    if (SECOND) return;
+    float* dst = sg.n_seg == 1 ? state + (size_t)write_slots[sg.e] * slot_stride + (size_t)h * head_f : seg_state + ((size_t)blockIdx.x * H + h) * head_f;
+#pragma unroll
+    for (int c = 0; c < DS_COLS; ++c) {
+        if (c0 + c >= vdim) continue;
+        float* at = dst + (size_t)(c0 + c) * dim + d0;
+#pragma unroll
+        for (int i = 0; i < DS_ROWS; i += 4) {
+            float4 x;
+            il_f2_get(S[c][i / 2], x.x, x.y);
+            il_f2_get(S[c][i / 2 + 1], x.z, x.w);
+            if (rows4) {
+                if (d0 + i < dim) *reinterpret_cast<float4*>(at + i) = x;
+            } else {
+                if (d0 + i < dim) at[i] = x.x;
+                if (d0 + i + 1 < dim) at[i + 1] = x.y;
+                if (d0 + i + 2 < dim) at[i + 2] = x.z;
+                if (d0 + i + 3 < dim) at[i + 3] = x.w;
+            }
+        }
+    }
+}
+
 // In place: x[t, c] = silu(x[t, c]) for the first `cols` columns of float32 rows (the recurrences' inputs, as a pass of its own).
 __global__ void silu_cols_kernel(float* x, int ld, int cols, int T) {
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
@@ -689,11 +907,31 @@ IL_EXPORT int il_matrix_state_scan(int mode, const float* q, const float* k, con
     if (E <= 0) return IL_OK;
     if (e0 < 0) return IL_BAD_ARG;
     // seg_len > 0 (decayed sum, register form only): the entries' tokens in segments of seg_len, n_tiles of them at most
-    // (a bound is enough), seg_state float32 [n_tiles, H, vdim, dim] scratch; two passes.
+    // (a bound is enough), seg_state float32 [n_tiles, H, vdim, dim] scratch; three launches.
     if (seg_len > 0 && (mode != 0 || generic || single || dim > 256 || n_tiles <= 0 || !seg_state || seg_len % 8)) return IL_BAD_ARG;
     if (H <= 0 || G <= 0 || H % G || dim <= 0 || vdim <= 0 || (mode != 0 && mode != 1 && mode != 3 && mode != 4)) return IL_BAD_ARG;
     if (mode == 3 && (vdim < 2 || in_act)) return IL_BAD_ARG;
     if (mode == 4 ? (!decay || !gdec || G != H || in_act || ld_g < H * dim) : mode == 0 ? !decay : (!beta || !gdec)) return IL_BAD_ARG;
+    const auto prefix = [&]() {
+        const int head_f = dim * vdim;
+        decay_prefix_kernel<<<dim3((head_f + 255) / 256, H, E), 256, 0, stream>>>(decay, state, (size_t)slot_stride, write_slots, qstart, H, head_f, e0,
+                                                                                  seg_len, seg_state);
+    };
+    if (seg_len > 0 && dim > 32 && dim <= 128) {
+        // (16 rows of a column a lane: smaller keys would leave lanes idle, larger ones would need 16 lanes a column)
+#define DS_RUN(LS, SECOND)                                                                                                                     \
+        decay_segment_kernel<LS, SECOND><<<dim3(n_tiles, H, (vdim + (SR_THREADS >> LS) * DS_COLS - 1) / ((SR_THREADS >> LS) * DS_COLS)), SR_THREADS, 0, \
+                                           stream>>>(q, k, v, ld_q, ld_k, ld_v, H, G, dim, vdim, in_act, decay, state, (size_t)slot_stride, read_slots,  \
+                                                     write_slots, qstart, out, ldo, e0, E, seg_len, seg_state)
+        if (dim > 64) DS_RUN(3, false); else DS_RUN(2, false);
+        IL_LAUNCH_CHECK();
+        prefix();
+        IL_LAUNCH_CHECK();
+        if (dim > 64) DS_RUN(3, true); else DS_RUN(2, true);
+#undef DS_RUN
+        IL_LAUNCH_CHECK();
+        return IL_OK;
+    }
     if (dim <= 256 && !generic) {
         // Rows of a column per lane (8 or 16) and lanes per column (a power of two up to 16) that cover dim. Few blocks (one
         // long prompt) of the decayed sum take the narrower lanes: twice the warps, each with half the products per token
@@ -721,6 +959,8 @@ IL_EXPORT int il_matrix_state_scan(int mode, const float* q, const float* k, con
         if (mode == 0) {
             if (dpt == 8) SR_PICK(0, 8); else SR_PICK(0, 16);
             if (seg_len > 0) {                    // the second pass: what each segment's start contributes
+                IL_LAUNCH_CHECK();
+                prefix();
                 IL_LAUNCH_CHECK();
                 if (log_split <= 3) { if (dpt == 8) sr_launch<2, 8, 8, 8>(SR_ARGS); else sr_launch<2, 16, 8, 8>(SR_ARGS); }
                 else { if (dpt == 8) sr_launch<2, 8, 8, 16>(SR_ARGS); else sr_launch<2, 16, 8, 16>(SR_ARGS); }

@@ -1544,7 +1544,7 @@ def matrix_state_scan(mode: int, q: torch.Tensor, k: torch.Tensor, v: torch.Tens
     one that runs beyond a key size of 256) instead of the one that keeps it in registers. Entries first_entry ..
     first_entry + n_entries - 1 are run; `single`: each of them brings one token (the form made for decoding).
     seg_len > 0 (SCAN_DECAY, key sizes up to 256): every entry's tokens are walked in segments of seg_len at once, each from
-    nothing, and a second launch adds what the state at a segment's start contributes (the sum is linear in it);
+    nothing, and two more launches add what the state at a segment's start contributes (the sum is linear in it);
     `n_tiles` bounds the number of segments, `seg_state` is float32 scratch of n_tiles * heads * vdim * dim."""
     _need_cuda(q, k, v, decay, beta, gdec, state, read_slots, write_slots, entry_qstart, out)
     _i32("matrix_state_scan", read_slots, write_slots, entry_qstart)
@@ -1576,7 +1576,12 @@ def matrix_state_scan(mode: int, q: torch.Tensor, k: torch.Tensor, v: torch.Tens
              _ptr(entry_qstart), n_entries, _ptr(out), out.stride(0), int(generic), first_entry, int(single), seg_len, n_tiles,
              _ptr(seg_state), ld_g, _stream()), "matrix_state_scan")
     if seg_len > 0:
-        count_launches(1)                         # the second pass
+        count_launches(2)                         # the segments' ends and the second pass
+
+
+def scan_in_segments(ctx, mode: int, dim: int) -> bool:
+    """Whether `matrix_state_scan_step` walks this step's prompt portions in segments: by the step's shape alone."""
+    return mode == SCAN_DECAY and dim <= 256 and ctx.T - ctx.n_decode >= 2 * SCAN_SEGMENT
 
 
 def matrix_state_scan_step(ctx, *args, **kw) -> None:
@@ -1588,7 +1593,7 @@ def matrix_state_scan_step(ctx, *args, **kw) -> None:
         matrix_state_scan(*args, n_entries=n_dec, first_entry=0, single=True, **kw)
     if E > n_dec:
         mode, dim, vdim, n_heads = args[0], args[6], args[7], args[4]
-        if (mode == SCAN_DECAY and not kw.get("generic") and dim <= 256 and ctx.T - n_dec >= 2 * SCAN_SEGMENT):
+        if not kw.get("generic") and scan_in_segments(ctx, mode, dim):
             n_tiles = ctx.prompt_tiles(SCAN_SEGMENT)
             scratch = ctx.ws.flat("scan_segment_state", n_tiles * n_heads * vdim * dim, torch.float32)
             matrix_state_scan(*args, n_entries=E - n_dec, first_entry=n_dec, single=False, seg_len=SCAN_SEGMENT, n_tiles=n_tiles,

@@ -98,7 +98,9 @@ class DecayLinearAttention(_FusableEnds, Mixer):
         proj = self._project(x, ctx.ws.rows("dla_proj", T, 2 * nqk + 2 * nv, torch.float32))
         o = ctx.ws.rows("dla_o", T, nv, torch.float32)
         in_act = 1
-        if T > self.ACT_PASS_ROWS:                # many rows: the activation as a pass of its own (the same function), not in the token loop
+        # many rows: the activation as a pass of its own (the same function), not in the token loop of eight blocks a head; the kernel
+        # that walks segments is two blocks a head and applies it as it stages the inputs
+        if T > self.ACT_PASS_ROWS and not (32 < self.dk <= 128 and ops.scan_in_segments(ctx, ops.SCAN_DECAY, self.dk)):
             ops.silu_cols(proj, 2 * nqk + nv)
             in_act = 0
         ops.matrix_state_scan_step(ctx, ops.SCAN_DECAY, proj[:, :nqk], proj[:, nqk: 2 * nqk], proj[:, 2 * nqk: 2 * nqk + nv], self.nh, self.nh,

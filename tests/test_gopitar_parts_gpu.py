@@ -232,6 +232,34 @@ def test_decayed_sum_in_segments(cuda_device, H, d, dv):
     assert torch.equal(state[6], before[6]) and torch.equal(state[7], before[7])
 
 
+@pytest.mark.parametrize("H,d,dv", [(2, 33, 7), (1, 64, 130), (2, 50, 66), (3, 65, 5), (1, 100, 64), (2, 127, 129), (1, 128, 68)])
+def test_decayed_sum_in_segments_four_columns_a_lane(cuda_device, H, d, dv):
+    """The same at key sizes of 33 to 128, which run the kernel with four columns a lane: rows that fill no lane, columns that
+    fill no block, rows and outputs that are no whole 16-byte pieces."""
+    test_decayed_sum_in_segments(cuda_device, H, d, dv)
+
+
+def test_segments_apply_the_activation_as_they_stage(cuda_device):
+    """silu inside the kernel that walks segments against the pass of its own in front of it: the same numbers."""
+    from infinilm_b200 import ops
+    dev = cuda_device
+    torch.manual_seed(5)
+    H, d, dv, lens = 2, 64, 64, [150, 40]
+    T = sum(lens)
+    qkv = torch.randn(T, H * (2 * d + dv), device=dev)
+    qstart, _ = _step_arrays(lens, dev)
+    outs = []
+    for in_act in (0, 1):
+        x, state, out = qkv.clone(), torch.zeros(3, H, dv, d, device=dev), torch.empty(T, H * dv, device=dev)
+        if not in_act:
+            ops.silu_cols(x, x.shape[1])
+        ops.matrix_state_scan(ops.SCAN_DECAY, x[:, :H * d], x[:, H * d: 2 * H * d], x[:, 2 * H * d:], H, H, d, dv, in_act, torch.tensor([0.9, 0.99], device=dev), None,
+                              None, state, _i32([0, 0], dev), _i32([1, 2], dev), qstart, 2, out, seg_len=64, n_tiles=4,
+                              seg_state=torch.empty(4 * H * dv * d, device=dev))
+        outs.append((out, state))
+    assert torch.equal(outs[0][0], outs[1][0]) and torch.equal(outs[0][1], outs[1][1])
+
+
 @pytest.mark.parametrize("out_dtype", [torch.float32, torch.bfloat16])
 def test_group_norm_gate_head_gate_softcap_sum(cuda_device, out_dtype):
     from infinilm_b200 import ops
