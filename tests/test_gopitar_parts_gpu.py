@@ -196,6 +196,31 @@ def test_scan_of_a_batch_equals_each_alone(cuda_device, scan_kernel):
         a += n
 
 
+@pytest.mark.parametrize("last", [26, 27, 50])
+def test_short_conv_one_token_a_thread_and_eight(cuda_device, last):
+    """64 rows (one token a thread), 65 and 88 (eight): single tokens that move their state on beside portions, from held states."""
+    from infinilm_b200 import ops
+    dev = cuda_device
+    torch.manual_seed(last)
+    C, taps, lens = 130, 4, [1, 1, 1, 1, 1, 33, last]
+    E, T = len(lens), sum(lens)
+    x, w = torch.randn(T, C), torch.randn(C, taps)
+    state = torch.randn(E + 1, taps - 1, C, device=dev)
+    state[0] = 0
+    before = state.clone()
+    qstart, tok_entry = _step_arrays(lens, dev)
+    rd, wr = _i32([0] + list(range(2, E + 1)), dev), _i32(list(range(1, E + 1)), dev)
+    out = torch.empty(T, C, device=dev)
+    ops.short_conv(x.to(dev), 0, w.to(dev), state, 0, rd, tok_entry, qstart, out, 0, 1, C, C, 0, write_slots=wr)
+    a = 0
+    for e, n in enumerate(lens):
+        u = torch.cat([before[int(rd[e])].cpu(), x[a:a + n]]).double()
+        want = P.short_conv(u, w.double())[taps - 1:]
+        assert float((out[a:a + n].cpu().double() - want).abs().max()) <= 1e-5 * float(want.abs().max() + 1), (e, n)
+        assert torch.equal(state[int(wr[e])].cpu(), u[1:].float() if n == 1 else before[int(wr[e])].cpu()), e
+        a += n
+
+
 @pytest.mark.parametrize("H,d,dv", [(2, 32, 32), (3, 8, 40), (1, 128, 64), (2, 20, 12), (2, 10, 6), (1, 250, 9)])
 def test_decayed_sum_in_segments(cuda_device, H, d, dv):
     """Long portions walked in segments that run at once, with the second pass that adds each segment's start: several
