@@ -30,6 +30,7 @@ __global__ void attn_tile_kernel(const TA* qkv, int row_stride, TA* __restrict__
                                  const float* __restrict__ dist_bias, int dist_far, float cap, int HW, int KS, int async) {
     extern __shared__ __align__(16) float sm[];
     il_pdl_wait();
+    il_pdl_launch_dependents();                   // (a product behind may ask for its weights meanwhile)
     constexpr int RS = at_row(HDP), PIECES = HDP / 4, NV = (HDP + 63) / 64;
     const int G = nh / nkv, n_hb = (G + HW - 1) / HW;
     const int t = blockIdx.x, g = blockIdx.y / n_hb, hb = blockIdx.y - g * n_hb;

@@ -59,12 +59,14 @@ constexpr int FR_WS = FR_CHUNKS * FR_CS + 4, FR_XS = FR_CHUNKS * FR_CS, FR_THREA
 __host__ __device__ constexpr int fr_stage_floats(int M) { return FR_ROWS * FR_WS + M * FR_XS; }
 __host__ __device__ constexpr int fr_smem_floats(int M, int stages) { return stages * fr_stage_floats(M) + M * FR_CHUNKS * FR_ROWS; }
 
-template <int MT, bool VEC>
+// GLU: W holds N gate rows and then N up rows; a block's 8 rows are 4 gate rows and the 4 up rows that go with them, and the output is
+// act(gate) * up as the SwiGLU kernel computes it from the two products (one launch less between a step's products).
+template <int MT, bool VEC, bool GLU>
 __global__ void __launch_bounds__(FR_THREADS) gemm_f32_rows_kernel(const float* A, int lda, const float* __restrict__ W, int ldw,
                                                                    float* __restrict__ C, int ldc, const float* __restrict__ bias, float alpha,
-                                                                   int M, int N, int K, int stages, int early) {
+                                                                   int M, int N, int K, int stages, int early, int act, float limit, float act_alpha) {
     extern __shared__ __align__(16) float sm[];
-    const int tid = threadIdx.x, n0 = blockIdx.x * FR_ROWS;
+    const int tid = threadIdx.x, n0 = blockIdx.x * (GLU ? FR_ROWS / 2 : FR_ROWS);
     const int n = tid & 7, c = tid >> 3;
     const int stage_f = fr_stage_floats(M);
     float* red = sm + (size_t)stages * stage_f;   // [M][FR_CHUNKS][FR_ROWS]
@@ -75,7 +77,8 @@ __global__ void __launch_bounds__(FR_THREADS) gemm_f32_rows_kernel(const float* 
 #pragma unroll 4
         for (int i = 0; i < FR_ROWS * FR_ROUND / 4 / FR_THREADS; ++i) {
             const int idx = tid + i * FR_THREADS, row = idx / (FR_ROUND / 4), kk = (idx % (FR_ROUND / 4)) * 4;
-            const int gn = min(n0 + row, N - 1);  // rows past the end are computed and dropped
+            // rows past the end are computed and dropped
+            const int gn = GLU ? (row < FR_ROWS / 2 ? 0 : N) + min(n0 + row % (FR_ROWS / 2), N - 1) : min(n0 + row, N - 1);
             f32_cp_piece<VEC>(base + 4u * (row * FR_WS + (kk / F32_CHUNK) * FR_CS + kk % F32_CHUNK), W + (size_t)gn * ldw, r * FR_ROUND + kk, K);
         }
     };
@@ -88,6 +91,7 @@ __global__ void __launch_bounds__(FR_THREADS) gemm_f32_rows_kernel(const float* 
     };
     if (early) load_w(0);
     il_pdl_wait();
+    il_pdl_launch_dependents();                   // (the kernel behind may ask for its own weights meanwhile)
     if (!early) load_w(0);
     load_x(0);
     f32_commit();
@@ -126,8 +130,15 @@ __global__ void __launch_bounds__(FR_THREADS) gemm_f32_rows_kernel(const float* 
             for (int i = 0; i < FR_CHUNKS; ++i) tot = __fadd_rn(tot, red[(om * FR_CHUNKS + i) * FR_ROWS + on]);
         }
     }
-    il_pdl_tail();
-    if (om < M && n0 + on < N) C[(size_t)om * ldc + n0 + on] = __fmaf_rn(alpha, tot, bias ? bias[n0 + on] : 0.f);
+    if constexpr (GLU) {
+        const int n = min(n0 + (on & 3), N - 1);
+        const float y = __fmaf_rn(alpha, tot, bias ? bias[on < 4 ? n : N + n] : 0.f), up = __shfl_down_sync(0xffffffffu, y, 4);
+        if (om < M && on < 4 && n0 + on < N)
+            C[(size_t)om * ldc + n0 + on] = act == IL_ACT_CLAMPED ? il_clamped_glu(y, up, limit, act_alpha)
+                                            : act == IL_ACT_GELU_TANH ? il_gelu_tanh_mul(y, up) : y / (1.f + expf(-y)) * up;
+    } else if (om < M && n0 + on < N) {
+        C[(size_t)om * ldc + n0 + on] = __fmaf_rn(alpha, tot, bias ? bias[n0 + on] : 0.f);
+    }
 }
 
 // ---- more rows: tiles of 32 WM x 32 WN, K dealt out to KG groups of warps ------------------------------------------------------
@@ -257,8 +268,8 @@ __global__ void __launch_bounds__(FT_THREADS, FtShape<WM, WN, KG>::BLOCKS) gemm_
 struct F32Args {
     const float *A, *W, *bias;
     float* C;
-    int lda, ldw, ldc, M, N, K, early;
-    float alpha;
+    int lda, ldw, ldc, M, N, K, early, act;
+    float alpha, limit, act_alpha;
     cudaStream_t stream;
 };
 
@@ -275,13 +286,17 @@ static cudaError_t f32_allow_smem(const void* kernel, int bytes, bool* done) {
     return e;
 }
 
-template <int MT, bool VEC> static cudaError_t f32_launch_rows(const F32Args& a) {
+template <int MT, bool VEC, bool GLU> static cudaError_t f32_launch_rows_as(const F32Args& a) {
     static bool done[64];
     const int stages = a.K > FR_ROUND ? 2 : 1;
-    cudaError_t e = f32_allow_smem((const void*)gemm_f32_rows_kernel<MT, VEC>, fr_smem_floats(MT, 2) * 4, done);
+    cudaError_t e = f32_allow_smem((const void*)gemm_f32_rows_kernel<MT, VEC, GLU>, fr_smem_floats(MT, 2) * 4, done);
     if (e != cudaSuccess) return e;
-    return il_launch(gemm_f32_rows_kernel<MT, VEC>, dim3((a.N + FR_ROWS - 1) / FR_ROWS), dim3(FR_THREADS), (size_t)fr_smem_floats(a.M, stages) * 4,
-                     a.stream, a.A, a.lda, a.W, a.ldw, a.C, a.ldc, a.bias, a.alpha, a.M, a.N, a.K, stages, a.early);
+    constexpr int ROWS = GLU ? FR_ROWS / 2 : FR_ROWS;
+    return il_launch(gemm_f32_rows_kernel<MT, VEC, GLU>, dim3((a.N + ROWS - 1) / ROWS), dim3(FR_THREADS), (size_t)fr_smem_floats(a.M, stages) * 4,
+                     a.stream, a.A, a.lda, a.W, a.ldw, a.C, a.ldc, a.bias, a.alpha, a.M, a.N, a.K, stages, a.early, a.act, a.limit, a.act_alpha);
+}
+template <int MT, bool VEC> static cudaError_t f32_launch_rows(const F32Args& a) {
+    return a.act ? f32_launch_rows_as<MT, VEC, true>(a) : f32_launch_rows_as<MT, VEC, false>(a);
 }
 
 template <int WM, int WN, int KG, bool VEC> static cudaError_t f32_launch_tile(const F32Args& a) {
@@ -312,11 +327,14 @@ template <bool VEC> static cudaError_t f32_dispatch(const F32Args& a) {
     return f32_launch_tile<4, 2, 1, VEC>(a);
 }
 
+// act: 0, or the gate of a gated product (M <= 16): W is [2N, K], gate rows, then up rows, bias [2N].
+// w_static: W was written long before (a model's weights), not by the kernel in front of this one in the stream.
 IL_EXPORT int il_gemm_f32(const float* A, int lda, const float* W, int ldw, float* C, int ldc, const float* bias,
-                          float alpha, int M, int N, int K, int w_static, cudaStream_t stream) {
+                          float alpha, int M, int N, int K, int act, float limit, float act_alpha, int w_static, cudaStream_t stream) {
     if (M <= 0 || N <= 0) return IL_OK;
     if (K <= 0 || lda < K || ldw < K || ldc < N) return IL_BAD_ARG;
-    const F32Args a{A, W, bias, C, lda, ldw, ldc, M, N, K, w_static, alpha, stream};
+    if (act && (M > 16 || act < IL_ACT_SILU || act > IL_ACT_CLAMPED)) return IL_UNSUPPORTED;
+    const F32Args a{A, W, bias, C, lda, ldw, ldc, M, N, K, w_static, act, alpha, limit, act_alpha, stream};
     const bool vec = !(lda & 3) && !(ldw & 3) && !((uintptr_t)A & 15) && !((uintptr_t)W & 15);
     const cudaError_t e = vec ? f32_dispatch<true>(a) : f32_dispatch<false>(a);
     if (e != cudaSuccess) return 1000 + (int)e;

@@ -573,24 +573,29 @@ def gate_pack(y: torch.Tensor, head_dim: int, gate: Optional[torch.Tensor], g_of
 
 
 def gemm_f32(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, alpha: float = 1.0,
-             bias: Optional[torch.Tensor] = None, w_static: bool = False) -> None:
+             bias: Optional[torch.Tensor] = None, w_static: bool = False, glu: int = 0, act_params=None) -> None:
     """out[M,N] = alpha * a[M,K] @ w[N,K]^T (+ bias), all float32, FP32 pipes only. `w_static`: w is a model's weight, not what
-    the kernel launched just before writes, and may be read while that kernel still runs."""
+    the kernel launched just before writes, and may be read while that kernel still runs.
+    glu (ACT_SILU / ACT_GELU_TANH / ACT_CLAMPED with act_params; up to 16 rows): w is [2N,K] (gate rows, then up rows) and
+    out[M,N] = act(gate) * up, as `swiglu` computes it from the products."""
     _need_cuda(a, w, out, bias)
     M, K = a.shape
-    N = w.shape[0]
+    N = w.shape[0] // 2 if glu else w.shape[0]
     if a.dtype != torch.float32 or w.dtype != torch.float32 or out.dtype != torch.float32:
         raise KernelError("gemm_f32: float32 tensors")
     if w.shape[1] != K or out.shape != (M, N):
         raise KernelError(f"gemm_f32: shapes a{tuple(a.shape)} w{tuple(w.shape)} out{tuple(out.shape)}")
     if a.stride(1) != 1 or w.stride(1) != 1 or out.stride(1) != 1:
         raise KernelError("gemm_f32: innermost dimension must be contiguous")
-    if bias is not None and (bias.dtype != torch.float32 or bias.numel() != N):
-        raise KernelError("gemm_f32: bias float32 [N]")
+    if bias is not None and (bias.dtype != torch.float32 or bias.numel() != w.shape[0]):
+        raise KernelError("gemm_f32: bias float32, one per weight row")
+    if glu and (M > SKINNY_MAX_ROWS or int(glu) not in (ACT_SILU, ACT_GELU_TANH, ACT_CLAMPED) or w.shape[0] % 2):
+        raise KernelError("gemm_f32: a gate goes with up to 16 rows")
+    limit, act_alpha = _act_args(glu, act_params)
     f = _fn("gemm_f32", "il_gemm_f32", [_c_void_p, _c_int, _c_void_p, _c_int, _c_void_p, _c_int, _c_void_p, _c_float,
-                                        _c_int, _c_int, _c_int, _c_int, _c_void_p])
+                                        _c_int, _c_int, _c_int, _c_int, _c_float, _c_float, _c_int, _c_void_p])
     _check(f(_ptr(a), a.stride(0), _ptr(w), w.stride(0), _ptr(out), out.stride(0), _ptr(bias), alpha, M, N, K,
-             int(w_static), _stream()), "gemm_f32")
+             int(glu), limit, act_alpha, int(w_static), _stream()), "gemm_f32")
 
 
 _ones_k = {}

@@ -78,6 +78,9 @@ class SwiGLU(FeedForward):
                                              ctx.ws.rows("sumsq_ffn", T, (self.hidden + 15) // 16, torch.float32), w_static=True)
             return self.down(act, ctx.ws.rows("ffn_branch", T, self.hidden, self.dtype))
         act = ctx.ws.rows("ffn_act", T, self.inter, self.dtype)
+        if self.dtype == torch.float32 and T <= ops.SKINNY_MAX_ROWS:        # a few rows: the gate in the product's epilogue
+            ops.gemm_f32(x, self.gate_up.weight, act, 1.0, self.gate_up.bias, w_static=True, glu=self.act, act_params=self.act_params)
+            return self.down(act, ctx.ws.rows("ffn_branch", T, self.hidden, self.dtype))
         if self.dtype == torch.bfloat16 and ops.mid_ok(T, self.hidden):
             # 17..128 rows: gate and up on the tcgen05 tensor cores as two accumulators in the same lanes, SiLU(gate)*up in
             # the epilogue (measured against the library product followed by the SwiGLU kernel at 8B sizes: 44.6 against

@@ -118,6 +118,20 @@ def test_gemm_f32_shapes(cuda_device, M, N, K, off):
     assert torch.equal(again, out[:, :N]) and torch.equal(one[0], out[M - 1, :N])
 
 
+@pytest.mark.parametrize("M", [1, 4, 7, 16])
+@pytest.mark.parametrize("act", [1, 2, 3])
+@pytest.mark.parametrize("I,K", [(4, 64), (7, 100), (130, 1028), (9, 33)])
+def test_gemm_f32_gated(cuda_device, M, act, I, K):
+    """The gate in the product's epilogue: what the product and then the gate's kernel give, bit for bit."""
+    g = torch.Generator(device="cuda").manual_seed(M + I)
+    x, w, b = (torch.randn(*n, device="cuda", generator=g) for n in ((M, K), (2 * I, K), (2 * I,)))
+    out, gu, ref = torch.full((M, I + 1), float("nan"), device="cuda"), torch.empty(M, 2 * I, device="cuda"), torch.empty(M, I, device="cuda")
+    ops.gemm_f32(x, w, out[:, :I], 0.3, b, glu=act, act_params=(7.0, 1.7))
+    ops.gemm_f32(x, w, gu, 0.3, b)
+    ops.swiglu(gu, ref, act, (7.0, 1.7))
+    assert torch.equal(out[:, :I], ref) and bool(out[:, I].isnan().all())
+
+
 # -- rope + cache write --------------------------------------------------------------------------
 def _paged_setup(E, lens, nkv, hd, page, dtype, seed, n_extra_pages=3):
     """Random block tables over shuffled pages for entries with the given kv lengths."""
