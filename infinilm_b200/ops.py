@@ -857,7 +857,7 @@ def _norm_args(norm_in: Optional[NormedInput], M: int):
 def gemm_skinny(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, alpha: float = 1.0,
                 bias: Optional[torch.Tensor] = None, glu: int = 0, norm_in: Optional[NormedInput] = None, act_params=None,
                 w_static: bool = False) -> None:
-    """out[M,N] = alpha * x[M,K] @ w[N,K]^T (+ bias) for M <= 16 bfloat16 rows; out bfloat16 or float32.
+    """out[M,N] = alpha * x[M,K] @ w[N,K]^T (+ bias) for M <= 16 bfloat16 rows (with a gate `skinny_glu_ok`); out bfloat16 or float32.
     glu (True, or ACT_SILU / ACT_GELU_TANH / ACT_CLAMPED with act_params): w is [2N,K] (gate rows, then up rows) and out[M,N] = act(gate) * up;
     ACT_RELU2: w is [N,K] and out is relu(.)^2 of the product (bfloat16).
     norm_in: x is `norm_in.xw`, and the results are divided by the rms that its sums give.
@@ -871,6 +871,16 @@ def gemm_skinny(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, alpha: floa
         raise KernelError("gemm_skinny: innermost dimension must be contiguous")
     if bias is not None and (bias.dtype != torch.float32 or bias.numel() != w.shape[0]):
         raise KernelError("gemm_skinny: bias float32, one per weight row")
+    if M > SKINNY_MAX_ROWS and glu and int(glu) != ACT_RELU2:
+        if out.dtype != torch.bfloat16 or not narrow_ok(M, K):
+            raise KernelError(f"gemm_skinny: {M} rows of {K} columns")
+        limit, act_alpha = _act_args(glu, act_params)
+        f = _fn("gemm_narrow", "il_gemm_narrow_glu", [_c_void_p, _c_int, _c_void_p, _c_int, _c_void_p, _c_int, _c_void_p, _c_float, _c_int, _c_int,
+                                                      _c_int, _c_int, _c_float, _c_float, _c_void_p, _c_int, _c_int, _c_float, _c_int, _c_void_p])
+        np_, nb, nw, ne = _norm_args(norm_in, M)
+        _check(f(_ptr(x), x.stride(0), _ptr(w), w.stride(0), _ptr(out), out.stride(0), _ptr(bias), alpha, M, N, K, int(glu), limit, act_alpha,
+                 np_, nb, nw, ne, int(w_static), _stream()), "gemm_narrow_glu")
+        return
     f = _fn("gemm_skinny", "il_gemm_skinny", [_c_void_p, _c_int, _c_void_p, _c_int, _c_void_p, _c_int, _c_int, _c_void_p,
                                               _c_float, _c_int, _c_int, _c_int, _c_int, _c_void_p, _c_int, _c_int, _c_float,
                                               _c_float, _c_float, _c_int, _c_void_p])
@@ -880,15 +890,36 @@ def gemm_skinny(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, alpha: floa
              M, N, K, int(glu), np_, nb, nw, ne, limit, act_alpha, int(w_static), _stream()), "gemm_skinny")
 
 
+# 17 to 48 rows of a narrow model: the fused products (gated, rotating, adding into the residual) take these rows too where
+# the model is NARROW_FROM to NARROW_WIDTH wide. Every block brings the activations in: measured at 1,024 wide against the tcgen05 and
+# library products, which still want their norms, 6.4 / 7.7 us at 17 rows and 8.5 / 10.2 at 48 for gate+up, 3.0 / 3.8 and 5.0 / 3.8 for
+# 1,024 x 1,024 into the residual; at 64 rows 10.0 / 8.6. With 4,096 columns into the residual 7.8 / 9.1 at 17 rows, 8.6 / 8.7 at 32 and
+# 11.2 / 8.1 at 48, so that product ends at NARROW_LONG_ROWS. Below NARROW_FROM, half the narrowest model in use, nothing was measured
+# and 17 rows keep the norm kernels.
+NARROW_MAX_ROWS, NARROW_LONG_ROWS, NARROW_FROM, NARROW_WIDTH = 48, 32, 512, 1024
+
+
+def narrow_ok(M: int, K: int) -> bool:
+    """Whether the fused products of a model K wide take M rows, more than the few of `skinny_ok`."""
+    return SKINNY_MAX_ROWS < M <= NARROW_MAX_ROWS and NARROW_FROM <= K <= NARROW_WIDTH and K % 8 == 0
+
+
+def skinny_glu_ok(M: int, K: int) -> bool:
+    """Whether `gemm_skinny` takes this shape with a gate."""
+    return skinny_ok(M, K) or narrow_ok(M, K)
+
+
 def skinny_resid_ok(M: int, K: int, width: int) -> bool:
     """Whether `gemm_skinny_resid` takes this shape."""
+    if narrow_ok(M, width):
+        return K % 8 == 0 and (K <= NARROW_WIDTH or (K <= 4 * NARROW_WIDTH and M <= NARROW_LONG_ROWS))
     return 0 < M <= SKINNY_MAX_ROWS and K % 8 == 0 and (width + 15) // 16 <= NORM_MAX_BLOCKS
 
 
 def gemm_skinny_resid(x: torch.Tensor, w: torch.Tensor, alpha: float, bias: Optional[torch.Tensor], resid: torch.Tensor,
                       branch_scale: float, norm_weight: torch.Tensor, eps: float, xw: torch.Tensor,
                       sumsq: torch.Tensor, w_static: bool = False) -> NormedInput:
-    """The last product of a branch (up to 16 bfloat16 rows) with the residual add and the next RMSNorm's inputs in its
+    """The last product of a branch (`skinny_resid_ok` bfloat16 rows) with the residual add and the next RMSNorm's inputs in its
     epilogue: resid (float32 [M,H], in place) += branch_scale * bf16(alpha * x @ w^T + bias); xw = resid * norm_weight;
     sumsq[m][b] = sum of resid[m]^2 over columns 16b..16b+15. Returns what the next product needs to finish the norm.
     w_static: as for gemm_skinny."""
@@ -907,8 +938,10 @@ def gemm_skinny_resid(x: torch.Tensor, w: torch.Tensor, alpha: float, bias: Opti
     if bias is not None and (bias.dtype != torch.float32 or bias.numel() != H):
         raise KernelError("gemm_skinny_resid: bias float32 [H]")
     _contig("resid", resid), _contig("xw", xw), _contig("sumsq", sumsq), _contig("norm_weight", norm_weight)
-    f = _fn("gemm_skinny", "il_gemm_skinny_resid", [_c_void_p, _c_int, _c_void_p, _c_int, _c_void_p, _c_float, _c_int, _c_int, _c_int,
-                                                    _c_void_p, _c_float, _c_void_p, _c_int, _c_void_p, _c_void_p, _c_int, _c_void_p])
+    many = M > SKINNY_MAX_ROWS
+    f = _fn("gemm_narrow" if many else "gemm_skinny", "il_gemm_narrow_resid" if many else "il_gemm_skinny_resid",
+            [_c_void_p, _c_int, _c_void_p, _c_int, _c_void_p, _c_float, _c_int, _c_int, _c_int,
+             _c_void_p, _c_float, _c_void_p, _c_int, _c_void_p, _c_void_p, _c_int, _c_void_p])
     _check(f(_ptr(x), x.stride(0), _ptr(w), w.stride(0), _ptr(bias), alpha, M, H, K, _ptr(resid), branch_scale, _ptr(norm_weight),
              kind_of(norm_weight.dtype), _ptr(xw), _ptr(sumsq), int(w_static), _stream()), "gemm_skinny_resid")
     return NormedInput(xw, sumsq, H, eps)
@@ -916,7 +949,7 @@ def gemm_skinny_resid(x: torch.Tensor, w: torch.Tensor, alpha: float, bias: Opti
 
 def skinny_rope_ok(M: int, K: int, head_dim: int, rot_dim: int) -> bool:
     """Whether `gemm_skinny_rope` takes this shape: a few rows, rotary and head sizes in steps of 16."""
-    return 0 < M <= SKINNY_MAX_ROWS and K % 8 == 0 and head_dim % 16 == 0 and rot_dim % 16 == 0 and 0 <= rot_dim <= head_dim
+    return (skinny_ok(M, K) or narrow_ok(M, K)) and head_dim % 16 == 0 and rot_dim % 16 == 0 and 0 <= rot_dim <= head_dim
 
 
 def gemm_skinny_rope(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, alpha: float, bias: Optional[torch.Tensor],
@@ -924,7 +957,7 @@ def gemm_skinny_rope(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, alpha:
                      page_size: int, n_heads: int, n_kv_heads: int, head_dim: int, rot_dim: int,
                      inv_freq: Optional[torch.Tensor], mscale: float, norm_in: Optional[NormedInput] = None,
                      w_static: bool = False) -> None:
-    """The q/k/v projection of up to 16 bfloat16 rows with what `rope_store` does in its epilogue: out[M, (heads + 2
+    """The q/k/v projection of a few bfloat16 rows (`skinny_rope_ok`) with what `rope_store` does in its epilogue: out[M, (heads + 2
     kv_heads) * head_dim] = alpha * x @ w^T (+ bias), q and k rotated, k and v written to their cache slots (if `cache`).
     w_static: as for gemm_skinny."""
     _need_cuda(x, w, out, bias, tok_pos, tok_entry, block_table, cache, inv_freq)
@@ -945,7 +978,8 @@ def gemm_skinny_rope(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, alpha:
         _contig("cache", cache)
         if cache.dtype != torch.bfloat16 or tuple(cache.shape[1:]) != (2, n_kv_heads, page_size, head_dim):
             raise KernelError("gemm_skinny_rope: cache bfloat16 [pages,2,kv_heads,page,head_dim]")
-    f = _fn("gemm_skinny", "il_gemm_skinny_rope",
+    many = M > SKINNY_MAX_ROWS
+    f = _fn("gemm_narrow" if many else "gemm_skinny", "il_gemm_narrow_rope" if many else "il_gemm_skinny_rope",
             [_c_void_p, _c_int, _c_void_p, _c_int, _c_void_p, _c_int, _c_void_p, _c_float, _c_int, _c_int, _c_void_p, _c_void_p,
              _c_void_p, _c_int, _c_void_p, _c_int, _c_int, _c_int, _c_int, _c_int, _c_void_p, _c_float, _c_void_p, _c_int, _c_int,
              _c_float, _c_int, _c_void_p])
