@@ -7,6 +7,11 @@
 // Cache layout of one layer: [page][0=K,1=V][kv head = 1][slot in page][width of B].
 #include "common.cuh"
 
+// Bound by latency: a block a token, few tokens in a decode step. The row's elements stay in registers where they fit (LN_KEEP a thread), so
+// the row is read once, both sums go through one reduction, and the weights, cold by the time a layer comes round again, are asked for before the
+// wait for the kernel in front (an ordinary launch where the caller does not vouch for them); longer rows are read twice. Asked for with the row
+// instead, nothing was gained.
+constexpr int LN_KEEP = 4;
 template <typename TA>
 __global__ void latent_norm_store_kernel(const TA* proj, int row_stride, int off_a, int n_a, int off_b, int n_b,
                                          const void* __restrict__ w_a, const void* __restrict__ w_b, int w_kind, float eps,
@@ -25,48 +30,87 @@ __global__ void latent_norm_store_kernel(const TA* proj, int row_stride, int off
             kdst = cache + (size_t)page * 2 * plane + (size_t)(pos % page_size) * n_b;
         }
     }
+    float wa[LN_KEEP], x[LN_KEEP];
+    const int n = n_a + n_b;
+    const bool keep = n <= LN_KEEP * (int)blockDim.x;
+#pragma unroll
+    for (int u = 0; u < LN_KEEP; ++u) {
+        const int i = threadIdx.x + u * blockDim.x;
+        wa[u] = !keep || i >= n ? 0.f : i < n_a ? il_load_any(w_a, w_kind, i) : il_load_any(w_b, w_kind, i - n_a);
+    }
     il_pdl_begin();
     const TA* row = proj + (size_t)t * row_stride;
     float sa = 0.f, sb = 0.f;
-    for (int i = threadIdx.x; i < n_a; i += blockDim.x) {
-        const float x = il_to_f(row[off_a + i]);
-        sa += x * x;
+    if (keep) {
+#pragma unroll
+        for (int u = 0; u < LN_KEEP; ++u) {
+            const int i = threadIdx.x + u * blockDim.x;
+            x[u] = i >= n ? 0.f : il_to_f(row[i < n_a ? off_a + i : off_b + i - n_a]);
+        }
+#pragma unroll
+        for (int u = 0; u < LN_KEEP; ++u) {
+            if (threadIdx.x + u * blockDim.x < n_a) sa += x[u] * x[u];
+            else sb += x[u] * x[u];
+        }
+        sa = il_warp_sum(sa), sb = il_warp_sum(sb);
+        const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+        if (lane == 0) red[warp] = sa, red[16 + warp] = sb;
+        __syncthreads();
+        sa = il_warp_sum(lane < nw ? red[lane] : 0.f), sb = il_warp_sum(lane < nw ? red[16 + lane] : 0.f);
+    } else {
+        for (int i = threadIdx.x; i < n_a; i += blockDim.x) {
+            const float v = il_to_f(row[off_a + i]);
+            sa += v * v;
+        }
+        for (int i = threadIdx.x; i < n_b; i += blockDim.x) {
+            const float v = il_to_f(row[off_b + i]);
+            sb += v * v;
+        }
+        sa = il_block_sum(sa, red);
+        sb = il_block_sum(sb, red);
     }
-    for (int i = threadIdx.x; i < n_b; i += blockDim.x) {
-        const float x = il_to_f(row[off_b + i]);
-        sb += x * x;
-    }
-    sa = il_block_sum(sa, red);
-    sb = il_block_sum(sb, red);
     const float ra = n_a > 0 ? rsqrtf(sa / (float)n_a + eps) : 0.f, rb = rsqrtf(sb / (float)n_b + eps);
-    for (int i = threadIdx.x; i < n_a; i += blockDim.x)
-        out_a[(size_t)t * n_a + i] = il_from_f<TA>(il_to_f(row[off_a + i]) * ra * il_load_any(w_a, w_kind, i));
-    for (int i = threadIdx.x; i < n_b; i += blockDim.x) {
-        const TA v = il_from_f<TA>(il_to_f(row[off_b + i]) * rb * il_load_any(w_b, w_kind, i));
+    const auto put_b = [&](int i, float y) {
+        const TA v = il_from_f<TA>(y);
         if (out_b) out_b[(size_t)t * n_b + i] = v;
         if (kdst) {
             kdst[i] = v;
             kdst[plane + i] = v;
         }
+    };
+    if (keep) {
+#pragma unroll
+        for (int u = 0; u < LN_KEEP; ++u) {
+            const int i = threadIdx.x + u * blockDim.x;
+            if (i < n_a) out_a[(size_t)t * n_a + i] = il_from_f<TA>(x[u] * ra * wa[u]);
+            else if (i < n) put_b(i - n_a, x[u] * rb * wa[u]);
+        }
+        return;
     }
+    for (int i = threadIdx.x; i < n_a; i += blockDim.x)
+        out_a[(size_t)t * n_a + i] = il_from_f<TA>(il_to_f(row[off_a + i]) * ra * il_load_any(w_a, w_kind, i));
+    for (int i = threadIdx.x; i < n_b; i += blockDim.x) put_b(i, il_to_f(row[off_b + i]) * rb * il_load_any(w_b, w_kind, i));
 }
 
+// w_static: the weights were written long before, not by the kernel in front of this one.
 IL_EXPORT int il_latent_norm_store(const void* proj, int act_kind, int row_stride, int off_a, int n_a, int off_b, int n_b, const void* w_a,
                                    const void* w_b, int w_kind, float eps, void* out_a, void* out_b, const int* tok_pos,
                                    const int* tok_entry, const int* block_table, int bt_stride, void* cache, int page_size, int T,
-                                   cudaStream_t stream) {
+                                   int w_static, cudaStream_t stream) {
     if (T <= 0) return IL_OK;
     if (n_b <= 0 || n_a < 0 || page_size <= 0 || (n_a > 0 && !out_a)) return IL_BAD_ARG;
     const int threads = (n_a + n_b) >= 1024 ? 256 : 128;
+    cudaError_t e;
     if (act_kind == IL_F32)
-        IL_LAUNCH(latent_norm_store_kernel<float>, T, threads, 0, stream, (const float*)proj, row_stride, off_a, n_a, off_b, n_b, w_a, w_b,
-                  w_kind, eps, (float*)out_a, (float*)out_b, tok_pos, tok_entry, block_table, bt_stride, (float*)cache, page_size);
+        e = il_launch_as(w_static != 0, latent_norm_store_kernel<float>, dim3(T), dim3(threads), 0, stream, (const float*)proj, row_stride, off_a, n_a, off_b, n_b, w_a,
+                         w_b, w_kind, eps, (float*)out_a, (float*)out_b, tok_pos, tok_entry, block_table, bt_stride, (float*)cache, page_size);
     else if (act_kind == IL_BF16)
-        IL_LAUNCH(latent_norm_store_kernel<__nv_bfloat16>, T, threads, 0, stream, (const __nv_bfloat16*)proj, row_stride, off_a, n_a, off_b,
-                  n_b, w_a, w_b, w_kind, eps, (__nv_bfloat16*)out_a, (__nv_bfloat16*)out_b, tok_pos, tok_entry, block_table, bt_stride,
-                  (__nv_bfloat16*)cache, page_size);
+        e = il_launch_as(w_static != 0, latent_norm_store_kernel<__nv_bfloat16>, dim3(T), dim3(threads), 0, stream, (const __nv_bfloat16*)proj, row_stride, off_a, n_a,
+                         off_b, n_b, w_a, w_b, w_kind, eps, (__nv_bfloat16*)out_a, (__nv_bfloat16*)out_b, tok_pos, tok_entry, block_table, bt_stride,
+                         (__nv_bfloat16*)cache, page_size);
     else
         return IL_BAD_ARG;
+    if (e != cudaSuccess) return 1000 + (int)e;
     IL_LAUNCH_CHECK();
     return IL_OK;
 }

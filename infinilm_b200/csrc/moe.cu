@@ -255,6 +255,8 @@ __device__ __forceinline__ void moe_sort_body(int* sh, const int* idx, int n_slo
     int* cur = sh + E;
     for (int e = threadIdx.x; e < E; e += blockDim.x) cnt[e] = 0;
     __syncthreads();
+    const bool once = SL == 1 && n_slots <= (int)blockDim.x;          // a decode step: a slot a thread, its choice read once
+    const int mine = once && (int)threadIdx.x < n_slots ? idx[threadIdx.x] : -1;
     // (SL slots of a thread asked for at a time: one after the other the slots of a long portion are a chain of round trips to
     // memory; a decode step has at most one a thread)
     for (int i0 = threadIdx.x; i0 < n_slots; i0 += SL * blockDim.x) {
@@ -262,21 +264,33 @@ __device__ __forceinline__ void moe_sort_body(int* sh, const int* idx, int n_slo
 #pragma unroll
         for (int u = 0; u < SL; ++u) {
             const int i = i0 + u * blockDim.x;
-            e[u] = i < n_slots ? idx[i] : -1;
+            e[u] = once ? mine : i < n_slots ? idx[i] : -1;
         }
 #pragma unroll
         for (int u = 0; u < SL; ++u)
             if (e[u] >= 0 && e[u] < E) atomicAdd(&cnt[e[u]], 1);
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
-        int a = 0;
-        for (int e = 0; e < E; ++e) {
-            group_off[e] = a;
-            cur[e] = a;
-            a += cnt[e];
+    // the groups' first places: one warp, 32 counts at a time. (One thread that walked them was a chain of E loads and adds; with this, a
+    // choice read once and the latent rows' norm in registers 4 layers of 64 experts, 8 requests: 26.1 -> 25.9 ms for their prompts and 31 decode steps.)
+    if (threadIdx.x < 32) {
+        const int lane = threadIdx.x;
+        int before = 0;
+        for (int e0 = 0; e0 < E; e0 += 32) {
+            const int n = e0 + lane < E ? cnt[e0 + lane] : 0;
+            int incl = n;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int up = __shfl_up_sync(0xffffffffu, incl, o);
+                if (lane >= o) incl += up;
+            }
+            if (e0 + lane < E) {
+                group_off[e0 + lane] = before + incl - n;
+                cur[e0 + lane] = before + incl - n;
+            }
+            before += __shfl_sync(0xffffffffu, incl, 31);
         }
-        group_off[E] = a;
+        if (lane == 0) group_off[E] = before;
     }
     __syncthreads();
     // the order of the rows inside an expert's range is whatever the atomics give: a row's result does not depend on it
@@ -286,7 +300,7 @@ __device__ __forceinline__ void moe_sort_body(int* sh, const int* idx, int n_slo
 #pragma unroll
         for (int u = 0; u < SL; ++u) {
             const int i = i0 + u * blockDim.x;
-            e[u] = i < n_slots ? idx[i] : -1;
+            e[u] = once ? mine : i < n_slots ? idx[i] : -1;
             w[u] = (wt_of_pos && i < n_slots) ? wt[i] : 0.f;
         }
 #pragma unroll

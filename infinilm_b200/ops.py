@@ -1120,10 +1120,10 @@ def embed_pair_pos(ids: torch.Tensor, tok_pos: torch.Tensor, tok_entry: torch.Te
 def latent_norm_store(proj: torch.Tensor, off_a: int, n_a: int, off_b: int, n_b: int, w_a: Optional[torch.Tensor],
                       w_b: torch.Tensor, eps: float, out_a: Optional[torch.Tensor], out_b: Optional[torch.Tensor],
                       tok_pos: torch.Tensor, tok_entry: torch.Tensor, block_table: torch.Tensor, cache: Optional[torch.Tensor],
-                      page_size: int) -> None:
+                      page_size: int, w_static: bool = False) -> None:
     """Per row of `proj`: columns [off_a, off_a + n_a) and [off_b, off_b + n_b) are each divided by their root mean
     square (f32) and multiplied by `w_a` / `w_b`. The first goes to `out_a` [T, n_a]; the second to `out_b` (if given) and
-    into the token's slot of `cache` [pages, 2, 1, page, n_b], K plane and V plane alike."""
+    into the token's slot of `cache` [pages, 2, 1, page, n_b], K plane and V plane alike. w_static: w_a and w_b are weights, as for gemm_skinny."""
     _need_cuda(proj, w_a, w_b, out_a, out_b, tok_pos, tok_entry, block_table, cache)
     T = proj.shape[0]
     if proj.stride(1) != 1 or off_a + n_a > proj.shape[1] or off_b + n_b > proj.shape[1]:
@@ -1143,10 +1143,10 @@ def latent_norm_store(proj: torch.Tensor, off_a: int, n_a: int, off_b: int, n_b:
             raise KernelError("latent_norm_store: cache [pages,2,1,page,n_b] of proj's dtype")
     f = _fn("latent", "il_latent_norm_store", [_c_void_p, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_void_p, _c_void_p, _c_int,
                                                _c_float, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_int, _c_void_p, _c_int,
-                                               _c_int, _c_void_p])
+                                               _c_int, _c_int, _c_void_p])
     _check(f(_ptr(proj), kind_of(proj.dtype), proj.stride(0), off_a, n_a, off_b, n_b, _ptr(w_a), _ptr(w_b), kind_of(w_b.dtype), eps,
              _ptr(out_a), _ptr(out_b), _ptr(tok_pos), _ptr(tok_entry), _ptr(block_table), block_table.shape[1], _ptr(cache), page_size,
-             T, _stream()), "latent_norm_store")
+             T, int(w_static), _stream()), "latent_norm_store")
 
 
 def latent_rope_store(proj: torch.Tensor, off_q: int, n_heads: int, q_dim: int, off_b: int, n_b: int, rot_part: int, head_dim: int,

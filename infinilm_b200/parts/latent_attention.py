@@ -143,7 +143,7 @@ class LatentAttention(Mixer):
                                   cache.storage if cache.writable else None, cache.page_size)
         else:
             ops.latent_norm_store(proj, 0, self.qr, self.n_q, self.r, self.nq, self.nkv, self.eps, cq, None, ctx.tok_pos, ctx.tok_entry,
-                                  cache.block_table, cache.storage if cache.writable else None, cache.page_size)
+                                  cache.block_table, cache.storage if cache.writable else None, cache.page_size, w_static=True)
         q = proj[:, :self.n_q] if self.direct_q else self.up_q(cq, ws.rows("lat_q", T, H * self.d, dt))
         # heads [T, H, columns]: the queries without their rotated part, and the first r columns of what stands against the cache
         q_heads, qlat_heads = q.view(T, H, self.dq)[:, :, :self.d], q_lat.view(T, H, self.hd)[:, :, :self.r]
