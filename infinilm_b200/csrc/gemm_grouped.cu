@@ -9,7 +9,7 @@
 // epilogue: a factor per row of A, or - scale_by_place - per place of the sorted order. Products accumulate in f32 in the order of K whatever the tile, one accumulator per
 // output element, so a row's result does not depend on what else is in the batch. float32 runs on the FP32 pipes
 // (FFMA); bfloat16 runs on the tensor cores (mma.sync m16n8k16, operands staged by cp.async in a three-stage ring: a
-// block streams a tile of 64 weight rows over all of K once, against up to 32 rows of its group, which is what a decode
+// block streams a tile of 64 weight rows over all of K once, against up to 16 or 32 rows of its group, which is what a decode
 // step's few rows per expert need - the weights of the experts that were chosen are read once, at the rate the memory
 // gives); bfloat16 operands that are not 16-byte aligned are widened to f32 in shared memory (exact) and run the FFMA loop.
 #include "common.cuh"
@@ -47,16 +47,35 @@ __global__ void __launch_bounds__(128) gemm_grouped_mma_kernel(const __nv_bfloat
     int g, r0, r1;
     if (group_off) {                              // (the groups' ranges come from the sort kernel before this one)
         il_pdl_begin();
-        if (tid == 0) {
-            int tile = blockIdx.y, gg = 0, a = 0, b = 0;
-            for (; gg < n_groups; ++gg) {
-                a = group_off[gg];
-                b = group_off[gg + 1];
-                const int nt = (b - a + BM - 1) / BM;
-                if (tile < nt) break;
-                tile -= nt;
+        // The tile's group, by one warp, two groups a lane (one thread that walked the groups was a chain of up to n_groups reads in every
+        // block, the surplus ones too: 8 tokens to 6 of 64 experts of 2 x 1,408 x 2,048, gate+up 74.7 us, 69.4 with this and tiles of 16 rows; one
+        // token's six experts 26.1 and, the other way, 18.6 us, now 22.8 and 11.9).
+        if (warp == 0) {
+            int tile = blockIdx.y;
+            if (lane == 0) sh_g = n_groups;
+            __syncwarp();
+            for (int g0 = 0; g0 < n_groups; g0 += 64) {
+                const int gg = g0 + 2 * lane;
+                const int o0 = group_off[min(gg, n_groups)], o1 = group_off[min(gg + 1, n_groups)], o2 = group_off[min(gg + 2, n_groups)];
+                const int t0 = (o1 - o0 + BM - 1) / BM, t1 = (o2 - o1 + BM - 1) / BM;
+                int incl = t0 + t1;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const int up = __shfl_up_sync(0xffffffffu, incl, o);
+                    if (lane >= o) incl += up;
+                }
+                const unsigned hit = __ballot_sync(0xffffffffu, tile < incl);
+                if (hit) {
+                    if (lane == __ffs(hit) - 1) {
+                        const int in = tile - (incl - t0 - t1);
+                        sh_g = in < t0 ? gg : gg + 1;
+                        sh_r0 = in < t0 ? o0 + in * BM : o1 + (in - t0) * BM;
+                        sh_r1 = in < t0 ? o1 : o2;
+                    }
+                    break;
+                }
+                tile -= __shfl_sync(0xffffffffu, incl, 31);
             }
-            sh_g = gg, sh_r0 = a + tile * BM, sh_r1 = b;
         }
         __syncthreads();
         g = sh_g, r0 = sh_r0, r1 = sh_r1;
@@ -75,17 +94,12 @@ __global__ void __launch_bounds__(128) gemm_grouped_mma_kernel(const __nv_bfloat
     const __nv_bfloat16* a_src[A_CH];
     const __nv_bfloat16* w_src[W_CH];
 #pragma unroll
-    for (int i = 0; i < A_CH; ++i) {
-        const int ch = tid + i * 128, r = ch >> 3, p = r0 + r;
-        a_src[i] = p < r1 ? Ag + (size_t)(a_rows ? a_rows[p] : p) * lda + (ch & 7) * 8 : nullptr;
-    }
-#pragma unroll
     for (int i = 0; i < W_CH; ++i) {
         const int ch = tid + i * 128, r = ch >> 3, half = r / BN, gn = n0 + (r - half * BN);
         w_src[i] = gn < N ? Wg + (size_t)(half * N + gn) * ldw + (ch & 7) * 8 : nullptr;
     }
     const int n_kb = (K + BK - 1) / BK;
-    auto issue = [&](int kb) {
+    auto issue_a = [&](int kb) {
         if (kb < n_kb) {
             const uint32_t st = sbase + (kb % STAGES) * STAGE_BYTES;
             const int k0 = kb * BK;
@@ -95,6 +109,13 @@ __global__ void __launch_bounds__(128) gemm_grouped_mma_kernel(const __nv_bfloat
                 const uint32_t dst = st + (ch >> 3) * ROW + (ch & 7) * 16;
                 if (a_src[i] && k0 + (ch & 7) * 8 < K) cp16(dst, a_src[i] + k0); else zero16(dst);
             }
+        }
+        commit();
+    };
+    auto issue_w = [&](int kb) {
+        if (kb < n_kb) {
+            const uint32_t st = sbase + (kb % STAGES) * STAGE_BYTES;
+            const int k0 = kb * BK;
 #pragma unroll
             for (int i = 0; i < W_CH; ++i) {
                 const int ch = tid + i * 128;
@@ -102,7 +123,6 @@ __global__ void __launch_bounds__(128) gemm_grouped_mma_kernel(const __nv_bfloat
                 if (w_src[i] && k0 + (ch & 7) * 8 < K) cp16(dst, w_src[i] + k0); else zero16(dst);
             }
         }
-        commit();
     };
     float acc[MT][2][4], acc2[GLU ? MT : 1][2][4];
 #pragma unroll
@@ -115,14 +135,22 @@ __global__ void __launch_bounds__(128) gemm_grouped_mma_kernel(const __nv_bfloat
                 if (GLU) acc2[i][j][k] = 0.f;
             }
 #pragma unroll
-    for (int s = 0; s < STAGES - 1; ++s) issue(s);
+    for (int s = 0; s < STAGES - 1; ++s) issue_w(s);                     // the weights need no list of rows
+#pragma unroll
+    for (int i = 0; i < A_CH; ++i) {
+        const int ch = tid + i * 128, r = ch >> 3, p = r0 + r;
+        a_src[i] = p < r1 ? Ag + (size_t)(a_rows ? a_rows[p] : p) * lda + (ch & 7) * 8 : nullptr;
+    }
+#pragma unroll
+    for (int s = 0; s < STAGES - 1; ++s) issue_a(s);
     const int mat = lane >> 3, rr = lane & 7;
     const uint32_t a_off = ((mat & 1) * 8 + rr) * ROW + (mat >> 1) * 16;                       // A fragment: rows (mat&1)*8.., k (mat>>1)*8..
     const uint32_t b_off = A_BYTES + (warp * 16 + (mat >> 1) * 8 + rr) * ROW + (mat & 1) * 16; // B fragment: weight rows (mat>>1)*8.., k (mat&1)*8..
     for (int kb = 0; kb < n_kb; ++kb) {
         wait<STAGES - 2>();
         __syncthreads();                          // stage kb has landed for everyone, and everyone is done with stage kb - 1
-        issue(kb + STAGES - 1);
+        issue_w(kb + STAGES - 1);
+        issue_a(kb + STAGES - 1);
         const uint32_t st = sbase + (kb % STAGES) * STAGE_BYTES;
 #pragma unroll
         for (int kk = 0; kk < BK / 16; ++kk) {
@@ -323,7 +351,12 @@ IL_EXPORT int il_gemm_grouped(const void* A, int act_kind, int lda, long long a_
     if (act_kind == IL_BF16 && K % 8 == 0 && lda % 8 == 0 && ldw % 8 == 0 && a_gs % 8 == 0 && w_gs % 8 == 0 && !((uintptr_t)A & 15) &&
         !((uintptr_t)W & 15)) {
         // rows of 16-byte chunks: the tensor-core kernel. Few rows a group (a decode step): tiles of 32 rows; else 64.
+        // (and of 16 where a group has a few rows of them at most: half the stores of zeros and reads of rows that are none; 40 tokens to 6 of 64 experts:
+        // gate+up 139.7 us with 32, 131.2 with 16)
         const bool few = group_off ? M <= 32 * n_groups : M <= 32;
+        if (group_off ? M <= 4 * n_groups : M <= 16)
+            return glu ? launch_mma<16, true>(A, lda, a_gs, a_rows, W, ldw, w_gs, C, ldc, c_gs, group_off, n_groups, M, N, K, gate, ld_gate, gate_gs, gate_ns, row_scale, scale_by_place, stream)
+                       : launch_mma<16, false>(A, lda, a_gs, a_rows, W, ldw, w_gs, C, ldc, c_gs, group_off, n_groups, M, N, K, gate, ld_gate, gate_gs, gate_ns, row_scale, scale_by_place, stream);
         if (glu)
             return few ? launch_mma<32, true>(A, lda, a_gs, a_rows, W, ldw, w_gs, C, ldc, c_gs, group_off, n_groups, M, N, K, gate, ld_gate, gate_gs, gate_ns, row_scale, scale_by_place, stream)
                        : launch_mma<64, true>(A, lda, a_gs, a_rows, W, ldw, w_gs, C, ldc, c_gs, group_off, n_groups, M, N, K, gate, ld_gate, gate_gs, gate_ns, row_scale, scale_by_place, stream);

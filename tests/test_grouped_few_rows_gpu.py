@@ -1,0 +1,70 @@
+"""Products over many groups of a few rows: every tile finds its group, among up to hundreds, and a row has the same bits in any tile."""
+import math
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _layout(G, M, seed):
+    """Groups of 0 to 2 rows, one of 16, one of 17 and the last of the rest."""
+    g = torch.Generator().manual_seed(seed)
+    counts = torch.randint(0, 3, (G,), generator=g)
+    counts[G // 2], counts[G // 3] = 16, 17
+    counts[-1] = 0
+    over = int(counts.sum()) - M
+    for i in range(G):
+        cut = min(max(over, 0), int(counts[i])) if i not in (G // 2, G // 3) else 0
+        counts[i] -= cut
+        over -= cut
+    counts[-1] += max(-over, 0)
+    return torch.cat([torch.zeros(1, dtype=torch.int64), counts.cumsum(0)])
+
+
+@pytest.mark.parametrize("G,M", [(12, 48), (63, 100), (64, 100), (65, 70), (128, 300), (300, 330)])
+@pytest.mark.parametrize("N,K,glu", [(40, 96, True), (72, 1408, False), (130, 64, True)])
+def test_ragged(cuda_device, G, M, N, K, glu):
+    from infinilm_b200 import ops
+    off = _layout(G, M, G + N)
+    M = int(off[-1])
+    assert M <= 4 * G                                      # tiles of 16 rows
+    g = torch.Generator().manual_seed(K)
+    a = torch.randn(M + 3, K, generator=g).bfloat16()
+    w = (torch.randn(G, (2 if glu else 1) * N, K, generator=g) * 2 / math.sqrt(K)).bfloat16()
+    rows = torch.randint(0, M + 3, (M,), generator=g, dtype=torch.int32)
+    scale = 0.5 + torch.rand(M + 3, generator=g)
+    out = torch.full((M + 1, N), float("nan"), device="cuda", dtype=torch.bfloat16)
+    ops.gemm_grouped(a.cuda(), w.cuda(), out[:M], group_off=off.to(torch.int32).cuda(), a_rows=rows.cuda(), n_rows=M, glu=glu, row_scale=scale.cuda())
+    for e in range(G):
+        lo, hi = int(off[e]), int(off[e + 1])
+        if lo == hi:
+            continue
+        r = rows[lo:hi].long()
+        y = (a[r].double() @ w[e].double().t()) * scale[r].double()[:, None]
+        if glu:
+            gt, up = y[:, :N].bfloat16().double(), y[:, N:].bfloat16().double()
+            y = gt * torch.sigmoid(gt) * up
+        # rounded to bfloat16 once; with a gate its two products before that
+        assert float((out[lo:hi].cpu().double() - y).abs().amax()) <= (3 if glu else 1) * 2.0 ** -8 * max(float(y.abs().amax()), 1e-3)
+    assert bool(out[M].isnan().all())
+    # the same rows as one group alone, with as many more rows as make the tiles larger
+    e = G // 3
+    lo, hi = int(off[e]), int(off[e + 1])
+    many = torch.cat([rows[lo:hi], rows[:1].expand(60)])
+    alone = torch.empty(len(many), N, device="cuda", dtype=torch.bfloat16)
+    ops.gemm_grouped(a.cuda(), w[e:e + 1].cuda(), alone, group_off=torch.tensor([0, len(many)], dtype=torch.int32, device="cuda"), a_rows=many.cuda(),
+                     n_rows=len(many), glu=glu, row_scale=scale.cuda())
+    assert torch.equal(alone[:hi - lo], out[lo:hi])
+
+
+@pytest.mark.parametrize("M", [1, 15, 16, 17, 32, 33])
+def test_batched(cuda_device, M):
+    from infinilm_b200 import ops
+    G, K, N = 5, 72, 100
+    g = torch.Generator().manual_seed(M)
+    a, w = torch.randn(M, G, K, generator=g).bfloat16(), (torch.randn(G, N, K, generator=g) * 0.2).bfloat16()
+    out = torch.empty(M, G, N, device="cuda", dtype=torch.bfloat16)
+    ops.gemm_grouped(a.cuda(), w.cuda(), out)
+    ref = torch.einsum("mgk,gnk->mgn", a.double(), w.double())
+    assert float((out.cpu().double() - ref).abs().amax()) <= 2.0 ** -8 * float(ref.abs().amax())
