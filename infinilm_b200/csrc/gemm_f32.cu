@@ -4,15 +4,17 @@
 //
 // One order of summation for every shape, so that a row's result is bit-identical whatever else is in the batch: K is cut
 // into chunks of 64; in a chunk the products at even and at odd k are two chains of fused multiply-adds in the order of k
-// (one packed instruction serves both), the chunk's sum is even + odd, and the chunks' sums are added in their order. Chunks
-// are what the kernels below spread over threads: no sum ever waits for K products in a row, and the rounding error is that
-// of chains of 32 and K / 64 instead of one of K.
+// (one packed instruction serves both), the chunk's sum is even + odd, the chunks' sums are added in their order over the first
+// f32_share(K) chunks and over the others, and the two shares' sums are added. Chunks are what the kernels below spread over threads and
+// shares what they spread over blocks: no sum ever waits for K products in a row, and the rounding error is that of chains of 32 and
+// K / 128 (up to 1,024 columns, one share: K / 64) instead of one of K.
 //
 // Up to 16 rows the kernel is bound by the bytes of W (gemm_f32_rows_kernel); beyond, by the FP32 pipes and, where there
 // are few tiles, by how many SMs get one (gemm_f32_tile_kernel).
 #include "common.cuh"
 
 constexpr int F32_CHUNK = 64;
+__host__ __device__ constexpr int f32_share(int K) { return K <= 16 * F32_CHUNK ? 16 : 16 * ((K + 32 * F32_CHUNK - 1) / (32 * F32_CHUNK)); }
 
 __device__ __forceinline__ void f32_cp16(uint32_t dst, const void* src, int bytes) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst), "l"(src), "r"(bytes));
@@ -99,7 +101,7 @@ __global__ void __launch_bounds__(FR_THREADS) gemm_f32_rows_kernel(const float* 
     f32_commit();
 
     const int on = tid & 7, om = tid >> 3;        // the output this thread adds up (om < M)
-    float tot = 0.f;
+    float tot = 0.f, first = 0.f;                 // first: the first share's sum, once it is done (rounds are 16 chunks, shares whole rounds)
     for (int r = 0; r < rounds; ++r) {
         f32_wait<1>();
         __syncthreads();
@@ -129,7 +131,9 @@ __global__ void __launch_bounds__(FR_THREADS) gemm_f32_rows_kernel(const float* 
 #pragma unroll
             for (int i = 0; i < FR_CHUNKS; ++i) tot = __fadd_rn(tot, red[(om * FR_CHUNKS + i) * FR_ROWS + on]);
         }
+        if ((r + 1) * FR_CHUNKS == f32_share(K) && r + 1 < rounds) first = tot, tot = 0.f;
     }
+    tot = __fadd_rn(first, tot);
     if constexpr (GLU) {
         const int n = min(n0 + (on & 3), N - 1);
         const float y = __fmaf_rn(alpha, tot, bias ? bias[on < 4 ? n : N + n] : 0.f), up = __shfl_down_sync(0xffffffffu, y, 4);
@@ -145,32 +149,50 @@ __global__ void __launch_bounds__(FR_THREADS) gemm_f32_rows_kernel(const float* 
 // Eight warps; a warp holds 32 x 32 outputs (a lane 8 x 4: rows l/8 + 4i, columns l%8 + 8j) of one group's chunks, fed by a ring
 // of stages of 16 k for every group, 16-byte asynchronous copies, rows padded to 20 floats (a lane's loads run along k, where the
 // packed multiply-adds want their pairs, and no two lanes of a phase share a bank group). With KG > 1 the groups' chunk sums meet in
-// shared memory after every round of KG chunks and are added in the order of the chunks.
+// shared memory after every round of KG chunks and are added in the order of the chunks. The first share's sums wait for the second's
+// in shared memory or, KG 1, where it has no room for them, in C (the same thread's elements, once over the whole of K). SPLIT: two blocks, a cluster, take a share each and the sums meet through their
+// shared memory, where the tiles leave SMs idle or alone: 800 rows to 1,024
+// columns, K = 4,096, 278 -> 225 us; 61 rows 51 -> 27; 300 rows to 2,048 columns, K = 2,048, 130 -> 115.
 constexpr int FT_BK = 16, FT_RS = FT_BK + 4, FT_THREADS = 256;
 template <int WM, int WN, int KG> struct FtShape {
     static_assert(WM * WN * KG == 8, "eight warps");
     static constexpr int BM = 32 * WM, BN = 32 * WN, STAGES = KG > 1 ? 3 : 4;
     static constexpr int STAGE = KG * (BM + BN) * FT_RS, RSR = BN + 8;
-    static constexpr int SMEM = (STAGES * STAGE + (KG > 1 ? KG * BM * RSR : BM * BN)) * 4;
+    static constexpr int SMEM = (STAGES * STAGE + (KG > 1 ? KG * BM * RSR : 0) + BM * BN) * 4;
     static constexpr int BLOCKS = 2 * SMEM <= 224 * 1024 ? 2 : 1;     // an SM's worth: two where both fit
 };
 
-template <int WM, int WN, int KG, bool VEC>
+__device__ __forceinline__ float f32_peer(uint32_t addr, uint32_t rank) {
+    uint32_t at;
+    float v;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(at) : "r"(addr), "r"(rank));
+    asm volatile("ld.shared::cluster.f32 %0, [%1];\n" : "=f"(v) : "r"(at) : "memory");
+    return v;
+}
+__device__ __forceinline__ void f32_cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+}
+
+// MODE 0: one share; 1: two, one after the other; 2: a cluster's.
+template <int WM, int WN, int KG, int MODE, bool VEC>
 __global__ void __launch_bounds__(FT_THREADS, FtShape<WM, WN, KG>::BLOCKS) gemm_f32_tile_kernel(const float* A, int lda, const float* __restrict__ W, int ldw,
-                                                                   float* __restrict__ C, int ldc, const float* __restrict__ bias, float alpha,
+                                                                   float* C, int ldc, const float* __restrict__ bias, float alpha,
                                                                    int M, int N, int K) {
     using S = FtShape<WM, WN, KG>;
+    constexpr bool SPLIT = MODE == 2;
     constexpr int BM = S::BM, BN = S::BN, ST = S::STAGES, GROUP = (BM + BN) * FT_RS;
     extern __shared__ __align__(16) float sm[];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int g = warp / (WM * WN), wm = warp % (WM * WN) / WN, wn = warp % WN;
     const int lm = lane >> 3, ln = lane & 7;
     const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
-    const int steps = ((K + F32_CHUNK * KG - 1) / (F32_CHUNK * KG)) * (F32_CHUNK / FT_BK);
+    // (shares are whole rounds of KG chunks; a cluster's block z has share z)
+    const int k0 = SPLIT ? (int)blockIdx.z * f32_share(K) * F32_CHUNK : 0, k_own = SPLIT && blockIdx.z == 0 ? f32_share(K) * F32_CHUNK : K - k0;
+    const int steps = ((k_own + F32_CHUNK * KG - 1) / (F32_CHUNK * KG)) * (F32_CHUNK / FT_BK), share_steps = f32_share(K) / KG * (F32_CHUNK / FT_BK);
 
     auto load = [&](int s) {
         const uint32_t base = (uint32_t)__cvta_generic_to_shared(sm + (size_t)(s % ST) * S::STAGE);
-        const int k_round = (s / (F32_CHUNK / FT_BK)) * KG * F32_CHUNK + (s % (F32_CHUNK / FT_BK)) * FT_BK;
+        const int k_round = k0 + (s / (F32_CHUNK / FT_BK)) * KG * F32_CHUNK + (s % (F32_CHUNK / FT_BK)) * FT_BK;
 #pragma unroll
         for (int i = 0; i < KG * (BM + BN) * 4 / FT_THREADS; ++i) {
             const int idx = tid + i * FT_THREADS, gg = idx / ((BM + BN) * 4), rem = idx % ((BM + BN) * 4), row = rem >> 2, q = rem & 3;
@@ -193,6 +215,7 @@ __global__ void __launch_bounds__(FT_THREADS, FtShape<WM, WN, KG>::BLOCKS) gemm_
     // k, and 32 registers fewer let two blocks share an SM. Else outputs tid + 256 i of the tile, in registers.
     constexpr int OUT = BM * BN / FT_THREADS;
     float* red = sm + ST * S::STAGE;              // KG 1: [32][256]; else [KG][BM][RSR]
+    float* first = red + KG * BM * S::RSR;        // KG > 1: this thread's sums of the first share
     float tot[KG > 1 ? OUT : 1];
 #pragma unroll
     for (int i = 0; i < OUT; ++i) {
@@ -254,15 +277,51 @@ __global__ void __launch_bounds__(FT_THREADS, FtShape<WM, WN, KG>::BLOCKS) gemm_
                     }
             }
         }
+        if (MODE == 1 && s + 1 == share_steps && s + 1 < steps) {
+#pragma unroll
+            for (int i = 0; i < OUT; ++i) {
+                if (KG > 1) {
+                    first[i * FT_THREADS + tid] = tot[KG > 1 ? i : 0];
+                    tot[KG > 1 ? i : 0] = 0.f;
+                } else {
+                    const int row = wm * 32 + lm + 4 * (i / 4), col = wn * 32 + ln + 8 * (i % 4);
+                    if (m0 + row < M && n0 + col < N) C[(size_t)(m0 + row) * ldc + n0 + col] = red[i * FT_THREADS + tid];
+                    red[i * FT_THREADS + tid] = 0.f;
+                }
+            }
+        }
     }
     il_pdl_tail();
+    float* mine = KG > 1 ? sm : red;              // SPLIT: this block's sums for the other to read
+    const uint32_t at = (uint32_t)__cvta_generic_to_shared(mine + tid);
+    if (SPLIT) {
+        f32_wait<0>();
+        __syncthreads();                          // (the stages are read)
+        if (KG > 1) {
+#pragma unroll
+            for (int i = 0; i < OUT; ++i) mine[i * FT_THREADS + tid] = tot[KG > 1 ? i : 0];
+        }
+        f32_cluster_sync();
+    }
+    const bool second = MODE == 1 && steps > share_steps;
 #pragma unroll
     for (int i = 0; i < OUT; ++i) {
+        if (SPLIT && (i & 1) != (int)blockIdx.z) continue;     // block z stores every second of a thread's outputs
         const int e = tid + i * FT_THREADS;
         const int row = KG == 1 ? wm * 32 + lm + 4 * (i / 4) : e / BN, col = KG == 1 ? wn * 32 + ln + 8 * (i % 4) : e % BN;
         const int gm = m0 + row, gn = n0 + col;
-        if (gm < M && gn < N) C[(size_t)gm * ldc + gn] = __fmaf_rn(alpha, KG > 1 ? tot[KG > 1 ? i : 0] : red[i * FT_THREADS + tid], bias ? bias[gn] : 0.f);
+        float v = KG > 1 ? tot[KG > 1 ? i : 0] : red[i * FT_THREADS + tid];
+        if (SPLIT) {
+            const float other = f32_peer(at + 4u * i * FT_THREADS, blockIdx.z ^ 1);
+            v = blockIdx.z ? __fadd_rn(other, v) : __fadd_rn(v, other);
+        }
+        if (gm < M && gn < N) {
+            float* c = C + (size_t)gm * ldc + gn;
+            if (second) v = __fadd_rn(KG > 1 ? first[i * FT_THREADS + tid] : *c, v);
+            *c = __fmaf_rn(alpha, v, bias ? bias[gn] : 0.f);
+        }
     }
+    if (SPLIT) f32_cluster_sync();                // (no block leaves while its sums are read)
 }
 
 struct F32Args {
@@ -299,32 +358,64 @@ template <int MT, bool VEC> static cudaError_t f32_launch_rows(const F32Args& a)
     return a.act ? f32_launch_rows_as<MT, VEC, true>(a) : f32_launch_rows_as<MT, VEC, false>(a);
 }
 
-template <int WM, int WN, int KG, bool VEC> static cudaError_t f32_launch_tile(const F32Args& a) {
+template <int WM, int WN, int KG, int MODE, bool VEC> static cudaError_t f32_launch_tile_as(const F32Args& a) {
     using S = FtShape<WM, WN, KG>;
     static bool done[64];
-    cudaError_t e = f32_allow_smem((const void*)gemm_f32_tile_kernel<WM, WN, KG, VEC>, S::SMEM, done);
+    const auto kernel = gemm_f32_tile_kernel<WM, WN, KG, MODE, VEC>;
+    constexpr bool SPLIT = MODE == 2;
+    cudaError_t e = f32_allow_smem((const void*)kernel, S::SMEM, done);
     if (e != cudaSuccess) return e;
-    return il_launch(gemm_f32_tile_kernel<WM, WN, KG, VEC>, dim3((a.N + S::BN - 1) / S::BN, (a.M + S::BM - 1) / S::BM), dim3(FT_THREADS), (size_t)S::SMEM,
-                     a.stream, a.A, a.lda, a.W, a.ldw, a.C, a.ldc, a.bias, a.alpha, a.M, a.N, a.K);
+    const dim3 grid((a.N + S::BN - 1) / S::BN, (a.M + S::BM - 1) / S::BM, SPLIT ? 2 : 1);
+    if (!SPLIT) return il_launch(kernel, grid, dim3(FT_THREADS), (size_t)S::SMEM, a.stream, a.A, a.lda, a.W, a.ldw, a.C, a.ldc, a.bias, a.alpha, a.M, a.N, a.K);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(FT_THREADS);
+    cfg.dynamicSmemBytes = S::SMEM;
+    cfg.stream = a.stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 1, attr[0].val.clusterDim.y = 1, attr[0].val.clusterDim.z = 2;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = il_pdl_enabled() ? 2 : 1;
+    return cudaLaunchKernelEx(&cfg, kernel, a.A, a.lda, a.W, a.ldw, a.C, a.ldc, a.bias, a.alpha, a.M, a.N, a.K);
+}
+template <int WM, int WN, int KG, bool VEC> static cudaError_t f32_launch_tile(const F32Args& a, bool split) {
+    if (split) return f32_launch_tile_as<WM, WN, KG, 2, VEC>(a);
+    return a.K > f32_share(a.K) * F32_CHUNK ? f32_launch_tile_as<WM, WN, KG, 1, VEC>(a) : f32_launch_tile_as<WM, WN, KG, 0, VEC>(a);
 }
 
 template <bool VEC> static cudaError_t f32_dispatch(const F32Args& a) {
     if (a.M <= 16)
         return a.M == 1 ? f32_launch_rows<1, VEC>(a) : a.M == 2 ? f32_launch_rows<2, VEC>(a) : a.M <= 4 ? f32_launch_rows<4, VEC>(a)
              : a.M <= 8 ? f32_launch_rows<8, VEC>(a) : f32_launch_rows<16, VEC>(a);
-    // The tile by what a wave of blocks was measured to take (us for K = 1,024 on a B200): one block on an SM, two on an SM.
+    // The tile, and whether K is cut, by what a wave of blocks was measured to take (us for K = 1,024 on a B200): one block on an SM, two on an SM.
     //   128 x 64: 78, 138    64 x 64 (K in 2): 50, 74    64 x 32 (K in 4): 25, 49    32 x 32 (K in 8): 14, 28
     // Large tiles do more work a byte, small ones give more SMs work: 61 rows to 1,024 columns 78 / 42 / 25 / 14 us, 2,048 rows to
     // 8,192 columns 908 / 954 / 1,309 / 1,425 us (37.9 TFLOP/s; one accumulator a product and plain loads took 389 us and 1.7 ms).
-    const auto cost = [&](int bm, int bn, float one, float two) {
-        const long long tiles = (long long)((a.M + bm - 1) / bm) * ((a.N + bn - 1) / bn), rest = tiles % 296;
-        return (float)(tiles / 296) * two + (rest == 0 ? 0.f : rest <= 148 ? one : two);
-    };
-    const float c0 = cost(128, 64, 78.f, 138.f), c1 = cost(64, 64, 50.f, 74.f), c2 = cost(64, 32, 25.f, 49.f), c3 = cost(32, 32, 14.f, 28.f);
-    if (c3 <= c2 && c3 <= c1 && c3 <= c0) return f32_launch_tile<1, 1, 8, VEC>(a);
-    if (c2 <= c1 && c2 <= c0) return f32_launch_tile<2, 1, 4, VEC>(a);
-    if (c1 <= c0) return f32_launch_tile<2, 2, 2, VEC>(a);
-    return f32_launch_tile<4, 2, 1, VEC>(a);
+    // Cut, there are twice the blocks of half the time and some 5 us a wave for their ends; more than two waves whole are as good.
+    const int share = f32_share(a.K) * F32_CHUNK;
+    const float whole = (float)a.K / 1024.f, part = (float)share / 1024.f;
+    static constexpr int BM[4] = {32, 64, 64, 128}, BN[4] = {32, 32, 64, 64};
+    static constexpr float ONE[4] = {14.f, 25.f, 50.f, 78.f}, TWO[4] = {28.f, 49.f, 74.f, 138.f};
+    int best = -1;
+    float best_us = 0.f;
+    for (int cut = 0; cut < (a.K > share ? 2 : 1); ++cut)
+        for (int i = 0; i < 4; ++i) {
+            const long long tiles = (long long)((a.M + BM[i] - 1) / BM[i]) * ((a.N + BN[i] - 1) / BN[i]), blocks = tiles << cut, rest = blocks % 296;
+            if (cut && tiles > 2 * 296) continue;
+            const float waves = (float)(blocks / 296) * TWO[i] + (rest == 0 ? 0.f : rest <= 148 ? ONE[i] : TWO[i]);
+            const float us = cut ? waves * part + 5.f * (float)((blocks + 295) / 296) : waves * whole;
+            if (best < 0 || us < best_us) best = cut * 4 + i, best_us = us;
+        }
+    const bool split = best >= 4;
+    switch (best & 3) {
+        case 0: return f32_launch_tile<1, 1, 8, VEC>(a, split);
+        case 1: return f32_launch_tile<2, 1, 4, VEC>(a, split);
+        case 2: return f32_launch_tile<2, 2, 2, VEC>(a, split);
+        default: return f32_launch_tile<4, 2, 1, VEC>(a, split);
+    }
 }
 
 // act: 0, or the gate of a gated product (M <= 16): W is [2N, K], gate rows, then up rows, bias [2N].
