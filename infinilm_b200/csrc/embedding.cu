@@ -24,7 +24,7 @@ __global__ void embed_kernel(const int* __restrict__ ids, const TW* __restrict__
 
 // The same in 16-byte pieces, one a thread (256 x 16 bytes of a row a block): element by element a row of 4,096 was sixteen loads of 2
 // bytes a thread on as many SMs as the step has tokens. Bound by latency in a decode step; with the wider blocks of embed_pair_pos below 32 steps of 8
-// requests of a model 2,048 wide (4 layers of 64 experts) went from 25.91 to 25.75 ms, 8 of a model 4,096 wide from 112.1 to 111.0 on average.
+// requests of a model 2,048 wide (4 layers of 64 experts) went from 25.91 to 25.75 ms; at 4,096 wide the step's time did not change measurably.
 template <typename TW>
 __global__ void __launch_bounds__(256) embed_vec_kernel(const int* __restrict__ ids, const TW* __restrict__ table, float scale,
                                                         float* __restrict__ out, int H, int V, int round_bf16) {
