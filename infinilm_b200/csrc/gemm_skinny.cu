@@ -145,7 +145,7 @@ __host__ __device__ constexpr bool gs_gated(int glu) { return glu >= IL_ACT_SILU
 // NT: 8-row groups of x (1: M <= 8, 2: M <= 16). GLU: 0 plain, 4 plain with relu(.)^2, 5 plain with gelu_tanh(.) * a table's row; 1 SwiGLU, 2 the same with the tanh form of GELU as the gate, 3 with the clamped gate (act_limit, act_alpha) (W holds N gate rows, then N up rows). U: blocks in flight.
 // NRM: the activations may come without their norm's 1/rms (`ni`); the SwiGLU form always can, the plain form as a variant of its own.
 template <int NT, int GLU, int U, typename TO, bool NRM, bool EARLY>
-__global__ void __launch_bounds__(GS_WARPS * 32, EARLY && NT == 1 && U == 4 ? 4 : 2) gemm_skinny_kernel(const __nv_bfloat16* __restrict__ x, int ldx,
+__global__ void __launch_bounds__(GS_WARPS * 32, EARLY && NT == 1 && U == 4 ? 4 : 2) gemm_skinny_kernel(const __nv_bfloat16* x, int ldx,
                                                                     const __nv_bfloat16* __restrict__ W, int ldw, TO* __restrict__ out,
                                                                     int ldo, const float* __restrict__ bias, float alpha, int M, int N, int K,
                                                                     const GsNormIn ni, float act_limit, float act_alpha, const GsRowMul rm) {
@@ -456,7 +456,7 @@ IL_EXPORT int il_gemm_skinny_rope(const void* x, int ldx, const void* W, int ldw
 // place); xw = resid * norm_w as bfloat16; sumsq[m][block] = sum of resid^2 over the block's 16 columns. N = the width of
 // the residual stream. What add_rmsnorm does, but for the division by the rms, which the next product applies.
 template <int NT, int U, int WARPS, bool EARLY>
-__global__ void __launch_bounds__(WARPS * 32, WARPS > 8 ? 1 : 2) gemm_skinny_resid_kernel(const __nv_bfloat16* __restrict__ x, int ldx,
+__global__ void __launch_bounds__(WARPS * 32, WARPS > 8 ? 1 : 2) gemm_skinny_resid_kernel(const __nv_bfloat16* x, int ldx,
                                                                           const __nv_bfloat16* __restrict__ W, int ldw,
                                                                           const float* __restrict__ bias, float alpha, int M, int N, int K,
                                                                           float* resid, float bscale, const void* __restrict__ norm_w,

@@ -1,0 +1,45 @@
+"""Kernels that may become resident while the kernel in front still runs: what that kernel writes is never read through a
+`const __restrict__` pointer, whose loads the compiler may move above the wait (checked in the sources, no GPU)."""
+import os
+import re
+
+import pytest
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "infinilm_b200", "csrc")
+# Parameters that no kernel of a step writes: weights and tables of the model (and of a request's sampling), and the step's descriptors,
+# which the host copies to the device.
+WRITTEN_LONG_BEFORE = {
+    "W", "w", "bias", "norm_w", "w_a", "w_b", "wq", "wk", "wb", "wn", "corr", "sink", "dist_bias", "table", "pair_table", "inv_freq", "freq", "decay",
+    "A_log", "dt_bias", "mix", "out_w", "in_next", "vec",
+    "temperature", "top_k", "top_p", "uniform",
+    "tok_pos", "tok_entry", "block_table", "entry_qstart", "entry_kvlen", "qstart", "read_slots", "write_slots", "rows", "src_idx",
+}
+WAIT = re.compile(r"il_pdl_wait|il_pdl_begin|sm_small_begin|gs_begin|griddepcontrol\.wait")
+KERNEL = re.compile(r"__global__\s+void\s+(?:__launch_bounds__\((?:[^()]|\([^()]*\))*\)\s*)?(\w+)\s*\(([^{]*?)\)\s*\{", re.S)
+FILES = ["gemm_skinny.cu"]
+
+
+def _waiting_kernels(name):
+    with open(os.path.join(CSRC, name), encoding="utf-8") as fh:
+        text = re.sub(r"//[^\n]*", "", fh.read())
+    for m in KERNEL.finditer(text):
+        at, depth = m.end(), 1
+        while depth:
+            depth += {"{": 1, "}": -1}.get(text[at], 0)
+            at += 1
+        if WAIT.search(text[m.end():at]):
+            yield m.group(1), m.group(2)
+
+
+@pytest.mark.parametrize("name", FILES)
+def test_what_the_kernel_in_front_writes_is_not_read_only(name):
+    found, bad = 0, []
+    for kernel, params in _waiting_kernels(name):
+        found += 1
+        for p in params.split(","):
+            if "__restrict__" in p and re.search(r"\bconst\b", p):
+                arg = re.search(r"(\w+)\s*$", p).group(1)
+                if arg not in WRITTEN_LONG_BEFORE:
+                    bad.append(f"{kernel}: {arg}")
+    assert found, "no kernel with a wait was found"
+    assert not bad, bad

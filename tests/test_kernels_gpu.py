@@ -708,3 +708,46 @@ def test_gemm_mid_swiglu(cuda_device, M, I, K, bm, nb):
     act = torch.empty(M, I, device="cuda", dtype=torch.bfloat16)
     ops.swiglu(gu, act)
     close(out, act.float(), "bfloat16")
+
+
+@pytest.mark.parametrize("M,I", [(9, 4096), (16, 4096), (13, 8192), (8, 8192), (3, 4104)])
+def test_replayed_chain_of_products_that_let_the_next_one_in(cuda_device, M, I):
+    """Gate+up, whose kernel lets the next one in right after its own wait, and the product into the residual, whose later rounds read
+    what gate+up wrote: a replayed chain over the same buffers gives the bits of the same launches one at a time."""
+    g = torch.Generator(device="cuda").manual_seed(M)
+    H, L = 1024, 6
+    gu = [(torch.randn(2 * I, H, device="cuda", generator=g) / 16).bfloat16() for _ in range(L)]
+    down = [(torch.randn(H, I, device="cuda", generator=g) / math.sqrt(I)).bfloat16() for _ in range(L)]
+    nw = torch.ones(H, device="cuda")
+    resid, xw = torch.empty(M, H, device="cuda"), torch.empty(M, H, device="cuda", dtype=torch.bfloat16)
+    sq, act = torch.empty(M, H // 16, device="cuda"), torch.empty(M, I, device="cuda", dtype=torch.bfloat16)
+    first = torch.empty(M, H, device="cuda")
+
+    def chain(alone):
+        resid.copy_(first)
+        xw.copy_(first)
+        sq.copy_((first * first).view(M, -1, 16).sum(-1))
+        for i in range(L):
+            ops.gemm_skinny(xw, gu[i], act, glu=1, norm_in=ops.NormedInput(xw, sq, H, 1e-5), w_static=True)
+            if alone:
+                torch.cuda.synchronize()
+            ops.gemm_skinny_resid(act, down[i], 1.0, None, resid, 0.5, nw, 1e-5, xw, sq, w_static=True)
+            if alone:
+                torch.cuda.synchronize()
+
+    first.copy_(torch.randn(M, H, device="cuda", generator=g))
+    stream = torch.cuda.Stream()
+    stream.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(stream):
+        chain(True)
+    torch.cuda.current_stream().wait_stream(stream)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        chain(False)
+    for _ in range(20):
+        first.copy_(torch.randn(M, H, device="cuda", generator=g))
+        chain(True)
+        want = (resid.clone(), xw.clone(), act.clone())
+        act.fill_(3.0)
+        graph.replay()
+        assert torch.equal(resid, want[0]) and torch.equal(xw, want[1]) and torch.equal(act, want[2])
