@@ -161,12 +161,12 @@ __device__ __forceinline__ void ad_merge_row(float* fs, float* comb, const float
     __syncwarp();
 }
 
-// (qkv, and o_part / ml_part in the merge, are written by the kernel before and read after a wait that is not the
+// (qkv, the newest token's slot of the cache, and o_part / ml_part in the merge, are written by the kernel before and read after a wait that is not the
 // kernel's first statement: they are not declared __restrict__, so that no load of them is treated as read-only
 // data and scheduled above the wait.)
 template <bool SIG, bool CAP>
 __global__ void __launch_bounds__(AD_WARPS * 32) attn_decode_kernel(
-    const __nv_bfloat16* qkv, int row_stride, const __nv_bfloat16* __restrict__ cache,
+    const __nv_bfloat16* qkv, int row_stride, const __nv_bfloat16* cache,
     const int* __restrict__ block_table, int bt_stride, const int* __restrict__ entry_kvlen, int nh, int nkv,
     float scale_log2, int window, int pages_per_split, int n_splits, float* __restrict__ o_part,
     float* __restrict__ ml_part, const __grid_constant__ CUtensorMap kv_map, const __grid_constant__ CUtensorMap kv_page_map,

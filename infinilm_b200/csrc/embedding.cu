@@ -4,7 +4,7 @@
 #include "common.cuh"
 
 template <typename TW>
-__global__ void embed_kernel(const int* __restrict__ ids, const TW* __restrict__ table, float scale,
+__global__ void embed_kernel(const int* ids, const TW* __restrict__ table, float scale,
                              float* __restrict__ out, int H, int V, int round_bf16) {
     il_pdl_begin();
     const int t = blockIdx.x;
@@ -26,7 +26,7 @@ __global__ void embed_kernel(const int* __restrict__ ids, const TW* __restrict__
 // bytes a thread on as many SMs as the step has tokens. Bound by latency in a decode step; with the wider blocks of embed_pair_pos below 32 steps of 8
 // requests of a model 2,048 wide (4 layers of 64 experts) went from 25.91 to 25.75 ms; at 4,096 wide the step's time did not change measurably.
 template <typename TW>
-__global__ void __launch_bounds__(256) embed_vec_kernel(const int* __restrict__ ids, const TW* __restrict__ table, float scale,
+__global__ void __launch_bounds__(256) embed_vec_kernel(const int* ids, const TW* __restrict__ table, float scale,
                                                         float* __restrict__ out, int H, int V, int round_bf16) {
     constexpr int VEC = 16 / sizeof(TW);
     il_pdl_begin();
@@ -77,7 +77,7 @@ IL_EXPORT int il_embed(const int* ids, const void* table, int table_kind, float 
 // token_ids[rows[i]] = src[src_idx[i]]: puts tokens that were sampled on the device (and not read by the host yet)
 // into the next step's token list. Out-of-vocabulary values are caught by the gather above.
 __global__ void patch_tokens_kernel(int* __restrict__ token_ids, const int* __restrict__ rows, const int* __restrict__ src_idx,
-                                    const int* __restrict__ src, int n) {
+                                    const int* src, int n) {
     il_pdl_begin();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) token_ids[rows[i]] = src[src_idx[i]];
@@ -97,7 +97,7 @@ IL_EXPORT int il_patch_tokens(int* token_ids, const int* rows, const int* src_id
 // 0: none); the block of that first token reads it and then writes the entry's last token there, so the read of an entry
 // always comes before its write, and no other block touches the slot.
 template <typename TW>
-__global__ void embed_pair_pos_kernel(const int* __restrict__ ids, const int* __restrict__ tok_pos, const int* __restrict__ tok_entry,
+__global__ void embed_pair_pos_kernel(const int* ids, const int* __restrict__ tok_pos, const int* __restrict__ tok_entry,
                                       const int* __restrict__ entry_qstart, const TW* __restrict__ table, float scale,
                                       const TW* __restrict__ pair_table, int buckets, long long mul_prev, long long mul_cur,
                                       int* prev_state, const int* __restrict__ read_slots, const int* __restrict__ write_slots,

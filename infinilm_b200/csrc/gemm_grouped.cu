@@ -32,10 +32,10 @@ template <int BM, bool GLU> constexpr int smem_bytes() { return STAGES * (BM + (
 }  // namespace ggm
 
 template <int BM, bool GLU>
-__global__ void __launch_bounds__(128) gemm_grouped_mma_kernel(const __nv_bfloat16* A, int lda, long long a_gs, const int* __restrict__ a_rows,
+__global__ void __launch_bounds__(128) gemm_grouped_mma_kernel(const __nv_bfloat16* A, int lda, long long a_gs, const int* a_rows,
                                                                const __nv_bfloat16* __restrict__ W, int ldw, long long w_gs,
                                                                __nv_bfloat16* __restrict__ C, int ldc, long long c_gs,
-                                                               const int* __restrict__ group_off, int n_groups, int M, int N, int K,
+                                                               const int* group_off, int n_groups, int M, int N, int K,
                                                                const __nv_bfloat16* gate, int ld_gate, long long gate_gs, int gate_ns, const float* row_scale,
                                                                int scale_by_place) {
     using namespace ggm;
@@ -213,9 +213,9 @@ __global__ void __launch_bounds__(128) gemm_grouped_mma_kernel(const __nv_bfloat
 }
 
 template <typename TA, bool GLU>
-__global__ void __launch_bounds__(256) gemm_grouped_kernel(const TA* A, int lda, long long a_gs, const int* __restrict__ a_rows,
+__global__ void __launch_bounds__(256) gemm_grouped_kernel(const TA* A, int lda, long long a_gs, const int* a_rows,
                                                            const TA* __restrict__ W, int ldw, long long w_gs, TA* __restrict__ C, int ldc,
-                                                           long long c_gs, const int* __restrict__ group_off, int n_groups, int M, int N,
+                                                           long long c_gs, const int* group_off, int n_groups, int M, int N,
                                                            int K, const TA* gate, int ld_gate, long long gate_gs, int gate_ns, const float* row_scale,
                                                            int scale_by_place) {
     constexpr int BM = 64, BN = 64, BK = 16, TM = 4, TN = 4;

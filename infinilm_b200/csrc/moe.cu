@@ -229,7 +229,7 @@ __global__ void __launch_bounds__(WARPS * 32) moe_route_kernel(const TA* x, int 
 // The choice alone, for logits that a matrix product has written already (z [T, ldz] f32, the bias still to be added):
 // a warp a token, its row of logits in shared memory.
 template <int WARPS>
-__global__ void __launch_bounds__(WARPS * 32) moe_select_kernel(const float* __restrict__ z, int ldz, const void* __restrict__ bias, int b_kind,
+__global__ void __launch_bounds__(WARPS * 32) moe_select_kernel(const float* z, int ldz, const void* __restrict__ bias, int b_kind,
                                                                int* __restrict__ idx, float* __restrict__ wt, int T, int E, int top, int rule,
                                                                float out_scale) {
     extern __shared__ __align__(16) float sm[];   // [WARPS][E]

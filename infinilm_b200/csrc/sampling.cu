@@ -29,7 +29,7 @@ __device__ __forceinline__ int sp_block_sum_int(int v, int* sh) {
     return t;
 }
 
-__global__ void __launch_bounds__(SP_THREADS) sample_kernel(const float* __restrict__ logits, int ld, int V,
+__global__ void __launch_bounds__(SP_THREADS) sample_kernel(const float* logits, int ld, int V,
                                                             const float* __restrict__ temperature,
                                                             const int* __restrict__ top_k, const float* __restrict__ top_p,
                                                             const float* __restrict__ uniform, int* __restrict__ out) {

@@ -1037,7 +1037,7 @@ IL_EXPORT int il_matrix_state_scan(int mode, const float* q, const float* k, con
 template <typename TG, typename TO>
 __global__ void group_norm_gate_kernel(const float* x, int ldx, const void* __restrict__ w, int w_kind, int n_w, float eps,
                                        const TG* gate, int ldg, int g_off, int act, TO* __restrict__ out, int ldo, int group,
-                                       const float* __restrict__ den_floor, float x_scale, float den_eps) {
+                                       const float* den_floor, float x_scale, float den_eps) {
     __shared__ float red[32];
     sm_small_begin();
     const int t = blockIdx.x, j0 = blockIdx.y * group;

@@ -73,7 +73,7 @@ __global__ void relu2_kernel(const TA* z, TA* out, size_t total_vec) {
 
 // out[t, n] = gelu_tanh(z[t, n]) * table[ids[t], off + n] for n < dim, 0 for dim <= n < ldo: a token's own row of a table, gated (z f32).
 template <typename TA>
-__global__ void gelu_row_kernel(const float* z, int ldz, const int* __restrict__ ids, const TA* __restrict__ table, int ldt, int off, int dim, int vocab,
+__global__ void gelu_row_kernel(const float* z, int ldz, const int* ids, const TA* __restrict__ table, int ldt, int off, int dim, int vocab,
                                 TA* __restrict__ out, int ldo, unsigned total) {
     il_pdl_wait();
     const unsigned stride = gridDim.x * blockDim.x;
@@ -102,7 +102,7 @@ __device__ __forceinline__ void gr_st4(__nv_bfloat16* p, float4 v) {
     *reinterpret_cast<uint2*>(p) = make_uint2(*reinterpret_cast<const uint32_t*>(&a), *reinterpret_cast<const uint32_t*>(&b));
 }
 template <typename TA>
-__global__ void gelu_row4_kernel(const float* z, int ldz, const int* __restrict__ ids, const TA* __restrict__ table, int ldt, int off, int dim, int vocab,
+__global__ void gelu_row4_kernel(const float* z, int ldz, const int* ids, const TA* __restrict__ table, int ldt, int off, int dim, int vocab,
                                  TA* __restrict__ out, int ldo, unsigned total4) {
     il_pdl_wait();
     const unsigned stride = gridDim.x * blockDim.x, ld4 = (unsigned)ldo >> 2;
