@@ -163,10 +163,12 @@ static inline int sm_grid(size_t total, int threads) {
 
 // write_slots (may be null): entries that bring a single token get their state moved on by this kernel; the others (and
 // all of them, without write_slots) by il_short_conv_state.
+// w_static: the taps and the step's descriptors were written long before, not by the kernel in front of this one in the stream: the tiled
+// form, which reads them before its wait, is then launched to overlap with that kernel, else as an ordinary launch.
 IL_EXPORT int il_short_conv(const void* x, int x_kind, int ldx, int x_off, const float* w, int taps, float* state,
                             long long slot_stride, int st_off, int st_ld, const int* read_slots, const int* write_slots, const int* tok_entry,
                             const int* qstart, void* out, int out_kind, int ldo, int out_off, int n_seg, int seg_in, int n_seg2, int seg_in2,
-                            int seg_out, int act, int T, cudaStream_t stream) {
+                            int seg_out, int act, int T, int w_static, cudaStream_t stream) {
     if (T <= 0 || n_seg <= 0) return IL_OK;
     if (taps < 1 || taps > SM_MAX_TAPS || seg_in <= 0 || seg_out < seg_in || n_seg2 < 0 || (n_seg2 > 0 && (seg_in2 <= 0 || seg_out < seg_in2)))
         return IL_BAD_ARG;
@@ -178,9 +180,11 @@ IL_EXPORT int il_short_conv(const void* x, int x_kind, int ldx, int x_off, const
         // 23.6 -> 21.3 ms for eight requests with 32 new tokens on Gopitar).
         const int per = T <= 64 ? 1 : 8;
         const dim3 tgrid((cols_all + 127) / 128, (T + per - 1) / per);
+        cudaError_t e = cudaSuccess;
 #define SC_TILE2(TI_, TO_, TAPS_, TT_)                                                                                                               \
-        IL_LAUNCH((short_conv_tile_kernel<TI_, TO_, TAPS_, TT_>), tgrid, 128, 0, stream, (const TI_*)x, ldx, x_off, w, state, (size_t)slot_stride, st_off, \
-                  st_ld, read_slots, write_slots, tok_entry, qstart, (TO_*)out, ldo, out_off, n_seg, seg_in, n_seg2, seg_in2, seg_out, act, T)
+        e = il_launch_as(w_static != 0, short_conv_tile_kernel<TI_, TO_, TAPS_, TT_>, tgrid, dim3(128), 0, stream, (const TI_*)x, ldx, x_off, w, state, \
+                         (size_t)slot_stride, st_off, st_ld, read_slots, write_slots, tok_entry, qstart, (TO_*)out, ldo, out_off, n_seg, seg_in, n_seg2, \
+                         seg_in2, seg_out, act, T)
 #define SC_TILE(TI_, TO_, TAPS_)                                                                           \
         do {                                                                                               \
             if (per == 1) SC_TILE2(TI_, TO_, TAPS_, 1); else SC_TILE2(TI_, TO_, TAPS_, 8);                 \
@@ -196,6 +200,7 @@ IL_EXPORT int il_short_conv(const void* x, int x_kind, int ldx, int x_off, const
         else if (x_kind == IL_BF16 && out_kind == IL_F32) { SC_TAPS(__nv_bfloat16, float) }
         else if (x_kind == IL_BF16 && out_kind == IL_BF16) { SC_TAPS(__nv_bfloat16, __nv_bfloat16) }
         else return IL_BAD_ARG;
+        if (e != cudaSuccess) return 1000 + (int)e;
         IL_LAUNCH_CHECK();
         return IL_OK;
     }
@@ -435,7 +440,7 @@ __global__ void __launch_bounds__(SR_THREADS) matrix_state_scan_reg_kernel(
         q0 = qstart[e];
         n = qstart[e + 1] - q0;
     }
-    if (SR_CHUNK == 1) sm_small_begin();          // (the form for single tokens is launched to overlap with the kernel in front)
+    if (SR_CHUNK == 1) sm_small_begin();          // (the form for single tokens is launched to overlap with the kernel in front, where that one wrote none of the above)
     if (n <= 0) return;
     const int hq = h / (H / G);
     const bool live = c < vdim;
@@ -663,11 +668,11 @@ __global__ void __launch_bounds__(SR_THREADS) matrix_state_scan_reg_kernel(
 }
 
 template <int MODE, int DPT, int CH, int MS>
-static void sr_launch(dim3 grid, size_t smem, cudaStream_t stream, const float* q, const float* k, const float* v, int ld_q, int ld_k, int ld_v,
+static void sr_launch(dim3 grid, size_t smem, bool w_static, cudaStream_t stream, const float* q, const float* k, const float* v, int ld_q, int ld_k, int ld_v,
                       int H, int G, int dim, int vdim, int in_act, const float* decay, const float* beta, const float* gdec, float* state,
                       size_t slot_stride, const int* read_slots, const int* write_slots, const int* qstart, float* out, int ldo, int log_split,
                       int e0, int n_ent, int seg_len, float* seg_state, int ld_g) {
-    il_launch_as(CH == 1, matrix_state_scan_reg_kernel<MODE, DPT, CH, MS>, grid, dim3(SR_THREADS), smem, stream, q, k, v, ld_q, ld_k, ld_v, H, G, dim, vdim,
+    il_launch_as(CH == 1 && w_static, matrix_state_scan_reg_kernel<MODE, DPT, CH, MS>, grid, dim3(SR_THREADS), smem, stream, q, k, v, ld_q, ld_k, ld_v, H, G, dim, vdim,
                  in_act, decay, beta, gdec, state, slot_stride, read_slots, write_slots, qstart, out, ldo, log_split, e0, n_ent, seg_len, seg_state, ld_g);
 }
 
@@ -925,7 +930,9 @@ IL_EXPORT int il_matrix_state_scan(int mode, const float* q, const float* k, con
                                    int dim, int vdim, int in_act, const float* decay, const float* beta, const float* gdec, float* state,
                                    long long slot_stride, const int* read_slots, const int* write_slots, const int* qstart, int E,
                                    float* out, int ldo, int generic, int e0, int single, int seg_len, int n_tiles, float* seg_state,
-                                   int ld_g, cudaStream_t stream) {
+                                   int ld_g, int w_static, cudaStream_t stream) {
+    // w_static: decays and descriptors (slots, qstart) were written long before, not by the kernel in front of this one in the stream: the
+    // form for single tokens is then launched to overlap with that kernel, else as an ordinary launch.
     // mode 4: `gdec` holds the decays per token and key channel (float32 rows of H * dim, row stride ld_g), `decay` the bonus
     // [H, dim]; G = H.
     if (E <= 0) return IL_OK;
@@ -972,7 +979,7 @@ IL_EXPORT int il_matrix_state_scan(int mode, const float* q, const float* k, con
         const int ch = single ? 1 : 8;
         const size_t smem_r = ((size_t)ch * ((mode == 4 ? 3 : 2) * ((dpt + 4) << log_split) + cpb) + ((2 * ch + 3) & ~3)) * sizeof(float);
         const dim3 grid_r(seg_len > 0 ? n_tiles : E, H, (vdim + cpb - 1) / cpb);
-#define SR_ARGS grid_r, smem_r, stream, q, k, v, ld_q, ld_k, ld_v, H, G, dim, vdim, in_act, decay, beta, gdec, state, (size_t)slot_stride, \
+#define SR_ARGS grid_r, smem_r, w_static != 0, stream, q, k, v, ld_q, ld_k, ld_v, H, G, dim, vdim, in_act, decay, beta, gdec, state, (size_t)slot_stride, \
                 read_slots, write_slots, qstart, out, ldo, log_split, e0, E, seg_len, seg_state, ld_g
         // (the widest split a variant is built for sizes its staging registers: 8 lanes up to dim = 8 DPT, 16 beyond)
 #define SR_PICK(MODE_, DPT_)                                                                                     \

@@ -1497,13 +1497,16 @@ def _i32(name: str, *ts: torch.Tensor) -> None:
 
 def short_conv(x: torch.Tensor, x_off: int, w: torch.Tensor, state: torch.Tensor, st_off: int, read_slots: torch.Tensor,
                tok_entry: torch.Tensor, entry_qstart: torch.Tensor, out: torch.Tensor, out_off: int, n_seg: int, seg_in: int,
-               seg_out: int, act: int = 0, n_seg2: int = 0, seg_in2: int = 0, write_slots: Optional[torch.Tensor] = None) -> None:
+               seg_out: int, act: int = 0, n_seg2: int = 0, seg_in2: int = 0, write_slots: Optional[torch.Tensor] = None,
+               w_static: bool = False) -> None:
     """Causal convolution over time of n_seg * seg_in (+ n_seg2 * seg_in2) channels of `x` (columns from x_off), per channel,
     with weights w float32 [channels, taps] whose last column meets the current token. Inputs before a step's first row come
     from `state` (float32 [slots, taps-1, all channels], this call's channels from column st_off; slot read_slots[entry]).
     Written to `out` from column out_off as segments of seg_out columns each, the surplus zero. act 1: silu.
     `write_slots`: entries that bring ONE token have their state moved on here, in slot write_slots[entry] (the thread that
-    reads such an entry's state is the only one that does); `short_conv_state` then only has the other entries to do."""
+    reads such an entry's state is the only one that does); `short_conv_state` then only has the other entries to do.
+    w_static: w and the step's descriptors (slots, entries, starts) are not what the kernel launched just before writes, and may be read
+    while that kernel still runs."""
     _need_cuda(x, w, state, read_slots, tok_entry, entry_qstart, out, write_slots)
     _i32("short_conv", read_slots, tok_entry, entry_qstart)
     if write_slots is not None:
@@ -1519,10 +1522,10 @@ def short_conv(x: torch.Tensor, x_off: int, w: torch.Tensor, state: torch.Tensor
         raise KernelError("short_conv: column ranges do not fit")
     f = _fn("seqmix", "il_short_conv", [_c_void_p, _c_int, _c_int, _c_int, _c_void_p, _c_int, _c_void_p, _c_ll, _c_int, _c_int,
                                         _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_int, _c_int, _c_int, _c_int, _c_int,
-                                        _c_int, _c_int, _c_int, _c_int, _c_int, _c_void_p])
+                                        _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_void_p])
     _check(f(_ptr(x), kind_of(x.dtype), x.stride(0), x_off, _ptr(w), taps, _ptr(state), state.stride(0), st_off, state.shape[2],
              _ptr(read_slots), _ptr(write_slots if taps > 1 else None), _ptr(tok_entry), _ptr(entry_qstart), _ptr(out), kind_of(out.dtype),
-             out.stride(0), out_off, n_seg, seg_in, n_seg2, seg_in2, seg_out, act, T, _stream()), "short_conv")
+             out.stride(0), out_off, n_seg, seg_in, n_seg2, seg_in2, seg_out, act, T, int(w_static), _stream()), "short_conv")
 
 
 def short_conv_state(x: torch.Tensor, x_off: int, n_channels: int, taps: int, state: torch.Tensor, st_off: int,
@@ -1570,7 +1573,8 @@ def matrix_state_scan(mode: int, q: torch.Tensor, k: torch.Tensor, v: torch.Tens
                       vdim: int, in_act: int, decay: Optional[torch.Tensor], beta: Optional[torch.Tensor],
                       gdec: Optional[torch.Tensor], state: torch.Tensor, read_slots: torch.Tensor, write_slots: torch.Tensor,
                       entry_qstart: torch.Tensor, n_entries: int, out: torch.Tensor, generic: bool = False, first_entry: int = 0,
-                      single: bool = False, seg_len: int = 0, n_tiles: int = 0, seg_state: Optional[torch.Tensor] = None) -> None:
+                      single: bool = False, seg_len: int = 0, n_tiles: int = 0, seg_state: Optional[torch.Tensor] = None,
+                      w_static: bool = False) -> None:
     """A recurrence over a float32 state S [dim, vdim] per (request, head), token by token in each entry's order.
     SCAN_DECAY: S = decay[h] S + k v^T, o = S^T q. SCAN_DELTA: S = g S; u = beta (v - S^T k); S += k u^T; o = S^T q.
     SCAN_GATED: S = g S + beta k [v, 1]^T, o = S^T q with g, beta per token and head (`gdec`, `beta`); the state and the output
@@ -1584,7 +1588,9 @@ def matrix_state_scan(mode: int, q: torch.Tensor, k: torch.Tensor, v: torch.Tens
     first_entry + n_entries - 1 are run; `single`: each of them brings one token (the form made for decoding).
     seg_len > 0 (SCAN_DECAY, key sizes up to 256): every entry's tokens are walked in segments of seg_len at once, each from
     nothing, and two more launches add what the state at a segment's start contributes (the sum is linear in it);
-    `n_tiles` bounds the number of segments, `seg_state` is float32 scratch of n_tiles * heads * vdim * dim."""
+    `n_tiles` bounds the number of segments, `seg_state` is float32 scratch of n_tiles * heads * vdim * dim.
+    w_static (`single`): decay and the descriptors (slots, starts) are not what the kernel launched just before writes, and may be read
+    while that kernel still runs."""
     _need_cuda(q, k, v, decay, beta, gdec, state, read_slots, write_slots, entry_qstart, out)
     _i32("matrix_state_scan", read_slots, write_slots, entry_qstart)
     for t in (q, k, v, out, state):
@@ -1609,11 +1615,11 @@ def matrix_state_scan(mode: int, q: torch.Tensor, k: torch.Tensor, v: torch.Tens
     f = _fn("seqmix", "il_matrix_state_scan", [_c_int, _c_void_p, _c_void_p, _c_void_p, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int,
                                                _c_int, _c_int, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_ll, _c_void_p, _c_void_p,
                                                _c_void_p, _c_int, _c_void_p, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_void_p,
-                                               _c_void_p])
+                                               _c_int, _c_int, _c_void_p])
     _check(f(mode, _ptr(q), _ptr(k), _ptr(v), q.stride(0), k.stride(0), v.stride(0), n_heads, n_qk_heads, dim, vdim, in_act,
              _ptr(decay), _ptr(beta), _ptr(gdec), _ptr(state), state.stride(0), _ptr(read_slots), _ptr(write_slots),
              _ptr(entry_qstart), n_entries, _ptr(out), out.stride(0), int(generic), first_entry, int(single), seg_len, n_tiles,
-             _ptr(seg_state), ld_g, _stream()), "matrix_state_scan")
+             _ptr(seg_state), ld_g, int(w_static), _stream()), "matrix_state_scan")
     if seg_len > 0:
         count_launches(2)                         # the segments' ends and the second pass
 
@@ -1629,7 +1635,7 @@ def matrix_state_scan_step(ctx, *args, **kw) -> None:
     once (`SCAN_SEGMENT` tokens; the choice rests on the step's shape alone, so a replayed step makes it the same way)."""
     n_dec, E = ctx.n_decode, ctx.n_entries
     if n_dec > 0:
-        matrix_state_scan(*args, n_entries=n_dec, first_entry=0, single=True, **kw)
+        matrix_state_scan(*args, n_entries=n_dec, first_entry=0, single=True, w_static=True, **kw)
     if E > n_dec:
         mode, dim, vdim, n_heads = args[0], args[6], args[7], args[4]
         if not kw.get("generic") and scan_in_segments(ctx, mode, dim):

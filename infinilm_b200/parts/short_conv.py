@@ -47,7 +47,7 @@ class ShortConv:
             raise ValueError("short convolution: the segments do not add up to the channels")
         wr = state.write_slots if state.writable else None
         ops.short_conv(x, x_off, self.weight, state.storage, 0, state.read_slots, ctx.tok_entry, ctx.entry_qstart, out, 0, n1, s1, so, act,
-                       n_seg2=n2, seg_in2=s2, write_slots=wr)
+                       n_seg2=n2, seg_in2=s2, write_slots=wr, w_static=True)
         if wr is not None and ctx.n_entries > ctx.n_decode:
             ops.short_conv_state(x, x_off, self.channels, self.taps, state.storage, 0, state.read_slots, wr, ctx.entry_qstart,
                                  ctx.n_entries - ctx.n_decode, first_entry=ctx.n_decode)

@@ -45,3 +45,13 @@ def test_what_the_kernel_in_front_writes_is_not_read_only(name):
 
 def test_the_kernels_are_found():
     assert sum(1 for name in FILES for _ in _waiting_kernels(name)) >= 50
+
+
+@pytest.mark.parametrize("op", ["gemm_f32", "gemm_skinny", "gemm_skinny_resid", "gemm_skinny_rope", "gemm_skinny_gelu_row", "latent_norm_store",
+                                "short_conv", "matrix_state_scan"])
+def test_reading_before_the_wait_is_for_the_caller_to_allow(op):
+    """Kernels that read weights before their wait overlap with the kernel in front only where the caller says that it wrote none of them."""
+    import inspect
+
+    from infinilm_b200 import ops
+    assert inspect.signature(getattr(ops, op)).parameters["w_static"].default is False

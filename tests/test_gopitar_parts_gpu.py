@@ -221,6 +221,47 @@ def test_short_conv_one_token_a_thread_and_eight(cuda_device, last):
         a += n
 
 
+def test_taps_and_decays_from_the_kernel_in_front(cuda_device):
+    """Taps and decays that the launch just before writes - a 32-bit product, which lets the next kernel in as soon as it starts - in a
+    replayed graph: nothing is read before it is there."""
+    from infinilm_b200 import ops
+    dev = cuda_device
+    torch.manual_seed(3)
+    C, taps, E, H, d, K = 1024, 4, 16, 16, 64, 8192
+    a, w = torch.empty(16, K, device=dev), torch.randn(C * taps // 16, K, device=dev) / K ** 0.5
+    wd = torch.randn(H, K, device=dev) / K ** 0.5
+    x, w_out, decay = torch.randn(E, C, device=dev), torch.empty(16, C * taps // 16, device=dev), torch.empty(1, H, device=dev)
+    conv_state, state = torch.randn(E + 1, taps - 1, C, device=dev), torch.randn(E + 1, H, d, d, device=dev)
+    qstart, tok_entry = _step_arrays([1] * E, dev)
+    rd, wr = _i32(list(range(1, E + 1)), dev), _i32([0] * E, dev)
+    q, k, v = (torch.randn(E, H * d, device=dev) for _ in range(3))
+    conv, o = torch.empty(E, C, device=dev), torch.empty(E, H * d, device=dev)
+
+    def run(alone):
+        ops.gemm_f32(a, w, w_out)
+        if alone:
+            torch.cuda.synchronize()
+        ops.short_conv(x, 0, w_out.view(C, taps), conv_state, 0, rd, tok_entry, qstart, conv, 0, 1, C, C, 0)
+        ops.gemm_f32(a[:1], wd, decay)
+        if alone:
+            torch.cuda.synchronize()
+        ops.matrix_state_scan(ops.SCAN_DECAY, q, k, v, H, H, d, d, 0, decay.view(H), None, None, state, rd, wr, qstart, E, o, single=True)
+
+    a.normal_()
+    run(True)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        run(False)
+    for _ in range(10):
+        a.normal_()
+        run(True)
+        want = conv.clone(), o.clone()
+        w_out.zero_(), decay.zero_()
+        graph.replay()
+        assert torch.equal(conv, want[0]) and torch.equal(o, want[1])
+
+
 @pytest.mark.parametrize("H,d,dv", [(2, 32, 32), (3, 8, 40), (1, 128, 64), (2, 20, 12), (2, 10, 6), (1, 250, 9)])
 def test_decayed_sum_in_segments(cuda_device, H, d, dv):
     """Long portions walked in segments that run at once, with the second pass that adds each segment's start: several
