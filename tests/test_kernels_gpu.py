@@ -370,6 +370,31 @@ def test_attention_plain_tiles(cuda_device, nh, nkv, hd, starts, qlens):
     close(out.cpu(), c["ref"], "float32")
 
 
+@pytest.mark.parametrize("nh,nkv,hd", [(16, 2, 64), (3, 1, 32), (5, 1, 36), (6, 2, 20), (7, 1, 128), (9, 1, 64), (8, 8, 64), (2, 1, 100), (4, 1, 256)])
+@pytest.mark.parametrize("mode", ["plain", "window", "cap", "sink", "sigmoid", "bias"])
+def test_attention_plain_of_a_token_alone_and_among_others(cuda_device, nh, nkv, hd, mode):
+    """Heads that share a block with 1 to 8 others: a token's result is the same bits alone (a warp for every running sum) and among
+    hundreds (a warp for two of them)."""
+    c = _attn_case("float32", nh, nkv, hd, [300, 0, 33, 511, 64], [1, 280, 40, 1, 90], None, 13, dominate=True)
+    g = torch.Generator(device="cuda").manual_seed(hd)
+    kw = {"plain": {}, "window": {}, "cap": {"cap": 5.0}, "sink": {"sink": torch.randn(nh, device="cuda", generator=g)}, "sigmoid": {"sigmoid": True},
+          "bias": {"dist_bias": torch.randn(65, nh, device="cuda", generator=g)}}[mode]
+    window = 150 if mode == "window" else None
+
+    def run(at):
+        out = torch.full((len(at), nh * hd), float("nan"), device="cuda")
+        ops.attention_plain(c["qkv"][at].contiguous(), out, c["cache"], c["bt"], c["tok_pos"][at].contiguous(), c["tok_entry"][at].contiguous(), c["page"], nh, nkv, hd,
+                            1 / math.sqrt(hd), window, **kw)
+        return out
+
+    every = torch.arange(c["T"], device="cuda")
+    among = run(every)
+    assert bool(torch.isfinite(among).all())
+    for t in (0, 1, 31, 33, 150, 280, 281, 320, 321, c["T"] - 1):
+        assert torch.equal(run(every[t:t + 1])[0], among[t]), t
+    assert torch.equal(run(every[240:290]), among[240:290])
+
+
 @pytest.mark.parametrize("nh,nkv,hd", SHAPES)
 @pytest.mark.parametrize("window", [None, 21])
 def test_attention_prefill_bf16(cuda_device, nh, nkv, hd, window):
