@@ -43,9 +43,13 @@ class PagedAttend:
     FAST_MAX_GROUP = 64
     _warned_plain = False
 
-    # Up to here one split, which writes the output itself: more would save each warp a few pages, but cost the merge's launch
-    # (0.5B sizes, one request of 64 cached tokens: 3.6 us a layer in one split, 3.6 + 2.3 in four with their merge).
-    ONE_SPLIT_PAGES = 16
+    # Up to here one split, which writes the output itself: more would save each warp a few pages, but cost the merge's launch. A replayed
+    # step plans for 16 pages at least. Measured, us a layer of a replayed step in one split and in up to four with their merge, 1 / 8 / 16 requests:
+    # 16 heads on 2 of 64, 1,024 wide, some 40 cached tokens 16.6, 18.4 / 18.7, 20.8 / 23.2, 25.7, some 220 tokens 18.7, 19.1 / 20.9, 21.8; 12 on 12, 768 wide,
+    # 220 tokens 18.0, 17.9 / 19.6, 20.9; 64 on 8, 4,096 wide, 40 tokens 76.7, 78.7 / 85.6, 84.8 / 104.8, 107.1. Larger heads keep the splits: 32 on 2 of 128,
+    # 4,096 wide, 40 tokens 90.3, 77.2 / 112.9, 82.9 / 126.6, 103.1, 220 tokens 97.6, 78.9 / 123.8, 93.4 (the products that overlap with an unmerged attention
+    # of few blocks then run slower than the merge takes); 16 on 2 of 128, 2,048 wide, 30.3, 32.0 / 34.4, 35.2 / 42.8, 42.4.
+    ONE_SPLIT_PAGES, ONE_SPLIT_HEAD = 16, 64
     WAVE_FILL = 2.0 / 3.0                         # share of the blocks the device holds at once that the splits aim at
 
     def __init__(self, dtype, n_heads: int, n_kv_heads: int, head_dim: int, scale: float, window: Optional[int] = None,
@@ -73,8 +77,8 @@ class PagedAttend:
         """Splits of the keys for `base` blocks per split: as many as fill the wanted share of one wave of blocks
         (`resident`: what the device runs at once, from the occupancy query), never more - a second, part-filled wave
         costs more in partials than it gains - and at least four pages a split.
-        A few pages are one split: its block writes the output itself."""
-        if max_pages <= self.ONE_SPLIT_PAGES:
+        A few pages of small heads are one split: its block writes the output itself."""
+        if max_pages <= self.ONE_SPLIT_PAGES and self.hd <= self.ONE_SPLIT_HEAD:
             return 1
         target = max(1, int(resident * self.WAVE_FILL))
         return max(1, min(target // base, (max_pages + 3) // 4, 128))
