@@ -894,9 +894,12 @@ def gemm_skinny(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, alpha: floa
 # the model is NARROW_FROM to NARROW_WIDTH wide. Every block brings the activations in: measured at 1,024 wide against the tcgen05 and
 # library products, which still want their norms, 6.4 / 7.7 us at 17 rows and 8.5 / 10.2 at 48 for gate+up, 3.0 / 3.8 and 5.0 / 3.8 for
 # 1,024 x 1,024 into the residual; at 64 rows 10.0 / 8.6. With 4,096 columns into the residual 7.8 / 9.1 at 17 rows, 8.6 / 8.7 at 32 and
-# 11.2 / 8.1 at 48, so that product ends at NARROW_LONG_ROWS. Below NARROW_FROM, half the narrowest model in use, nothing was measured
-# and 17 rows keep the norm kernels.
-NARROW_MAX_ROWS, NARROW_LONG_ROWS, NARROW_FROM, NARROW_WIDTH = 48, 32, 512, 1024
+# 11.2 / 8.1 at 48, so that product ends at NARROW_LONG_ROWS. Whole replayed steps, us a layer with these products and with the others, 17 / 32 / 48 rows:
+# 512 wide with 2,048 in the feed-forward 19.5, 33.3 / 22.1, 33.5 / 28.0, 33.8; 768 with 3,072 23.2, 34.0 / 26.7, 37.1 / 34.1, 37.5; 1,024 with 4,096
+# 26.4, 41.9 / 29.8, 42.2 / 39.8, 41.7. Below NARROW_FROM nothing was measured and 17 rows keep the norm kernels. Gate+up is a block for 32 columns: with more
+# than one block an SM (NARROW_GLU_COLUMNS) and more than NARROW_LONG_ROWS rows it loses (1,024 with 8,192: 42.3, 50.4 / 46.5, 48.0 / 55.4, 50.2;
+# 896 with 4,736 at 33 and 48 rows 40.4, 43.4 / 40.7, 44.0, with 5,632 45.6, 41.7 / 44.6, 44.9) and is left to the tcgen05 product.
+NARROW_MAX_ROWS, NARROW_LONG_ROWS, NARROW_FROM, NARROW_WIDTH, NARROW_GLU_COLUMNS = 48, 32, 512, 1024, 148 * 32
 
 
 def narrow_ok(M: int, K: int) -> bool:
@@ -904,9 +907,9 @@ def narrow_ok(M: int, K: int) -> bool:
     return SKINNY_MAX_ROWS < M <= NARROW_MAX_ROWS and NARROW_FROM <= K <= NARROW_WIDTH and K % 8 == 0
 
 
-def skinny_glu_ok(M: int, K: int) -> bool:
-    """Whether `gemm_skinny` takes this shape with a gate."""
-    return skinny_ok(M, K) or narrow_ok(M, K)
+def skinny_glu_ok(M: int, K: int, N: int = 0) -> bool:
+    """Whether a gated product of M rows of K columns to N (0: not asked) goes to `gemm_skinny`, which takes them whatever N is."""
+    return skinny_ok(M, K) or (narrow_ok(M, K) and (M <= NARROW_LONG_ROWS or N <= NARROW_GLU_COLUMNS))
 
 
 def skinny_resid_ok(M: int, K: int, width: int) -> bool:

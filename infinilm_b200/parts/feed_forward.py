@@ -57,14 +57,14 @@ class SwiGLU(FeedForward):
         self.down.set(t[self.n_down], t.get("down_proj.bias"))
 
     def accepts_normed(self, T):
-        return self.dtype == torch.bfloat16 and ops.skinny_glu_ok(T, self.hidden)
+        return self.dtype == torch.bfloat16 and ops.skinny_glu_ok(T, self.hidden, self.inter)
 
     def fuses_tail(self, T):
-        return self.dtype == torch.bfloat16 and ops.skinny_glu_ok(T, self.hidden) and ops.skinny_resid_ok(T, self.inter, self.hidden)
+        return self.dtype == torch.bfloat16 and ops.skinny_glu_ok(T, self.hidden, self.inter) and ops.skinny_resid_ok(T, self.inter, self.hidden)
 
     def forward(self, x, ctx, tail=None):
         T = x.shape[0]
-        if self.dtype == torch.bfloat16 and ops.skinny_glu_ok(T, self.hidden):
+        if self.dtype == torch.bfloat16 and ops.skinny_glu_ok(T, self.hidden, self.inter):
             # decode: gate and up rows streamed together, SiLU(gate)*up in the epilogue
             act = ctx.ws.rows("ffn_act", T, self.inter, self.dtype)
             if isinstance(x, ops.NormedInput):
