@@ -48,8 +48,7 @@ __global__ void __launch_bounds__(128) gemm_grouped_mma_kernel(const __nv_bfloat
     if (group_off) {                              // (the groups' ranges come from the sort kernel before this one)
         il_pdl_begin();
         // The tile's group, by one warp, two groups a lane (one thread that walked the groups was a chain of up to n_groups reads in every
-        // block, the surplus ones too: 8 tokens to 6 of 64 experts of 2 x 1,408 x 2,048, gate+up 74.7 us, 69.4 with this and tiles of 16 rows; one
-        // token's six experts 26.1 and, the other way, 18.6 us, now 22.8 and 11.9).
+        // block, the surplus ones too; the rule that chooses the tile has the figures).
         if (warp == 0) {
             int tile = blockIdx.y;
             if (lane == 0) sh_g = n_groups;
@@ -99,12 +98,14 @@ __global__ void __launch_bounds__(128) gemm_grouped_mma_kernel(const __nv_bfloat
         w_src[i] = gn < N ? Wg + (size_t)(half * N + gn) * ldw + (ch & 7) * 8 : nullptr;
     }
     const int n_kb = (K + BK - 1) / BK;
+    const bool half = BM == 32 && r1 - r0 <= 16;  // a tile of 32 rows with at most 16: its upper half is neither staged nor multiplied
     auto issue_a = [&](int kb) {
         if (kb < n_kb) {
             const uint32_t st = sbase + (kb % STAGES) * STAGE_BYTES;
             const int k0 = kb * BK;
 #pragma unroll
             for (int i = 0; i < A_CH; ++i) {
+                if (i > 0 && half) break;             // (128 threads: 16 rows a turn)
                 const int ch = tid + i * 128;
                 const uint32_t dst = st + (ch >> 3) * ROW + (ch & 7) * 16;
                 if (a_src[i] && k0 + (ch & 7) * 8 < K) cp16(dst, a_src[i] + k0); else zero16(dst);
@@ -159,6 +160,7 @@ __global__ void __launch_bounds__(128) gemm_grouped_mma_kernel(const __nv_bfloat
             if (GLU) ldsm4(b2[0], b2[1], b2[2], b2[3], st + b_off + W_BYTES + kk * 32);
 #pragma unroll
             for (int mt = 0; mt < MT; ++mt) {
+                if (mt > 0 && half) break;
                 uint32_t a[4];
                 ldsm4(a[0], a[1], a[2], a[3], st + a_off + mt * 16 * ROW + kk * 32);
                 mma(acc[mt][0], a, b[0], b[1]);
@@ -351,10 +353,12 @@ IL_EXPORT int il_gemm_grouped(const void* A, int act_kind, int lda, long long a_
     if (act_kind == IL_BF16 && K % 8 == 0 && lda % 8 == 0 && ldw % 8 == 0 && a_gs % 8 == 0 && w_gs % 8 == 0 && !((uintptr_t)A & 15) &&
         !((uintptr_t)W & 15)) {
         // rows of 16-byte chunks: the tensor-core kernel. Few rows a group (a decode step): tiles of 32 rows; else 64.
-        // (and of 16 where a group has a few rows of them at most: half the stores of zeros and reads of rows that are none; 40 tokens to 6 of 64 experts:
-        // gate+up 139.7 us with 32, 131.2 with 16)
+        // A tile of 32 whose group has at most 16 rows left for it leaves its upper half out. Gate+up / back in us of tokens to 6 of 64 experts of 2 x 1,408 x 2,048, with
+        // whole tiles and so: 1 token 27.2 / 19.4, 22.2 / 13.7; 8 tokens 77.9 / 47.4, 74.7 / 43.7; 40 spread 134.3 / 74.9, 132.5 / 66.8; 40 on twelve of the experts
+        // 36.2 / 24.6, 34.2 / 21.5. (Tiles of 16 wherever groups have few rows on average: 74.8 / 47.6, 132.3 / 71.1, but 51.4 / 23.3 for the twelve, whose weights
+        // they stage twice.) Batched, every group has M rows: tiles of 16 up to there.
         const bool few = group_off ? M <= 32 * n_groups : M <= 32;
-        if (group_off ? M <= 4 * n_groups : M <= 16)
+        if (!group_off && M <= 16)
             return glu ? launch_mma<16, true>(A, lda, a_gs, a_rows, W, ldw, w_gs, C, ldc, c_gs, group_off, n_groups, M, N, K, gate, ld_gate, gate_gs, gate_ns, row_scale, scale_by_place, stream)
                        : launch_mma<16, false>(A, lda, a_gs, a_rows, W, ldw, w_gs, C, ldc, c_gs, group_off, n_groups, M, N, K, gate, ld_gate, gate_gs, gate_ns, row_scale, scale_by_place, stream);
         if (glu)

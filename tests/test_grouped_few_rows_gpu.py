@@ -28,7 +28,7 @@ def test_ragged(cuda_device, G, M, N, K, glu):
     from infinilm_b200 import ops
     off = _layout(G, M, G + N)
     M = int(off[-1])
-    assert M <= 4 * G                                      # tiles of 16 rows
+    assert M <= 4 * G                                      # few rows a group
     g = torch.Generator().manual_seed(K)
     a = torch.randn(M + 3, K, generator=g).bfloat16()
     w = (torch.randn(G, (2 if glu else 1) * N, K, generator=g) * 2 / math.sqrt(K)).bfloat16()
@@ -68,3 +68,36 @@ def test_batched(cuda_device, M):
     ops.gemm_grouped(a.cuda(), w.cuda(), out)
     ref = torch.einsum("mgk,gnk->mgn", a.double(), w.double())
     assert float((out.cpu().double() - ref).abs().amax()) <= 2.0 ** -8 * float(ref.abs().amax())
+
+
+@pytest.mark.parametrize("glu", [False, True])
+@pytest.mark.parametrize("N,K", [(64, 64), (100, 1408)])
+def test_groups_at_the_edges_of_tiles(cuda_device, N, K, glu):
+    """A tile of 32 rows with at most 16 leaves its upper half out: groups of 1 to 65 rows together in tiles of 32 (many groups) and of 64 (few), against
+    float64 and with the same bits."""
+    from infinilm_b200 import ops
+    counts = [1, 15, 16, 17, 0, 31, 32, 33, 48, 49, 64, 65, 2]
+    M, many = sum(counts), [0] * 20
+    g = torch.Generator().manual_seed(N)
+    a = torch.randn(M, K, generator=g).bfloat16()
+    w = (torch.randn(len(counts), (2 if glu else 1) * N, K, generator=g) * 2 / math.sqrt(K)).bfloat16()
+    outs = []
+    for pad, rows in ((many, M), ([], M), ([], 64 * M)):           # (n_rows bounds the places and chooses the tile)
+        off = torch.tensor([0] + counts + pad).cumsum(0)
+        wide = torch.cat([w, w[:1].expand(len(pad), -1, -1)]).contiguous()
+        out = torch.full((rows + 1, N), float("nan"), device="cuda", dtype=torch.bfloat16)
+        src = torch.cat([a, a[:1].expand(rows - M, -1)]).contiguous()
+        ops.gemm_grouped(src.cuda(), wide.cuda(), out[:rows], group_off=off.to(torch.int32).cuda(), n_rows=rows, glu=glu)
+        outs.append(out[:M])
+        assert bool(out[M:].isnan().all())
+        assert torch.equal(outs[-1], outs[0])
+    at = 0
+    for e, n in enumerate(counts):
+        if n:
+            y = a[at:at + n].double() @ w[e].double().t()
+            if glu:
+                gt, up = y[:, :N].bfloat16().double(), y[:, N:].bfloat16().double()
+                y = gt * torch.sigmoid(gt) * up
+            # rounded to bfloat16 once; with a gate its two products before that
+            assert float((outs[0][at:at + n].cpu().double() - y).abs().amax()) <= (3 if glu else 1) * 2.0 ** -8 * float(y.abs().amax())
+        at += n
