@@ -404,11 +404,12 @@ template <bool VEC> static cudaError_t f32_dispatch(const F32Args& a) {
     for (int cut = 0; cut < (a.K > share ? 2 : 1); ++cut)
         for (int i = 0; i < 4; ++i) {
             const long long tiles = (long long)((a.M + BM[i] - 1) / BM[i]) * ((a.N + BN[i] - 1) / BN[i]), blocks = tiles << cut, rest = blocks % 296;
-            if (cut && tiles > 2 * 296) continue;
+            if ((cut && tiles > 2 * 296) || (a.M + BM[i] - 1) / BM[i] > 65535) continue;     // (millions of rows: the taller tiles, a grid has 65,535 rows)
             const float waves = (float)(blocks / 296) * TWO[i] + (rest == 0 ? 0.f : rest <= 148 ? ONE[i] : TWO[i]);
             const float us = cut ? waves * part + 5.f * (float)((blocks + 295) / 296) : waves * whole;
             if (best < 0 || us < best_us) best = cut * 4 + i, best_us = us;
         }
+    if (best < 0) return cudaErrorInvalidConfiguration;
     const bool split = best >= 4;
     switch (best & 3) {
         case 0: return f32_launch_tile<1, 1, 8, VEC>(a, split);

@@ -24,3 +24,18 @@ def test_shares(cuda_device, M, N, K):
     few = torch.empty(9, N, device="cuda")
     ops.gemm_f32(x[5:14].contiguous(), w, few, 0.5, b)
     assert torch.equal(few, out[5:14, :N])
+
+
+def test_millions_of_rows(cuda_device):
+    """More rows than 65,535 tiles of 32 or 64 have: the taller tiles take them."""
+    from infinilm_b200 import ops
+    M, N, K = 4_300_000, 32, 4
+    g = torch.Generator(device="cuda").manual_seed(1)
+    x, w = torch.randn(M, K, device="cuda", generator=g), torch.randn(N, K, device="cuda", generator=g)
+    out = torch.full((M, N), float("nan"), device="cuda")
+    ops.gemm_f32(x, w, out)
+    for at in (0, 4_194_240 - 8, M - 20):
+        few = torch.empty(16, N, device="cuda")
+        ops.gemm_f32(x[at:at + 16], w, few)
+        assert torch.equal(out[at:at + 16], few)
+    assert not bool(out.isnan().any())
