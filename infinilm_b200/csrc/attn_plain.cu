@@ -116,8 +116,10 @@ __global__ void __launch_bounds__(R == 1 ? 512 : 256, R == 1 ? 2 : 4) attn_tile_
                 p = in ? __fdiv_rn(1.f, __fadd_rn(1.f, expf(-s))) : 0.f;
             } else {
                 const float mn = fmaxf(m[u], il_warp_max(in ? s : -INFINITY));
-                const float corr = expf(__fadd_rn(m[u], -mn));           // exp(-inf) = 0 on the first tile
-                p = in ? expf(__fadd_rn(s, -mn)) : 0.f;
+                // exp(-inf) = 0 on the first tile; a tile whose scores are all -inf (a bias that masks) leaves the sum as it is
+                const float ref = mn == -INFINITY ? 0.f : mn;
+                const float corr = mn == -INFINITY ? 1.f : expf(__fadd_rn(m[u], -mn));
+                p = in ? expf(__fadd_rn(s, -ref)) : 0.f;
                 l[u] = __fmaf_rn(l[u], corr, p);
                 m[u] = mn;
                 const il_f2 c2 = il_f2_dup(corr);
@@ -159,7 +161,7 @@ __global__ void __launch_bounds__(R == 1 ? 512 : 256, R == 1 ? 2 : 4) attn_tile_
         const float m0 = m[0];
         for (int i = 1; i < R * KS; ++i) m[0] = fmaxf(m[0], sm[(size_t)(i * HW + hs) * (HDP + 4) + HDP]);
         if (!SIG) {
-            const float c = expf(__fadd_rn(m0, -m[0]));
+            const float c = m0 == -INFINITY ? 0.f : expf(__fadd_rn(m0, -m[0]));
             l[0] = __fmul_rn(l[0], c);
 #pragma unroll
             for (int v = 0; v < NV; ++v) acc[0][v] = il_f2_mul(acc[0][v], il_f2_dup(c));
@@ -167,7 +169,7 @@ __global__ void __launch_bounds__(R == 1 ? 512 : 256, R == 1 ? 2 : 4) attn_tile_
         for (int i = 1; i < R * KS; ++i) {
             const float* other = sm + (size_t)(i * HW + hs) * (HDP + 4);
             const float mi = other[HDP];
-            const float c = SIG ? 1.f : mi == -INFINITY && m[0] != -INFINITY ? 0.f : expf(__fadd_rn(mi, -m[0]));
+            const float c = SIG ? 1.f : mi == -INFINITY ? 0.f : expf(__fadd_rn(mi, -m[0]));
             l[0] = __fmaf_rn(c, other[HDP + 1], l[0]);
 #pragma unroll
             for (int v = 0; v < NV; ++v)

@@ -395,6 +395,26 @@ def test_attention_plain_of_a_token_alone_and_among_others(cuda_device, nh, nkv,
     assert torch.equal(run(every[240:290]), among[240:290])
 
 
+@pytest.mark.parametrize("nh,nkv,hd", [(16, 2, 64), (3, 1, 32), (4, 1, 256)])
+@pytest.mark.parametrize("masked", [1, 40, 100, 200])
+def test_attention_plain_with_a_bias_that_masks_the_nearest_keys(cuda_device, nh, nkv, hd, masked):
+    """A bias of -inf on the nearest keys, one to whole tiles of them: they have no weight, and the others' softmax is what it is without them."""
+    c = _attn_case("float32", nh, nkv, hd, [0], [300], None, 14)
+    bias = torch.randn(256, nh, generator=torch.Generator().manual_seed(masked))
+    bias[:masked] = float("-inf")
+    at = torch.arange(masked, 300)
+    out = torch.empty(len(at), nh * hd, device="cuda")
+    ops.attention_plain(c["qkv"][at].contiguous(), out, c["cache"], c["bt"], c["tok_pos"][at].contiguous(), c["tok_entry"][at].contiguous(), c["page"], nh, nkv, hd,
+                        1 / math.sqrt(hd), dist_bias=bias.cuda())
+    pages = c["cache"].cpu()[c["bt"][0].cpu().long()].double()              # [pages, 2, kv heads, page, hd]
+    k, v = (pages[:, i].permute(1, 0, 2, 3).reshape(nkv, -1, hd)[:, :300].repeat_interleave(nh // nkv, 0) for i in (0, 1))
+    q = c["qkv"].cpu()[at, :nh * hd].double().view(-1, nh, hd).transpose(0, 1)
+    dist = at[:, None] - torch.arange(300)[None]
+    s = q @ k.transpose(1, 2) / math.sqrt(hd) + bias.double()[dist.clamp(0, 255)].permute(2, 0, 1)
+    ref = torch.softmax(s.masked_fill(dist < 0, float("-inf")), -1) @ v
+    close(out.cpu(), ref.transpose(0, 1).reshape(len(at), nh * hd).float(), "float32")
+
+
 @pytest.mark.parametrize("nh,nkv,hd", SHAPES)
 @pytest.mark.parametrize("window", [None, 21])
 def test_attention_prefill_bf16(cuda_device, nh, nkv, hd, window):
