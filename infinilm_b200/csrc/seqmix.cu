@@ -697,7 +697,7 @@ __device__ __forceinline__ bool ds_find(int tile, int e0, int n_ent, int seg_len
 // segments before its own: 390 MB of reads a layer for two portions of 2,100 and 2,900 tokens, where this pass moves 80.)
 __global__ void decay_prefix_kernel(const float* __restrict__ decay, float* state, size_t slot_stride, const int* __restrict__ write_slots,
                                     const int* __restrict__ qstart, int H, int head_f, int e0, int seg_len, float* seg_state) {
-    const int e = e0 + blockIdx.z, h = blockIdx.y, i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int e = e0 + blockIdx.x, h = blockIdx.y, i = blockIdx.z * blockDim.x + threadIdx.x;
     int first = 0;
     for (int f = e0; f < e; ++f) first += (qstart[f + 1] - qstart[f] + seg_len - 1) / seg_len;
     const int len = qstart[e + 1] - qstart[e], n_seg = (len + seg_len - 1) / seg_len;
@@ -945,7 +945,7 @@ IL_EXPORT int il_matrix_state_scan(int mode, const float* q, const float* k, con
     if (mode == 4 ? (!decay || !gdec || G != H || in_act || ld_g < H * dim) : mode == 0 ? !decay : (!beta || !gdec)) return IL_BAD_ARG;
     const auto prefix = [&]() {
         const int head_f = dim * vdim;
-        decay_prefix_kernel<<<dim3((head_f + 255) / 256, H, E), 256, 0, stream>>>(decay, state, (size_t)slot_stride, write_slots, qstart, H, head_f, e0,
+        decay_prefix_kernel<<<dim3(E, H, (head_f + 255) / 256), 256, 0, stream>>>(decay, state, (size_t)slot_stride, write_slots, qstart, H, head_f, e0,
                                                                                   seg_len, seg_state);
     };
     if (seg_len > 0 && dim > 32 && dim <= 128) {

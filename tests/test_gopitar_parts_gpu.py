@@ -305,6 +305,23 @@ def test_decayed_sum_in_segments_four_columns_a_lane(cuda_device, H, d, dv):
     test_decayed_sum_in_segments(cuda_device, H, d, dv)
 
 
+@pytest.mark.parametrize("d", [8, 40])
+def test_decayed_sum_in_segments_of_very_many_entries(cuda_device, d):
+    """More entries than a grid has rows, a token each: the state is what the token brings."""
+    from infinilm_b200 import ops
+    dev = cuda_device
+    E, dv = 65_600, 4
+    g = torch.Generator(device="cuda").manual_seed(d)
+    q, k, v = (torch.randn(E, n, device=dev, generator=g) for n in (d, d, dv))
+    qstart, slots = torch.arange(E + 1, device=dev, dtype=torch.int32), torch.arange(1, E + 1, device=dev, dtype=torch.int32)
+    state, out = torch.zeros(E + 1, 1, dv, d, device=dev), torch.empty(E, dv, device=dev)
+    ops.matrix_state_scan(ops.SCAN_DECAY, q, k, v, 1, 1, d, dv, 0, torch.tensor([0.9], device=dev), None, None, state, torch.zeros_like(slots), slots, qstart, E, out,
+                          seg_len=8, n_tiles=E, seg_state=torch.empty(E * dv * d, device=dev))
+    assert torch.equal(state[1:, 0], v[:, :, None] * k[:, None, :])
+    dot = (q.double() * k.double()).sum(1, keepdim=True) * v.double()
+    assert float((out.double() - dot).abs().max()) <= (d + 2) * 2.0 ** -24 * float((q.abs().double() * k.abs().double()).sum(1).max() * v.abs().max())
+
+
 def test_segments_apply_the_activation_as_they_stage(cuda_device):
     """silu inside the kernel that walks segments against the pass of its own in front of it: the same numbers."""
     from infinilm_b200 import ops
