@@ -971,7 +971,7 @@ IL_EXPORT int il_matrix_state_scan(int mode, const float* q, const float* k, con
         int dpt = dim <= 32 ? 8 : 16;
         if ((mode == 0 || mode == 4) && dim > 32 && dim <= 128) {       // (the channel decay, like the decayed sum, has no sum over the lanes between a token's updates)
             const int cols16 = SR_THREADS / ((dim + 15) / 16 <= 1 ? 1 : (dim <= 32 ? 2 : dim <= 64 ? 4 : 8));
-            if ((long long)(seg_len > 0 ? n_tiles : E) * H * ((vdim + cols16 - 1) / cols16) <= 148) dpt = 8;     // at most one block an SM otherwise
+            if ((long long)E * H * ((vdim + cols16 - 1) / cols16) <= 148) dpt = 8;     // at most one block an SM otherwise
         }
         int log_split = 0;
         while ((dpt << log_split) < dim) ++log_split;
@@ -993,8 +993,7 @@ IL_EXPORT int il_matrix_state_scan(int mode, const float* q, const float* k, con
                 IL_LAUNCH_CHECK();
                 prefix();
                 IL_LAUNCH_CHECK();
-                if (log_split <= 3) { if (dpt == 8) sr_launch<2, 8, 8, 8>(SR_ARGS); else sr_launch<2, 16, 8, 8>(SR_ARGS); }
-                else { if (dpt == 8) sr_launch<2, 8, 8, 16>(SR_ARGS); else sr_launch<2, 16, 8, 16>(SR_ARGS); }
+                if (dpt == 8) sr_launch<2, 8, 8, 8>(SR_ARGS); else sr_launch<2, 16, 8, 16>(SR_ARGS);      // (key sizes up to 32, or beyond 128)
             }
         } else if (mode == 1) {
             if (dpt == 8) SR_PICK(1, 8); else SR_PICK(1, 16);
