@@ -95,6 +95,43 @@ def test_rotated_and_stored(cuda_device, nh, nkv, hd, rot, M):
     assert torch.equal(caches[0] == 0, caches[1] == 0)
 
 
+@pytest.mark.parametrize("K", [512, 1016, 1024])
+@pytest.mark.parametrize("M", [17, 24, 32, 33, 48])
+@pytest.mark.parametrize("with_cache,with_bias", [(True, True), (False, True), (True, False)])
+def test_rotated_rows_whose_norm_is_unfinished(cuda_device, M, K, with_cache, with_bias):
+    """Rows whose 1/rms differ by orders of magnitude, up to the widest model: row by row against float64, rounded to bfloat16 and then rotated."""
+    from infinilm_b200 import ops
+    nh, nkv, hd, rot, page = 4, 2, 64, 32, 16
+    N = (nh + 2 * nkv) * hd
+    g = torch.Generator().manual_seed(M + K)
+    pos = torch.tensor([(11 * i) % 63 for i in range(M)], dtype=torch.int32)
+    bt = torch.randperm(M * 4, generator=g).view(M, 4).to(torch.int32).cuda()
+    x = torch.randn(M, K, generator=g).bfloat16()
+    w = (torch.randn(N, K, generator=g) / math.sqrt(K)).bfloat16()
+    bias = torch.randn(N, generator=g) * 1e-3 if with_bias else None
+    sq = (torch.rand(M, 64, generator=g) + 0.5) * 10.0 ** (torch.arange(M).view(M, 1) % 7 - 3).float()
+    inv = (1.0 / (10000.0 ** (torch.arange(rot // 2, dtype=torch.float64) * 2 / rot))).float()
+    out = torch.full((M, N), float("nan"), device="cuda", dtype=torch.bfloat16)
+    cache = torch.zeros(M * 4, 2, nkv, page, hd, dtype=torch.bfloat16, device="cuda") if with_cache else None
+    ops.gemm_skinny_rope(x.cuda(), w.cuda(), out, 0.75, None if bias is None else bias.cuda(), pos.cuda(), torch.arange(M, dtype=torch.int32).cuda(), bt, cache, page,
+                         nh, nkv, hd, rot, inv.cuda(), 1.1, norm_in=ops.NormedInput(x.cuda(), sq.cuda(), 1024, 1e-5))
+    y = 0.75 * torch.rsqrt(sq.double().sum(1, keepdim=True) / 1024 + 1e-5) * (x.double() @ w.double().t()) + (bias.double() if bias is not None else 0.0)
+    y = y.view(M, nh + 2 * nkv, hd)
+    ang = pos.double().view(M, 1, 1) * inv.double()
+    lo, hi = y[..., :rot // 2], y[..., rot // 2:rot]
+    turned = torch.cat([(lo * ang.cos() - hi * ang.sin()) * 1.1, (hi * ang.cos() + lo * ang.sin()) * 1.1, y[..., rot:]], -1)
+    ref = torch.cat([turned[:, :nh + nkv], y[:, nh + nkv:]], 1)
+    got = out.cpu().double().view(M, nh + 2 * nkv, hd)
+    # two roundings to bfloat16 of values within the head's largest (the second of two rotated ones), and the angle's rounding (63 radians: 63 x 2^-23 at most)
+    assert bool(((got - ref).abs() <= 3 * 2.0 ** -8 * ref.abs().amax(-1, keepdim=True)).all())
+    if with_cache:
+        for m in range(M):
+            p = int(bt[m, int(pos[m]) // page])
+            assert torch.equal(cache[p, 0, :, int(pos[m]) % page].cpu(), out[m].view(-1, hd)[nh:nh + nkv].cpu())
+            assert torch.equal(cache[p, 1, :, int(pos[m]) % page].cpu(), out[m].view(-1, hd)[nh + nkv:].cpu())
+        assert int((cache != 0).any(-1).sum()) == 2 * nkv * M
+
+
 def test_step_with_and_without_the_norm_in_its_products(cuda_device):
     """A model 512 wide in portions of 17 to 48 rows, with rows either side of them, against the plain model, with the fused products and with the kernels
     they stand for."""
