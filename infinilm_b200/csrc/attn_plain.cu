@@ -20,8 +20,8 @@
 // read the same keys and values from shared memory, where asynchronous copies bring the next round while this one is
 // worked on (bfloat16, and sizes whose rows are not whole 16-byte pieces, are widened by plain loads instead). In the scores a lane
 // is a key, in the weighted sum a pair of columns. What bounds it is the chain of a tile - scores, maximum, exponentials, sum -
-// where one key at a time paid that chain and a trip to memory for every key: 16 heads on 2 of 64, one token over 80 keys 84 us, now 7.7; 800 tokens of
-// four prompts 1.3 ms, now 70 us.
+// where one key at a time paid that chain and a trip to memory for every key: 16 heads on 2 of 64, one token over 80 keys 84 us, now 7.7; some 800 tokens of
+// four prompts 1.3 ms, now 72 us.
 constexpr int AT_KEYS = 32;
 __host__ __device__ constexpr int at_row(int hdp) { return hdp + 4; }          // floats of a staged row: an odd number of 16-byte pieces
 __host__ __device__ constexpr int at_round_floats(int hdp, int ks) { return 2 * ks * AT_KEYS * at_row(hdp); }

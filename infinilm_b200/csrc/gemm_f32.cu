@@ -54,7 +54,7 @@ __device__ __forceinline__ float f32_halves(il_f2 v) {
 // A) to shared memory, a thread sums one chunk of one W row with all M rows of A, and the chunk sums are added in order.
 // The next round's copies are in flight meanwhile, and the first round's W is asked for before the wait for the kernel in
 // front where the caller says that W is no kernel's output (`early`). Rows and chunks are padded so that the eight lanes of a load phase hit eight banks groups.
-// Measured, one row, weights not in cache: 8,192 x 1,024 in 10.3 us (3.3 TB/s), 73,448 x 1,024 in 69 us (4.4 TB/s); one accumulator
+// Measured, one row, weights not in cache: 8,192 x 1,024 in 10.5 us (3.2 TB/s), 73,448 x 1,024 in 76 us (4.0 TB/s); one accumulator
 // that walked all of K with plain loads took 740 us on average over a step's products of 1,024 and 4,096 k.
 constexpr int FR_ROWS = 8, FR_CHUNKS = 16, FR_ROUND = FR_CHUNKS * F32_CHUNK, FR_CS = F32_CHUNK + 4;
 constexpr int FR_WS = FR_CHUNKS * FR_CS + 4, FR_XS = FR_CHUNKS * FR_CS, FR_THREADS = FR_ROWS * FR_CHUNKS;

@@ -727,8 +727,10 @@ __global__ void decay_prefix_kernel(const float* __restrict__ decay, float* stat
 // the arithmetic, which runs two rows an instruction (packed f32); a head is two blocks instead of eight, so the inputs'
 // activation fits into the staging (no pass of its own); and the outputs of 8 tokens are summed over the lanes of a column by
 // halving (28 shuffles for 32 outputs) and leave as 16 bytes a lane. SECOND: o_t += decay^(t - t0 + 1) S_start^T q_t.
-// Measured at 16 heads of 128 x 128, portions of 2,100 and 2,900 tokens, a layer: 110 + 11 (prefix) + 57 us; the register form took
-// 279 + 142 us, and the activation's own pass 45. The arithmetic alone is about 130 us at the FP32 pipes' rate.
+// Measured at 16 heads of 128 x 128, portions of 2,100 and 2,900 tokens in one step, a layer: 332 us in a replayed graph (under the counters 227 + 18
+// (prefix) + 113), 264 us for two of 2,048; the register form took 995 and 823 with the activation in its loop. In a pass that brings the two
+// prompts in steps of 4,096 and 904 tokens, us a layer and step: 110 + 11 + 57, and 279 + 142 and 45 for the activation's own pass before. The
+// arithmetic of both passes over 5,000 tokens is some 140 us at the FP32 pipes' rate.
 constexpr int DS_COLS = 4, DS_CHUNK = 8, DS_ROWS = 16, DS_SEG = DS_ROWS + 4;
 template <int LOG_SPLIT, bool SECOND>
 __global__ void __launch_bounds__(SR_THREADS) decay_segment_kernel(const float* __restrict__ q, const float* __restrict__ k, const float* __restrict__ v,
