@@ -26,6 +26,50 @@ constexpr int AT_KEYS = 32;
 __host__ __device__ constexpr int at_row(int hdp) { return hdp + 4; }          // floats of a staged row: an odd number of 16-byte pieces
 __host__ __device__ constexpr int at_round_floats(int hdp, int ks) { return 2 * ks * AT_KEYS * at_row(hdp); }
 
+// What both kernels of these sizes do with a tile's scores, its weights and the running sums: one text, and the roundings spelled out, so that a
+// token has the same bits from either.
+// A lane's key: its score from the dot product's two halves, the sum's new maximum, the weight. `bias`: the key's, or null.
+template <bool SIG, bool CAP, int NV>
+__device__ __forceinline__ float at_weight(float d0, float d1, bool in, float scale, float cap, const float* bias, float& m, float& l, il_f2 (&acc)[NV]) {
+    float s = __fmul_rn(__fadd_rn(d0, d1), scale);
+    if (CAP) s = __fmul_rn(cap, tanhf(__fdiv_rn(s, cap)));
+    if (bias) s = __fadd_rn(s, *bias);
+    if constexpr (SIG) return in ? __fdiv_rn(1.f, __fadd_rn(1.f, expf(-s))) : 0.f;
+    const float mn = fmaxf(m, il_warp_max(in ? s : -INFINITY));
+    // exp(-inf) = 0 on the first tile; a tile whose scores are all -inf (a bias that masks) leaves the sum as it is
+    const float ref = mn == -INFINITY ? 0.f : mn;
+    const float corr = mn == -INFINITY ? 1.f : expf(__fadd_rn(m, -mn));
+    const float p = in ? expf(__fadd_rn(s, -ref)) : 0.f;
+    l = __fmaf_rn(l, corr, p);
+    m = mn;
+    const il_f2 c2 = il_f2_dup(corr);
+#pragma unroll
+    for (int v = 0; v < NV; ++v) acc[v] = il_f2_mul(acc[v], c2);
+    return p;
+}
+// The first of a head's sums brought to the maximum m of all of them; then each other one's factor.
+template <bool SIG, int NV> __device__ __forceinline__ void at_first(float m0, float m, float& l, il_f2 (&acc)[NV]) {
+    if (SIG) return;
+    const float c = m0 == -INFINITY ? 0.f : expf(__fadd_rn(m0, -m));
+    l = __fmul_rn(l, c);
+#pragma unroll
+    for (int v = 0; v < NV; ++v) acc[v] = il_f2_mul(acc[v], il_f2_dup(c));
+}
+template <bool SIG> __device__ __forceinline__ float at_factor(float mi, float m) { return SIG ? 1.f : mi == -INFINITY ? 0.f : expf(__fadd_rn(mi, -m)); }
+template <typename TA, bool SIG, int NV>
+__device__ __forceinline__ void at_store(TA* orow, int hd, int lane, const float* sink, float m, float l, const il_f2 (&acc)[NV]) {
+    if (sink) l = __fadd_rn(l, expf(__fadd_rn(*sink, -m)));      // (+inf when the sink towers over every score: the row is then zero)
+    const float inv = SIG ? 1.f : __fdiv_rn(1.f, l);
+#pragma unroll
+    for (int v = 0; v < NV; ++v) {
+        float a, b;
+        il_f2_get(acc[v], a, b);
+        const int d = 2 * lane + 64 * v;
+        if (d < hd) orow[d] = il_from_f<TA>(__fmul_rn(a, inv));
+        if (d + 1 < hd) orow[d + 1] = il_from_f<TA>(__fmul_rn(b, inv));
+    }
+}
+
 template <typename TA, int HDP, bool SIG, bool CAP, int R>
 __global__ void __launch_bounds__(R == 1 ? 512 : 256, R == 1 ? 2 : 4) attn_tile_kernel(const TA* qkv, int row_stride, TA* __restrict__ out, const TA* cache, const int* __restrict__ block_table,
                                  int bt_stride, const int* __restrict__ tok_pos, const int* __restrict__ tok_entry, int page_size, int page_shift,
@@ -107,25 +151,8 @@ __global__ void __launch_bounds__(R == 1 ? 512 : 256, R == 1 ? 2 : 4) attn_tile_
             }
             float d0, d1;
             il_f2_get(il_f2_add(s2[0], s2[1]), d0, d1);
-            // (roundings spelled out: the same bits from both forms of this kernel)
-            float s = __fmul_rn(__fadd_rn(d0, d1), scale);
-            if (CAP) s = __fmul_rn(cap, tanhf(__fdiv_rn(s, cap)));
-            if (dist_bias && in) s = __fadd_rn(s, dist_bias[(size_t)min(n_keys - 1 - kk, dist_far) * nh + j]);
-            float p;
-            if constexpr (SIG) {
-                p = in ? __fdiv_rn(1.f, __fadd_rn(1.f, expf(-s))) : 0.f;
-            } else {
-                const float mn = fmaxf(m[u], il_warp_max(in ? s : -INFINITY));
-                // exp(-inf) = 0 on the first tile; a tile whose scores are all -inf (a bias that masks) leaves the sum as it is
-                const float ref = mn == -INFINITY ? 0.f : mn;
-                const float corr = mn == -INFINITY ? 1.f : expf(__fadd_rn(m[u], -mn));
-                p = in ? expf(__fadd_rn(s, -ref)) : 0.f;
-                l[u] = __fmaf_rn(l[u], corr, p);
-                m[u] = mn;
-                const il_f2 c2 = il_f2_dup(corr);
-#pragma unroll
-                for (int v = 0; v < NV; ++v) acc[u][v] = il_f2_mul(acc[u][v], c2);
-            }
+            const float* bias = dist_bias && in ? dist_bias + (size_t)min(n_keys - 1 - kk, dist_far) * nh + j : nullptr;
+            const float p = at_weight<SIG, CAP, NV>(d0, d1, in, scale, cap, bias, m[u], l[u], acc[u]);
             ps[lane] = p;
             __syncwarp();
             const float* vr = sm + (r & 1) * round_f + half_f + ks * AT_KEYS * RS + 2 * lane;
@@ -160,16 +187,10 @@ __global__ void __launch_bounds__(R == 1 ? 512 : 256, R == 1 ? 2 : 4) attn_tile_
         if (ks != 0) return;
         const float m0 = m[0];
         for (int i = 1; i < R * KS; ++i) m[0] = fmaxf(m[0], sm[(size_t)(i * HW + hs) * (HDP + 4) + HDP]);
-        if (!SIG) {
-            const float c = m0 == -INFINITY ? 0.f : expf(__fadd_rn(m0, -m[0]));
-            l[0] = __fmul_rn(l[0], c);
-#pragma unroll
-            for (int v = 0; v < NV; ++v) acc[0][v] = il_f2_mul(acc[0][v], il_f2_dup(c));
-        }
+        at_first<SIG, NV>(m0, m[0], l[0], acc[0]);
         for (int i = 1; i < R * KS; ++i) {
             const float* other = sm + (size_t)(i * HW + hs) * (HDP + 4);
-            const float mi = other[HDP];
-            const float c = SIG ? 1.f : mi == -INFINITY ? 0.f : expf(__fadd_rn(mi, -m[0]));
+            const float c = at_factor<SIG>(other[HDP], m[0]);
             l[0] = __fmaf_rn(c, other[HDP + 1], l[0]);
 #pragma unroll
             for (int v = 0; v < NV; ++v)
@@ -177,18 +198,165 @@ __global__ void __launch_bounds__(R == 1 ? 512 : 256, R == 1 ? 2 : 4) attn_tile_
                     acc[0][v] = il_f2_fma(il_f2_dup(c), *reinterpret_cast<const il_f2*>(other + 2 * lane + 64 * v), acc[0][v]);
         }
     }
-    if (!live) return;
-    if (sink) l[0] = __fadd_rn(l[0], expf(__fadd_rn(sink[j], -m[0])));   // (+inf when the sink towers over every score: the row is then zero)
-    const float inv = SIG ? 1.f : __fdiv_rn(1.f, l[0]);
-    TA* orow = out + (size_t)t * nh * hd + (size_t)j * hd;
-#pragma unroll
-    for (int v = 0; v < NV; ++v) {
-        float a, b;
-        il_f2_get(acc[0][v], a, b);
-        const int d = 2 * lane + 64 * v;
-        if (d < hd) orow[d] = il_from_f<TA>(a * inv);
-        if (d + 1 < hd) orow[d + 1] = il_from_f<TA>(b * inv);
+    if (live) at_store<TA, SIG, NV>(out + (size_t)t * nh * hd + (size_t)j * hd, hd, lane, sink ? sink + j : nullptr, m[0], l[0], acc[0]);
+}
+
+// The same for many tokens of heads that share no keys, or few do: there a block of the kernel above is 1 to 4 warps and 140 KB of tiles, one block an
+// SM, and keys staged for them alone. Here a warp has a (token, head), holds all its running sums (V) and reads keys and values from memory, through L1: in the
+// scores eight columns of its key's row a lane and load, in the weighted sum whole rows. What bounds it is the lines that the loads of 32 rows touch in L1; the
+// (token, head) pairs an SM holds cover each other's chains.
+constexpr int AT_DIRECT_WARPS = 4;
+// Four elements p[0 .. 3] of a row as two pairs, zeros from `left` on. VEC: left is a multiple of 4 and the row aligned to four elements.
+__device__ __forceinline__ void at_load4(const float* p, int left, bool vec, il_f2& lo, il_f2& hi) {
+    if (vec) {
+        const float4 x = *reinterpret_cast<const float4*>(p);
+        lo = il_f2_make(x.x, x.y), hi = il_f2_make(x.z, x.w);
+    } else {
+        lo = il_f2_make(p[0], left > 1 ? p[1] : 0.f), hi = il_f2_make(left > 2 ? p[2] : 0.f, left > 3 ? p[3] : 0.f);
     }
+}
+__device__ __forceinline__ void at_load4(const __nv_bfloat16* p, int left, bool vec, il_f2& lo, il_f2& hi) {
+    if (vec) {
+        const uint2 x = *reinterpret_cast<const uint2*>(p);
+        const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&x.x)), b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&x.y));
+        lo = il_f2_make(a.x, a.y), hi = il_f2_make(b.x, b.y);
+    } else {
+        lo = il_f2_make(il_to_f(p[0]), left > 1 ? il_to_f(p[1]) : 0.f), hi = il_f2_make(left > 2 ? il_to_f(p[2]) : 0.f, left > 3 ? il_to_f(p[3]) : 0.f);
+    }
+}
+// Eight elements as four pairs: one load of 32 (16) bytes, aligned to as many.
+__device__ __forceinline__ void at_load8(const float* p, il_f2 (&a)[4]) {
+    float x[8];
+    asm volatile("ld.global.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];\n"
+                 : "=f"(x[0]), "=f"(x[1]), "=f"(x[2]), "=f"(x[3]), "=f"(x[4]), "=f"(x[5]), "=f"(x[6]), "=f"(x[7]) : "l"(p));
+#pragma unroll
+    for (int i = 0; i < 4; ++i) a[i] = il_f2_make(x[2 * i], x[2 * i + 1]);
+}
+__device__ __forceinline__ void at_load8(const __nv_bfloat16* p, il_f2 (&a)[4]) {
+    const uint4 q = *reinterpret_cast<const uint4*>(p);
+    const unsigned w[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const float2 x = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&w[i]));
+        a[i] = il_f2_make(x.x, x.y);
+    }
+}
+__device__ __forceinline__ il_f2 at_load2(const float* p, int left, bool vec) {
+    if (vec) {
+        const float2 x = *reinterpret_cast<const float2*>(p);
+        return il_f2_make(x.x, x.y);
+    }
+    return il_f2_make(p[0], left > 1 ? p[1] : 0.f);
+}
+__device__ __forceinline__ il_f2 at_load2(const __nv_bfloat16* p, int left, bool vec) {
+    if (vec) {
+        const float2 x = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(p));
+        return il_f2_make(x.x, x.y);
+    }
+    return il_f2_make(il_to_f(p[0]), left > 1 ? il_to_f(p[1]) : 0.f);
+}
+
+template <typename TA, int HDP, bool SIG, bool CAP, int V>
+__global__ void __launch_bounds__(AT_DIRECT_WARPS * 32) attn_direct_kernel(const TA* qkv, int row_stride, TA* __restrict__ out, const TA* cache,
+                                                                          const int* __restrict__ block_table, int bt_stride, const int* __restrict__ tok_pos,
+                                                                          const int* __restrict__ tok_entry, int page_size, int page_shift, int nh, int nkv, int hd,
+                                                                          float scale, int window, const float* __restrict__ sink,
+                                                                          const float* __restrict__ dist_bias, int dist_far, float cap, int vec) {
+    constexpr int NV = (HDP + 63) / 64;
+    __shared__ __align__(16) float qs_all[AT_DIRECT_WARPS][HDP], ps_all[AT_DIRECT_WARPS][AT_KEYS];
+    il_pdl_wait();
+    il_pdl_launch_dependents();
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int t = blockIdx.x, j = blockIdx.y * AT_DIRECT_WARPS + warp;
+    if (j >= nh) return;
+    const int g = j / (nh / nkv);
+    float* qs = qs_all[warp];
+    float* ps = ps_all[warp];
+    const TA* qrow = qkv + (size_t)t * row_stride + (size_t)j * hd;
+    for (int d = lane; d < HDP; d += 32) qs[d] = d < hd ? il_to_f(qrow[d]) : 0.f;
+    const int pos = tok_pos[t];
+    const int* bt = block_table + (size_t)tok_entry[t] * bt_stride;
+    const int lo = il_mask_lo(pos, window), n_keys = pos - lo + 1, tiles = (n_keys + AT_KEYS - 1) / AT_KEYS;
+    const size_t page_elems = (size_t)2 * nkv * page_size * hd, v_off = (size_t)nkv * page_size * hd;
+    float m[V], l[V];
+    il_f2 acc[V][NV];
+#pragma unroll
+    for (int u = 0; u < V; ++u) {
+        m[u] = -INFINITY, l[u] = 0.f;
+#pragma unroll
+        for (int v = 0; v < NV; ++v) acc[u][v] = 0ull;
+    }
+    __syncwarp();
+    for (int t0 = 0; t0 < tiles; t0 += V) {
+#pragma unroll
+        for (int u = 0; u < V; ++u) {             // tile i of the keys goes to running sum i % V
+            const int tile = t0 + u;
+            if (V > 1 && tile >= tiles) break;
+            const int kk = tile * AT_KEYS + lane;
+            const bool in = kk < n_keys;
+            const int kp = lo + (in ? kk : 0), pi = page_shift >= 0 ? kp >> page_shift : kp / page_size;
+            const TA* krow = cache + (size_t)bt[pi] * page_elems + ((size_t)g * page_size + (kp - pi * page_size)) * hd;
+            il_f2 s2[2] = {0ull, 0ull};
+            if (vec == 2) {
+#pragma unroll 4
+                for (int d = 0; d < HDP; d += 8) {
+                    if (d >= hd) break;
+                    il_f2 a[4];
+                    at_load8(krow + d, a);
+                    const ulonglong2 b0 = *reinterpret_cast<const ulonglong2*>(qs + d), b1 = *reinterpret_cast<const ulonglong2*>(qs + d + 4);
+                    s2[0] = il_f2_fma(a[0], b0.x, s2[0]);
+                    s2[1] = il_f2_fma(a[1], b0.y, s2[1]);
+                    s2[0] = il_f2_fma(a[2], b1.x, s2[0]);
+                    s2[1] = il_f2_fma(a[3], b1.y, s2[1]);
+                }
+            } else {
+#pragma unroll 4
+                for (int d = 0; d < HDP; d += 4) {
+                    if (d >= hd) break;
+                    il_f2 a0, a1;
+                    at_load4(krow + d, hd - d, vec, a0, a1);
+                    const ulonglong2 b = *reinterpret_cast<const ulonglong2*>(qs + d);
+                    s2[0] = il_f2_fma(a0, b.x, s2[0]);
+                    s2[1] = il_f2_fma(a1, b.y, s2[1]);
+                }
+            }
+            float d0, d1;
+            il_f2_get(il_f2_add(s2[0], s2[1]), d0, d1);
+            const float* bias = dist_bias && in ? dist_bias + (size_t)min(n_keys - 1 - kk, dist_far) * nh + j : nullptr;
+            ps[lane] = at_weight<SIG, CAP, NV>(d0, d1, in, scale, cap, bias, m[u], l[u], acc[u]);
+            __syncwarp();
+            const unsigned long long row = reinterpret_cast<unsigned long long>(krow);
+            const int n = min(AT_KEYS, n_keys - tile * AT_KEYS);
+#pragma unroll 4
+            for (int key = 0; key < n; ++key) {
+                const TA* vrow = reinterpret_cast<const TA*>(__shfl_sync(0xffffffffu, row, key)) + v_off;
+                const il_f2 w = il_f2_dup(ps[key]);
+#pragma unroll
+                for (int v = 0; v < NV; ++v) {
+                    const int d = 2 * lane + 64 * v;
+                    if (d < hd) acc[u][v] = il_f2_fma(w, at_load2(vrow + d, hd - d, vec), acc[u][v]);
+                }
+            }
+            __syncwarp();                         // ps is written again in the next tile
+        }
+    }
+    if (!SIG)
+#pragma unroll
+        for (int u = 0; u < V; ++u) l[u] = il_warp_sum(l[u]);
+    if (V > 1) {
+        const float m0 = m[0];
+#pragma unroll
+        for (int u = 1; u < V; ++u) m[0] = fmaxf(m[0], m[u]);
+        at_first<SIG, NV>(m0, m[0], l[0], acc[0]);
+#pragma unroll
+        for (int u = 1; u < V; ++u) {
+            const float c = at_factor<SIG>(m[u], m[0]);
+            l[0] = __fmaf_rn(c, l[u], l[0]);
+#pragma unroll
+            for (int v = 0; v < NV; ++v) acc[0][v] = il_f2_fma(il_f2_dup(c), acc[u][v], acc[0][v]);
+        }
+    }
+    at_store<TA, SIG, NV>(out + (size_t)t * nh * hd + (size_t)j * hd, hd, lane, sink ? sink + j : nullptr, m[0], l[0], acc[0]);
 }
 
 // Warps that share a head in a block of 8 warps, as many as shared memory holds tiles for; and the running sums of a head: twice as many where
@@ -197,6 +365,9 @@ __global__ void __launch_bounds__(R == 1 ? 512 : 256, R == 1 ? 2 : 4) attn_tile_
 __host__ __device__ constexpr int at_fit(int hdp) { return hdp <= 32 ? 8 : hdp == 64 ? 4 : hdp == 128 ? 2 : 1; }
 __host__ __device__ constexpr int at_warps_a_head(int hdp, int HW) { return 8 / HW < at_fit(hdp) ? 8 / HW : at_fit(hdp); }
 __host__ __device__ constexpr int at_sums(int hdp, int HW) { return 2 * at_warps_a_head(hdp, HW) <= at_fit(hdp) && 16 / HW >= 2 * at_warps_a_head(hdp, HW) ? 2 * at_warps_a_head(hdp, HW) : at_warps_a_head(hdp, HW); }
+
+static_assert(at_sums(256, 1) == 1 && at_sums(256, 4) == 1 && at_sums(128, 1) == 2 && at_sums(128, 2) == 2 && at_sums(64, 1) == 4 && at_sums(64, 2) == 4 &&
+              at_sums(32, 1) == 8, "attn_direct_kernel's sums");
 
 struct AtArgs {
     const void *qkv, *cache;
@@ -229,11 +400,44 @@ static cudaError_t at_launch_as(const AtArgs& a, int HW, int n_hb, int KS) {
                      (TA*)a.out, (const TA*)a.cache, a.block_table, a.bt_stride, a.tok_pos, a.tok_entry, a.page_size, shift, a.nh, a.nkv, a.hd, a.scale,
                      a.window, a.sink, a.dist_bias, a.dist_far, a.cap, HW, KS, async);
 }
+template <typename TA, int HDP, bool SIG, bool CAP, int V>
+static cudaError_t at_launch_direct(const AtArgs& a) {
+    int shift = -1;
+    if ((a.page_size & (a.page_size - 1)) == 0)
+        for (shift = 0; (1 << shift) < a.page_size; ++shift) {}
+    const uintptr_t at = (uintptr_t)a.cache;       // columns of a row that a load may take: 8, 4, 1
+    const int vec = a.hd % 8 == 0 && !(at & (8 * sizeof(TA) - 1)) ? 2 : a.hd % 4 == 0 && !(at & (4 * sizeof(TA) - 1)) ? 1 : 0;
+    return il_launch(attn_direct_kernel<TA, HDP, SIG, CAP, V>, dim3(a.T, (a.nh + AT_DIRECT_WARPS - 1) / AT_DIRECT_WARPS), dim3(AT_DIRECT_WARPS * 32), (size_t)0,
+                     a.stream, (const TA*)a.qkv, a.row_stride, (TA*)a.out, (const TA*)a.cache, a.block_table, a.bt_stride, a.tok_pos, a.tok_entry, a.page_size,
+                     shift, a.nh, a.nkv, a.hd, a.scale, a.window, a.sink, a.dist_bias, a.dist_far, a.cap, vec);
+}
+// Whether a step runs the kernel that stages nothing: where few heads share a kv head and the tiles' blocks, about one an SM there, are so many waves (0: never).
+// A long context is a longer chain for its one warp a head than for the tiles' several, so the waves wanted grow with the contexts the block table has room for
+// (`keys`), up to 512. bfloat16 tiles are widened by plain loads as they are staged, which float32 leaves to asynchronous copies: fewer waves. Measured, tiles / direct / key by
+// key as it was before both, us:
+//   float32  256: 8 heads on 8, 1,024 tokens 9,580 / 1,102 / 1,213, 64 single tokens over 500 keys 679 / 658 / 1,013; 8 on 4 3,006 / 1,110 / 1,201; 9 on 3 1,852 / 1,252 / 1,378, 300
+//            tokens 200 / 212 / 264; 8 on 2 1,104 / 1,123 / 1,233
+//            128: 8 on 8, 1,024 tokens 2,277 / 831 / 1,079, 64 single tokens 164 / 551 / 926; 12 on 12, 64 tokens 41 / 34 / 52; 8 on 4, 1,024 tokens 784 / 837 / 1,079
+//            64: 16 on 16, 1,024 tokens 1,421 / 748 / 1,587, 64 single tokens 96 / 305 / 722, 30 tokens 19 / 13 / 24; 16 on 8, 1,024 tokens 647 / 746 / 1,555
+//            32: 32 on 32, 1,024 tokens 1,725 / 1,386 / 2,700, after 2,000 cached 5,882 / 6,662 / 12,229, 64 tokens 59 / 21 / 43
+//   bfloat16 256: 8 on 8 18,118 / 1,015 / 1,278; 8 on 2 1,733 / 1,066 / 1,267, 300 tokens 189 / 182 / 278    128: 8 on 4 1,462 / 739 / 1,193; 9 on 3, 300 tokens 103 / 154 / 268
+//            64: 16 on 8 991 / 683 / 1,759, 64 single tokens 77 / 147 / 377; 9 on 3 322 / 442 / 1,111    32: 32 on 32 2,345 / 1,213 / 2,909; 16 on 8 401 / 621 / 1,570
+__host__ __device__ constexpr int at_direct_waves(int hdp, int HW, int bytes) {
+    if (bytes == 4) return hdp == 256 ? (HW <= 2 ? 2 : HW == 3 ? 12 : 0) : HW > 1 ? 0 : hdp == 128 ? 10 : hdp == 64 ? 20 : 40;
+    return hdp == 256 ? (HW <= 2 ? 2 : HW <= 4 ? HW : 0) : HW > 2 ? 0 : hdp == 128 ? 2 * HW : hdp == 64 ? (HW == 1 ? 4 : 16) : HW == 1 ? 8 : 0;
+}
+static bool at_direct(int hdp, int HW, int bytes, long long blocks, long long keys) {
+    const long long waves = at_direct_waves(hdp, HW, bytes);
+    if (waves == 0 || blocks < 148 || (bytes == 4 && hdp == 32 && keys > 1024)) return false;
+    return blocks * 512 >= 148 * waves * (keys < 512 ? keys : 512);
+}
 template <typename TA, int HDP, bool SIG, bool CAP>
 static cudaError_t at_launch(const AtArgs& a) {
     const int G = a.nh / a.nkv, HW = G < 8 ? G : 8, n_hb = (G + HW - 1) / HW;
     const long long blocks = (long long)a.T * a.nkv * n_hb;
     const int KS = at_warps_a_head(HDP, HW), sums = at_sums(HDP, HW);
+    // (wherever the other kernel is taken a head has at_fit(HDP) running sums)
+    if (at_direct(HDP, HW, sizeof(TA), blocks, (long long)a.bt_stride * a.page_size)) return at_launch_direct<TA, HDP, SIG, CAP, at_fit(HDP)>(a);
     // Few (token, kv head) pairs, less than two blocks an SM: a warp for every sum.
     if (sums == KS || blocks < 2 * 148) return at_launch_as<TA, HDP, SIG, CAP, 1>(a, HW, n_hb, sums);
     if constexpr (HDP < 256) return at_launch_as<TA, HDP, SIG, CAP, 2>(a, HW, n_hb, KS);

@@ -395,6 +395,35 @@ def test_attention_plain_of_a_token_alone_and_among_others(cuda_device, nh, nkv,
     assert torch.equal(run(every[240:290]), among[240:290])
 
 
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+@pytest.mark.parametrize("nh,nkv,hd", [(8, 8, 256), (6, 3, 256), (9, 3, 256), (8, 2, 200), (4, 4, 250), (20, 20, 80), (8, 4, 128), (5, 5, 65), (16, 16, 64), (16, 8, 64), (6, 6, 36), (7, 7, 33), (32, 32, 32),
+                                       (9, 9, 10)])
+@pytest.mark.parametrize("mode", ["plain", "window", "cap", "sink", "sigmoid", "bias"])
+def test_attention_plain_of_heads_that_share_few_keys(cuda_device, dtype, nh, nkv, hd, mode):
+    """One to four heads a kv head, where many tokens run the kernel that stages nothing: rows of whole 8- and 4-element pieces and others, against the reference (plain and
+    windowed) and the bits of a token alone."""
+    window = 150 if mode == "window" else None
+    c = _attn_case(dtype, nh, nkv, hd, [300, 0, 33, 511, 64], [1, 280, 40, 1, 190], window, 15, dominate=True)
+    g = torch.Generator(device="cuda").manual_seed(hd)
+    bias = torch.randn(65, nh, device="cuda", generator=g)
+    bias[7] = float("-inf")
+    kw = {"cap": {"cap": 5.0}, "sink": {"sink": torch.randn(nh, device="cuda", generator=g)}, "sigmoid": {"sigmoid": True}, "bias": {"dist_bias": bias}}.get(mode, {})
+
+    def run(at):
+        out = torch.full((len(at), nh * hd), float("nan"), device="cuda", dtype=DT[dtype])
+        ops.attention_plain(c["qkv"][at].contiguous(), out, c["cache"], c["bt"], c["tok_pos"][at].contiguous(), c["tok_entry"][at].contiguous(), c["page"], nh, nkv, hd,
+                            1 / math.sqrt(hd), window, **kw)
+        return out
+
+    every = torch.arange(c["T"], device="cuda")
+    among = run(every)
+    if mode in ("plain", "window"):
+        close(among.cpu(), c["ref"], dtype)
+    assert bool(torch.isfinite(among).all())
+    for t in (0, 1, 32, 33, 280, 281, 320, 321, 322, c["T"] - 1):
+        assert torch.equal(run(every[t:t + 1])[0], among[t]), t
+
+
 @pytest.mark.parametrize("nh,nkv,hd", [(16, 2, 64), (3, 1, 32), (4, 1, 256)])
 @pytest.mark.parametrize("masked", [1, 40, 100, 200])
 def test_attention_plain_with_a_bias_that_masks_the_nearest_keys(cuda_device, nh, nkv, hd, masked):
