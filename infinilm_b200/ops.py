@@ -574,7 +574,8 @@ def gate_pack(y: torch.Tensor, head_dim: int, gate: Optional[torch.Tensor], g_of
 
 def gemm_f32(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, alpha: float = 1.0,
              bias: Optional[torch.Tensor] = None, w_static: bool = False, glu: int = 0, act_params=None) -> None:
-    """out[M,N] = alpha * a[M,K] @ w[N,K]^T (+ bias), all float32, FP32 pipes only. `w_static`: w is a model's weight, not what
+    """out[M,N] = alpha * a[M,K] @ w[N,K]^T (+ bias), all float32, with the error of 32-bit multiply-adds (each operand
+    as three bfloat16 pieces on the tensor cores, sums in float32). `w_static`: w is a model's weight, not what
     the kernel launched just before writes, and may be read while that kernel still runs.
     glu (ACT_SILU / ACT_GELU_TANH / ACT_CLAMPED with act_params; up to 16 rows): w is [2N,K] (gate rows, then up rows) and
     out[M,N] = act(gate) * up, as `swiglu` computes it from the products."""
@@ -593,9 +594,9 @@ def gemm_f32(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, alpha: float =
         raise KernelError("gemm_f32: a gate goes with up to 16 rows")
     limit, act_alpha = _act_args(glu, act_params)
     f = _fn("gemm_f32", "il_gemm_f32", [_c_void_p, _c_int, _c_void_p, _c_int, _c_void_p, _c_int, _c_void_p, _c_float,
-                                        _c_int, _c_int, _c_int, _c_int, _c_float, _c_float, _c_int, _c_void_p])
+                                        _c_int, _c_int, _c_int, _c_int, _c_float, _c_float, _c_int, _c_void_p, _c_void_p])
     _check(f(_ptr(a), a.stride(0), _ptr(w), w.stride(0), _ptr(out), out.stride(0), _ptr(bias), alpha, M, N, K,
-             int(glu), limit, act_alpha, int(w_static), _stream()), "gemm_f32")
+             int(glu), limit, act_alpha, int(w_static), _ptr(stream_status(out.device)), _stream()), "gemm_f32")
 
 
 _ones_k = {}

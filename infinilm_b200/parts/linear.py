@@ -2,7 +2,7 @@
 
 Parity with InfiniLM: `csrc/layers/linear/base_linear.cpp:35-44` and
 `csrc/layers/quantization/none_quantization.cpp:26-46` (weight [out,in], optional bias, a scale
-`alpha` passed into the product). The float32 path runs the FFMA kernel of this package. On the
+`alpha` passed into the product). The float32 path runs this package's 32-bit product. On the
 bfloat16 path up to 16 rows (decode) run this package's weight-streaming kernel, 17 to 256 rows run
 its tcgen05/TMA kernels where that is enabled (the output head: `gemm_mid` up to 64 rows, `gemm_tc5`
 beyond), and everything else calls the library matrix product, as InfiniLM does for its linears.
