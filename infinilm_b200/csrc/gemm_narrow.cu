@@ -2,7 +2,9 @@
 //   gated   out[M,N] = act(alpha * x . Wg^T + bg) * (alpha * x . Wu^T + bu),  W = [Wg; Wu], K <= 1,024
 //   rope    the q/k/v projection, q and k rotated, k and v written to the paged cache, K <= 1,024
 //   resid   resid += bscale * bf16(alpha * x . W^T + b), xw = resid * norm weight, sums of the residual's squares, K <= 1,024
-//           (up to 32 rows: K <= 4,096)
+//           (in steps of 64, or up to 32 rows: K <= 4,096)
+// Two forms: on tcgen05 with K over a cluster (gemm_narrow_tc5.cuh), which more rows and the long product take (gc_ok has the times), and
+// the one below.
 // They do for these rows what the fused forms of the weight-streaming kernels do for up to 16, and take the same unfinished
 // norms (the activations times a weight, to be divided by the rms that `GnNormIn` gives).
 //
@@ -15,7 +17,7 @@
 // A 24-layer model 1,024 wide, 40 requests arriving and leaving: 71.8 ms of steps before, 66.2 with these; its layer's products of 17 rows
 // (gate+up / o / down, by themselves) 7.7 / 3.8 / 9.1 us before, 6.4 / 3.0 / 7.8 now, and two norms and a rotation less. With the
 // activations read from L2 by every tile of weights instead of staged once a block the steps took 69.4; with the long product's K cut
-// over a cluster of two blocks 71.5.
+// over a cluster of two blocks 71.5. With the tcgen05 form, which takes 40 rows' long product from the library too, 60.1.
 #include "common.cuh"
 
 constexpr int GN_SLAB = 512, GN_STAGES = 3, GN_MAX_ROWS = 48, GN_MAX_K = 4096;
@@ -51,6 +53,8 @@ struct GnArgs {
     const void* norm_w;
     int norm_w_kind;
 };
+
+#include "gemm_narrow_tc5.cuh"
 
 __device__ __forceinline__ void gn_mma(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
     asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
@@ -299,24 +303,36 @@ static bool gn_bad(const GnArgs& a) {
            ((uintptr_t)a.W & 15) || (a.ni.partial && (a.ni.n_partial <= 0 || a.ni.n_partial > 64));
 }
 
+// cluster: blocks a tile of the tcgen05 form (0: whether and how many is chosen here; negative: the mma.sync form). From which number of rows
+// the tcgen05 form is taken: us at 17 / 32 / 40 / 48 rows, mma.sync and tcgen05, 1,024 wide with 4,096 in the feed-forward, replayed in a row:
+//   gated 6.5, 7.6, 8.4, 9.5 and 6.9, 6.6, 7.6, 7.5; rotated 3.9, 4.5, 5.2, 6.5 and 4.3, 4.4, 4.6, 4.6;
+//   into the residual K = 1,024 3.0, 3.4, 3.9, 5.0 and 4.0, 4.2, 4.6, 4.6; K = 4,096 7.8, 8.6, -, - and 5.9, 6.1, 6.2, 6.4.
+static bool gc_ok(const GnArgs& a, int cluster, const int* status, int rows_from) {
+    return cluster >= 0 && status && a.K % 64 == 0 && (cluster > 0 || a.M >= rows_from);
+}
+
 // Up to 48 rows (made for 17 and more), K <= 1,024. W [2N, K]: gate rows, then up rows; bias [2N] or null; act: 1 SiLU, 2 the tanh form of
 // GELU, 3 the clamped gate. norm_partial: see GnNormIn. w_static: W was written long before, not by the kernel in front of this one.
 IL_EXPORT int il_gemm_narrow_glu(const void* x, int ldx, const void* W, int ldw, void* out, int ldo, const float* bias, float alpha, int M, int N, int K,
                                  int act, float act_limit, float act_alpha, const float* norm_partial, int n_partial, int norm_h, float norm_eps,
-                                 int w_static, cudaStream_t stream) {
+                                 int w_static, int cluster, int* status, cudaStream_t stream) {
     if (M <= 0 || N <= 0) return IL_OK;
     GnArgs a = {};
     a.x = (const __nv_bfloat16*)x, a.W = (const __nv_bfloat16*)W, a.out = (__nv_bfloat16*)out, a.bias = bias;
     a.ldx = ldx, a.ldw = ldw, a.ldo = ldo, a.M = M, a.N = N, a.K = K, a.alpha = alpha, a.act = act, a.act_limit = act_limit, a.act_alpha = act_alpha;
     a.ni = GnNormIn{norm_partial, n_partial, norm_partial ? 1.f / (float)norm_h : 0.f, norm_eps};
     if (gn_bad(a) || K > 2 * GN_SLAB || ldo < N || act < 1 || act > 3 || (norm_partial && norm_h <= 0)) return IL_UNSUPPORTED;
+    if (gc_ok(a, cluster, status, 25)) {
+        const int tiles = (N + 63) / 64;
+        return gc_rows<GN_GLU, 2>(a, 2 * N, tiles, cluster > 0 ? cluster : gc_cluster(tiles, K), w_static != 0, status, stream);
+    }
     return gn_rows<GN_GLU, 4, 4, 2>(a, (N + 31) / 32, w_static != 0, stream);
 }
 
 IL_EXPORT int il_gemm_narrow_rope(const void* x, int ldx, const void* W, int ldw, void* out, int ldo, const float* bias, float alpha, int M, int K,
                                   const int* tok_pos, const int* tok_entry, const int* block_table, int bt_stride, void* cache, int page_size, int nh,
                                   int nkv, int hd, int rot, const float* inv_freq, float mscale, const float* norm_partial, int n_partial, int norm_h,
-                                  float norm_eps, int w_static, cudaStream_t stream) {
+                                  float norm_eps, int w_static, int cluster, int* status, cudaStream_t stream) {
     if (M <= 0) return IL_OK;
     GnArgs a = {};
     a.x = (const __nv_bfloat16*)x, a.W = (const __nv_bfloat16*)W, a.out = (__nv_bfloat16*)out, a.bias = bias;
@@ -326,13 +342,18 @@ IL_EXPORT int il_gemm_narrow_rope(const void* x, int ldx, const void* W, int ldw
     if (gn_bad(a) || K > 2 * GN_SLAB || ldo < a.N || (norm_partial && norm_h <= 0)) return IL_UNSUPPORTED;
     if (nh <= 0 || nkv <= 0 || hd <= 0 || (hd & 15) || rot < 0 || rot > hd || (rot & 15) || page_size <= 0) return IL_UNSUPPORTED;
     if (rot > 0 && !inv_freq) return IL_BAD_ARG;
+    if (gc_ok(a, cluster, status, 33) && rot == hd && (hd == 64 || hd == 128)) {
+        const int tiles = nh + 2 * nkv, c = cluster > 0 ? cluster : gc_cluster(tiles, K);
+        return hd == 64 ? gc_rows<GN_ROPE, 1>(a, a.N, tiles, c, w_static != 0, status, stream) : gc_rows<GN_ROPE, 2>(a, a.N, tiles, c, w_static != 0, status, stream);
+    }
     return gn_rows<GN_ROPE, 1, 8, 2>(a, a.N / 16, w_static != 0, stream);
 }
 
 // N = width of the residual stream (a multiple of nothing: the last block may be ragged); sumsq [M][ceil(N / 16)]. K <= 1,024, or
-// with up to 32 rows K <= 4,096.
+// K in steps of 64 or up to 32 rows, K <= 4,096.
 IL_EXPORT int il_gemm_narrow_resid(const void* x, int ldx, const void* W, int ldw, const float* bias, float alpha, int M, int N, int K, float* resid,
-                                   float bscale, const void* norm_w, int norm_w_kind, void* xw, float* sumsq, int w_static, cudaStream_t stream) {
+                                   float bscale, const void* norm_w, int norm_w_kind, void* xw, float* sumsq, int w_static, int cluster, int* status,
+                                   cudaStream_t stream) {
     if (M <= 0 || N <= 0) return IL_OK;
     GnArgs a = {};
     a.x = (const __nv_bfloat16*)x, a.W = (const __nv_bfloat16*)W, a.out = (__nv_bfloat16*)xw, a.bias = bias;
@@ -340,6 +361,10 @@ IL_EXPORT int il_gemm_narrow_resid(const void* x, int ldx, const void* W, int ld
     a.resid = resid, a.sumsq = sumsq, a.bscale = bscale, a.norm_w = norm_w, a.norm_w_kind = norm_w_kind;
     if (gn_bad(a) || K > GN_MAX_K || !resid || !norm_w || !xw || !sumsq) return IL_UNSUPPORTED;
     if (norm_w_kind != IL_F32 && norm_w_kind != IL_BF16) return IL_BAD_ARG;
+    if (gc_ok(a, cluster, status, K > 2 * GN_SLAB ? 1 : 41)) {
+        const int tiles = (N + 63) / 64;
+        return gc_rows<GN_RESID, 1>(a, N, tiles, cluster > 0 ? cluster : gc_cluster(tiles, K), w_static != 0, status, stream);
+    }
     const int blocks = (N + 15) / 16;
     if (K <= 2 * GN_SLAB) return gn_rows<GN_RESID, 1, 8, 2>(a, blocks, w_static != 0, stream);
     return gn_rows<GN_RESID, 1, 16, GN_MAX_K / GN_SLAB>(a, blocks, w_static != 0, stream);

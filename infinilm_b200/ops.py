@@ -877,10 +877,10 @@ def gemm_skinny(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, alpha: floa
             raise KernelError(f"gemm_skinny: {M} rows of {K} columns")
         limit, act_alpha = _act_args(glu, act_params)
         f = _fn("gemm_narrow", "il_gemm_narrow_glu", [_c_void_p, _c_int, _c_void_p, _c_int, _c_void_p, _c_int, _c_void_p, _c_float, _c_int, _c_int,
-                                                      _c_int, _c_int, _c_float, _c_float, _c_void_p, _c_int, _c_int, _c_float, _c_int, _c_void_p])
+                                                      _c_int, _c_int, _c_float, _c_float, _c_void_p, _c_int, _c_int, _c_float, _c_int, _c_int, _c_void_p, _c_void_p])
         np_, nb, nw, ne = _norm_args(norm_in, M)
         _check(f(_ptr(x), x.stride(0), _ptr(w), w.stride(0), _ptr(out), out.stride(0), _ptr(bias), alpha, M, N, K, int(glu), limit, act_alpha,
-                 np_, nb, nw, ne, int(w_static), _stream()), "gemm_narrow_glu")
+                 np_, nb, nw, ne, int(w_static), narrow_cluster, _ptr(stream_status(x.device)), _stream()), "gemm_narrow_glu")
         return
     f = _fn("gemm_skinny", "il_gemm_skinny", [_c_void_p, _c_int, _c_void_p, _c_int, _c_void_p, _c_int, _c_int, _c_void_p,
                                               _c_float, _c_int, _c_int, _c_int, _c_int, _c_void_p, _c_int, _c_int, _c_float,
@@ -894,13 +894,20 @@ def gemm_skinny(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, alpha: floa
 # 17 to 48 rows of a narrow model: the fused products (gated, rotating, adding into the residual) take these rows too where
 # the model is NARROW_FROM to NARROW_WIDTH wide. Every block brings the activations in: measured at 1,024 wide against the tcgen05 and
 # library products, which still want their norms, 6.4 / 7.7 us at 17 rows and 8.5 / 10.2 at 48 for gate+up, 3.0 / 3.8 and 5.0 / 3.8 for
-# 1,024 x 1,024 into the residual; at 64 rows 10.0 / 8.6. With 4,096 columns into the residual 7.8 / 9.1 at 17 rows, 8.6 / 8.7 at 32 and
-# 11.2 / 8.1 at 48, so that product ends at NARROW_LONG_ROWS. Whole replayed steps, us a layer with these products and with the others, 17 / 32 / 48 rows:
+# 1,024 x 1,024 into the residual; at 64 rows 10.0 / 8.6. With 4,096 columns into the residual (mma.sync form) 7.8 / 9.1 at 17 rows, 8.6 / 8.7 at 32 and
+# 11.2 / 8.1 at 48, so that form ends at NARROW_LONG_ROWS; the tcgen05 form (K in steps of 64) takes 5.9, 6.1 and 6.4, without a norm behind it. Whole replayed steps, us a layer with these products and with the others, 17 / 32 / 48 rows:
 # 512 wide with 2,048 in the feed-forward 19.5, 33.3 / 22.1, 33.5 / 28.0, 33.8; 768 with 3,072 23.2, 34.0 / 26.7, 37.1 / 34.1, 37.5; 1,024 with 4,096
 # 26.4, 41.9 / 29.8, 42.2 / 39.8, 41.7. Below NARROW_FROM nothing was measured and 17 rows keep the norm kernels. Gate+up is a block for 32 columns: with more
 # than one block an SM (NARROW_GLU_COLUMNS) and more than NARROW_LONG_ROWS rows it loses (1,024 with 8,192: 42.3, 50.4 / 46.5, 48.0 / 55.4, 50.2;
 # 896 with 4,736 at 33 and 48 rows 40.4, 43.4 / 40.7, 44.0, with 5,632 45.6, 41.7 / 44.6, 44.9) and is left to the tcgen05 product.
 NARROW_MAX_ROWS, NARROW_LONG_ROWS, NARROW_FROM, NARROW_WIDTH, NARROW_GLU_COLUMNS = 48, 32, 512, 1024, 148 * 32
+
+
+narrow_cluster = 0                                # blocks a tile of the narrow products' tcgen05 form: 0 the kernel's choice, negative the other form (tests)
+
+
+def _narrow_args(many: bool, x: torch.Tensor):
+    return (narrow_cluster, _ptr(stream_status(x.device))) if many else ()
 
 
 def narrow_ok(M: int, K: int) -> bool:
@@ -916,7 +923,7 @@ def skinny_glu_ok(M: int, K: int, N: int = 0) -> bool:
 def skinny_resid_ok(M: int, K: int, width: int) -> bool:
     """Whether `gemm_skinny_resid` takes this shape."""
     if narrow_ok(M, width):
-        return K % 8 == 0 and (K <= NARROW_WIDTH or (K <= 4 * NARROW_WIDTH and M <= NARROW_LONG_ROWS))
+        return K % 8 == 0 and (K <= NARROW_WIDTH or (K <= 4 * NARROW_WIDTH and (M <= NARROW_LONG_ROWS or K % 64 == 0)))
     return 0 < M <= SKINNY_MAX_ROWS and K % 8 == 0 and (width + 15) // 16 <= NORM_MAX_BLOCKS
 
 
@@ -945,9 +952,9 @@ def gemm_skinny_resid(x: torch.Tensor, w: torch.Tensor, alpha: float, bias: Opti
     many = M > SKINNY_MAX_ROWS
     f = _fn("gemm_narrow" if many else "gemm_skinny", "il_gemm_narrow_resid" if many else "il_gemm_skinny_resid",
             [_c_void_p, _c_int, _c_void_p, _c_int, _c_void_p, _c_float, _c_int, _c_int, _c_int,
-             _c_void_p, _c_float, _c_void_p, _c_int, _c_void_p, _c_void_p, _c_int, _c_void_p])
+             _c_void_p, _c_float, _c_void_p, _c_int, _c_void_p, _c_void_p, _c_int] + [_c_int, _c_void_p] * many + [_c_void_p])
     _check(f(_ptr(x), x.stride(0), _ptr(w), w.stride(0), _ptr(bias), alpha, M, H, K, _ptr(resid), branch_scale, _ptr(norm_weight),
-             kind_of(norm_weight.dtype), _ptr(xw), _ptr(sumsq), int(w_static), _stream()), "gemm_skinny_resid")
+             kind_of(norm_weight.dtype), _ptr(xw), _ptr(sumsq), int(w_static), *_narrow_args(many, x), _stream()), "gemm_skinny_resid")
     return NormedInput(xw, sumsq, H, eps)
 
 
@@ -986,11 +993,11 @@ def gemm_skinny_rope(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, alpha:
     f = _fn("gemm_narrow" if many else "gemm_skinny", "il_gemm_narrow_rope" if many else "il_gemm_skinny_rope",
             [_c_void_p, _c_int, _c_void_p, _c_int, _c_void_p, _c_int, _c_void_p, _c_float, _c_int, _c_int, _c_void_p, _c_void_p,
              _c_void_p, _c_int, _c_void_p, _c_int, _c_int, _c_int, _c_int, _c_int, _c_void_p, _c_float, _c_void_p, _c_int, _c_int,
-             _c_float, _c_int, _c_void_p])
+             _c_float, _c_int] + [_c_int, _c_void_p] * many + [_c_void_p])
     np_, nb, nw, ne = _norm_args(norm_in, M)
     _check(f(_ptr(x), x.stride(0), _ptr(w), w.stride(0), _ptr(out), out.stride(0), _ptr(bias), alpha, M, K, _ptr(tok_pos),
              _ptr(tok_entry), _ptr(block_table), block_table.shape[1], _ptr(cache), page_size, n_heads, n_kv_heads, head_dim,
-             rot_dim, _ptr(inv_freq), mscale, np_, nb, nw, ne, int(w_static), _stream()), "gemm_skinny_rope")
+             rot_dim, _ptr(inv_freq), mscale, np_, nb, nw, ne, int(w_static), *_narrow_args(many, x), _stream()), "gemm_skinny_rope")
 
 
 def skinny_ok(M: int, K: int) -> bool:
