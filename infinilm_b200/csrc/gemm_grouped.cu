@@ -16,7 +16,7 @@
 
 // ---- bfloat16 on the tensor cores ---------------------------------------------------------------------------------
 namespace ggm {
-constexpr int BN = 64, BK = 64, STAGES = 3, ROW = BK * 2 + 16;      // a tile row: 64 bfloat16 and 16 bytes of padding (ldmatrix bank spread)
+constexpr int BN = 64, BK = 64, ROW = BK * 2 + 16;      // a tile row: 64 bfloat16 and 16 bytes of padding (ldmatrix bank spread)
 __device__ __forceinline__ void cp16(uint32_t dst, const void* src) { asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst), "l"(src)); }
 __device__ __forceinline__ void zero16(uint32_t dst) { asm volatile("st.shared.v4.u32 [%0], {%1,%1,%1,%1};\n" ::"r"(dst), "r"(0u)); }
 __device__ __forceinline__ void commit() { asm volatile("cp.async.commit_group;\n" ::); }
@@ -28,16 +28,16 @@ __device__ __forceinline__ void mma(float (&d)[4], const uint32_t (&a)[4], uint3
     asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
                  : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
-template <int BM, bool GLU> constexpr int smem_bytes() { return STAGES * (BM + (GLU ? 2 : 1) * BN) * ROW; }
+template <int BM, bool GLU, int STAGES> constexpr int smem_bytes() { return STAGES * (BM + (GLU ? 2 : 1) * BN) * ROW; }
 }  // namespace ggm
 
-template <int BM, bool GLU>
+template <int BM, bool GLU, int STAGES>
 __global__ void __launch_bounds__(128) gemm_grouped_mma_kernel(const __nv_bfloat16* A, int lda, long long a_gs, const int* a_rows,
                                                                const __nv_bfloat16* __restrict__ W, int ldw, long long w_gs,
                                                                __nv_bfloat16* __restrict__ C, int ldc, long long c_gs,
                                                                const int* group_off, int n_groups, int M, int N, int K,
                                                                const __nv_bfloat16* gate, int ld_gate, long long gate_gs, int gate_ns, const float* row_scale,
-                                                               int scale_by_place) {
+                                                               int scale_by_place, int early) {
     using namespace ggm;
     constexpr int MT = BM / 16, NW = GLU ? 2 : 1;
     constexpr int A_BYTES = BM * ROW, W_BYTES = BN * ROW, STAGE_BYTES = A_BYTES + NW * W_BYTES;
@@ -45,8 +45,8 @@ __global__ void __launch_bounds__(128) gemm_grouped_mma_kernel(const __nv_bfloat
     __shared__ int sh_g, sh_r0, sh_r1;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     int g, r0, r1;
-    if (group_off) {                              // (the groups' ranges come from the sort kernel before this one)
-        il_pdl_begin();
+    if (group_off) {                              // (the groups' ranges come from the sort kernel before this one, or, early, from one before that)
+        if (!early) il_pdl_begin();
         // The tile's group, by one warp, two groups a lane (one thread that walked the groups was a chain of up to n_groups reads in every
         // block, the surplus ones too; the rule that chooses the tile has the figures).
         if (warp == 0) {
@@ -55,7 +55,8 @@ __global__ void __launch_bounds__(128) gemm_grouped_mma_kernel(const __nv_bfloat
             __syncwarp();
             for (int g0 = 0; g0 < n_groups; g0 += 64) {
                 const int gg = g0 + 2 * lane;
-                const int o0 = group_off[min(gg, n_groups)], o1 = group_off[min(gg + 1, n_groups)], o2 = group_off[min(gg + 2, n_groups)];
+                // (through the L2: early, there was no wait behind which the SM's own cache holds nothing older)
+                const int o0 = __ldcg(group_off + min(gg, n_groups)), o1 = __ldcg(group_off + min(gg + 1, n_groups)), o2 = __ldcg(group_off + min(gg + 2, n_groups));
                 const int t0 = (o1 - o0 + BM - 1) / BM, t1 = (o2 - o1 + BM - 1) / BM;
                 int incl = t0 + t1;
 #pragma unroll
@@ -78,7 +79,10 @@ __global__ void __launch_bounds__(128) gemm_grouped_mma_kernel(const __nv_bfloat
         }
         __syncthreads();
         g = sh_g, r0 = sh_r0, r1 = sh_r1;
-        if (g >= n_groups) return;
+        if (g >= n_groups) {
+            if (early) il_pdl_wait();             // (no block leaves before the kernel in front is done: the next one counts on that)
+            return;
+        }
     } else {
         g = blockIdx.z, r0 = blockIdx.y * BM, r1 = M;
         il_pdl_begin();
@@ -137,6 +141,7 @@ __global__ void __launch_bounds__(128) gemm_grouped_mma_kernel(const __nv_bfloat
             }
 #pragma unroll
     for (int s = 0; s < STAGES - 1; ++s) issue_w(s);                     // the weights need no list of rows
+    if (early && group_off) il_pdl_begin();
 #pragma unroll
     for (int i = 0; i < A_CH; ++i) {
         const int ch = tid + i * 128, r = ch >> 3, p = r0 + r;
@@ -326,20 +331,22 @@ IL_EXPORT int il_gemm_grouped_max_tiles(int M, int n_groups) { return (M + 63) /
 template <int BM, bool GLU>
 static int launch_mma(const void* A, int lda, long long a_gs, const int* a_rows, const void* W, int ldw, long long w_gs, void* C, int ldc,
                       long long c_gs, const int* group_off, int n_groups, int M, int N, int K, const void* gate, int ld_gate, long long gate_gs,
-                      int gate_ns, const float* row_scale, int scale_by_place, cudaStream_t stream) {
-    constexpr int smem = ggm::smem_bytes<BM, GLU>();
+                      int gate_ns, const float* row_scale, int scale_by_place, int early, cudaStream_t stream) {
+    // Stages of the ring for few rows a group without a gate: four, so that four blocks fit on an SM. (8 tokens to 6 of 64 experts, 2,048 x 1,408 back,
+    // us with 3 / 4 / 5 stages and 5 / 4 / 3 blocks an SM: 42.8, 36.8, 41.4, the number of blocks that a last wave leaves over; 40 tokens 65.9, 67.0, 67.6.)
+    constexpr int STAGES = BM == 32 && !GLU ? 4 : 3, smem = ggm::smem_bytes<BM, GLU, STAGES>();
     static bool attr_set[64];
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev >= 0 && dev < 64 && !attr_set[dev]) {
-        cudaError_t e = cudaFuncSetAttribute(gemm_grouped_mma_kernel<BM, GLU>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        cudaError_t e = cudaFuncSetAttribute(gemm_grouped_mma_kernel<BM, GLU, STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
         if (e != cudaSuccess) return 1000 + (int)e;
         attr_set[dev] = true;
     }
     dim3 grid((N + ggm::BN - 1) / ggm::BN, group_off ? (M + BM - 1) / BM + n_groups : (M + BM - 1) / BM, group_off ? 1 : n_groups);
     if (grid.y > 65535 || grid.z > 65535) return IL_UNSUPPORTED;
-    IL_LAUNCH((gemm_grouped_mma_kernel<BM, GLU>), grid, 128, smem, stream, (const __nv_bfloat16*)A, lda, a_gs, a_rows, (const __nv_bfloat16*)W, ldw,
-              w_gs, (__nv_bfloat16*)C, ldc, c_gs, group_off, n_groups, M, N, K, (const __nv_bfloat16*)gate, ld_gate, gate_gs, gate_ns, row_scale, scale_by_place);
+    IL_LAUNCH((gemm_grouped_mma_kernel<BM, GLU, STAGES>), grid, 128, smem, stream, (const __nv_bfloat16*)A, lda, a_gs, a_rows, (const __nv_bfloat16*)W, ldw,
+              w_gs, (__nv_bfloat16*)C, ldc, c_gs, group_off, n_groups, M, N, K, (const __nv_bfloat16*)gate, ld_gate, gate_gs, gate_ns, row_scale, scale_by_place, early);
     IL_LAUNCH_CHECK();
     return IL_OK;
 }
@@ -347,7 +354,8 @@ static int launch_mma(const void* A, int lda, long long a_gs, const int* a_rows,
 IL_EXPORT int il_gemm_grouped(const void* A, int act_kind, int lda, long long a_gs, const int* a_rows, const void* W, int ldw, long long w_gs,
                               void* C, int ldc, long long c_gs, const int* group_off, int n_groups, int M, int N, int K, int glu,
                               const void* gate, int ld_gate, long long gate_gs, int gate_ns, const float* row_scale, int scale_by_place,
-                              cudaStream_t stream) {
+                              int early, cudaStream_t stream) {
+    // early: W and group_off were written before the kernel in front started, which may then still run while they are read.
     if (M <= 0 || N <= 0 || n_groups <= 0) return IL_OK;
     if (K <= 0 || (glu && gate)) return IL_BAD_ARG;
     if (act_kind == IL_BF16 && K % 8 == 0 && lda % 8 == 0 && ldw % 8 == 0 && a_gs % 8 == 0 && w_gs % 8 == 0 && !((uintptr_t)A & 15) &&
@@ -359,13 +367,13 @@ IL_EXPORT int il_gemm_grouped(const void* A, int act_kind, int lda, long long a_
         // they stage twice.) Batched, every group has M rows: tiles of 16 up to there.
         const bool few = group_off ? M <= 32 * n_groups : M <= 32;
         if (!group_off && M <= 16)
-            return glu ? launch_mma<16, true>(A, lda, a_gs, a_rows, W, ldw, w_gs, C, ldc, c_gs, group_off, n_groups, M, N, K, gate, ld_gate, gate_gs, gate_ns, row_scale, scale_by_place, stream)
-                       : launch_mma<16, false>(A, lda, a_gs, a_rows, W, ldw, w_gs, C, ldc, c_gs, group_off, n_groups, M, N, K, gate, ld_gate, gate_gs, gate_ns, row_scale, scale_by_place, stream);
+            return glu ? launch_mma<16, true>(A, lda, a_gs, a_rows, W, ldw, w_gs, C, ldc, c_gs, group_off, n_groups, M, N, K, gate, ld_gate, gate_gs, gate_ns, row_scale, scale_by_place, early, stream)
+                       : launch_mma<16, false>(A, lda, a_gs, a_rows, W, ldw, w_gs, C, ldc, c_gs, group_off, n_groups, M, N, K, gate, ld_gate, gate_gs, gate_ns, row_scale, scale_by_place, early, stream);
         if (glu)
-            return few ? launch_mma<32, true>(A, lda, a_gs, a_rows, W, ldw, w_gs, C, ldc, c_gs, group_off, n_groups, M, N, K, gate, ld_gate, gate_gs, gate_ns, row_scale, scale_by_place, stream)
-                       : launch_mma<64, true>(A, lda, a_gs, a_rows, W, ldw, w_gs, C, ldc, c_gs, group_off, n_groups, M, N, K, gate, ld_gate, gate_gs, gate_ns, row_scale, scale_by_place, stream);
-        return few ? launch_mma<32, false>(A, lda, a_gs, a_rows, W, ldw, w_gs, C, ldc, c_gs, group_off, n_groups, M, N, K, gate, ld_gate, gate_gs, gate_ns, row_scale, scale_by_place, stream)
-                   : launch_mma<64, false>(A, lda, a_gs, a_rows, W, ldw, w_gs, C, ldc, c_gs, group_off, n_groups, M, N, K, gate, ld_gate, gate_gs, gate_ns, row_scale, scale_by_place, stream);
+            return few ? launch_mma<32, true>(A, lda, a_gs, a_rows, W, ldw, w_gs, C, ldc, c_gs, group_off, n_groups, M, N, K, gate, ld_gate, gate_gs, gate_ns, row_scale, scale_by_place, early, stream)
+                       : launch_mma<64, true>(A, lda, a_gs, a_rows, W, ldw, w_gs, C, ldc, c_gs, group_off, n_groups, M, N, K, gate, ld_gate, gate_gs, gate_ns, row_scale, scale_by_place, early, stream);
+        return few ? launch_mma<32, false>(A, lda, a_gs, a_rows, W, ldw, w_gs, C, ldc, c_gs, group_off, n_groups, M, N, K, gate, ld_gate, gate_gs, gate_ns, row_scale, scale_by_place, early, stream)
+                   : launch_mma<64, false>(A, lda, a_gs, a_rows, W, ldw, w_gs, C, ldc, c_gs, group_off, n_groups, M, N, K, gate, ld_gate, gate_gs, gate_ns, row_scale, scale_by_place, early, stream);
     }
     dim3 grid((N + 63) / 64, group_off ? il_gemm_grouped_max_tiles(M, n_groups) : (M + 63) / 64, group_off ? 1 : n_groups);
     if (grid.y > 65535 || grid.z > 65535) return IL_UNSUPPORTED;

@@ -1410,7 +1410,8 @@ def moe_combine_resid(y: torch.Tensor, pos_of_slot: torch.Tensor, wt: torch.Tens
 
 def gemm_grouped(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, *, group_off: Optional[torch.Tensor] = None,
                  a_rows: Optional[torch.Tensor] = None, n_rows: Optional[int] = None, glu: bool = False,
-                 gate: Optional[torch.Tensor] = None, row_scale: Optional[torch.Tensor] = None, scale_by_place: bool = False) -> None:
+                 gate: Optional[torch.Tensor] = None, row_scale: Optional[torch.Tensor] = None, scale_by_place: bool = False,
+                 early: bool = False) -> None:
     """Products over groups, out_g = a_g w_g^T, w [G, N, K] (glu: [G, 2N, K], gate rows then up rows, out = silu(gate) * up).
     Ragged (`group_off` int32 [G + 1] on the device): the `n_rows` rows of `out` [n_rows, N] stand sorted by group, group g
     owning places group_off[g] .. group_off[g+1] - 1; the row of `a` [*, K] at a place is a_rows[place] (or the place).
@@ -1418,7 +1419,8 @@ def gemm_grouped(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, *, group_o
     out by its sigmoid; a gate [M, G] is one number per group and row.
     row_scale (ragged): float32 per row of `a` - or, with scale_by_place, per place of the sorted order; the products of a row
     are multiplied by its factor before the epilogue (the rstd of a norm the rows have not been divided by; the weight of a
-    choice that belongs to its expert's input)."""
+    choice that belongs to its expert's input).
+    early: w and group_off were written before the kernel launched just before this one started, and may be read while that one still runs."""
     _need_cuda(a, w, out, group_off, a_rows, gate, row_scale)
     if row_scale is not None and (group_off is None or row_scale.dtype != torch.float32 or not row_scale.is_contiguous()
                                   or row_scale.numel() < (int(n_rows if n_rows is not None else out.shape[0]) if scale_by_place else a.shape[0])):
@@ -1456,9 +1458,9 @@ def gemm_grouped(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, *, group_o
             ldg, g_gs = gate.stride(0), gate.stride(1)
     f = _fn("gemm_grouped", "il_gemm_grouped", [_c_void_p, _c_int, _c_int, _c_ll, _c_void_p, _c_void_p, _c_int, _c_ll, _c_void_p, _c_int,
                                                 _c_ll, _c_void_p, _c_int, _c_int, _c_int, _c_int, _c_int, _c_void_p, _c_int, _c_ll,
-                                                _c_int, _c_void_p, _c_int, _c_void_p])
+                                                _c_int, _c_void_p, _c_int, _c_int, _c_void_p])
     _check(f(_ptr(a), kind_of(a.dtype), lda, a_gs, _ptr(a_rows), _ptr(w), w.stride(1), w.stride(0), _ptr(out), ldc, c_gs, _ptr(group_off),
-             G, M, N, K, int(glu), _ptr(gate), ldg, g_gs, g_ns, _ptr(row_scale), int(scale_by_place), _stream()), "gemm_grouped")
+             G, M, N, K, int(glu), _ptr(gate), ldg, g_gs, g_ns, _ptr(row_scale), int(scale_by_place), int(early), _stream()), "gemm_grouped")
 
 
 # ----------------------------------------------------------------------------------------------

@@ -189,7 +189,7 @@ class RoutedExperts(FeedForward):
         else:
             ops.gemm_grouped(x if normed_in is None else x.xw, self.w_gate_up, act, group_off=group_off, a_rows=row_of_pos, n_rows=n_slots,
                              glu=True, row_scale=wt_of_pos if self.w_on_input else rstd, scale_by_place=self.w_on_input)
-            ops.gemm_grouped(act, self.w_down, y, group_off=group_off, n_rows=n_slots)
+            ops.gemm_grouped(act, self.w_down, y, group_off=group_off, n_rows=n_slots, early=True)     # (the sort was over when the product in front began)
         shared = self.shared.forward(x, ctx) if self.shared is not None else None
         if tail is not None:
             return ops.moe_combine_resid(y, pos_of_slot, wt, shared, tail.resid, tail.scale, tail.norm.weight, tail.norm.eps,
