@@ -455,17 +455,29 @@ IL_EXPORT int il_gemm_skinny_rope(const void* x, int ldx, const void* W, int ldw
 // y = alpha * x . W^T (+ bias), rounded to bfloat16 as the product alone would store it; resid += bscale * y (float32, in
 // place); xw = resid * norm_w as bfloat16; sumsq[m][block] = sum of resid^2 over the block's 16 columns. N = the width of
 // the residual stream. What add_rmsnorm does, but for the division by the rms, which the next product applies.
-template <int NT, int U, int WARPS, bool EARLY>
+// CL > 1: a cluster of CL blocks takes the 16 rows of W, CL * WARPS warps sharing K; all partial sums go to the first block's shared
+// memory, which finishes them.
+__device__ __forceinline__ void gs_cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;\n" ::: "memory"); }
+__device__ __forceinline__ void gs_cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory"); }
+__device__ __forceinline__ void gs_put2(float* p, float a, float b) {     // to the same place of the cluster's first block
+    uint32_t at;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(at) : "r"((uint32_t)__cvta_generic_to_shared(p)), "r"(0));
+    asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};\n" ::"r"(at), "f"(a), "f"(b) : "memory");
+}
+
+template <int NT, int U, int WARPS, bool EARLY, int CL>
 __global__ void __launch_bounds__(WARPS * 32, WARPS > 8 ? 1 : 2) gemm_skinny_resid_kernel(const __nv_bfloat16* x, int ldx,
                                                                           const __nv_bfloat16* __restrict__ W, int ldw,
                                                                           const float* __restrict__ bias, float alpha, int M, int N, int K,
                                                                           float* resid, float bscale, const void* __restrict__ norm_w,
                                                                           int norm_w_kind, __nv_bfloat16* __restrict__ xw,
                                                                           float* __restrict__ sumsq) {
-    __shared__ float part[WARPS][NT][16][8];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    constexpr int SHARES = CL * WARPS;
+    __shared__ __align__(8) float part[SHARES][NT][16][8];
+    const int rank = CL > 1 ? blockIdx.x % CL : 0, tile = blockIdx.x / CL;
+    const int warp = rank * WARPS + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     const int r = lane >> 2, c = lane & 3;
-    const int n0 = blockIdx.x * 16;
+    const int n0 = tile * 16;
     const __nv_bfloat16* wrow[2];
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
@@ -474,12 +486,13 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS > 8 ? 1 : 2) gemm_skinny_res
         wrow[h] = W + (size_t)n * ldw;
     }
     uint4 a[U][2], b[U][NT];
-    if (EARLY) gs_round_w<U, WARPS>(a, wrow, warp, c, K);
+    if (EARLY) gs_round_w<U, SHARES>(a, wrow, warp, c, K);
+    if (CL > 1) gs_cluster_arrive();              // (waited for before the first access to another block's memory)
     gs_begin<EARLY>();
     // What the epilogue adds to - the residual, the norm's weight, the bias of this thread's (row, column) - is asked for
     // now: read after the main loop it cost the kernel a round trip to memory at its very end.
     const int e_nl = threadIdx.x & 15, e_m = threadIdx.x >> 4, e_n = n0 + e_nl;
-    const bool e_live = (int)threadIdx.x < NT * 8 * 16 && e_m < M && e_n < N;
+    const bool e_live = rank == 0 && (int)threadIdx.x < NT * 8 * 16 && e_m < M && e_n < N;
     const float e_resid = e_live ? resid[(size_t)e_m * N + e_n] : 0.f;
     const float e_w = e_live ? il_load_any(norm_w, norm_w_kind, e_n) : 0.f;
     const float e_bias = (e_live && bias) ? bias[e_n] : 0.f;
@@ -493,23 +506,35 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS > 8 ? 1 : 2) gemm_skinny_res
         for (int q = 0; q < 4; ++q) acc[t][q] = 0.f;
     const int nkb = (K + 31) >> 5;
     if (EARLY) {
-        gs_round_x<NT, U, WARPS>(b, xrow, warp, c, K);
+        gs_round_x<NT, U, SHARES>(b, xrow, warp, c, K);
         gs_round_mma<NT, U>(acc, a, b);
     }
-    for (int kb0 = warp + (EARLY ? WARPS * U : 0); kb0 < nkb; kb0 += WARPS * U) {
+    for (int kb0 = warp + (EARLY ? SHARES * U : 0); kb0 < nkb; kb0 += SHARES * U) {
         uint4 a[U][2], b[U][NT];
-        gs_round_both<NT, U, WARPS>(a, b, wrow, xrow, kb0, c, K);
+        gs_round_both<NT, U, SHARES>(a, b, wrow, xrow, kb0, c, K);
         gs_round_mma<NT, U>(acc, a, b);
     }
     gs_tail<EARLY>();
+    if (CL > 1) {
+        gs_cluster_wait();
 #pragma unroll
-    for (int t = 0; t < NT; ++t) {
-        part[warp][t][r][c * 2] = acc[t][0];
-        part[warp][t][r][c * 2 + 1] = acc[t][1];
-        part[warp][t][r + 8][c * 2] = acc[t][2];
-        part[warp][t][r + 8][c * 2 + 1] = acc[t][3];
+        for (int t = 0; t < NT; ++t) {
+            gs_put2(&part[warp][t][r][c * 2], acc[t][0], acc[t][1]);
+            gs_put2(&part[warp][t][r + 8][c * 2], acc[t][2], acc[t][3]);
+        }
+        gs_cluster_arrive();
+        gs_cluster_wait();
+        if (rank > 0) return;
+    } else {
+#pragma unroll
+        for (int t = 0; t < NT; ++t) {
+            part[warp][t][r][c * 2] = acc[t][0];
+            part[warp][t][r][c * 2 + 1] = acc[t][1];
+            part[warp][t][r + 8][c * 2] = acc[t][2];
+            part[warp][t][r + 8][c * 2 + 1] = acc[t][3];
+        }
+        __syncthreads();
     }
-    __syncthreads();
     // one thread per (row, column): 16 consecutive lanes share a row and add up its squares by shuffles; warps beyond the
     // NT * 8 * 16 pairs have nothing to do and leave as a whole
     if ((int)threadIdx.x >= NT * 8 * 16) return;
@@ -520,7 +545,7 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS > 8 ? 1 : 2) gemm_skinny_res
     if (m < M && n < N) {
         float s0 = 0.f;
 #pragma unroll
-        for (int w = 0; w < WARPS; ++w) s0 += part[w][t][nl][mc];
+        for (int w = 0; w < SHARES; ++w) s0 += part[w][t][nl][mc];
         const float y = __bfloat162float(__float2bfloat16_rn(alpha * s0 + e_bias));
         h = e_resid + bscale * y;
         resid[(size_t)m * N + n] = h;
@@ -531,7 +556,7 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS > 8 ? 1 : 2) gemm_skinny_res
     sq += __shfl_xor_sync(0xffffffffu, sq, 4);
     sq += __shfl_xor_sync(0xffffffffu, sq, 2);
     sq += __shfl_xor_sync(0xffffffffu, sq, 1);
-    if (nl == 0 && m < M) sumsq[(size_t)m * gridDim.x + blockIdx.x] = sq;
+    if (nl == 0 && m < M) sumsq[(size_t)m * (gridDim.x / CL) + tile] = sq;
 }
 
 // N = width of the residual stream; sumsq gets [M][ceil(N / 16)] floats (at most 256 a row: N <= 4096).
@@ -542,21 +567,44 @@ IL_EXPORT int il_gemm_skinny_resid(const void* x, int ldx, const void* W, int ld
     if (M > 16 || K <= 0 || (K & 7) || (ldx & 7) || (ldw & 7) || ldx < K || ldw < K) return IL_UNSUPPORTED;
     if ((N + 15) / 16 > GS_NORM_MAX_PARTIALS || !resid || !norm_w || !xw || !sumsq) return IL_UNSUPPORTED;
     if (norm_w_kind != IL_F32 && norm_w_kind != IL_BF16) return IL_BAD_ARG;
-    const auto go = [&](auto kernel, int warps, bool early) {
-        return il_launch_as(w_static || !early, kernel, dim3((N + 15) / 16), dim3(warps * 32), 0, stream, (const __nv_bfloat16*)x, ldx, (const __nv_bfloat16*)W, ldw, bias, alpha,
-                         M, N, K, resid, bscale, norm_w, norm_w_kind, (__nv_bfloat16*)xw, sumsq);
+    const auto go = [&](auto kernel, int warps, bool early, int cluster) {
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3((N + 15) / 16 * cluster);
+        cfg.blockDim = dim3(warps * 32);
+        cfg.stream = stream;
+        cudaLaunchAttribute attr[2];
+        int n = 0;
+        if ((w_static || !early) && il_pdl_enabled()) {
+            attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+            attr[n++].val.programmaticStreamSerializationAllowed = 1;
+        }
+        if (cluster > 1) {
+            attr[n].id = cudaLaunchAttributeClusterDimension;
+            attr[n].val.clusterDim.x = cluster, attr[n].val.clusterDim.y = 1, attr[n].val.clusterDim.z = 1;
+            ++n;
+        }
+        cfg.attrs = attr;
+        cfg.numAttrs = n;
+        return cudaLaunchKernelEx(&cfg, kernel, (const __nv_bfloat16*)x, ldx, (const __nv_bfloat16*)W, ldw, bias, alpha, M, N, K, resid, bscale, norm_w,
+                                  norm_w_kind, (__nv_bfloat16*)xw, sumsq);
     };
-    const bool wide = K > GS_EARLY_K(8) && (N + 15) / 16 <= 148;      // fewer blocks than SMs: 16 warps a block
+    // Fewer tiles than SMs: 16 warps share K, in one block or, where that would leave half the SMs idle and for up to 8 rows, in a cluster of
+    // two: the same bits. (Us, one block and two, 1 / 8 / 16 rows: 1,024 x 4,096 3.8, 4.2, 5.5 and 3.3, 3.6, 4.8; a replayed step of 24 layers
+    // 1,024 wide 387 and 380 with one row, 509 and 480 with 8, 643 and 656 with 16. 2,048 x 8,192, 128 tiles, 8.2, 8.9, 9.7 and 7.5, 7.7, 9.0 by
+    // itself, but nothing in a step, where gate+up's blocks start later for it.)
+    const int tiles = (N + 15) / 16;
+    const bool wide = K > GS_EARLY_K(8) && tiles <= 148, pair = wide && tiles <= 74 && M <= 8;
     cudaError_t e;
     if (M <= 8)
-        e = wide                   ? go(gemm_skinny_resid_kernel<1, 8, 16, true>, 16, true)
-            : K <= GS_EARLY_K(4)   ? go(gemm_skinny_resid_kernel<1, 4, GS_WARPS, true>, GS_WARPS, true)
-            : K <= GS_EARLY_K(8)   ? go(gemm_skinny_resid_kernel<1, 8, GS_WARPS, true>, GS_WARPS, true)
-                                   : go(gemm_skinny_resid_kernel<1, 8, GS_WARPS, false>, GS_WARPS, false);
+        e = pair                   ? go(gemm_skinny_resid_kernel<1, 8, GS_WARPS, true, 2>, GS_WARPS, true, 2)
+            : wide                 ? go(gemm_skinny_resid_kernel<1, 8, 16, true, 1>, 16, true, 1)
+            : K <= GS_EARLY_K(4)   ? go(gemm_skinny_resid_kernel<1, 4, GS_WARPS, true, 1>, GS_WARPS, true, 1)
+            : K <= GS_EARLY_K(8)   ? go(gemm_skinny_resid_kernel<1, 8, GS_WARPS, true, 1>, GS_WARPS, true, 1)
+                                   : go(gemm_skinny_resid_kernel<1, 8, GS_WARPS, false, 1>, GS_WARPS, false, 1);
     else
-        e = wide                 ? go(gemm_skinny_resid_kernel<2, 4, 16, true>, 16, true)
-            : K <= GS_EARLY_K(4) ? go(gemm_skinny_resid_kernel<2, 4, GS_WARPS, true>, GS_WARPS, true)
-                                 : go(gemm_skinny_resid_kernel<2, 4, GS_WARPS, false>, GS_WARPS, false);
+        e = wide                 ? go(gemm_skinny_resid_kernel<2, 4, 16, true, 1>, 16, true, 1)
+            : K <= GS_EARLY_K(4) ? go(gemm_skinny_resid_kernel<2, 4, GS_WARPS, true, 1>, GS_WARPS, true, 1)
+                                 : go(gemm_skinny_resid_kernel<2, 4, GS_WARPS, false, 1>, GS_WARPS, false, 1);
     if (e != cudaSuccess) return 1000 + (int)e;
     IL_LAUNCH_CHECK();
     return IL_OK;
