@@ -250,9 +250,37 @@ __global__ void sigmoid_gate_kernel(TA* y, const TA* g, int ldg, int n, long lon
     }
 }
 
+// 16 bytes a thread and load (n, ldg multiples of that); the same arithmetic. 3,935 rows of 2,048 in bfloat16: 26.6 us one element at a
+// time, 11.8 so.
+template <typename TA>
+__global__ void sigmoid_gate_vec_kernel(TA* y, const TA* g, int ldg, int n_vec, long long total_vec) {
+    constexpr int VEC = 16 / sizeof(TA);
+    il_pdl_begin();
+    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total_vec; i += (long long)gridDim.x * blockDim.x) {
+        const long long t = i / n_vec;
+        const int c = (int)(i - t * n_vec) * VEC;
+        uint4 yq = reinterpret_cast<uint4*>(y)[i];
+        const uint4 gq = *reinterpret_cast<const uint4*>(g + (size_t)t * ldg + c);
+        TA* yp = reinterpret_cast<TA*>(&yq);
+        const TA* gp = reinterpret_cast<const TA*>(&gq);
+#pragma unroll
+        for (int k = 0; k < VEC; ++k) yp[k] = il_from_f<TA>(il_to_f(yp[k]) / (1.f + expf(-il_to_f(gp[k]))));
+        reinterpret_cast<uint4*>(y)[i] = yq;
+    }
+}
+
 IL_EXPORT int il_sigmoid_gate(void* y, int act_kind, const void* g, int ldg, int T, int n, cudaStream_t stream) {
     if (T <= 0 || n <= 0) return IL_OK;
     const long long total = (long long)T * n;
+    const int vec = act_kind == IL_F32 ? 4 : 8;
+    if ((act_kind == IL_F32 || act_kind == IL_BF16) && n % vec == 0 && ldg % vec == 0 && !(((uintptr_t)y | (uintptr_t)g) & 15)) {
+        const long long b = (total / vec + 255) / 256;
+        const int blocks = (int)(b > 148 * 32 ? 148 * 32 : b);
+        if (act_kind == IL_F32) IL_LAUNCH(sigmoid_gate_vec_kernel<float>, blocks, 256, 0, stream, (float*)y, (const float*)g, ldg, n / vec, total / vec);
+        else IL_LAUNCH(sigmoid_gate_vec_kernel<__nv_bfloat16>, blocks, 256, 0, stream, (__nv_bfloat16*)y, (const __nv_bfloat16*)g, ldg, n / vec, total / vec);
+        IL_LAUNCH_CHECK();
+        return IL_OK;
+    }
     const int blocks = (int)((total + 255) / 256 > 148 * 16 ? 148 * 16 : (total + 255) / 256);
     if (act_kind == IL_F32)
         IL_LAUNCH(sigmoid_gate_kernel<float>, blocks, 256, 0, stream, (float*)y, (const float*)g, ldg, n, total);

@@ -131,6 +131,22 @@ __global__ void add_bias_kernel(TA* __restrict__ y, const void* __restrict__ b, 
     }
 }
 
+// 16 bytes of y a thread (N a multiple of that, so a piece lies in one row); the bias stays in the caches. 4,096 and 904 rows
+// of 2,560 in bfloat16: 11.3 us on average one element at a time, 8.0 so.
+template <typename TA>
+__global__ void add_bias_vec_kernel(TA* __restrict__ y, const void* __restrict__ b, int b_kind, int n_vec, size_t total_vec) {
+    constexpr int VEC = 16 / sizeof(TA);
+    const size_t stride = (size_t)gridDim.x * blockDim.x;
+    for (size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x; idx < total_vec; idx += stride) {
+        uint4 q = reinterpret_cast<uint4*>(y)[idx];
+        TA* p = reinterpret_cast<TA*>(&q);
+        const int n = (int)(idx % n_vec) * VEC;
+#pragma unroll
+        for (int k = 0; k < VEC; ++k) p[k] = il_from_f<TA>(il_to_f(p[k]) + il_load_any(b, b_kind, n + k));
+        reinterpret_cast<uint4*>(y)[idx] = q;
+    }
+}
+
 static inline int grid_for(size_t total, int threads) {
     size_t g = (total + threads - 1) / threads;
     const size_t cap = 148 * 16;
@@ -174,6 +190,15 @@ IL_EXPORT int il_add_bias(void* y, int act_kind, const void* bias, int bias_kind
     if (T <= 0) return IL_OK;
     if (N <= 0) return IL_BAD_ARG;
     const size_t total = (size_t)T * N;
+    const int vec = act_kind == IL_F32 ? 4 : 8;
+    if ((act_kind == IL_F32 || act_kind == IL_BF16) && N % vec == 0 && !((uintptr_t)y & 15)) {
+        size_t g = (total / vec + 255) / 256;
+        if (g > 148 * 32) g = 148 * 32;
+        if (act_kind == IL_F32) add_bias_vec_kernel<float><<<(int)g, 256, 0, stream>>>((float*)y, bias, bias_kind, N / vec, total / vec);
+        else add_bias_vec_kernel<__nv_bfloat16><<<(int)g, 256, 0, stream>>>((__nv_bfloat16*)y, bias, bias_kind, N / vec, total / vec);
+        IL_LAUNCH_CHECK();
+        return IL_OK;
+    }
     const int threads = 256, grid = grid_for(total, threads);
     if (act_kind == IL_F32)
         add_bias_kernel<float><<<grid, threads, 0, stream>>>((float*)y, bias, bias_kind, N, total);
