@@ -439,7 +439,13 @@ static cudaError_t at_launch(const AtArgs& a) {
     // (wherever the other kernel is taken a head has at_fit(HDP) running sums)
     if (at_direct(HDP, HW, sizeof(TA), blocks, (long long)a.bt_stride * a.page_size)) return at_launch_direct<TA, HDP, SIG, CAP, at_fit(HDP)>(a);
     // Few (token, kv head) pairs, less than two blocks an SM: a warp for every sum.
-    if (sums == KS || blocks < 2 * 148) return at_launch_as<TA, HDP, SIG, CAP, 1>(a, HW, n_hb, sums);
+    if (sums == KS || blocks < 2 * 148) {
+        // Eight heads a block read their tiles from one SM's shared memory, which bounds a round of tiles; where SMs are idle four do (the same
+        // sums, so the same bits). 16 heads on 2 of 64, one to eight tokens over 66 / 450 / 2,000 keys, us: 6.3 / 20.2 / 75.6 with eight, 5.3 / 15.7 / 57.4
+        // with four, 5.5 / 16.0 / 57.7 with two, whose few threads bring the tiles in more slowly; 32 on 2 of 128: 9.5 / 33.3 / 128.5, 7.9 / 25.9 / 97.5.
+        const int hw = HW == 8 && (long long)a.T * a.nkv * ((G + 3) / 4) <= 148 ? 4 : HW;
+        return at_launch_as<TA, HDP, SIG, CAP, 1>(a, hw, (G + hw - 1) / hw, sums);
+    }
     if constexpr (HDP < 256) return at_launch_as<TA, HDP, SIG, CAP, 2>(a, HW, n_hb, KS);
     return cudaErrorInvalidValue;                 // (not reached: one sum a head at 256)
 }

@@ -395,6 +395,24 @@ def test_attention_plain_of_a_token_alone_and_among_others(cuda_device, nh, nkv,
     assert torch.equal(run(every[240:290]), among[240:290])
 
 
+@pytest.mark.parametrize("nh,nkv,hd", [(8, 1, 128), (13, 1, 64), (16, 2, 80), (32, 2, 128), (40, 4, 36)])
+def test_attention_plain_where_blocks_of_eight_heads_become_blocks_of_four(cuda_device, nh, nkv, hd):
+    """As many tokens as give the 148 SMs a block of four heads each, one fewer and one more, whole and ragged last blocks of heads: the reference, and
+    the bits of the same tokens among more."""
+    edge = 148 // (nkv * -(-(nh // nkv) // 4))
+    c = _attn_case("float32", nh, nkv, hd, [70, 0, 33], [edge - 1, 1, 40], None, 14, dominate=True)
+
+    def run(n):
+        out = torch.full((n, nh * hd), float("nan"), device="cuda")
+        ops.attention_plain(c["qkv"][:n], out, c["cache"], c["bt"], c["tok_pos"][:n], c["tok_entry"][:n], c["page"], nh, nkv, hd, 1 / math.sqrt(hd))
+        return out
+
+    among = run(c["T"])
+    close(among.cpu(), c["ref"], "float32")
+    for n in (1, edge - 1, edge, edge + 1):
+        assert torch.equal(run(n), among[:n]), n
+
+
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 @pytest.mark.parametrize("nh,nkv,hd", [(8, 8, 256), (6, 3, 256), (9, 3, 256), (8, 2, 200), (4, 4, 250), (20, 20, 80), (8, 4, 128), (5, 5, 65), (16, 16, 64), (16, 8, 64), (6, 6, 36), (7, 7, 33), (32, 32, 32),
                                        (9, 9, 10)])
