@@ -106,7 +106,7 @@ def test_groups_at_the_edges_of_tiles(cuda_device, N, K, glu):
 @pytest.mark.parametrize("T", [1, 8, 40])
 def test_early_reads_in_a_replayed_chain(cuda_device, T):
     """Layers of sort, gate+up and back product over the same buffers, the back product reading its weights and groups while gate+up still
-    runs: replayed as a graph, the bits of the same launches one at a time."""
+    runs: replayed as a graph, the bits of the same launches one at a time. (A choice's row is looked up by its place: the sort's atomics order an expert's rows.)"""
     from infinilm_b200 import ops
     E, top, W, F, L = 16, 4, 256, 192, 6
     g = torch.Generator().manual_seed(T)
@@ -114,19 +114,20 @@ def test_early_reads_in_a_replayed_chain(cuda_device, T):
     wgu = [(torch.randn(E, 2 * F, W, generator=g) / W ** 0.5).bfloat16().cuda() for _ in range(L)]
     wd = [(torch.randn(E, W, F, generator=g) / F ** 0.5).bfloat16().cuda() for _ in range(L)]
     x = torch.randn(T, W, generator=g).bfloat16().cuda()
-    off, pos, row = torch.empty(E + 1, dtype=torch.int32, device="cuda"), torch.empty(T * top, dtype=torch.int32, device="cuda"), torch.empty(T * top, dtype=torch.int32, device="cuda")
+    off, row = torch.empty(E + 1, dtype=torch.int32, device="cuda"), torch.empty(T * top, dtype=torch.int32, device="cuda")
+    pos = [torch.empty(T * top, dtype=torch.int32, device="cuda") for _ in range(L)]
     act, y = torch.empty(T * top, F, dtype=torch.bfloat16, device="cuda"), [torch.empty(T * top, W, dtype=torch.bfloat16, device="cuda") for _ in range(L)]
 
     def run(wait):
         for i in range(L):
-            ops.moe_sort(choices[i], E, off, pos, row)
+            ops.moe_sort(choices[i], E, off, pos[i], row)
             wait()
             ops.gemm_grouped(x, wgu[i], act, group_off=off, a_rows=row, n_rows=T * top, glu=True)
             wait()
             ops.gemm_grouped(act, wd[i], y[i], group_off=off, n_rows=T * top, early=True)
             wait()
     run(torch.cuda.synchronize)
-    want = [t.clone() for t in y]
+    want = [t[p.long()] for t, p in zip(y, pos)]
     graph = torch.cuda.CUDAGraph()
     with torch.cuda.graph(graph):
         run(lambda: None)
@@ -135,4 +136,4 @@ def test_early_reads_in_a_replayed_chain(cuda_device, T):
             t.zero_()
         graph.replay()
         torch.cuda.synchronize()
-        assert all(torch.equal(a, b) for a, b in zip(y, want))
+        assert all(torch.equal(t[p.long()], b) for t, p, b in zip(y, pos, want))
