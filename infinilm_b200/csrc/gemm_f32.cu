@@ -124,8 +124,8 @@ __device__ __forceinline__ void f32_mma(float (&d)[4], const uint32_t (&a)[4], u
 // NT: groups of 8 rows of A; STAGE: taken apart in shared memory. GLU: W holds N gate rows and then N up rows; a tile's 16 rows are 8 gate rows and the 8 up rows that go with
 // them, and the output is act(gate) * up as the SwiGLU kernel computes it from the two products (one launch less between a step's products).
 template <int NT, bool STAGE, bool VEC, bool GLU>
-__global__ void __launch_bounds__(FR_THREADS, 2) gemm_f32_rows_kernel(const float* A, int lda, const float* __restrict__ W, int ldw,
-                                                                      float* __restrict__ C, int ldc, const float* __restrict__ bias, float alpha,
+__global__ void __launch_bounds__(FR_THREADS, 2) gemm_f32_rows_kernel(const float* A, int lda, const float* W, int ldw,
+                                                                      float* C, int ldc, const float* bias, float alpha,
                                                                       int M, int N, int K, int tiles, int cluster, int early, int act, float limit, float act_alpha) {
     constexpr int OUT = FR_TILE * NT * 8;         // outputs of a tile: [row of W, of the first eight][which eight][row of A]; thread e adds up output e
     extern __shared__ __align__(16) unsigned char fr_sm[];
@@ -346,7 +346,7 @@ __device__ __forceinline__ void f32_columns(uint32_t (&r)[8], uint32_t taddr) {
 // SHARES 0: a block a tile; else K's number of shares, which the blocks of a cluster take one or two each.
 template <int SHARES, bool VEC>
 __global__ void __launch_bounds__(FT_THREADS, 1) gemm_f32_tile_kernel(const float* A, int lda, const float* W, int ldw,
-                                                                      float* C, int ldc, const float* __restrict__ bias, float alpha,
+                                                                      float* C, int ldc, const float* bias, float alpha,
                                                                       int M, int N, int K, int m_tiles, int units, int own, int early, int* status) {
     constexpr bool SPLIT = SHARES > 0;
     extern __shared__ __align__(1024) unsigned char smem_raw[];
