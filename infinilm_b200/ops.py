@@ -857,12 +857,13 @@ def _norm_args(norm_in: Optional[NormedInput], M: int):
 
 def gemm_skinny(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, alpha: float = 1.0,
                 bias: Optional[torch.Tensor] = None, glu: int = 0, norm_in: Optional[NormedInput] = None, act_params=None,
-                w_static: bool = False) -> None:
+                w_static: bool = False, cluster: int = 0) -> None:
     """out[M,N] = alpha * x[M,K] @ w[N,K]^T (+ bias) for M <= 16 bfloat16 rows (with a gate `skinny_glu_ok`); out bfloat16 or float32.
     glu (True, or ACT_SILU / ACT_GELU_TANH / ACT_CLAMPED with act_params): w is [2N,K] (gate rows, then up rows) and out[M,N] = act(gate) * up;
     ACT_RELU2: w is [N,K] and out is relu(.)^2 of the product (bfloat16).
     norm_in: x is `norm_in.xw`, and the results are divided by the rms that its sums give.
-    w_static: w is a model's weight, not what the kernel launched just before writes, and may be read while that kernel still runs."""
+    w_static: w is a model's weight, not what the kernel launched just before writes, and may be read while that kernel still runs.
+    cluster (more than 16 rows): blocks that share a tile of the tcgen05 form, 0 the kernel's choice, negative the form without tcgen05."""
     _need_cuda(x, w, out, bias)
     M, K = x.shape
     N = w.shape[0] // 2 if glu and int(glu) != ACT_RELU2 else w.shape[0]
@@ -880,7 +881,7 @@ def gemm_skinny(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, alpha: floa
                                                       _c_int, _c_int, _c_float, _c_float, _c_void_p, _c_int, _c_int, _c_float, _c_int, _c_int, _c_void_p, _c_void_p])
         np_, nb, nw, ne = _norm_args(norm_in, M)
         _check(f(_ptr(x), x.stride(0), _ptr(w), w.stride(0), _ptr(out), out.stride(0), _ptr(bias), alpha, M, N, K, int(glu), limit, act_alpha,
-                 np_, nb, nw, ne, int(w_static), narrow_cluster, _ptr(stream_status(x.device)), _stream()), "gemm_narrow_glu")
+                 np_, nb, nw, ne, int(w_static), cluster, _ptr(stream_status(x.device)), _stream()), "gemm_narrow_glu")
         return
     f = _fn("gemm_skinny", "il_gemm_skinny", [_c_void_p, _c_int, _c_void_p, _c_int, _c_void_p, _c_int, _c_int, _c_void_p,
                                               _c_float, _c_int, _c_int, _c_int, _c_int, _c_void_p, _c_int, _c_int, _c_float,
@@ -903,13 +904,6 @@ def gemm_skinny(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, alpha: floa
 NARROW_MAX_ROWS, NARROW_LONG_ROWS, NARROW_FROM, NARROW_WIDTH, NARROW_GLU_COLUMNS = 48, 32, 512, 1024, 148 * 32
 
 
-narrow_cluster = 0                                # blocks a tile of the narrow products' tcgen05 form: 0 the kernel's choice, negative the other form (tests)
-
-
-def _narrow_args(many: bool, x: torch.Tensor):
-    return (narrow_cluster, _ptr(stream_status(x.device))) if many else ()
-
-
 def narrow_ok(M: int, K: int) -> bool:
     """Whether the fused products of a model K wide take M rows, more than the few of `skinny_ok`."""
     return SKINNY_MAX_ROWS < M <= NARROW_MAX_ROWS and NARROW_FROM <= K <= NARROW_WIDTH and K % 8 == 0
@@ -929,11 +923,11 @@ def skinny_resid_ok(M: int, K: int, width: int) -> bool:
 
 def gemm_skinny_resid(x: torch.Tensor, w: torch.Tensor, alpha: float, bias: Optional[torch.Tensor], resid: torch.Tensor,
                       branch_scale: float, norm_weight: torch.Tensor, eps: float, xw: torch.Tensor,
-                      sumsq: torch.Tensor, w_static: bool = False) -> NormedInput:
+                      sumsq: torch.Tensor, w_static: bool = False, cluster: int = 0) -> NormedInput:
     """The last product of a branch (`skinny_resid_ok` bfloat16 rows) with the residual add and the next RMSNorm's inputs in its
     epilogue: resid (float32 [M,H], in place) += branch_scale * bf16(alpha * x @ w^T + bias); xw = resid * norm_weight;
     sumsq[m][b] = sum of resid[m]^2 over columns 16b..16b+15. Returns what the next product needs to finish the norm.
-    w_static: as for gemm_skinny."""
+    w_static, cluster: as for gemm_skinny."""
     _need_cuda(x, w, bias, resid, norm_weight, xw, sumsq)
     M, K = x.shape
     H = w.shape[0]
@@ -949,12 +943,12 @@ def gemm_skinny_resid(x: torch.Tensor, w: torch.Tensor, alpha: float, bias: Opti
     if bias is not None and (bias.dtype != torch.float32 or bias.numel() != H):
         raise KernelError("gemm_skinny_resid: bias float32 [H]")
     _contig("resid", resid), _contig("xw", xw), _contig("sumsq", sumsq), _contig("norm_weight", norm_weight)
-    many = M > SKINNY_MAX_ROWS
+    many = (cluster, _ptr(stream_status(x.device))) if M > SKINNY_MAX_ROWS else ()
     f = _fn("gemm_narrow" if many else "gemm_skinny", "il_gemm_narrow_resid" if many else "il_gemm_skinny_resid",
             [_c_void_p, _c_int, _c_void_p, _c_int, _c_void_p, _c_float, _c_int, _c_int, _c_int,
-             _c_void_p, _c_float, _c_void_p, _c_int, _c_void_p, _c_void_p, _c_int] + [_c_int, _c_void_p] * many + [_c_void_p])
+             _c_void_p, _c_float, _c_void_p, _c_int, _c_void_p, _c_void_p, _c_int] + [_c_int, _c_void_p][:len(many)] + [_c_void_p])
     _check(f(_ptr(x), x.stride(0), _ptr(w), w.stride(0), _ptr(bias), alpha, M, H, K, _ptr(resid), branch_scale, _ptr(norm_weight),
-             kind_of(norm_weight.dtype), _ptr(xw), _ptr(sumsq), int(w_static), *_narrow_args(many, x), _stream()), "gemm_skinny_resid")
+             kind_of(norm_weight.dtype), _ptr(xw), _ptr(sumsq), int(w_static), *many, _stream()), "gemm_skinny_resid")
     return NormedInput(xw, sumsq, H, eps)
 
 
@@ -967,10 +961,10 @@ def gemm_skinny_rope(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, alpha:
                      tok_pos: torch.Tensor, tok_entry: torch.Tensor, block_table: torch.Tensor, cache: Optional[torch.Tensor],
                      page_size: int, n_heads: int, n_kv_heads: int, head_dim: int, rot_dim: int,
                      inv_freq: Optional[torch.Tensor], mscale: float, norm_in: Optional[NormedInput] = None,
-                     w_static: bool = False) -> None:
+                     w_static: bool = False, cluster: int = 0) -> None:
     """The q/k/v projection of a few bfloat16 rows (`skinny_rope_ok`) with what `rope_store` does in its epilogue: out[M, (heads + 2
     kv_heads) * head_dim] = alpha * x @ w^T (+ bias), q and k rotated, k and v written to their cache slots (if `cache`).
-    w_static: as for gemm_skinny."""
+    w_static, cluster: as for gemm_skinny."""
     _need_cuda(x, w, out, bias, tok_pos, tok_entry, block_table, cache, inv_freq)
     M, K = x.shape
     N = (n_heads + 2 * n_kv_heads) * head_dim
@@ -989,15 +983,15 @@ def gemm_skinny_rope(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, alpha:
         _contig("cache", cache)
         if cache.dtype != torch.bfloat16 or tuple(cache.shape[1:]) != (2, n_kv_heads, page_size, head_dim):
             raise KernelError("gemm_skinny_rope: cache bfloat16 [pages,2,kv_heads,page,head_dim]")
-    many = M > SKINNY_MAX_ROWS
+    many = (cluster, _ptr(stream_status(x.device))) if M > SKINNY_MAX_ROWS else ()
     f = _fn("gemm_narrow" if many else "gemm_skinny", "il_gemm_narrow_rope" if many else "il_gemm_skinny_rope",
             [_c_void_p, _c_int, _c_void_p, _c_int, _c_void_p, _c_int, _c_void_p, _c_float, _c_int, _c_int, _c_void_p, _c_void_p,
              _c_void_p, _c_int, _c_void_p, _c_int, _c_int, _c_int, _c_int, _c_int, _c_void_p, _c_float, _c_void_p, _c_int, _c_int,
-             _c_float, _c_int] + [_c_int, _c_void_p] * many + [_c_void_p])
+             _c_float, _c_int] + [_c_int, _c_void_p][:len(many)] + [_c_void_p])
     np_, nb, nw, ne = _norm_args(norm_in, M)
     _check(f(_ptr(x), x.stride(0), _ptr(w), w.stride(0), _ptr(out), out.stride(0), _ptr(bias), alpha, M, K, _ptr(tok_pos),
              _ptr(tok_entry), _ptr(block_table), block_table.shape[1], _ptr(cache), page_size, n_heads, n_kv_heads, head_dim,
-             rot_dim, _ptr(inv_freq), mscale, np_, nb, nw, ne, int(w_static), *_narrow_args(many, x), _stream()), "gemm_skinny_rope")
+             rot_dim, _ptr(inv_freq), mscale, np_, nb, nw, ne, int(w_static), *many, _stream()), "gemm_skinny_rope")
 
 
 def skinny_ok(M: int, K: int) -> bool:

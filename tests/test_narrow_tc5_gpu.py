@@ -9,10 +9,8 @@ pytestmark = pytest.mark.gpu
 
 @pytest.fixture
 def cut(request):
-    from infinilm_b200 import ops
-    ops.narrow_cluster = request.param
     yield request.param
-    ops.narrow_cluster = 0
+    from infinilm_b200 import ops
     ops.check_status(torch.device("cuda:0"))
 
 
@@ -30,7 +28,7 @@ def test_gated(cuda_device, cut, M, N, K):
     b = torch.randn(2 * N, device="cuda", generator=g) * 0.1 if M % 2 else None
     sq = (torch.rand(M, 64, device="cuda", generator=g) + 0.5) * 16
     out = torch.full((M, N + 2), float("nan"), device="cuda", dtype=torch.bfloat16)
-    ops.gemm_skinny(x, w, out[:, :N], 0.7, b, glu=1, norm_in=ops.NormedInput(x, sq, 1024, 1e-5), w_static=bool(M % 2))
+    ops.gemm_skinny(x, w, out[:, :N], 0.7, b, glu=1, norm_in=ops.NormedInput(x, sq, 1024, 1e-5), w_static=bool(M % 2), cluster=cut)
     z = 0.7 * torch.rsqrt(sq.double().sum(1, keepdim=True) / 1024 + 1e-5) * (x.double() @ w.double().t()) + (b.double() if b is not None else 0.0)
     ref = z[:, :N] * torch.sigmoid(z[:, :N]) * z[:, N:]
     assert _rel(out[:, :N], ref) <= 2.0 ** -8 and bool(out[:, N:].isnan().all())     # rounded to bfloat16 once
@@ -46,7 +44,7 @@ def test_into_the_residual(cuda_device, cut, M, N, K):
     b = torch.randn(N, device="cuda", generator=g) if M % 2 else None
     r0, nw = torch.randn(M, N, device="cuda", generator=g), 1 + 0.3 * torch.randn(N, device="cuda", generator=g)
     r, xw, sq = r0.clone(), torch.empty(M, N, device="cuda", dtype=torch.bfloat16), torch.empty(M, (N + 15) // 16, device="cuda")
-    ops.gemm_skinny_resid(x, w, 0.6, b, r, 0.35, nw, 1e-5, xw, sq, w_static=True)
+    ops.gemm_skinny_resid(x, w, 0.6, b, r, 0.35, nw, 1e-5, xw, sq, w_static=True, cluster=cut)
     y = 0.6 * (x.double() @ w.double().t()) + (b.double() if b is not None else 0.0)
     assert float((r.double() - (r0.double() + 0.35 * y)).abs().amax()) <= 2.0 ** -8 * 0.35 * float(y.abs().amax())     # the branch is rounded to bfloat16
     assert _rel(xw, r.double() * nw.double()) <= 2.0 ** -8
@@ -76,7 +74,7 @@ def test_rotated_and_stored(cuda_device, cut, nh, nkv, hd, M, with_cache):
     ops.rope_store(ref, pos, ent, bt, caches[0], page, nh, nkv, hd, hd, inv, 1.1)
     out = torch.full((M, N), float("nan"), device="cuda", dtype=torch.bfloat16)
     ops.gemm_skinny_rope(x, w, out, 0.75, bias, pos, ent, bt, caches[1] if with_cache else None, page, nh, nkv, hd, hd, inv, 1.1,
-                         norm_in=ops.NormedInput(x, sq, 528, 1e-5), w_static=True)
+                         norm_in=ops.NormedInput(x, sq, 528, 1e-5), w_static=True, cluster=cut)
     scale = float(ref.float().abs().amax())
     assert float((out.float() - ref.float()).abs().amax()) <= 2.0 ** -7 * scale
     if with_cache:
