@@ -128,7 +128,7 @@ __global__ void rope_store_kernel(TA* __restrict__ qkv, int row_stride, const in
     }
 }
 
-// The same for many tokens (prompt portions): a block's latency does not matter there, how many blocks an SM holds
+// The same for many tokens (prompt portions) where the pairs are not whole 16-byte pieces: a block's latency does not matter there, how many blocks an SM holds
 // does; two passes (rotate in place, then copy k and v to the cache in 16-byte pieces), 256 threads, few registers.
 template <typename TA>
 __global__ void rope_store_many_kernel(TA* __restrict__ qkv, int row_stride, const int* __restrict__ tok_pos,
@@ -192,6 +192,111 @@ __global__ void rope_store_many_kernel(TA* __restrict__ qkv, int row_stride, con
     }
 }
 
+// The same where the rotated pairs come in whole 16-byte pieces: one pass, a thread an item (a piece of the first half of a
+// rotated head and the piece it pairs with, a piece of v, or a piece of k that is not rotated), several tokens a block where a
+// token has few items. The row has just been written and lies in the L2, so what bounds it is loads in flight: the first of a
+// thread are asked for before the angles are computed (8B sizes, 2,048 tokens, without that 10.5 us).
+// Two passes before / so, us: 32 heads on 2 of 128 bfloat16, 600 / 2,048 / 8,192 tokens 4.2 / 9.2 / 32.1 and 3.6 / 8.1 / 27.4; 16 on 2 of 64 2.9 / 5.7 /
+// 16.5 and 2.7 / 3.5 / 9.9; the same in float32 2.9 / 5.7 / 16.4 and 2.9 / 5.3 / 15.8; 65 tokens 2.4 to 3.1 and 2.3 to 2.4.
+constexpr int ROPE_WIDE_TOKENS = 8;
+template <typename TA>
+__global__ void __launch_bounds__(512) rope_store_wide_kernel(TA* qkv, int row_stride, const int* tok_pos, const int* tok_entry, const int* block_table, int bt_stride,
+                                                              TA* cache, int page_size, int T, int nh, int nkv, int hd, int rot, const float* inv_freq, float mscale,
+                                                              int tokens, int items) {
+    constexpr int VEC = 16 / sizeof(TA);
+    __shared__ __align__(16) float cs[ROPE_WIDE_TOKENS * 128], sn[ROPE_WIDE_TOKENS * 128];        // rot <= head_dim <= 256
+    __shared__ TA* slot[ROPE_WIDE_TOKENS];        // a token's K slot of kv head 0, or null: nothing to store
+    const int t0 = blockIdx.x * tokens, n = min(tokens, T - t0), half = rot >> 1;
+    const size_t head_step = (size_t)page_size * hd;
+    const int hp = half / VEC, n_rot = (nh + nkv) * hp, cpr = hd / VEC, tail = (hd - rot) / VEC;
+    struct Item { TA* from; int tok, head, i, step; };      // step: columns to the piece it is rotated with, 0: none, it is copied; i: its column in a slot
+    const auto item = [&](int idx) {
+        Item it;
+        it.tok = idx / items;
+        int k = idx - it.tok * items;
+        TA* const row = qkv + (size_t)(t0 + it.tok) * row_stride;
+        if (k < n_rot) {
+            const int j = k / hp;
+            it.i = (k - j * hp) * VEC, it.head = j - nh, it.step = half;
+            it.from = row + (size_t)j * hd + it.i;
+        } else {                                  // v (kv heads nkv .. 2 nkv - 1), then what the rotation does not touch of k
+            k -= n_rot;
+            const bool v = k < nkv * cpr;
+            if (!v) k -= nkv * cpr;
+            const int per = v ? cpr : tail, g = k / per;
+            it.i = (v ? 0 : rot) + (k - g * per) * VEC, it.head = (v ? nkv : 0) + g, it.step = 0;
+            it.from = row + (size_t)(nh + it.head) * hd + it.i;
+        }
+        return it;
+    };
+    il_pdl_begin();
+    // the first item's pieces are on their way while the angles are computed
+    int idx = threadIdx.x;
+    Item it;
+    uint4 a, b;
+    if (idx < n * items) {
+        it = item(idx);
+        a = *reinterpret_cast<const uint4*>(it.from);
+        if (it.step) b = *reinterpret_cast<const uint4*>(it.from + half);
+    }
+    for (int i = threadIdx.x; i < n * half; i += blockDim.x) {
+        const int tok = i / half;
+        float s, c;
+        sincosf((float)tok_pos[t0 + tok] * inv_freq[i - tok * half], &s, &c);
+        sn[i] = s * mscale;
+        cs[i] = c * mscale;
+    }
+    if (threadIdx.x < n) {
+        TA* at = nullptr;
+        if (cache) {
+            const int pos = tok_pos[t0 + threadIdx.x], page = block_table[(size_t)tok_entry[t0 + threadIdx.x] * bt_stride + pos / page_size];
+            if (page >= 0) at = cache + (size_t)page * 2 * nkv * head_step + (size_t)(pos % page_size) * hd;     // the host reserves every page a step touches
+        }
+        slot[threadIdx.x] = at;
+    }
+    __syncthreads();
+    while (idx < n * items) {
+        TA* const at = slot[it.tok];
+        TA* const to = at + (size_t)it.head * head_step + it.i;       // (K's heads, then V's)
+        if (it.step) {
+            TA *ap = reinterpret_cast<TA*>(&a), *bp = reinterpret_cast<TA*>(&b);
+            const float *c = cs + it.tok * half + it.i, *s = sn + it.tok * half + it.i;
+#pragma unroll
+            for (int e = 0; e < VEC; ++e) {
+                const float x1 = il_to_f(ap[e]), x2 = il_to_f(bp[e]);
+                ap[e] = il_from_f<TA>(x1 * c[e] - x2 * s[e]);
+                bp[e] = il_from_f<TA>(x2 * c[e] + x1 * s[e]);
+            }
+            *reinterpret_cast<uint4*>(it.from) = a;
+            *reinterpret_cast<uint4*>(it.from + half) = b;
+            if (it.head >= 0 && at) {
+                *reinterpret_cast<uint4*>(to) = a;
+                *reinterpret_cast<uint4*>(to + half) = b;
+            }
+        } else if (at) {
+            *reinterpret_cast<uint4*>(to) = a;
+        }
+        idx += blockDim.x;
+        if (idx < n * items) {
+            it = item(idx);
+            a = *reinterpret_cast<const uint4*>(it.from);
+            if (it.step) b = *reinterpret_cast<const uint4*>(it.from + half);
+        }
+    }
+}
+template <typename TA>
+static int rope_store_wide(void* qkv, int row_stride, const int* tok_pos, const int* tok_entry, const int* block_table, int bt_stride, void* cache, int page_size, int T,
+                           int nh, int nkv, int hd, int rot, const float* inv_freq, float mscale, cudaStream_t stream) {
+    constexpr int VEC = 16 / sizeof(TA);
+    const int items = (nh + nkv) * (rot / 2 / VEC) + (cache ? nkv * ((2 * hd - rot) / VEC) : 0);
+    if (items == 0) return IL_OK;
+    const int tokens = items > 256 / 2 ? 1 : min(256 / items, ROPE_WIDE_TOKENS), threads = min((tokens * items + 31) / 32 * 32, 512);
+    IL_LAUNCH(rope_store_wide_kernel<TA>, (T + tokens - 1) / tokens, threads, 0, stream, (TA*)qkv, row_stride, tok_pos, tok_entry, block_table, bt_stride, (TA*)cache,
+              page_size, T, nh, nkv, hd, rot, inv_freq, mscale, tokens, items);
+    IL_LAUNCH_CHECK();
+    return IL_OK;
+}
+
 IL_EXPORT int il_rope_store(void* qkv, int act_kind, int row_stride, const int* tok_pos, const int* tok_entry,
                             const int* block_table, int bt_stride, void* cache, int page_size, int T, int nh,
                             int nkv, int hd, int rot, const float* inv_freq, float mscale, cudaStream_t stream) {
@@ -201,6 +306,11 @@ IL_EXPORT int il_rope_store(void* qkv, int act_kind, int row_stride, const int* 
     if (row_stride < (nh + 2 * nkv) * hd || hd % 16 != 0 || row_stride % 8 != 0) return IL_BAD_ARG;
     constexpr int MANY = 64;                      // from here on: the two-pass kernel for throughput
     if (T > MANY) {
+        const int vec = act_kind == IL_F32 ? 4 : 8;
+        if ((act_kind == IL_F32 || act_kind == IL_BF16) && rot % (2 * vec) == 0 && !(((uintptr_t)qkv | (uintptr_t)cache) & 15)) {
+            const auto wide = act_kind == IL_F32 ? rope_store_wide<float> : rope_store_wide<__nv_bfloat16>;
+            return wide(qkv, row_stride, tok_pos, tok_entry, block_table, bt_stride, cache, page_size, T, nh, nkv, hd, rot, inv_freq, mscale, stream);
+        }
         if (act_kind == IL_F32)
             IL_LAUNCH(rope_store_many_kernel<float>, T, 256, 0, stream, (float*)qkv, row_stride, tok_pos, tok_entry, block_table, bt_stride,
                       (float*)cache, page_size, nh, nkv, hd, rot, inv_freq, mscale);
