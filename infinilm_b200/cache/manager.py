@@ -49,6 +49,16 @@ class PagePool:
         self._held[p] = True
         return p
 
+    def take(self, n: int) -> List[int]:
+        """`n` pages at once, all or none: the ones that as many calls of `alloc` would give."""
+        if n > len(self._free):
+            raise OutOfPages(f"{n} pages wanted, {len(self._free)} free")
+        pop, held = self._free.popleft, self._held
+        pages = [pop() for _ in range(n)]
+        for p in pages:
+            held[p] = True
+        return pages
+
     def free(self, page: int) -> None:
         if not (0 <= page < self.n_pages) or not self._held[page]:
             raise CacheStateError(f"page {page} freed while not held")
@@ -101,7 +111,7 @@ class PageTable(list):
     that a step can copy the table into its descriptors without walking it: with hundreds of live requests, lists turned
     into arrays every step were most of a decode step's host time. The array is what the kernels read: a page of the
     manager is `sub` kernel pages that lie one behind the other, so page p stands there as p*sub .. p*sub+sub-1.
-    `append`, `tbl[i] = p` and `clear` keep the array in step; any other change marks it stale and `array()` rebuilds it."""
+    `append`, `extend`, `tbl[i] = p` and `clear` keep the array in step; any other change marks it stale and `array()` rebuilds it."""
 
     def __init__(self, *a, sub: int = 1):
         super().__init__(*a)
@@ -123,11 +133,26 @@ class PageTable(list):
     def append(self, p) -> None:
         n = len(self)
         super().append(p)
+        if self._stale:
+            return
         if (n + 1) * self.sub > self._arr.shape[0]:
             grown = np.empty(2 * self._arr.shape[0], dtype=np.int32)
             grown[:n * self.sub] = self._arr[:n * self.sub]
             self._arr = grown
         self._put(n, p)
+
+    def extend(self, pages) -> None:
+        n, pages = len(self), list(pages)
+        super().extend(pages)
+        if self._stale:
+            return
+        sub, end = self.sub, len(self) * self.sub
+        if end > self._arr.shape[0]:
+            grown = np.empty(max(2 * self._arr.shape[0], end), dtype=np.int32)
+            grown[:n * sub] = self._arr[:n * sub]
+            self._arr = grown
+        new = np.array(pages, dtype=np.int32)
+        self._arr[n * sub:end] = new if sub == 1 else np.where(new[:, None] < 0, -1, new[:, None] * sub + self._steps).ravel()
 
     def __setitem__(self, i, p) -> None:
         super().__setitem__(i, p)
@@ -145,7 +170,7 @@ class PageTable(list):
             self._stale = True
             return getattr(list, name)(self, *a, **k)
         return f
-    extend, insert, pop, remove = _touched("extend"), _touched("insert"), _touched("pop"), _touched("remove")
+    insert, pop, remove = _touched("insert"), _touched("pop"), _touched("remove")
     reverse, sort = _touched("reverse"), _touched("sort")
     __delitem__, __iadd__, __imul__ = _touched("__delitem__"), _touched("__iadd__"), _touched("__imul__")
     del _touched
@@ -311,8 +336,10 @@ class CacheManager:
                 raise OutOfPages(f"request {seq.seq_id!r} needs {n} more page(s) in cache group {g}, "
                                  f"{self.groups[g].pool.n_free} are free")
         for g, n in need.items():
-            for _ in range(n):
+            if n == 1:                            # a decode step's page
                 seq.tables[g].append(self.groups[g].pool.alloc())
+            elif n > 1:
+                seq.tables[g].extend(self.groups[g].pool.take(n))
 
     def commit(self, seq: SequenceCache, new_len: int) -> None:
         """The step that wrote positions < new_len has been issued: advance the length and give

@@ -10,6 +10,7 @@ from __future__ import annotations
 import ctypes
 from typing import Optional
 
+import numpy as np
 import torch
 
 from .csrc import build
@@ -1458,6 +1459,9 @@ def gemm_grouped(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, *, group_o
 
 
 # ----------------------------------------------------------------------------------------------
+_NP_DTYPES = {n: np.dtype(n) for n in ("int32", "int64", "uint8", "uint64")}
+
+
 def _np_ptr(a) -> _c_void_p:
     return _c_void_p(a.ctypes.data)
 
@@ -1475,7 +1479,7 @@ def step_fill(out, out_cap: int, E: int, Ep: int, Tp: int, order, n_tok, start, 
                         ("widths", widths, "int32"), ("tbl_ptr", tbl_ptr, "uint64"), ("tbl_len", tbl_len, "int32"),
                         ("scratch_page", scratch_page, "int32"), ("want", want, "int32"), ("want_off", want_off, "int32"),
                         ("offsets", offsets, "int32"), ("outs", outs, "int32"), ("out", out, "int32")):
-        if a.dtype.name != dt or not a.flags["C_CONTIGUOUS"]:
+        if a.dtype != _NP_DTYPES[dt] or not a.flags["C_CONTIGUOUS"]:
             raise KernelError(f"step_fill: {name} must be a contiguous {dt} array")
     if (len(order) != E or len(n_tok) != E or len(start) != E or len(slot) != E or len(fresh) != E or len(tok_off) != E + 1
             or len(want_off) != E + 1 or tbl_ptr.size != widths.size * E or tbl_len.size != widths.size * E
