@@ -97,7 +97,26 @@ __device__ __forceinline__ uint32_t pt_pack(float lo, float hi) {
     return *reinterpret_cast<uint32_t*>(&v);
 }
 
-template <bool SIG, bool LOGB, bool CAP>
+__device__ __forceinline__ void pt_cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+}
+__device__ __forceinline__ uint32_t pt_peer_of(uint32_t addr) {      // where the cluster's second block has it
+    uint32_t at;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, 1;\n" : "=r"(at) : "r"(addr));
+    return at;
+}
+__device__ __forceinline__ float pt_peer(uint32_t at) {
+    float v;
+    asm volatile("ld.shared::cluster.f32 %0, [%1];\n" : "=f"(v) : "r"(at) : "memory");
+    return v;
+}
+// Where the rows' sums of the second block lie for the first (over Q, P and the ring, which nothing reads any more): column c of row r,
+// and behind them m and l.
+constexpr int PT_SPLIT_ML = PT_ROWS * PT_HD * 4, PT_SPLIT_FROM = 4;
+static_assert(PT_SPLIT_ML + PT_ROWS * 8 <= PT_Q_BYTES + PT_P_BYTES + (PT_K_STAGES + PT_V_STAGES) * PT_K_BYTES, "the second block's sums");
+
+// SPLIT: a cluster of two blocks takes the tokens of one, each half of the key tiles (where there are PT_SPLIT_FROM; else the second leaves).
+template <bool SIG, bool LOGB, bool CAP, bool SPLIT = false>
 __global__ void __launch_bounds__(PT_THREADS, PT_BLOCKS_PER_SM) attn_prefill_tc5_kernel(
     const __grid_constant__ CUtensorMap kv_map, const __nv_bfloat16* __restrict__ qkv, int row_stride,
     __nv_bfloat16* __restrict__ out, const int* __restrict__ block_table, int bt_stride, const int* __restrict__ entry_qstart,
@@ -115,7 +134,8 @@ __global__ void __launch_bounds__(PT_THREADS, PT_BLOCKS_PER_SM) attn_prefill_tc5
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
     // which entry and which tokens: tiles are taken from the last to the first, the longest blocks start first
-    int tile = (int)gridDim.x - 1 - (int)blockIdx.x, e = first_entry;
+    const int rank = SPLIT ? (int)blockIdx.x & 1 : 0;
+    int tile = SPLIT ? ((int)gridDim.x - 1 - (int)blockIdx.x) >> 1 : (int)gridDim.x - 1 - (int)blockIdx.x, e = first_entry;
     for (; e < n_entries; ++e) {
         const int nt = (entry_qstart[e + 1] - entry_qstart[e] + tpt - 1) / tpt;
         if (tile < nt) break;
@@ -131,8 +151,17 @@ __global__ void __launch_bounds__(PT_THREADS, PT_BLOCKS_PER_SM) attn_prefill_tc5
     const int* bt = block_table + (size_t)e * bt_stride;
     const int bpos_first = start_pos + (tok0 - q0), bpos_last = bpos_first + n_tok - 1;
     const int blo = il_mask_lo(bpos_first, window);
-    const int page_first = blo / PT_PAGE, page_last = bpos_last / PT_PAGE;
-    const int n_tiles = (page_last - page_first) / PT_TILE_PAGES + 1;
+    const int page_last = bpos_last / PT_PAGE;
+    int page_first = blo / PT_PAGE, n_tiles = (page_last - page_first) / PT_TILE_PAGES + 1;
+    const bool split = SPLIT && n_tiles >= PT_SPLIT_FROM;
+    if (SPLIT) {
+        if (!split && rank) return;               // the whole block
+        if (split) {
+            const int first = (n_tiles + 1) >> 1;
+            if (rank) page_first += first * PT_TILE_PAGES;
+            n_tiles = rank ? n_tiles - first : first;
+        }
+    }
 
     unsigned char* q_smem = smem;
     unsigned char* p_smem = smem + PT_Q_BYTES;
@@ -216,6 +245,10 @@ __global__ void __launch_bounds__(PT_THREADS, PT_BLOCKS_PER_SM) attn_prefill_tc5
             ok = issue(j, 1);
             if (ok && j + 2 < n_tiles) ok = issue(j + 2, 0);
         }
+        if (split) {
+            __syncwarp();
+            pt_cluster_sync(), pt_cluster_sync();
+        }
     } else if (warp == 1) {
         // ---------------- tensor-core issue, scores: S(j) as soon as K(j) is there and the buffer has been read out ----------------
         // Two issuing threads, one for each kind of product: a wait on an mbarrier costs the thread about 200 clocks
@@ -247,6 +280,10 @@ __global__ void __launch_bounds__(PT_THREADS, PT_BLOCKS_PER_SM) attn_prefill_tc5
                 t5_commit(k_empty0 + 8 * s);                  // and the K slot is free
             }
         }
+        if (split) {
+            __syncwarp();
+            pt_cluster_sync(), pt_cluster_sync();
+        }
     } else if (warp == 2) {
         // ---------------- tensor-core issue, outputs: O += P.V(j) as soon as P(j) and V(j) are there ----------------
         if (lane == 0) {
@@ -266,6 +303,10 @@ __global__ void __launch_bounds__(PT_THREADS, PT_BLOCKS_PER_SM) attn_prefill_tc5
                 t5_commit(v_empty0 + 8 * s);                  // the V slot is free once these products have read it
                 t5_commit(o_done);                            // and so is P's place
             }
+        }
+        if (split) {
+            __syncwarp();
+            pt_cluster_sync(), pt_cluster_sync();
         }
     } else {
         // ---------------- softmax and output: warps 3..6 own tensor-memory lanes 32*(warp % 4) .. +31 ----------------
@@ -439,46 +480,82 @@ __global__ void __launch_bounds__(PT_THREADS, PT_BLOCKS_PER_SM) attn_prefill_tc5
             if (lane == 0) t5_mbar_arrive(p_full);
         }
         if (ok) {
-            if (!t5_mbar_wait(o_done, (uint32_t)(n_tiles - 1) & 1u, PT_SPIN)) {
-                atomicExch(status, 38);
-            } else {
-                t5_fence_after();
-                // a sink joins the denominator as one more key without a value: 2^(sink * log2(e) - m), its score not scaled
-                if (sink && rvalid) l += pt_ex2(fmaf(sink[g * G + hh], 1.4426950408889634f, -m));
-                const float inv = SIG ? 1.f : (l > 0.f) ? 1.f / l : 0.f;
-                // The rows go out through shared memory (Q's place: every product that reads Q is through): a thread owns a
-                // row of tensor memory, but 16-byte stores 8 KB apart cost a block 2 us; a warp's 32 rows are stored
-                // 32 / CH at a time instead, CH lanes a row, each row's bytes contiguous.
-                constexpr int CH = PT_HD / 8;                 // 16-byte chunks of a row
-                unsigned char* stage = q_smem + qd * 32 * (PT_HD * 2);
+            ok = t5_mbar_wait(o_done, (uint32_t)(n_tiles - 1) & 1u, PT_SPIN);
+            if (!ok) atomicExch(status, 38);
+            t5_fence_after();
+        }
+        // Split: the second block leaves its rows' sums in its shared memory, the first brings both to the larger reference and finishes them.
+        // (A row may see no key of the second half: m is -inf there and its share nothing; a row that is not there sees none of either.)
+        float f0 = 1.f, f1 = 0.f;
+        const uint32_t sums = SPLIT ? pt_peer_of(t5_smem(smem) + r * 4) : 0u;
+        if (split) {
+            __syncwarp();
+            if (rank && __all_sync(0xffffffffu, ok)) {
 #pragma unroll
                 for (int c0 = 0; c0 < PT_HD; c0 += 32) {
                     uint32_t ov[32];
                     t5_ld32(t_lane + PT_COL_O + c0, ov);
                     t5_wait_ld();
 #pragma unroll
-                    for (int c = 0; c < 32; c += 8) {
-                        uint4 v;
-                        v.x = pt_pack(__uint_as_float(ov[c]) * inv, __uint_as_float(ov[c + 1]) * inv);
-                        v.y = pt_pack(__uint_as_float(ov[c + 2]) * inv, __uint_as_float(ov[c + 3]) * inv);
-                        v.z = pt_pack(__uint_as_float(ov[c + 4]) * inv, __uint_as_float(ov[c + 5]) * inv);
-                        v.w = pt_pack(__uint_as_float(ov[c + 6]) * inv, __uint_as_float(ov[c + 7]) * inv);
-                        const int ch = (c0 + c) >> 3;
-                        *reinterpret_cast<uint4*>(stage + lane * (PT_HD * 2) + ((ch ^ (lane & 7)) << 4)) = v;
-                    }
+                    for (int c = 0; c < 32; ++c) *reinterpret_cast<uint32_t*>(smem + ((c0 + c) * PT_ROWS + r) * 4) = ov[c];
                 }
-                __syncwarp();
+                *reinterpret_cast<float*>(smem + PT_SPLIT_ML + r * 4) = m;
+                *reinterpret_cast<float*>(smem + PT_SPLIT_ML + (PT_ROWS + r) * 4) = l;
+            }
+            __syncwarp();
+            pt_cluster_sync();
+            if (!rank) {
+                const float m1 = pt_peer(sums + PT_SPLIT_ML), l1 = pt_peer(sums + PT_SPLIT_ML + PT_ROWS * 4), both = fmaxf(m, m1);
+                f0 = m == -INFINITY ? 0.f : pt_ex2(m - both);
+                f1 = m1 == -INFINITY ? 0.f : pt_ex2(m1 - both);
+                l = l * f0 + l1 * f1;
+                m = both;
+            }
+        }
+        if (ok && !(split && rank)) {
+            // a sink joins the denominator as one more key without a value: 2^(sink * log2(e) - m), its score not scaled
+            if (sink && rvalid) l += pt_ex2(fmaf(sink[g * G + hh], 1.4426950408889634f, -m));
+            const float inv = SIG ? 1.f : (l > 0.f) ? 1.f / l : 0.f;
+            // The rows go out through shared memory (Q's place: every product that reads Q is through): a thread owns a
+            // row of tensor memory, but 16-byte stores 8 KB apart cost a block 2 us; a warp's 32 rows are stored
+            // 32 / CH at a time instead, CH lanes a row, each row's bytes contiguous.
+            constexpr int CH = PT_HD / 8;                 // 16-byte chunks of a row
+            unsigned char* stage = q_smem + qd * 32 * (PT_HD * 2);
 #pragma unroll
-                for (int it = 0; it < CH; ++it) {
-                    const int wr = it * (32 / CH) + lane / CH, ch = lane % CH;      // row of this warp, chunk of the row
-                    const int rr = qd * 32 + wr;
-                    if (rr < rows_valid) {
-                        const int t2 = rr / G, h2 = rr - t2 * G;
-                        const uint4 v = *reinterpret_cast<const uint4*>(stage + wr * (PT_HD * 2) + ((ch ^ (wr & 7)) << 4));
-                        *reinterpret_cast<uint4*>(out + (size_t)(tok0 + t2) * nh * PT_HD + (size_t)(g * G + h2) * PT_HD + ch * 8) = v;
-                    }
+            for (int c0 = 0; c0 < PT_HD; c0 += 32) {
+                uint32_t ov[32];
+                t5_ld32(t_lane + PT_COL_O + c0, ov);
+                t5_wait_ld();
+                if (split) {
+#pragma unroll
+                    for (int c = 0; c < 32; ++c) ov[c] = __float_as_uint(__uint_as_float(ov[c]) * f0 + pt_peer(sums + (c0 + c) * (PT_ROWS * 4)) * f1);
+                }
+#pragma unroll
+                for (int c = 0; c < 32; c += 8) {
+                    uint4 v;
+                    v.x = pt_pack(__uint_as_float(ov[c]) * inv, __uint_as_float(ov[c + 1]) * inv);
+                    v.y = pt_pack(__uint_as_float(ov[c + 2]) * inv, __uint_as_float(ov[c + 3]) * inv);
+                    v.z = pt_pack(__uint_as_float(ov[c + 4]) * inv, __uint_as_float(ov[c + 5]) * inv);
+                    v.w = pt_pack(__uint_as_float(ov[c + 6]) * inv, __uint_as_float(ov[c + 7]) * inv);
+                    const int ch = (c0 + c) >> 3;
+                    *reinterpret_cast<uint4*>(stage + lane * (PT_HD * 2) + ((ch ^ (lane & 7)) << 4)) = v;
                 }
             }
+            __syncwarp();
+#pragma unroll
+            for (int it = 0; it < CH; ++it) {
+                const int wr = it * (32 / CH) + lane / CH, ch = lane % CH;      // row of this warp, chunk of the row
+                const int rr = qd * 32 + wr;
+                if (rr < rows_valid) {
+                    const int t2 = rr / G, h2 = rr - t2 * G;
+                    const uint4 v = *reinterpret_cast<const uint4*>(stage + wr * (PT_HD * 2) + ((ch ^ (wr & 7)) << 4));
+                    *reinterpret_cast<uint4*>(out + (size_t)(tok0 + t2) * nh * PT_HD + (size_t)(g * G + h2) * PT_HD + ch * 8) = v;
+                }
+            }
+        }
+        if (split) {                              // the second block's shared memory is read: it may leave
+            __syncwarp();
+            pt_cluster_sync();
         }
     }
     t5_fence_before();
@@ -515,7 +592,7 @@ IL_EXPORT int il_attn_prefill_tc5(const void* qkv, int row_stride, void* out, co
     if (dev >= 0 && dev < 64 && !attr_set[dev]) {
         cudaError_t e = cudaSuccess;
         for (auto k : {attn_prefill_tc5_kernel<false, false, false>, attn_prefill_tc5_kernel<true, false, false>, attn_prefill_tc5_kernel<true, true, false>,
-                       attn_prefill_tc5_kernel<false, false, true>}) {
+                       attn_prefill_tc5_kernel<false, false, true>, attn_prefill_tc5_kernel<false, false, false, true>}) {
             if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, PT_SMEM);
             if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
         }
@@ -525,6 +602,25 @@ IL_EXPORT int il_attn_prefill_tc5(const void* qkv, int row_stride, void* out, co
     CUtensorMap map;
     memcpy(&map, kv_map, sizeof(map));
     dim3 grid(n_tiles_total, nkv);
+    // All blocks on the device at once: the time is the longest block's chain of key tiles, which two blocks of a cluster halve; they pay with their
+    // starts and the sums handed over (heads of 128: twice as much). The table's width says how long a chain can be. One block / two, us: 16 heads on 2 of 64,
+    // 256 tokens (32 blocks) 9.3 / 9.7, behind 2,048 cached ones 38.4 / 22.8; 512 tokens 12.8 / 11.4, 1,024 20.4 / 17.4, 2,048 (256 blocks) 37.9 / 33.0, behind
+    // 6,144 138 / 127. 16 on 4 of 128: 512 tokens (64 blocks) 14.9 / 15.4, 1,024 (128) 22.3 / 22.5, behind as many 36.3 / 31.4, 256 behind 2,048 39.2 / 27.7,
+    // 2,048 (256) 43.3 / 49.1, behind 6,144 144 / 149; 32 on 2 of 128: 1,024 tokens (256) 25.5 / 35.5, behind as many 42.9 / 53.9.
+    const bool wide = HEAD_DIM > 64;
+    if (HEAD_DIM <= 128 && !sigmoid && !(cap > 0.f) && !dist_bias && n_tiles_total * (long long)nkv <= (wide ? 148 : 296) &&
+        bt_stride * (long long)PT_PAGE >= (wide ? 2048 : 512)) {
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(2 * n_tiles_total, nkv), cfg.blockDim = PT_THREADS, cfg.dynamicSmemBytes = PT_SMEM, cfg.stream = stream;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = 2, attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+        cfg.attrs = attr, cfg.numAttrs = 1;
+        const cudaError_t e = cudaLaunchKernelEx(&cfg, attn_prefill_tc5_kernel<false, false, false, true>, map, (const __nv_bfloat16*)qkv, row_stride,
+                                                 (__nv_bfloat16*)out, block_table, bt_stride, entry_qstart, entry_kvlen, first_entry, n_entries, nh, nkv,
+                                                 scale * 1.4426950408889634f, window, PT_ROWS / G, status, sink, dist_bias, dist_far, 1.f / scale, log_bias, 0.f);
+        return e != cudaSuccess ? 1000 + (int)e : IL_OK;
+    }
     (log_bias ? attn_prefill_tc5_kernel<true, true, false> : sigmoid ? attn_prefill_tc5_kernel<true, false, false>
               : cap > 0.f ? attn_prefill_tc5_kernel<false, false, true> : attn_prefill_tc5_kernel<false, false, false>)<<<grid, PT_THREADS, PT_SMEM, stream>>>(
         map, (const __nv_bfloat16*)qkv, row_stride, (__nv_bfloat16*)out, block_table, bt_stride, entry_qstart, entry_kvlen,
