@@ -128,6 +128,12 @@ __global__ void rope_store_kernel(TA* __restrict__ qkv, int row_stride, const in
     }
 }
 
+// A pair of a prompt portion rotated, x1 c - x2 s and x2 c + x1 s, written out in the rounding that both kernels for many tokens have: the products
+// x2 s and x2 c are rounded first. (Left to the compiler, the one below and the one in 16-byte pieces differed in bfloat16. The kernel for few tokens
+// rounds x1 s instead of x2 c.)
+__device__ __forceinline__ float rope_lo(float x1, float x2, float c, float s) { return __fmaf_rn(x1, c, -__fmul_rn(x2, s)); }
+__device__ __forceinline__ float rope_hi(float x1, float x2, float c, float s) { return __fmaf_rn(x1, s, __fmul_rn(x2, c)); }
+
 // The same for many tokens (prompt portions) where the pairs are not whole 16-byte pieces: a block's latency does not matter there, how many blocks an SM holds
 // does; two passes (rotate in place, then copy k and v to the cache in 16-byte pieces), 256 threads, few registers.
 template <typename TA>
@@ -156,8 +162,8 @@ __global__ void rope_store_many_kernel(TA* __restrict__ qkv, int row_stride, con
                 TA* base = row + (size_t)j * hd;
                 const float2 a = ld2(base + i), b = ld2(base + i + half);
                 const float s0 = sn[i], c0 = cs[i], s1 = sn[i + 1], c1 = cs[i + 1];
-                st2(base + i, make_float2(a.x * c0 - b.x * s0, a.y * c1 - b.y * s1));
-                st2(base + i + half, make_float2(b.x * c0 + a.x * s0, b.y * c1 + a.y * s1));
+                st2(base + i, make_float2(rope_lo(a.x, b.x, c0, s0), rope_lo(a.y, b.y, c1, s1)));
+                st2(base + i + half, make_float2(rope_hi(a.x, b.x, c0, s0), rope_hi(a.y, b.y, c1, s1)));
             }
         } else {
             const int n_pairs = (nh + nkv) * half;
@@ -264,8 +270,8 @@ __global__ void __launch_bounds__(512) rope_store_wide_kernel(TA* qkv, int row_s
 #pragma unroll
             for (int e = 0; e < VEC; ++e) {
                 const float x1 = il_to_f(ap[e]), x2 = il_to_f(bp[e]);
-                ap[e] = il_from_f<TA>(x1 * c[e] - x2 * s[e]);
-                bp[e] = il_from_f<TA>(x2 * c[e] + x1 * s[e]);
+                ap[e] = il_from_f<TA>(rope_lo(x1, x2, c[e], s[e]));
+                bp[e] = il_from_f<TA>(rope_hi(x1, x2, c[e], s[e]));
             }
             *reinterpret_cast<uint4*>(it.from) = a;
             *reinterpret_cast<uint4*>(it.from + half) = b;

@@ -33,3 +33,31 @@ def test_many_tokens_as_few_at_a_time(cuda_device, dtype, nh, nkv, hd, rot, T, c
             page = int(bt[ent[t], pos[t] // 16])
             if page >= 0:
                 assert torch.equal(caches[0][page, 0, :, pos[t] % 16].reshape(-1), many[t, nh * hd:(nh + nkv) * hd])
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("nh,nkv,hd,rot", [(16, 2, 64, 64), (32, 2, 128, 128), (4, 2, 80, 72)])
+def test_rounding_of_a_rotated_pair(cuda_device, dtype, nh, nkv, hd, rot):
+    """More than 64 tokens: x1 c - x2 s with x2 s rounded first, x2 c + x1 s with x2 c rounded first, bit for bit in both kernels and types (pairs in
+    whole 16-byte pieces or, the last shape in bfloat16, not)."""
+    from infinilm_b200 import ops
+    T, heads = 200, nh + nkv
+    g = torch.Generator(device="cuda").manual_seed(rot)
+    pos, ent = (torch.arange(T, device="cuda", dtype=torch.int32) * 37) % 3000, torch.zeros(T, device="cuda", dtype=torch.int32)
+    bt = torch.zeros(1, 200, device="cuda", dtype=torch.int32)
+    inv = (1.0 / (10000.0 ** (torch.arange(rot // 2, device="cuda", dtype=torch.float64) * 2 / rot))).float()
+
+    def rotated(x):
+        ops.rope_store(x, pos, ent, bt, None, 16, nh, nkv, hd, rot, inv, 1.1)
+        return x.view(T, nh + 2 * nkv, hd)[:, :heads]
+    one = torch.zeros(T, nh + 2 * nkv, hd, device="cuda")
+    one[:, :, :rot // 2] = 1
+    one = rotated(one.view(T, -1)).double()       # the angles' cosine and sine
+    c, s = one[..., :rot // 2], one[..., rot // 2:rot]
+    x = torch.randn(T, (nh + 2 * nkv) * hd, device="cuda", generator=g).to(dtype)
+    xd = x.view(T, nh + 2 * nkv, hd)[:, :heads].double().clone()
+    got = rotated(x)
+    x1, x2 = xd[..., :rot // 2], xd[..., rot // 2:rot]
+    # products of two float32 are exact in float64; adding rounds them to 53 bits before the rounding to 24, which no pair here is close enough to feel
+    assert torch.equal(got[..., :rot // 2], (x1 * c - (x2 * s).float().double()).float().to(dtype))
+    assert torch.equal(got[..., rot // 2:rot], ((x2 * c).float().double() + x1 * s).float().to(dtype))
