@@ -1210,14 +1210,18 @@ __global__ void __launch_bounds__(256) group_norm_gate_warp_kernel(const float* 
 }
 // Groups of thousands of columns: a block a (row, group), everything it reads asked for at once, 16 bytes of x a thread and piece. Bound by
 // memory for long portions: one group of 2,048 columns a row, prompts in steps of 4,096 and 904 rows, 34.4 us on average with 4-byte loads, 11.8 so.
-template <typename TG, typename TO, int PIECES>
-__global__ void __launch_bounds__(512) group_norm_gate_block_kernel(const float* x, int ldx, const void* __restrict__ w, int w_kind, int n_w, float eps,
+// The squares are added in the order of the kernel with one column a thread, whose blocks have four times as many threads as this has adders: an adder's
+// four columns are four of its threads, eight adders one of its warps - the same bits whichever of the two takes a row. PAIRS (1,028 to 2,044 columns,
+// and beyond 2,048): every second row of pieces is another thread's, which hands it to the adder through shared memory (2,000 rows of 8,192: 73.7 us with
+// the adders alone, 51.2 so; 4,096 of 2,044 30.6 and 26.6).
+template <typename TG, typename TO, int PIECES, bool PAIRS>
+__global__ void __launch_bounds__(PAIRS ? 512 : 256) group_norm_gate_block_kernel(const float* x, int ldx, const void* __restrict__ w, int w_kind, int n_w, float eps,
                                                                     const TG* gate, int ldg, int g_off, int act, TO* __restrict__ out, int ldo, int group) {
     __shared__ float red[32];
+    __shared__ float4 xs[PAIRS ? 256 * PIECES : 1];
     sm_small_begin();
-    const int t = blockIdx.x, j0 = blockIdx.y * group;
+    const int t = blockIdx.x, j0 = blockIdx.y * group, lane = threadIdx.x & 31, adders = PAIRS ? blockDim.x >> 1 : blockDim.x;
     float4 xv[PIECES], zv[PIECES], wv[PIECES];
-    float ss = 0.f;
 #pragma unroll
     for (int u = 0; u < PIECES; ++u) {
         const int j = (threadIdx.x + blockDim.x * u) * 4;
@@ -1229,9 +1233,33 @@ __global__ void __launch_bounds__(512) group_norm_gate_block_kernel(const float*
             wv[u] = w_kind == IL_F32 ? gn_load4((const float*)w + jw) : gn_load4((const __nv_bfloat16*)w + jw);
         }
     }
+    if (PAIRS) {
+        if ((int)threadIdx.x >= adders) {
 #pragma unroll
-    for (int u = 0; u < PIECES; ++u) ss += (xv[u].x * xv[u].x + xv[u].y * xv[u].y) + (xv[u].z * xv[u].z + xv[u].w * xv[u].w);
-    const float r = 1.f / sqrtf(il_block_sum(ss, red) / (float)group + eps);
+            for (int u = 0; u < PIECES; ++u) xs[threadIdx.x - adders + adders * u] = xv[u];
+        }
+        __syncthreads();
+    }
+    if ((int)threadIdx.x < adders) {
+        float4 ss = make_float4(0.f, 0.f, 0.f, 0.f);
+        const auto add = [&](const float4& v) {
+            ss.x = __fmaf_rn(v.x, v.x, ss.x), ss.y = __fmaf_rn(v.y, v.y, ss.y), ss.z = __fmaf_rn(v.z, v.z, ss.z), ss.w = __fmaf_rn(v.w, v.w, ss.w);
+        };
+#pragma unroll
+        for (int u = 0; u < PIECES; ++u) {
+            add(xv[u]);
+            if (PAIRS) add(xs[threadIdx.x + adders * u]);
+        }
+#pragma unroll
+        for (int o = 4; o > 0; o >>= 1) {
+            ss.x += __shfl_xor_sync(0xffffffffu, ss.x, o), ss.y += __shfl_xor_sync(0xffffffffu, ss.y, o);
+            ss.z += __shfl_xor_sync(0xffffffffu, ss.z, o), ss.w += __shfl_xor_sync(0xffffffffu, ss.w, o);
+        }
+        if ((lane & 7) == 0) red[threadIdx.x >> 3] = (ss.x + ss.z) + (ss.y + ss.w);
+    }
+    __syncthreads();
+    const float sum = il_warp_sum(lane < adders >> 3 ? red[lane] : 0.f);
+    const float r = 1.f / sqrtf(sum / (float)group + eps);
 #pragma unroll
     for (int u = 0; u < PIECES; ++u) {
         const int j = (threadIdx.x + blockDim.x * u) * 4;
@@ -1244,13 +1272,20 @@ __global__ void __launch_bounds__(512) group_norm_gate_block_kernel(const float*
         }
     }
 }
+// Threads of the kernel with one column a thread.
+static int group_norm_threads(int group) { return group >= 2048 ? 1024 : group >= 1024 ? 512 : group >= 256 ? 256 : group >= 128 ? 128 : 64; }
 
 template <typename TG, typename TO>
 static cudaError_t group_norm_gate_warp_launch(const float* x, int ldx, const void* w, int w_kind, int n_w, float eps, const void* gate, int ldg, int g_off,
                                                int act, void* out, int ldo, int group, int n_groups, int T, cudaStream_t stream) {
-    if (group > 512)                              // (up to 8,192)
-        return il_launch(group <= 4096 ? group_norm_gate_block_kernel<TG, TO, 2> : group_norm_gate_block_kernel<TG, TO, 4>, dim3(T, n_groups),
-                         dim3(group <= 2048 ? 256 : 512), 0, stream, x, ldx, w, w_kind, n_w, eps, (const TG*)gate, ldg, g_off, act, (TO*)out, ldo, group);
+    if (group > 512) {                            // (up to 8,192)
+        const int adders = group_norm_threads(group) / 4;
+        const bool pairs = group > 1024 && group != 2048;
+        return il_launch(group > 4096 ? group_norm_gate_block_kernel<TG, TO, 4, true> : pairs ? group_norm_gate_block_kernel<TG, TO, 2, true>
+                         : group > 8 * adders ? group_norm_gate_block_kernel<TG, TO, 4, false> : group_norm_gate_block_kernel<TG, TO, 2, false>,
+                         dim3(T, n_groups), dim3(pairs ? 2 * adders : adders), 0, stream, x, ldx, w, w_kind, n_w, eps, (const TG*)gate, ldg, g_off, act,
+                         (TO*)out, ldo, group);
+    }
     const auto kernel = group <= 128 ? group_norm_gate_warp_kernel<TG, TO, 1> : group <= 256 ? group_norm_gate_warp_kernel<TG, TO, 2>
                                                                                              : group_norm_gate_warp_kernel<TG, TO, 4>;
     const long long units = (long long)T * n_groups;
@@ -1282,7 +1317,7 @@ static int group_norm_gate_launch(const float* x, int ldx, const void* w, int w_
         return IL_OK;
     }
     // (a group of thousands of columns is one block: many threads, two to four columns each, keep its two passes short)
-    const int threads = group >= 2048 ? 1024 : group >= 1024 ? 512 : group >= 256 ? 256 : group >= 128 ? 128 : 64;
+    const int threads = group_norm_threads(group);
     const dim3 grid(T, n_groups);
 #define GN_ARGS x, ldx, w, w_kind, n_w, eps
     if (gate_kind == IL_F32 && out_kind == IL_F32)
