@@ -112,8 +112,12 @@ __device__ __forceinline__ float pt_peer(uint32_t at) {
 }
 // Where the rows' sums of the second block lie for the first (over Q, P and the ring, which nothing reads any more): column c of row r,
 // and behind them m and l.
-constexpr int PT_SPLIT_ML = PT_ROWS * PT_HD * 4, PT_SPLIT_FROM = 4;
+constexpr int PT_SPLIT_ML = PT_ROWS * PT_HD * 4;
 static_assert(PT_SPLIT_ML + PT_ROWS * 8 <= PT_Q_BYTES + PT_P_BYTES + (PT_K_STAGES + PT_V_STAGES) * PT_K_BYTES, "the second block's sums");
+constexpr bool PT_SPLITS = HEAD_DIM <= 128;       // head sizes that have that form
+// From so many key tiles of its own on, a block's keys are shared. Only the block's own tokens and window count: not the other requests of the step,
+// not whether it is replayed with a wider table. (The rule in il_attn_prefill_tc5 has the times.)
+constexpr int PT_SPLIT_FROM = HEAD_DIM > 64 ? 17 : 8;
 
 // SPLIT: a cluster of two blocks takes the tokens of one, each half of the key tiles (where there are PT_SPLIT_FROM; else the second leaves).
 template <bool SIG, bool LOGB, bool CAP, bool SPLIT = false>
@@ -571,9 +575,10 @@ IL_EXPORT int il_attn_prefill_tc5_rows() { return PT_ROWS; }
 
 // kv_map: the 128 bytes of the cache's third tensor map (il_attn_decode_kv_map: a page's K or V as tensor-core tiles), on the host.
 // n_tiles_total: sum over entries [first_entry, n_entries) of ceil(q_len / tpt), tpt = max(1, rows / (nh/nkv)), rows = il_attn_prefill_tc5_rows().
+// n_tiles_rule: the number by which it is decided whether blocks share keys: n_tiles_total, or a bound on it that a replayed and an eager step have alike.
 IL_EXPORT int il_attn_prefill_tc5(const void* qkv, int row_stride, void* out, const void* kv_map, const int* block_table,
                                   int bt_stride, const int* entry_qstart, const int* entry_kvlen, int page_size, int first_entry,
-                                  int n_entries, int n_tiles_total, int nh, int nkv, int hd, float scale, int window, int* status,
+                                  int n_entries, int n_tiles_total, int n_tiles_rule, int nh, int nkv, int hd, float scale, int window, int* status,
                                   const float* sink, const float* dist_bias, int dist_far, int sigmoid, const float* log_bias,
                                   float cap, cudaStream_t stream) {
     if (n_tiles_total <= 0 || first_entry >= n_entries) return IL_OK;
@@ -592,7 +597,7 @@ IL_EXPORT int il_attn_prefill_tc5(const void* qkv, int row_stride, void* out, co
     if (dev >= 0 && dev < 64 && !attr_set[dev]) {
         cudaError_t e = cudaSuccess;
         for (auto k : {attn_prefill_tc5_kernel<false, false, false>, attn_prefill_tc5_kernel<true, false, false>, attn_prefill_tc5_kernel<true, true, false>,
-                       attn_prefill_tc5_kernel<false, false, true>, attn_prefill_tc5_kernel<false, false, false, true>}) {
+                       attn_prefill_tc5_kernel<false, false, true>, attn_prefill_tc5_kernel<false, false, false, PT_SPLITS>}) {
             if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, PT_SMEM);
             if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
         }
@@ -603,20 +608,20 @@ IL_EXPORT int il_attn_prefill_tc5(const void* qkv, int row_stride, void* out, co
     memcpy(&map, kv_map, sizeof(map));
     dim3 grid(n_tiles_total, nkv);
     // All blocks on the device at once: the time is the longest block's chain of key tiles, which two blocks of a cluster halve; they pay with their
-    // starts and the sums handed over (heads of 128: twice as much). The table's width says how long a chain can be. One block / two, us: 16 heads on 2 of 64,
-    // 256 tokens (32 blocks) 9.3 / 9.7, behind 2,048 cached ones 38.4 / 22.8; 512 tokens 12.8 / 11.4, 1,024 20.4 / 17.4, 2,048 (256 blocks) 37.9 / 33.0, behind
-    // 6,144 138 / 127. 16 on 4 of 128: 512 tokens (64 blocks) 14.9 / 15.4, 1,024 (128) 22.3 / 22.5, behind as many 36.3 / 31.4, 256 behind 2,048 39.2 / 27.7,
-    // 2,048 (256) 43.3 / 49.1, behind 6,144 144 / 149; 32 on 2 of 128: 1,024 tokens (256) 25.5 / 35.5, behind as many 42.9 / 53.9.
-    const bool wide = HEAD_DIM > 64;
-    if (HEAD_DIM <= 128 && !sigmoid && !(cap > 0.f) && !dist_bias && n_tiles_total * (long long)nkv <= (wide ? 148 : 296) &&
-        bt_stride * (long long)PT_PAGE >= (wide ? 2048 : 512)) {
+    // starts and the sums handed over (heads of 128: twice as much). One block / two from PT_SPLIT_FROM tiles on, us, four in a row replayed: 16 heads on 2 of
+    // 64, 256 tokens (32 blocks) 10.8 / 10.8, behind 2,048 cached ones 40.4 / 24.1; 512 tokens 14.8 / 13.8, 1,024 22.5 / 18.4, 2,048 (256 blocks) 38.4 / 35.3,
+    // behind 6,144 138.8 / 130.0; four prompts of 64 to 400 13.8 / 13.8. 16 on 4 of 128: 512 tokens (64 blocks) 16.9 / 16.5, 1,024 (128) 24.1 / 24.1, 1,184 (148)
+    // 27.6 / 29.7 (a few blocks at the end are shared and the others meet on SMs; shared from 8 tiles on 26.1, but then 512 tokens of 32 heads on 2 take 20.5
+    // instead of 16.9), behind as many 38.4 / 33.3, 512 behind 1,024 30.7 / 24.6, 256 behind 2,048 41.5 / 29.7. More blocks than SMs, heads of 128, gain nothing.
+    if (PT_SPLITS && !sigmoid && !(cap > 0.f) && !dist_bias && n_tiles_rule * (long long)nkv <= (HEAD_DIM > 64 ? 148 : 296) &&
+        bt_stride > (PT_SPLIT_FROM - 1) * PT_TILE_PAGES) {        // (a narrower table holds no such chain: every block would be alone, with the same bits)
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3(2 * n_tiles_total, nkv), cfg.blockDim = PT_THREADS, cfg.dynamicSmemBytes = PT_SMEM, cfg.stream = stream;
         cudaLaunchAttribute attr[1];
         attr[0].id = cudaLaunchAttributeClusterDimension;
         attr[0].val.clusterDim.x = 2, attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
         cfg.attrs = attr, cfg.numAttrs = 1;
-        const cudaError_t e = cudaLaunchKernelEx(&cfg, attn_prefill_tc5_kernel<false, false, false, true>, map, (const __nv_bfloat16*)qkv, row_stride,
+        const cudaError_t e = cudaLaunchKernelEx(&cfg, attn_prefill_tc5_kernel<false, false, false, PT_SPLITS>, map, (const __nv_bfloat16*)qkv, row_stride,
                                                  (__nv_bfloat16*)out, block_table, bt_stride, entry_qstart, entry_kvlen, first_entry, n_entries, nh, nkv,
                                                  scale * 1.4426950408889634f, window, PT_ROWS / G, status, sink, dist_bias, dist_far, 1.f / scale, log_bias, 0.f);
         return e != cudaSuccess ? 1000 + (int)e : IL_OK;

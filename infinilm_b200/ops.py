@@ -770,10 +770,13 @@ def attention_prefill_tc5(qkv: torch.Tensor, out: torch.Tensor, kv_map: torch.Te
                           entry_qstart: torch.Tensor, entry_kvlen: torch.Tensor, first_entry: int, n_entries: int,
                           n_tiles_total: int, page_size: int, n_heads: int, n_kv_heads: int, head_dim: int, scale: float,
                           window: Optional[int], sink: Optional[torch.Tensor] = None, dist_bias: Optional[torch.Tensor] = None,
-                          sigmoid: bool = False, log_bias: Optional[torch.Tensor] = None, cap: Optional[float] = None) -> None:
+                          sigmoid: bool = False, log_bias: Optional[torch.Tensor] = None, cap: Optional[float] = None,
+                          n_tiles_rule: Optional[int] = None) -> None:
     """The same attention as `attention_prefill`, on tcgen05 tensor cores with tensor memory; `kv_map` is the cache's
     tensor map (`kv_tensor_map`). `log_bias` (with `sigmoid`, instead of dist_bias): float32 [3, heads] - r1, r2 and an offset pb:
-    the scaled score of a key n positions back gets pb - r1 ln(1 + r2 n), computed as it is needed. n_tiles_total = sum over the entries of ceil(q_len / (prefill_tc5_rows(head_dim) // (heads/kv_heads)))."""
+    the scaled score of a key n positions back gets pb - r1 ln(1 + r2 n), computed as it is needed. n_tiles_total = sum over the entries of ceil(q_len / (prefill_tc5_rows(head_dim) // (heads/kv_heads))).
+    n_tiles_rule: the number by which the kernel decides whether two blocks share a block's keys, n_tiles_total if not given; a caller that
+    launches the same portions with the exact number and with a bound on it gives the bound here both times, for the same order of sums."""
     _need_cuda(qkv, out, block_table, entry_qstart, entry_kvlen, sink, dist_bias, log_bias)
     if log_bias is not None and (not sigmoid or dist_bias is not None or log_bias.dtype != torch.float32 or tuple(log_bias.shape) != (3, n_heads)
                                  or not log_bias.is_contiguous()):
@@ -789,11 +792,11 @@ def attention_prefill_tc5(qkv: torch.Tensor, out: torch.Tensor, kv_map: torch.Te
         raise KernelError("attention_prefill_tc5: out [T, heads*head_dim]")
     _contig("qkv", qkv), _contig("out", out), _contig("block_table", block_table)
     f = _fn("attn_prefill_tc5", "il_attn_prefill_tc5",
-            [_c_void_p, _c_int, _c_void_p, _c_void_p, _c_void_p, _c_int, _c_void_p, _c_void_p, _c_int, _c_int, _c_int, _c_int,
+            [_c_void_p, _c_int, _c_void_p, _c_void_p, _c_void_p, _c_int, _c_void_p, _c_void_p, _c_int, _c_int, _c_int, _c_int, _c_int,
              _c_int, _c_int, _c_int, _c_float, _c_int, _c_void_p, _c_void_p, _c_void_p, _c_int, _c_int, _c_void_p, _c_float, _c_void_p], defines={"HEAD_DIM": head_dim})
     _check(f(_ptr(qkv), qkv.shape[1], _ptr(out), _c_void_p(kv_map.data_ptr() + 256), _ptr(block_table), block_table.shape[1],
-             _ptr(entry_qstart), _ptr(entry_kvlen), page_size, first_entry, n_entries, n_tiles_total, n_heads, n_kv_heads,
-             head_dim, scale, int(window or 0), _ptr(stream_status(qkv.device)), _ptr(sink), _ptr(dist_bias), 0 if dist_bias is None else dist_bias.shape[0] - 1,
+             _ptr(entry_qstart), _ptr(entry_kvlen), page_size, first_entry, n_entries, n_tiles_total,
+             n_tiles_total if n_tiles_rule is None else n_tiles_rule, n_heads, n_kv_heads, head_dim, scale, int(window or 0), _ptr(stream_status(qkv.device)), _ptr(sink), _ptr(dist_bias), 0 if dist_bias is None else dist_bias.shape[0] - 1,
              int(sigmoid), _ptr(log_bias), cap, _stream()), "attention_prefill_tc5")
 
 

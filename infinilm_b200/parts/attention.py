@@ -119,10 +119,12 @@ class PagedAttend:
             tpt = max(1, (ops.prefill_tc5_rows(self.hd) if tc5 else 64) // G)
             n_tiles = ctx.prompt_tiles(tpt)
             if tc5:
+                # (what a replayed step knows of its tiles, in an eager one too: both then add up in the same order)
+                most = (qkv.shape[0] - n_dec + tpt - 1) // tpt + E - n_dec - 1
                 ops.attention_prefill_tc5(qkv, out, cache.tma_map, cache.block_table, ctx.entry_qstart, ctx.entry_kvlen,
                                           n_dec, E, n_tiles, cache.page_size, self.nh, self.nkv, self.hd, self.scale,
                                           self.mask_arg, sink=self.sink, dist_bias=self.dist_bias if self.log_bias is None else None,
-                                          sigmoid=self.sigmoid, log_bias=self.log_bias, cap=self.cap)
+                                          sigmoid=self.sigmoid, log_bias=self.log_bias, cap=self.cap, n_tiles_rule=most)
             else:
                 ops.attention_prefill(qkv, out, cache.storage, cache.block_table, ctx.entry_qstart, ctx.entry_kvlen,
                                       n_dec, E, n_tiles, cache.page_size, self.nh, self.nkv, self.hd, self.scale,
