@@ -1,8 +1,10 @@
 // 32-bit matrix product on the bfloat16 tensor cores, with the error of 32-bit multiply-adds:
 //   C[M,N] = alpha * A[M,K] * W[N,K]^T (+ bias[N])
 // A and W are float32, row-major with K contiguous (the layout of activations and of checkpoint weights); nothing is stored in
-// fewer bits. Each operand is taken apart on its way to the tensor cores, x = h + m + l with h, m, l the bfloat16 nearest to x,
-// to x - h and to x - h - m: 24 bits, exactly x unless x is so small that l would lie below the bfloat16 range. Products of two
+// fewer bits. Each operand is taken apart on its way to the tensor cores, 2^23 x = h + m + l with h, m, l the bfloat16 nearest to 2^23 x,
+// to what h leaves and to what m leaves: 24 bits, exactly 2^23 x for every finite x below 2^105, the smallest ones too (the last bit of a
+// float32 is 2^-149 or more, that of l then 2^-126, the least bfloat16 that is not subnormal; without the factor, numbers below 2^-102
+// lost bits, which a large number on the other side made visible). Products of two
 // bfloat16 are exact in the tensor core; of the nine, three are below 2^-26 of the first and are left out.
 //
 // One order of summation for every kernel and shape, so that a row's result is bit-identical whatever else is in the batch:
@@ -17,8 +19,8 @@
 // 0.98e-7 (1.10e-7) and 1.12e-7 (1.35e-7); all positive 0.55e-7 (0.61e-7) and 0.59e-7 (0.65e-7). With the h h products of a whole
 // chunk in one accumulator: 1.03e-7, 1.36e-7 and 0.88e-7 at K = 1,024.
 //
-// A sum that is not finite, or smaller than 2^-80, may owe that to the pieces (an infinity has no remainder, a remainder can
-// fall below the range): it is computed again with 32-bit multiply-adds (f32_plain).
+// A sum that is not finite may owe that to the pieces (an infinity has no remainder) or to the factor 2^46 (sums of 2^82 and more): it is
+// computed again with 32-bit multiply-adds, in the same chunks (f32_plain).
 //
 // Up to 16 rows the kernel is bound by the bytes of W and by the instructions that take it apart (gemm_f32_rows_kernel,
 // mma.sync on fragments that come straight from memory); beyond, by shared memory: operands written, and read by the tensor core
@@ -43,25 +45,40 @@ __device__ __forceinline__ il_f2 f32_less(il_f2 x, uint32_t p) {      // x minus
     asm("sub.rn.f32x2 %0, %1, %2;\n" : "=l"(d) : "l"(x), "l"(il_f2_make(__uint_as_float(p << 16), __uint_as_float(p & 0xffff0000u))));
     return d;
 }
+constexpr float F32_SCALE = 0x1p23f, F32_UNSCALE = 0x1p-46f;          // of an operand; of a sum
+// (FUSED: the same pieces, the factor once more in the first subtraction instead of a scaled pair held for it - for the kernel that is short of registers,
+// 16 rows to 73,448 columns of K = 1,024: 111 us, 116 without; elsewhere it costs up to 2 %.)
+template <bool FUSED = false>
 __device__ __forceinline__ void f32_split(float a, float b, uint32_t& h, uint32_t& m, uint32_t& l) {
-    h = f32_pack(a, b);
-    il_f2 r = f32_less(il_f2_make(a, b), h);
+    il_f2 r;
+    if (FUSED) {
+        h = f32_pack(a * F32_SCALE, b * F32_SCALE);
+        r = il_f2_fma(il_f2_make(a, b), il_f2_dup(F32_SCALE), il_f2_make(__uint_as_float((h << 16) ^ 0x80000000u), __uint_as_float((h & 0xffff0000u) ^ 0x80000000u)));
+    } else {
+        r = il_f2_mul(il_f2_make(a, b), il_f2_dup(F32_SCALE));
+        il_f2_get(r, a, b);
+        h = f32_pack(a, b);
+        r = f32_less(r, h);
+    }
     il_f2_get(r, a, b);
     m = f32_pack(a, b);
     r = f32_less(r, m);
     il_f2_get(r, a, b);
     l = f32_pack(a, b);
 }
-__device__ __forceinline__ bool f32_suspect(float v) {
-    const uint32_t u = __float_as_uint(v) & 0x7fffffffu;
-    return u != 0u && u - (47u << 23) >= (255u - 47u) << 23;
-}
-// The sum by multiply-adds: even and odd k apart.
+__device__ __forceinline__ bool f32_suspect(float v) { return !(fabsf(v) < INFINITY); }
+// The sum by multiply-adds: even and odd k apart, chunk by chunk.
 __device__ __noinline__ float f32_plain(const float* a, const float* w, int K) {
-    float even = 0.f, odd = 0.f;
-    for (int k = 0; k + 1 < K; k += 2) even = __fmaf_rn(a[k], w[k], even), odd = __fmaf_rn(a[k + 1], w[k + 1], odd);
-    if (K & 1) even = __fmaf_rn(a[K - 1], w[K - 1], even);
-    return __fadd_rn(even, odd);
+    float sum = 0.f;
+    for (int c = 0; c < K; c += F32_CHUNK) {
+        float even = 0.f, odd = 0.f;
+        const int end = min(K, c + F32_CHUNK);
+        int k = c;
+        for (; k + 1 < end; k += 2) even = __fmaf_rn(a[k], w[k], even), odd = __fmaf_rn(a[k + 1], w[k + 1], odd);
+        if (k < end) even = __fmaf_rn(a[k], w[k], even);
+        sum = __fadd_rn(sum, __fadd_rn(even, odd));
+    }
+    return sum;
 }
 // Four floats row[k .. k+3], zeros past K. VEC: row + k is 16-byte aligned.
 __device__ __forceinline__ float4 f32_ld4(const float* p) {
@@ -108,9 +125,10 @@ __device__ __forceinline__ void f32_cluster_sync() {
 // chunks, a chunk a warp; a warp has the weights of two rounds in registers or on their way, across tiles, the first two asked
 // for before the wait for the kernel in front where the caller says that W is no kernel's output (`early`). Where the tiles are
 // few, the shares go to the blocks of a cluster.
-// Measured, weights not in cache, us (the kernel of multiply-adds before): one row, 2 x 4,096 gated columns of K = 1,024 8.9 (9.5), 73,448
-// columns 53 (69; 5.7 TB/s), 1,024 columns of K = 4,096 6.3 (5.8), of K = 1,024 3.2 (2.5); 8 rows 9.9 (17.8), 62 (116), 6.6 (9.9), 3.5 (3.9).
-// Some 250 instructions a warp for 4 KB of W bound the small ones.
+// Measured, weights not in cache, us (the kernel of multiply-adds before): one row, 2 x 4,096 gated columns of K = 1,024 9.6 (10.5), 73,448
+// columns 58.8 (71; 5.1 TB/s), 1,024 columns of K = 4,096 6.6 (6.0), of K = 1,024 3.3 (2.3); 8 rows to 73,448 columns 64 (87), K = 4,096 7.1 (9.9); 16 rows
+// 14.4 (22.8), 111 (156), K = 1,024 3.9 (5.2). Some 270 instructions a warp for 4 KB of W bound the small ones (counted from the source). Without the factor 2^23:
+// 9.5, 56.5, 6.4, 3.1; 63.6, 6.8; 13.7, 100, 3.6.
 constexpr int FR_WARPS = 8, FR_THREADS = FR_WARPS * 32, FR_TILE = 16, FR_ROUND = FR_WARPS * F32_CHUNK;
 // shared memory: a round's chunk sums; the shares' sums; two rounds of A's pieces, [16 k][piece][lane] 8 bytes
 constexpr int FR_X = FR_ROUND / 16 * 3 * 256;
@@ -219,16 +237,16 @@ __global__ void __launch_bounds__(FR_THREADS, 2) gemm_f32_rows_kernel(const floa
                 if (STAGE) {
                     xh[nt] = xs[kk * 96], xm[nt] = xs[kk * 96 + 32], xl[nt] = xs[kk * 96 + 64];
                 } else {
-                    f32_split(x[nt].x, x[nt].y, xh[nt].x, xm[nt].x, xl[nt].x);
-                    f32_split(x[nt].z, x[nt].w, xh[nt].y, xm[nt].y, xl[nt].y);
+                    f32_split<NT == 2>(x[nt].x, x[nt].y, xh[nt].x, xm[nt].x, xl[nt].x);
+                    f32_split<NT == 2>(x[nt].z, x[nt].w, xh[nt].y, xm[nt].y, xl[nt].y);
                 }
             }
             if (!STAGE && kk < 3) load_x(kk + 1);
             uint32_t h[4], m[4], l[4];
-            f32_split(v[kk].x, v[kk].y, h[0], m[0], l[0]);
-            f32_split(v[4 + kk].x, v[4 + kk].y, h[1], m[1], l[1]);
-            f32_split(v[kk].z, v[kk].w, h[2], m[2], l[2]);
-            f32_split(v[4 + kk].z, v[4 + kk].w, h[3], m[3], l[3]);
+            f32_split<NT == 2>(v[kk].x, v[kk].y, h[0], m[0], l[0]);
+            f32_split<NT == 2>(v[4 + kk].x, v[4 + kk].y, h[1], m[1], l[1]);
+            f32_split<NT == 2>(v[kk].z, v[kk].w, h[2], m[2], l[2]);
+            f32_split<NT == 2>(v[4 + kk].z, v[4 + kk].w, h[3], m[3], l[3]);
 #pragma unroll
             for (int nt = 0; nt < NT; ++nt) {
                 f32_mma(e[nt], l, xh[nt]);
@@ -297,7 +315,7 @@ __global__ void __launch_bounds__(FR_THREADS, 2) gemm_f32_rows_kernel(const floa
         if (rank == 0 && tid < OUT) {
             if (GLU) {
                 const int n = tile * (FR_TILE / 2) + row, nc = min(n, N - 1) + half * N;
-                if (m < M && f32_suspect(v)) v = f32_plain(A + (size_t)m * lda, W + (size_t)nc * ldw, K);
+                v = m < M && f32_suspect(v) ? f32_plain(A + (size_t)m * lda, W + (size_t)nc * ldw, K) : v * F32_UNSCALE;
                 const float y = __fmaf_rn(alpha, v, bias ? bias[nc] : 0.f), up = __shfl_down_sync(0xffffffffu, y, NT * 8);
                 if (m < M && !half && n < N)
                     C[(size_t)m * ldc + n] = act == IL_ACT_CLAMPED ? il_clamped_glu(y, up, limit, act_alpha)
@@ -305,7 +323,7 @@ __global__ void __launch_bounds__(FR_THREADS, 2) gemm_f32_rows_kernel(const floa
             } else {
                 const int n = tile * FR_TILE + row + 8 * half;
                 if (m < M && n < N) {
-                    if (f32_suspect(v)) v = f32_plain(A + (size_t)m * lda, W + (size_t)n * ldw, K);
+                    v = f32_suspect(v) ? f32_plain(A + (size_t)m * lda, W + (size_t)n * ldw, K) : v * F32_UNSCALE;
                     C[(size_t)m * ldc + n] = __fmaf_rn(alpha, v, bias ? bias[n] : 0.f);
                 }
             }
@@ -328,8 +346,8 @@ __global__ void __launch_bounds__(FR_THREADS, 2) gemm_f32_rows_kernel(const floa
 // What bounds it is shared memory: of a chunk the 24 products read 144 KB, the pieces are 72 KB written, and the 48 KB that come
 // from memory pass the same unit: some 2,300 clocks of 128 bytes, and a chunk takes 2,400 (the tensor core is busy for 1,750).
 // Larger tiles would read less, but their sums have no room: 128 x 64 in three accumulators twice and a total are 448 of 512 columns.
-// Measured, us (multiply-adds before): 627 rows to 8,192 columns of K = 1,024 115 (312), to 1,024 columns of K = 4,096 85 (224); 2,048
-// rows to 8,192 columns 312 (909; 110 against 38 TFLOP/s); 61 rows to 1,024 columns of K = 1,024 10.3 (13.6), of K = 4,096 17.5 (27.3).
+// Measured, us (multiply-adds before; without the factor 2^23): 627 rows to 1,024 columns of K = 4,096 87.6 (226; 85.4); 2,048 rows to 8,192 columns of
+// K = 1,024 317 (911; 318: 108 against 38 TFLOP/s); 61 rows to 1,024 columns of K = 1,024 10.6 (13.6; 10.5), of K = 4,096 17.8 (27.3; 17.7).
 constexpr int FT_BM = 128, FT_BN = 64, FT_STAGES = 3, FT_A = FT_BM * 128, FT_B = FT_BN * 128, FT_STAGE = 3 * (FT_A + FT_B);
 constexpr int FT_ACC_WARPS = 8, FT_CONV_WARPS = 8, FT_THREADS = (FT_ACC_WARPS + FT_CONV_WARPS + 2) * 32;
 constexpr int FT_ROWS = 2 * FT_CONV_WARPS, FT_WU = FT_BM / FT_ROWS, FT_XU = FT_BN / FT_ROWS;       // rows at a time; pieces of a row a thread, of W and of A
@@ -556,7 +574,7 @@ __global__ void __launch_bounds__(FT_THREADS, 1) gemm_f32_tile_kernel(const floa
                 for (int i = 0; i < 32; ++i)
                     if (i < rows) {
                         again |= f32_suspect(share[i]) ? 1u << i : 0u;
-                        to[(size_t)(unsigned)(i * ldc)] = __fmaf_rn(alpha, share[i], b);
+                        to[(size_t)(unsigned)(i * ldc)] = __fmaf_rn(alpha, share[i] * F32_UNSCALE, b);
                     }
                 for (; again; again &= again - 1) {
                     const int i = __ffs(again) - 1;
@@ -587,7 +605,7 @@ __global__ void __launch_bounds__(FT_THREADS, 1) gemm_f32_tile_kernel(const floa
 #pragma unroll
             for (int i = 0; i < 4; ++i)
                 if (gn + i < N) {
-                    if (f32_suspect(v[i])) v[i] = f32_plain(A + (size_t)gm * lda, W + (size_t)(gn + i) * ldw, K);
+                    v[i] = f32_suspect(v[i]) ? f32_plain(A + (size_t)gm * lda, W + (size_t)(gn + i) * ldw, K) : v[i] * F32_UNSCALE;
                     C[(size_t)gm * ldc + gn + i] = __fmaf_rn(alpha, v[i], bias ? bias[gn + i] : 0.f);
                 }
         }

@@ -576,7 +576,7 @@ def gate_pack(y: torch.Tensor, head_dim: int, gate: Optional[torch.Tensor], g_of
 def gemm_f32(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, alpha: float = 1.0,
              bias: Optional[torch.Tensor] = None, w_static: bool = False, glu: int = 0, act_params=None) -> None:
     """out[M,N] = alpha * a[M,K] @ w[N,K]^T (+ bias), all float32, with the error of 32-bit multiply-adds (each operand
-    as three bfloat16 pieces on the tensor cores, sums in float32). `w_static`: w is a model's weight, not what
+    as three bfloat16 pieces on the tensor cores, which hold every finite number; sums in float32, those that overflow by multiply-adds). `w_static`: w is a model's weight, not what
     the kernel launched just before writes, and may be read while that kernel still runs.
     glu (ACT_SILU / ACT_GELU_TANH / ACT_CLAMPED with act_params; up to 16 rows): w is [2N,K] (gate rows, then up rows) and
     out[M,N] = act(gate) * up, as `swiglu` computes it from the products."""
