@@ -97,9 +97,6 @@ __device__ __forceinline__ uint32_t pt_pack(float lo, float hi) {
     return *reinterpret_cast<uint32_t*>(&v);
 }
 
-__device__ __forceinline__ void pt_cluster_sync() {
-    asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;\n" ::: "memory");
-}
 __device__ __forceinline__ uint32_t pt_peer_of(uint32_t addr) {      // where the cluster's second block has it
     uint32_t at;
     asm volatile("mapa.shared::cluster.u32 %0, %1, 1;\n" : "=r"(at) : "r"(addr));
@@ -250,8 +247,7 @@ __global__ void __launch_bounds__(PT_THREADS, PT_BLOCKS_PER_SM) attn_prefill_tc5
             if (ok && j + 2 < n_tiles) ok = issue(j + 2, 0);
         }
         if (split) {
-            __syncwarp();
-            pt_cluster_sync(), pt_cluster_sync();
+            il_cluster_sync(), il_cluster_sync();
         }
     } else if (warp == 1) {
         // ---------------- tensor-core issue, scores: S(j) as soon as K(j) is there and the buffer has been read out ----------------
@@ -285,8 +281,7 @@ __global__ void __launch_bounds__(PT_THREADS, PT_BLOCKS_PER_SM) attn_prefill_tc5
             }
         }
         if (split) {
-            __syncwarp();
-            pt_cluster_sync(), pt_cluster_sync();
+            il_cluster_sync(), il_cluster_sync();
         }
     } else if (warp == 2) {
         // ---------------- tensor-core issue, outputs: O += P.V(j) as soon as P(j) and V(j) are there ----------------
@@ -309,8 +304,7 @@ __global__ void __launch_bounds__(PT_THREADS, PT_BLOCKS_PER_SM) attn_prefill_tc5
             }
         }
         if (split) {
-            __syncwarp();
-            pt_cluster_sync(), pt_cluster_sync();
+            il_cluster_sync(), il_cluster_sync();
         }
     } else {
         // ---------------- softmax and output: warps 3..6 own tensor-memory lanes 32*(warp % 4) .. +31 ----------------
@@ -506,8 +500,7 @@ __global__ void __launch_bounds__(PT_THREADS, PT_BLOCKS_PER_SM) attn_prefill_tc5
                 *reinterpret_cast<float*>(smem + PT_SPLIT_ML + r * 4) = m;
                 *reinterpret_cast<float*>(smem + PT_SPLIT_ML + (PT_ROWS + r) * 4) = l;
             }
-            __syncwarp();
-            pt_cluster_sync();
+            il_cluster_sync();
             if (!rank) {
                 const float m1 = pt_peer(sums + PT_SPLIT_ML), l1 = pt_peer(sums + PT_SPLIT_ML + PT_ROWS * 4), both = fmaxf(m, m1);
                 f0 = m == -INFINITY ? 0.f : pt_ex2(m - both);
@@ -558,8 +551,7 @@ __global__ void __launch_bounds__(PT_THREADS, PT_BLOCKS_PER_SM) attn_prefill_tc5
             }
         }
         if (split) {                              // the second block's shared memory is read: it may leave
-            __syncwarp();
-            pt_cluster_sync();
+            il_cluster_sync();
         }
     }
     t5_fence_before();

@@ -180,6 +180,21 @@ __device__ __forceinline__ il_f2 il_cap_log2_small(il_f2 s, const IlCapPoly& q) 
     return il_f2_mul(y, p);
 }
 
+// ---- the blocks of a cluster ------------------------------------------------------------------------
+// The aligned barriers want a warp's 32 lanes together, which code behind a branch or a loop that lanes left one by one does not promise: the warp meets first.
+__device__ __forceinline__ void il_cluster_arrive() {
+    __syncwarp();
+    asm volatile("barrier.cluster.arrive.release.aligned;\n" ::: "memory");
+}
+__device__ __forceinline__ void il_cluster_wait() {
+    __syncwarp();
+    asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+}
+__device__ __forceinline__ void il_cluster_sync() {
+    il_cluster_arrive();
+    il_cluster_wait();
+}
+
 // ---- programmatic dependent launch --------------------------------------------------------------
 // Kernels of the decode path are launched so that the next kernel in the stream may become resident
 // while this one drains (INFINILM_B200_PDL=0 turns it off). A kernel waits for its predecessor to have

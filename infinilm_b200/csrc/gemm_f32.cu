@@ -111,12 +111,6 @@ __device__ __forceinline__ float4 f32_peer4(uint32_t addr, uint32_t rank) {
     asm volatile("ld.shared::cluster.v4.f32 {%0,%1,%2,%3}, [%4];\n" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(at) : "memory");
     return v;
 }
-__device__ __forceinline__ void f32_cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;\n" ::: "memory"); }
-__device__ __forceinline__ void f32_cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory"); }
-__device__ __forceinline__ void f32_cluster_sync() {
-    f32_cluster_arrive();
-    f32_cluster_wait();
-}
 
 // ---- up to 16 rows: W streamed once -------------------------------------------------------------------------------------
 // A block owns tiles of 16 rows of W (the A operand of m16n8k16; lane l holds k 4 (l % 4) .. + 3 of every 16 for rows l / 4 and
@@ -182,7 +176,7 @@ __global__ void __launch_bounds__(FR_THREADS, 2) gemm_f32_rows_kernel(const floa
         if (0 < total) load_w(w[0]);
         if (1 < total) load_w(w[1]);
     }
-    if (cluster > 1) f32_cluster_arrive();        // (waited for before the first access to another block's memory)
+    if (cluster > 1) il_cluster_arrive();        // (waited for before the first access to another block's memory)
     il_pdl_wait();
     il_pdl_launch_dependents();                   // (the kernel behind may ask for its own weights meanwhile)
     if (!early) {
@@ -302,10 +296,10 @@ __global__ void __launch_bounds__(FR_THREADS, 2) gemm_f32_rows_kernel(const floa
         const int half = tid / (NT * 8) & 1, row = tid / (NT * 16), m = tid % (NT * 8);
         float v = 0.f;
         if (cluster > 1) {                        // (one tile a cluster)
-            f32_cluster_wait();
+            il_cluster_wait();
             if (rank > 0 && tid < OUT)
                 for (int sh = 0; sh < share; ++sh) f32_put(part + (rank * own_shares + sh) * OUT + tid, 0, part[sh * OUT + tid]);
-            f32_cluster_sync();
+            il_cluster_sync();
         }
         if (rank == 0 && tid < OUT) {
             const int all = (f32_chunks(K) + share_chunks - 1) / share_chunks;
@@ -586,7 +580,7 @@ __global__ void __launch_bounds__(FT_THREADS, 1) gemm_f32_tile_kernel(const floa
     }
     il_pdl_tail();
     if (SPLIT) {
-        f32_cluster_sync();
+        il_cluster_sync();
         // block `rank` finishes 64 / cluster columns: the shares in order
         const int cols = FT_BN / cluster, live = (chunks + share_chunks - 1) / share_chunks;
         const int nt = first / m_tiles, mt = first - nt * m_tiles;
@@ -609,7 +603,7 @@ __global__ void __launch_bounds__(FT_THREADS, 1) gemm_f32_tile_kernel(const floa
                     C[(size_t)gm * ldc + gn + i] = __fmaf_rn(alpha, v[i], bias ? bias[gn + i] : 0.f);
                 }
         }
-        f32_cluster_sync();                       // (no block leaves while its sums are read)
+        il_cluster_sync();                       // (no block leaves while its sums are read)
     }
     t5_fence_before();
     __syncthreads();

@@ -38,9 +38,6 @@ __device__ __forceinline__ float4 gc_peer(uint32_t addr, uint32_t rank) {
     asm volatile("ld.shared::cluster.v4.f32 {%0,%1,%2,%3}, [%4];\n" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(at) : "memory");
     return v;
 }
-__device__ __forceinline__ void gc_cluster_sync() {
-    asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;\n" ::: "memory");
-}
 
 // OPS: operands of 64 weight rows; NB: rows of x, a multiple of 16.
 template <int MODE, int OPS, int NB>
@@ -199,7 +196,7 @@ __global__ void __launch_bounds__(GC_THREADS, 1) gemm_narrow_tc5_kernel(const __
             }
         t5_fence_before();
     }
-    if (cut.cluster > 1) gc_cluster_sync();
+    if (cut.cluster > 1) il_cluster_sync();
     else __syncthreads();
     const uint32_t part_at = t5_smem(part);
     const auto sum = [&](int m, int row, float (&s)[4]) {         // four rows of the tile: the shares of K in their order
@@ -293,7 +290,7 @@ __global__ void __launch_bounds__(GC_THREADS, 1) gemm_narrow_tc5_kernel(const __
             if ((row & 15) == 0 && live) p.sumsq[(size_t)m * ((N + 15) / 16) + (n >> 4)] = sq;
         }
     }
-    if (cut.cluster > 1) gc_cluster_sync();       // (no block leaves while its sums are read)
+    if (cut.cluster > 1) il_cluster_sync();       // (no block leaves while its sums are read)
     else __syncthreads();
     if (warp == 3) {
         t5_fence_after();

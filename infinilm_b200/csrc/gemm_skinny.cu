@@ -457,8 +457,6 @@ IL_EXPORT int il_gemm_skinny_rope(const void* x, int ldx, const void* W, int ldw
 // the residual stream. What add_rmsnorm does, but for the division by the rms, which the next product applies.
 // CL > 1: a cluster of CL blocks takes the 16 rows of W, CL * WARPS warps sharing K; all partial sums go to the first block's shared
 // memory, which finishes them.
-__device__ __forceinline__ void gs_cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;\n" ::: "memory"); }
-__device__ __forceinline__ void gs_cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory"); }
 __device__ __forceinline__ void gs_put2(float* p, float a, float b) {     // to the same place of the cluster's first block
     uint32_t at;
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(at) : "r"((uint32_t)__cvta_generic_to_shared(p)), "r"(0));
@@ -487,7 +485,7 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS > 8 ? 1 : 2) gemm_skinny_res
     }
     uint4 a[U][2], b[U][NT];
     if (EARLY) gs_round_w<U, SHARES>(a, wrow, warp, c, K);
-    if (CL > 1) gs_cluster_arrive();              // (waited for before the first access to another block's memory)
+    if (CL > 1) il_cluster_arrive();              // (waited for before the first access to another block's memory)
     gs_begin<EARLY>();
     // What the epilogue adds to - the residual, the norm's weight, the bias of this thread's (row, column) - is asked for
     // now: read after the main loop it cost the kernel a round trip to memory at its very end.
@@ -516,14 +514,13 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS > 8 ? 1 : 2) gemm_skinny_res
     }
     gs_tail<EARLY>();
     if (CL > 1) {
-        gs_cluster_wait();
+        il_cluster_wait();
 #pragma unroll
         for (int t = 0; t < NT; ++t) {
             gs_put2(&part[warp][t][r][c * 2], acc[t][0], acc[t][1]);
             gs_put2(&part[warp][t][r + 8][c * 2], acc[t][2], acc[t][3]);
         }
-        gs_cluster_arrive();
-        gs_cluster_wait();
+        il_cluster_sync();
         if (rank > 0) return;
     } else {
 #pragma unroll
