@@ -205,20 +205,13 @@ __device__ __forceinline__ void il_cluster_sync() {
 // writes must then NOT be read through a `const __restrict__` pointer: such loads count as read-only data for the
 // whole kernel (ld.global.nc) and were seen scheduled above the wait, which replayed graphs then showed as wrong tokens. Measured on the 8B decode step at
 // batch 8: 3.65 ms so, 3.70 ms without; with every kernel letting its successor in at its very start
-// (IL_PDL_MODE 0) 6.7 ms, because waiting blocks of later kernels then crowd the SMs.
+// 6.7 ms, because waiting blocks of later kernels then crowd the SMs.
+// That il_pdl_begin waits and lets nobody in is counted on: a kernel behind one that uses it may read, before its own wait, what was written before that one
+// began (gemm_grouped's `early`).
 __device__ __forceinline__ void il_pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
 __device__ __forceinline__ void il_pdl_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
-// Where a kernel lets its successor in: IL_PDL_MODE 0 at its start, 1 after its main loop, 2 only by ending.
-#ifndef IL_PDL_MODE
-#define IL_PDL_MODE 1
-#endif
-__device__ __forceinline__ void il_pdl_begin() {
-    if (IL_PDL_MODE == 0) il_pdl_launch_dependents();
-    il_pdl_wait();
-}
-__device__ __forceinline__ void il_pdl_tail() {
-    if (IL_PDL_MODE == 1) il_pdl_launch_dependents();
-}
+__device__ __forceinline__ void il_pdl_begin() { il_pdl_wait(); }
+__device__ __forceinline__ void il_pdl_tail() { il_pdl_launch_dependents(); }
 
 #include <cstdlib>
 static inline bool il_pdl_enabled() {

@@ -8,7 +8,7 @@
 // sigmoid(G[m, g * gate_gs + n * gate_ns]) (gate_ns 0: one gate per group). `row_scale` multiplies a row's products before the
 // epilogue: a factor per row of A, or - scale_by_place - per place of the sorted order. Products accumulate in f32 in the order of K whatever the tile, one accumulator per
 // output element, so a row's result does not depend on what else is in the batch. float32 runs on the FP32 pipes
-// (FFMA); bfloat16 runs on the tensor cores (mma.sync m16n8k16, operands staged by cp.async in a three-stage ring: a
+// (FFMA); bfloat16 runs on the tensor cores (mma.sync m16n8k16, operands staged by cp.async in a ring of three stages, four for tiles of 32 rows without a gate: a
 // block streams a tile of 64 weight rows over all of K once, against up to 16 or 32 rows of its group, which is what a decode
 // step's few rows per expert need - the weights of the experts that were chosen are read once, at the rate the memory
 // gives); bfloat16 operands that are not 16-byte aligned are widened to f32 in shared memory (exact) and run the FFMA loop.
@@ -355,7 +355,8 @@ IL_EXPORT int il_gemm_grouped(const void* A, int act_kind, int lda, long long a_
                               void* C, int ldc, long long c_gs, const int* group_off, int n_groups, int M, int N, int K, int glu,
                               const void* gate, int ld_gate, long long gate_gs, int gate_ns, const float* row_scale, int scale_by_place,
                               int early, cudaStream_t stream) {
-    // early: W and group_off were written before the kernel in front started, which may then still run while they are read.
+    // early: W and group_off were written before the kernel in front passed its own wait, which may then still run while they are read; and that kernel lets
+    // its successor in only behind that wait (as this one does: il_pdl_begin, il_pdl_tail).
     if (M <= 0 || N <= 0 || n_groups <= 0) return IL_OK;
     if (K <= 0 || (glu && gate)) return IL_BAD_ARG;
     if (act_kind == IL_BF16 && K % 8 == 0 && lda % 8 == 0 && ldw % 8 == 0 && a_gs % 8 == 0 && w_gs % 8 == 0 && !((uintptr_t)A & 15) &&

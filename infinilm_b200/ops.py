@@ -1418,7 +1418,8 @@ def gemm_grouped(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, *, group_o
     row_scale (ragged): float32 per row of `a` - or, with scale_by_place, per place of the sorted order; the products of a row
     are multiplied by its factor before the epilogue (the rstd of a norm the rows have not been divided by; the weight of a
     choice that belongs to its expert's input).
-    early: w and group_off were written before the kernel launched just before this one started, and may be read while that one still runs."""
+    early: w and group_off were written before the kernel launched just before this one passed its wait for its own predecessor, and may be read while it
+    still runs. That kernel must be one that lets its successor in only behind that wait, as gemm_grouped itself does (rope_store of few tokens, for one, does not)."""
     _need_cuda(a, w, out, group_off, a_rows, gate, row_scale)
     if row_scale is not None and (group_off is None or row_scale.dtype != torch.float32 or not row_scale.is_contiguous()
                                   or row_scale.numel() < (int(n_rows if n_rows is not None else out.shape[0]) if scale_by_place else a.shape[0])):

@@ -55,3 +55,18 @@ def test_reading_before_the_wait_is_for_the_caller_to_allow(op):
 
     from infinilm_b200 import ops
     assert inspect.signature(getattr(ops, op)).parameters["w_static"].default is False
+
+
+def test_the_experts_gate_product_lets_its_successor_in_behind_its_wait():
+    """The experts' back product reads the groups' ranges before its wait: right only while the gate product in front of it, which waits with
+    il_pdl_begin, lets nobody in before that. No switch may change it."""
+    with open(os.path.join(CSRC, "common.cuh"), encoding="utf-8") as fh:
+        common = re.sub(r"//[^\n]*", "", fh.read())
+    with open(os.path.join(CSRC, "gemm_grouped.cu"), encoding="utf-8") as fh:
+        grouped = re.sub(r"//[^\n]*", "", fh.read())
+    body = re.search(r"void il_pdl_begin\(\)\s*\{([^}]*)\}", common).group(1)
+    assert body.split() == ["il_pdl_wait();"]
+    assert "il_pdl_launch_dependents" not in grouped and "griddepcontrol" not in grouped
+    for kernel in re.split(r"__global__", grouped)[1:]:
+        wait, tail = re.search(r"il_pdl_(?:wait|begin)\(", kernel), re.search(r"il_pdl_tail\(", kernel)
+        assert wait and (tail is None or wait.start() < tail.start())
