@@ -1013,6 +1013,11 @@ def stream_status(device) -> torch.Tensor:
     return _stream_status[key]
 
 
+# What a kernel whose bounded wait ran out leaves in its stream's status word: from, to, the kernel's file.
+STATUS_CODES = ((11, 14, "gemm_tc5"), (21, 21, "attn_decode"), (30, 39, "attn_prefill_tc5"), (51, 54, "gemm_mid"), (71, 75, "gemm_f32"),
+                (81, 83, "gemm_narrow_tc5"))
+
+
 def check_status(device) -> None:
     """Raises if a kernel with bounded waits (mbarriers of the TMA / tcgen05 kernels) gave up since the last check: its
     output is then not to be trusted. Reads one word from the device, so it synchronises; call it where the host
@@ -1024,7 +1029,8 @@ def check_status(device) -> None:
     code = int(t.item())
     if code:
         t.zero_()
-        raise KernelError(f"a kernel's bounded wait ran out (code {code}: 11-14 gemm_tc5, 21 attn_decode, 30-39 attn_prefill_tc5, 51-54 gemm_mid); the step's results are invalid")
+        who = next((name for lo, hi, name in STATUS_CODES if lo <= code <= hi), "no kernel known")
+        raise KernelError(f"a kernel's bounded wait ran out (code {code}: {who}); the step's results are invalid")
 
 
 TC5_MAX_ROWS = 256
