@@ -705,7 +705,7 @@ IL_EXPORT int il_moe_combine(const void* y, int act_kind, const int* pos_of_slot
                              int H, int top, const int* group_off, int n_real, const void* x, int ldx, const float* sgate, int ld_sg,
                              cudaStream_t stream) {
     if (T <= 0) return IL_OK;
-    if (H <= 0 || top <= 0 || (group_off && (!x || n_real < 0 || ldx < H))) return IL_BAD_ARG;
+    if (H <= 0 || top <= 0 || top > MOE_MAX_TOP || (group_off && (!x || n_real < 0 || ldx < H))) return IL_BAD_ARG;      // (a token's choices lie in shared memory)
     const int vec = (H % 4 == 0 && !((uintptr_t)y & 15) && !((uintptr_t)out & 15) && !((uintptr_t)shared_rows & 15) &&
                      (!group_off || (ldx % 4 == 0 && !((uintptr_t)x & 15)))) ? 1 : 0;
     if (vec && act_kind == IL_BF16 && H % 8 == 0 && T >= 256 && (!group_off || ldx % 8 == 0)) {

@@ -119,3 +119,20 @@ def test_combining_the_rows_of_many_tokens(cuda_device, T, H, top, shared, ident
     if shared:
         ref = ref + (torch.sigmoid(sg.double())[:, None] if sg is not None else 1.0) * sh.double()
     _close(out.cpu(), ref, "bfloat16")
+
+
+@pytest.mark.parametrize("T", [3, 300])
+def test_choices_of_a_token_end_at_the_room_for_them(cuda_device, T):
+    """32 choices are summed, 33 are refused: few tokens and many."""
+    from infinilm_b200 import ops
+    H = 64
+    g = torch.Generator().manual_seed(T)
+    for top in (32, 33):
+        y, wt = torch.randn(T * top, H, generator=g).bfloat16(), torch.rand(T, top, generator=g)
+        pos, out = torch.randperm(T * top, generator=g).to(torch.int32), torch.empty(T, H, dtype=torch.bfloat16, device="cuda")
+        if top == 33:
+            with pytest.raises(ops.KernelError):
+                ops.moe_combine(y.cuda(), pos.cuda(), wt.cuda(), None, out, top=top)
+            continue
+        ops.moe_combine(y.cuda(), pos.cuda(), wt.cuda(), None, out, top=top)
+        _close(out.cpu(), (wt.double()[:, :, None] * y.double()[pos.view(T, top).long()]).sum(1), "bfloat16")
