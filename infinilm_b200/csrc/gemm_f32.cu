@@ -23,8 +23,8 @@
 // computed again with 32-bit multiply-adds, in the same chunks (f32_plain).
 //
 // Up to 16 rows the kernel is bound by the bytes of W and by the instructions that take it apart (gemm_f32_rows_kernel,
-// mma.sync on fragments that come straight from memory); beyond, by shared memory: operands written, and read by the tensor core
-// (gemm_f32_tile_kernel, tcgen05).
+// mma.sync on fragments that come straight from memory); beyond, by those instructions and by shared memory, where the pieces are written
+// and read by the tensor core (gemm_f32_tile_kernel, tcgen05).
 #include "tcgen05.cuh"
 
 constexpr int F32_CHUNK = 64;
@@ -121,7 +121,7 @@ __device__ __forceinline__ float4 f32_peer4(uint32_t addr, uint32_t rank) {
 // few, the shares go to the blocks of a cluster.
 // Measured, weights not in cache, us (the kernel of multiply-adds before): one row, 2 x 4,096 gated columns of K = 1,024 9.6 (10.5), 73,448
 // columns 58.8 (71; 5.1 TB/s), 1,024 columns of K = 4,096 6.6 (6.0), of K = 1,024 3.3 (2.3); 8 rows to 73,448 columns 64 (87), K = 4,096 7.1 (9.9); 16 rows
-// 14.4 (22.8), 111 (156), K = 1,024 3.9 (5.2). Some 270 instructions a warp for 4 KB of W bound the small ones (counted from the source). Without the factor 2^23:
+// 14.4 (22.8), 111 (156), K = 1,024 3.9 (5.2). 371 instructions a warp for 4 KB of W (counted by the profiler) bound the small ones. Without the factor 2^23:
 // 9.5, 56.5, 6.4, 3.1; 63.6, 6.8; 13.7, 100, 3.6.
 constexpr int FR_WARPS = 8, FR_THREADS = FR_WARPS * 32, FR_TILE = 16, FR_ROUND = FR_WARPS * F32_CHUNK;
 // shared memory: a round's chunk sums; the shares' sums; two rounds of A's pieces, [16 k][piece][lane] 8 bytes
@@ -337,9 +337,9 @@ __global__ void __launch_bounds__(FR_THREADS, 2) gemm_f32_rows_kernel(const floa
 // accumulators of its own; warps 0-7 add these up, a running share in registers and, over several shares, the total in tensor memory. Blocks are persistent and
 // take tiles b, b + G, ..: the next tile's chunks are taken apart while this one's sums are written. SPLIT: a cluster takes a
 // tile, each block a share or two, and the shares meet in shared memory.
-// What bounds it is shared memory: of a chunk the 24 products read 144 KB, the pieces are 72 KB written, and the 48 KB that come
-// from memory pass the same unit: some 2,300 clocks of 128 bytes, and a chunk takes 2,400 (the tensor core is busy for 1,750).
-// Larger tiles would read less, but their sums have no room: 128 x 64 in three accumulators twice and a total are 448 of 512 columns.
+// Counters (2,048 rows to 8,192 columns of K = 1,024; a chunk takes 2,600 clocks under the profiler): 6,230 warp instructions a chunk keep the issue slots
+// busy for 60 %, mostly those that take operands apart; L1 and shared memory 55 % (of a chunk the 24 products read 144 KB and the pieces are 72 KB written),
+// the tensor pipe 30 %. Larger tiles would take less apart a product, but their sums have no room: 128 x 64 in three accumulators twice and a total are 448 of 512 columns.
 // Measured, us (multiply-adds before; without the factor 2^23): 627 rows to 1,024 columns of K = 4,096 87.6 (226; 85.4); 2,048 rows to 8,192 columns of
 // K = 1,024 317 (911; 318: 108 against 38 TFLOP/s); 61 rows to 1,024 columns of K = 1,024 10.6 (13.6; 10.5), of K = 4,096 17.8 (27.3; 17.7).
 constexpr int FT_BM = 128, FT_BN = 64, FT_STAGES = 3, FT_A = FT_BM * 128, FT_B = FT_BN * 128, FT_STAGE = 3 * (FT_A + FT_B);
